@@ -270,3 +270,65 @@ def test_stage_rotation_walks_resident_ctas_in_step(tiles, stages, G):
                 assert off == 0
             else:
                 assert k < stages and off == (lo - sk_lo(owner, units, G)) % stages
+
+
+# ---- pixel map and phase / bin polynomials of the mixed kernels (bp_tile.cuh) ----
+
+def pixel_map(mx, warp, lane, k):
+    """PixelMap: tile row, first tile column and row entry of a thread's k-th pixel pair."""
+    e = (warp >> 1) * 2 + ((lane >> 2) & 1)
+    row = (warp >> 1) * 2 * mx + ((lane >> 2) & 1) + 2 * k
+    col = (warp & 1) * 16 + ((lane >> 3) << 2) + (lane & 3)
+    mid = (e >> 1) * 2 * mx + (e & 1) + 2 * (mx // 2) - 4 * mx
+    return row, col, e, mid
+
+
+@pytest.mark.parametrize("mx", [1, 2, 4, 8])
+def test_pixel_map_covers_the_tile_once(mx):
+    seen = np.zeros((8 * mx, 64), dtype=int)
+    for warp in range(8):
+        for lane in range(32):
+            for k in range(mx):
+                row, col, e, mid = pixel_map(mx, warp, lane, k)
+                assert 0 <= e < 8 and row - 4 * mx == mid + 2 * (k - mx // 2)
+                seen[row, col] += 1
+                seen[row, col + 32] += 1
+    assert (seen == 1).all()
+
+
+@pytest.mark.parametrize("radius,dx,el,mx", [(8e3, 100.0 / 1023, 45.0, 8), (10e3, 0.08, 30.0, 8), (10e3, 0.08, 30.0, 4),
+                                             (8e3, 0.12, 5.0, 8), (1e3, 0.02, 30.0, 2)])
+def test_polynomials_match_the_exact_range(radius, dx, el, mx):
+    """write_poly_table's polynomials in the row step against the exact
+    range, in double: what is left is the far-field expansion's own error and
+    the k^3 term folded into the slope, below 2e-6 rad at these geometries
+    (the sine unit's own error is 4e-7 rad at best)."""
+    lam, kr = 34.2, 2 * math.pi * 2 * 9.28e9 / 299792458.0
+    fit = {8: 452.0 / 44.0, 4: 3.0, 2: 1.0, 1: 0.0}[mx]
+    for az in (0.0, 17.0, 45.0, 71.0, 90.0, 200.0):
+        a = radius * np.array([math.cos(math.radians(el)) * math.cos(math.radians(az)),
+                               math.cos(math.radians(el)) * math.sin(math.radians(az)), math.sin(math.radians(el))])
+        tx, ty = a[0] / radius * dx, a[1] / radius * dx
+        h, hr = 0.5 / radius, 0.5 / radius ** 2
+        n20, n11, n02 = tx * tx - dx * dx, 2 * tx * ty, ty * ty - dx * dx
+        q20, q11, q02 = -kr * h * n20, -kr * h * n11, -kr * h * n02
+        q30, q21 = -kr * hr * tx * n20, -kr * hr * (tx * n11 + ty * n20)
+        q12, q03 = -kr * hr * (tx * n02 + ty * n11), -kr * hr * ty * n02
+        sigma = lam / kr
+        for e in range(8):
+            i = (e >> 1) * 2 * mx + (e & 1) + 2 * (mx // 2) - 4 * mx
+            j = np.arange(-32, 32)
+            w = i * (q11 + i * q21) + j * (q02 + i * q12 + j * q03)
+            P0 = i * i * (q20 + i * q30) + j * w
+            an = 2 * i * (2 * q20 + 3 * i * q30) + 8 * fit * q30
+            pa = an + j * (2 * (q11 + 2 * i * q21) + 2 * j * q12)
+            pb = 4 * (q20 + 3 * i * q30) + j * 4 * q21
+            for k in range(mx):
+                m = k - mx // 2
+                Q = P0 + m * pa + m * m * pb
+                row = i + 2 * m
+                d = np.stack([np.full(64, row * dx), j * dx, np.zeros(64)])
+                exact = np.sqrt(((a[:, None] - d) ** 2).sum(0)) - radius
+                lin = -(tx * row + ty * j)
+                assert np.abs(Q / kr - (exact - lin)).max() * kr < 2e-6
+                assert np.abs(sigma * Q - lam * (exact - lin)).max() < 1e-6

@@ -9,34 +9,37 @@
 //     bracket [floor(bin), floor(bin)+1]  (CPU/MATLAB semantics, not the
 //     GPU kernel's roundf bracket, cuda_BackProjectionKernels.cuh:68-74).
 //
-// Design (one CTA = one pixel tile of (8*MX) x 64 pixels of one z-slice,
-// 256 threads = 8 warps, each thread MX rows (8 apart) x 2 columns (lane and
-// lane + 32, so the lanes of one gather are one column apart):
+// Design (one CTA = one pixel tile of (8*MX) x 64 pixels of one z-slice at a
+// time, 8 accumulating warps of MX x 2 pixels a thread and one producing warp):
 //  * pulses go through shared memory in stages of PB pulses, two stage
-//    buffers, each with three mbarriers: "full" (PB arrivals and the window
-//    bytes), "ready" (all 8 warps have put their windows into intercept
-//    form) and "empty" (all 8 warps have consumed the stage).  A warp waits
-//    only for the buffer it touches next, so the warps of a CTA drift up to
-//    a stage apart instead of meeting at a CTA barrier every stage (1.72 vs
-//    1.76 ms on the large workload, same image).  For each pulse slot of the next
-//    stage one warp (slot mod 8) computes the (tile, pulse) geometry record in
-//    FP64 (tile-centre range, unit vector, phase and bin steps reduced mod 1)
-//    and issues one cp.async.bulk copy of the pulse's range-bin window (the
-//    bins any pixel of the tile can touch: +-|tile half-diagonal|), so the
-//    FP64 work and the copy issue are spread evenly over the warps;
+//    buffers.  For each stage the producing warp writes the FP64 geometry
+//    records (tile-centre range, unit vector, phase and bin steps reduced mod
+//    1), the polynomial tables and one cp.async.bulk copy per pulse of the
+//    window of range bins any pixel of the tile can touch, rewrites the landed
+//    windows to intercept form and marks the buffer ready; the accumulating
+//    warps hand it back through the "empty" mbarrier, so they drift up to a
+//    stage apart and meet nowhere;
 //  * range profiles live in HBM as pair entries {rc[b], rc[b+1]-rc[b]}
-//    (float4); once a window lands its producing warp rewrites it in
-//    shared memory to intercept form {rc[b] - (n - W) slope, slope}, so one
+//    (float4); intercept form is {rc[b] - (n - W) slope, slope}, so one
 //    16-byte load and two FMAs on the window-centred bin interpolate;
-//  * per pixel-pulse all arithmetic is FP32: dR = (Rc - R0) - u.d + g with
-//    the FP64 per-tile part carried as a per-thread phase and bin base,
-//    g = e (h + t hr) the far-field remainder (exact sqrt form for near-field
-//    pulses); the phase stays in radians within a few multiples of pi of
-//    zero and goes straight to __sincosf; the floor of the bin comes from one
-//    round-down add whose result bits also form the shared-memory address;
+//  * per pixel-pulse all arithmetic is FP32: phase and bin of a thread's
+//    pixels are polynomials in the row step (write_poly_tables), the phase in
+//    radians within a few multiples of pi of zero goes straight to
+//    __sincosf; the floor of the bin comes from one round-down add whose
+//    result bits also form the shared-memory address (near-field pulses add
+//    the exact sqrt form of the remainder per pixel);
+//  * the 8 lanes of a shared-memory wavefront are a 2 x 4 pixel patch
+//    (PixelMap), so their 16-byte gathers rarely collide;
 //  * MX = 8 (64 x 64-pixel tiles) by default: the per-(tile, pulse) and
-//    per-(thread, pulse) work is spread over 16 pixels per thread;
-//  * complex64 results leave as float2 stores, 32 consecutive pixels per warp.
+//    per-(thread, pulse) work is spread over 16 pixels per thread.
+//
+// What bounds it (1024^2 pixels x 2048 pulses, 8 km, look direction along the
+// rows, the columns, ncu): 14.8 warp instructions per warp-pixel-pulse at 58%
+// of issue slots, shared memory's data pipe 80-86% busy (5.1-6.1 wavefronts,
+// 4 of them the 16-byte gather's floor), MUFU 62-65%, 18 warps per SM.  Rows
+// interleaved over the warps, a row of 32 lanes and one evaluation of the
+// range remainder per pixel took 18.0 instructions and 1.70-2.13 ms over the
+// same look directions, this 1.51-1.65 ms.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -48,12 +51,6 @@ namespace {
 
 using namespace tile;
 
-// pulses of a common-path stage unrolled together (0: the default per tile shape)
-#ifndef SARBP_FAST_UNROLL
-#define SARBP_FAST_UNROLL 0
-#endif
-constexpr int kFastUnroll = SARBP_FAST_UNROLL;
-
 // CTAs per SM the register budget is sized for when shared memory allows
 // more than one (launch bounds of the default instantiation)
 #ifndef SARBP_CTAS_PER_SM
@@ -61,19 +58,20 @@ constexpr int kFastUnroll = SARBP_FAST_UNROLL;
 #endif
 constexpr int kCtasPerSm = SARBP_CTAS_PER_SM;
 
-constexpr int kTabEntries = kBaseEntries;
+constexpr int kTabEntries = kPolyEntries;
 
 // Header of the shared memory: six mbarriers (full, ready and empty, two
 // buffers each) and the zero entry.
 constexpr int kHdr = 64;
 
-// Dynamic shared memory of the forward kernel: the header, two stage
-// buffers of PB records, base tables and windows, and two staging slots of
-// PB pre-pass records.
+// Threads of a forward CTA: kThreads consumers and one producing warp.
+constexpr int kFwdThreads = kThreads + 32;
+
+// Dynamic shared memory of the forward kernel: the header and two stage
+// buffers of PB records, tables and windows.
 __host__ __device__ constexpr size_t smem_bytes_of(int pb, int wsize) {
     return kHdr + 2 * static_cast<size_t>(pb) * (sizeof(PulseGeo) + kTabEntries * sizeof(float4)) +
-           2 * static_cast<size_t>(pb) * static_cast<size_t>(wsize) * 16 +
-           2 * static_cast<size_t>(pb) * sizeof(PulseGeo);
+           2 * static_cast<size_t>(pb) * static_cast<size_t>(wsize) * 16;
 }
 
 // pulse stages of split tiles walked in step across the resident CTAs
@@ -83,56 +81,53 @@ __host__ __device__ constexpr size_t smem_bytes_of(int pb, int wsize) {
 constexpr bool kRotate = SARBP_STAGE_ROTATION != 0;
 
 
-// One pulse into the thread's MX x 2 pixels.  The two columns l = 0, 1 (32 apart) of a
-// row form a pair and their geometry arithmetic and complex
+// One pulse into the thread's MX x 2 pixels (PixelMap).  The two columns
+// (32 apart) of a row form a pair whose phase, bin and complex
 // multiply-accumulate run as paired FP32 instructions (__ffma2_rn and
 // friends); the sine/cosine, the shared-memory gather and the interpolation
-// are per pixel.
-// Sign conventions avoid negations: nd2 = -|d|^2, so ne = t^2 - |d|^2 = -e,
-// ng = ne (h + t hr) = -g, and the phase / bin add -kr * ng, -lam * ng.
+// are per pixel.  Phase and bin of row k - kMid are P0 + k a + k^2 b
+// (write_poly_table); rows +-k share P0 + k^2 b.
 template <int MX, bool GATE, bool NEAR, bool CHECKED>
-__device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4 *base, uint32_t w_addr,
-                                                 uint32_t zero_addr, int warp, int lane, float lam, float j0f,
-                                                 const float2 (&nd2)[MX], float (&acc_re)[MX][2],
-                                                 float (&acc_im)[MX][2], int wsize, int W, unsigned *err) {
-    const float4 c0 = *reinterpret_cast<const float4 *>(&g.a8r);  // a8r, b32r, g8, e32
-    const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);   // tx, ty, h, hr
-    const float4 c2 = *reinterpret_cast<const float4 *>(&g.kr);   // kr, rc, lo, hi
-    // per-thread phase, bin and projection bases: row part + column part,
-    // each reduced in FP64 by the producer (|phase| <= 2 pi); the pair's
-    // second pixel is 32 columns on
-    const float4 rowv = base[warp];
-    const float P00 = rowv.x + reinterpret_cast<const float *>(base + kWarps)[lane];
-    const float B00 = fmaf(j0f, c0.w * (1.0f / 32.0f), rowv.y);
-    const float t00 = fmaf(j0f, c1.y, rowv.z);
-    float2 t2 = make_float2(t00, fmaf(32.0f, c1.y, t00));
-    float2 Pb = make_float2(P00, P00 + c0.y);
-    float2 Bb = make_float2(B00, B00 + c0.w);
-    const float2 TX8 = splat(8.0f * c1.x), A8 = splat(c0.x), G8 = splat(c0.z);
-    const float2 HR = splat(c1.w), H = splat(c1.z), NKR = splat(rowv.w), NLAM = splat(-lam);
-    const float2 MAGIC = splat(kRoundMagic);
+__device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4 *tab, uint32_t w_addr,
+                                                 uint32_t zero_addr, int entry, int col, const BpLaunch &L,
+                                                 float (&acc_re)[MX][2], float (&acc_im)[MX][2]) {
+    using M = PixelMap<MX>;
+    const float4 r0 = tab[2 * entry], r1 = tab[2 * entry + 1];
+    const float4 u0 = reinterpret_cast<const float4 *>(&g)[0], u1 = reinterpret_cast<const float4 *>(&g)[1];
+    const float j0 = static_cast<float>(col - kTY / 2);
+    const float2 J = make_float2(j0, j0 + static_cast<float>(kTY / 2));
+    const float s0 = r0.x + reinterpret_cast<const float *>(tab + kPolyCols)[col];
+    const float2 w = __ffma2_rn(J, __ffma2_rn(J, splat(u0.w), splat(r0.w)), splat(r0.z));
+    const float2 sJ = __fmul2_rn(J, splat(u0.z));
+    const float2 P0 = __ffma2_rn(J, w, make_float2(s0, s0 + u0.x));
+    const float2 B0 = __ffma2_rn(sJ, w, __ffma2_rn(J, splat(u0.y), splat(r0.y)));
+    const float2 v = __ffma2_rn(J, splat(u1.x), splat(r1.z));
+    const float2 Pa = __ffma2_rn(J, v, splat(r1.x)), Ba = __ffma2_rn(sJ, v, splat(r1.y));
+    const float2 Pb = __ffma2_rn(J, splat(u1.y), splat(r1.w)), Bb = __fmul2_rn(Pb, splat(u0.z));
     // B is the window-centred bin; shared address of pair entry floor(B) + W:
     // bits(B + 1.5*2^23, rounded down) * 16 + w_adj (mod 2^32)
-    const uint32_t w_adj = w_addr + (static_cast<uint32_t>(W) - kRoundMagicBits) * 16u;
-#pragma unroll
-    for (int k = 0; k < MX; ++k) {
-        if (k > 0) {
-            t2 = __fadd2_rn(t2, TX8);
-            Pb = __fadd2_rn(Pb, A8);
-            Bb = __fadd2_rn(Bb, G8);
-        }
-        float2 ng;
+    const uint32_t w_adj = w_addr + (static_cast<uint32_t>(L.W) - kRoundMagicBits) * 16u;
+    auto pixels = [&](int k, float2 P, float2 B) {
         if (NEAR) {
-            const float e0 = -fmaf(t2.x, t2.x, nd2[k].x), e1 = -fmaf(t2.y, t2.y, nd2[k].y);
-            const float s0 = c2.y - t2.x, s1 = c2.y - t2.y;
-            ng = make_float2(-e0 / (s0 + sqrtf(fmaf(s0, s0, e0))), -e1 / (s1 + sqrtf(fmaf(s1, s1, e1))));
-        } else {
-            const float2 ne = __ffma2_rn(t2, t2, nd2[k]);
-            ng = __fmul2_rn(ne, __ffma2_rn(t2, HR, H));
+            // exact remainder of the range, e = |d|^2 - t^2 >= 0
+            const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);  // tx, ty, h, hr
+            const float4 c2 = *reinterpret_cast<const float4 *>(&g.kr);  // kr, rc, lo, hi
+            const float fi = static_cast<float>(M::mid_row(entry) + M::kStep * (k - M::kMid));
+            const float di = fi * static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
+            const float lam = static_cast<float>(L.lambda);
+            float gl[2];
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const float fj = l ? J.y : J.x, dj = fj * dy;
+                const float t = fmaf(fi, c1.x, fj * c1.y);
+                const float e = -fmaf(t, t, -fmaf(di, di, dj * dj));
+                const float s = c2.y - t;
+                gl[l] = e / (s + sqrtf(fmaf(s, s, e)));
+            }
+            P = make_float2(fmaf(c2.x, gl[0], P.x), fmaf(c2.x, gl[1], P.y));
+            B = make_float2(fmaf(lam, gl[0], B.x), fmaf(lam, gl[1], B.y));
         }
-        const float2 P = __ffma2_rn(NKR, ng, Pb);
-        const float2 B = __ffma2_rn(NLAM, ng, Bb);
-        const float2 y = __fadd2_rd(B, MAGIC);
+        const float2 y = __fadd2_rd(B, splat(kRoundMagic));
         float2 RE, IM, CS, SN;  // the pair's interpolated samples and rotations
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
@@ -141,9 +136,11 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
             const float yl = l ? y.y : y.x;
             float sn, cs;
             __sincosf(Pl, &sn, &cs);
-            uint32_t addr = __float_as_uint(yl) * 16u + w_adj;
+            // on the multiply-add pipe: as a shift-add on the ALU 1529 vs 1516 us
+            uint32_t addr;
+            asm("mad.lo.u32 %0, %1, 16, %2;" : "=r"(addr) : "r"(__float_as_uint(yl)), "r"(w_adj));
             if (GATE) {
-                const bool valid = (Bl > c2.z) && (Bl < c2.w);
+                const bool valid = (Bl > u1.z) && (Bl < u1.w);
                 addr = valid ? addr : zero_addr;
             }
             if (CHECKED) {
@@ -151,14 +148,14 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
                 // [W - wp, W + wp] (its next entry too)
                 const uint32_t idx = __float_as_uint(yl) - kRoundMagicBits + static_cast<uint32_t>(g.wp);
                 if (idx > static_cast<uint32_t>(2 * g.wp)) {
-                    atomicOr(err, ERRBIT_BOUNDS);
+                    atomicOr(L.err, ERRBIT_BOUNDS);
                     addr = zero_addr;
                 }
             }
             // intercept-form entry {c, v'}: v(B) = c + B v'
-            const float4 v = lds128(addr);
-            const float re = fmaf(Bl, v.z, v.x);
-            const float im = fmaf(Bl, v.w, v.y);
+            const float4 e = lds128(addr);
+            const float re = fmaf(Bl, e.z, e.x);
+            const float im = fmaf(Bl, e.w, e.y);
             if (l) {
                 RE.y = re;
                 IM.y = im;
@@ -180,23 +177,31 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
         acc_re[k][1] = ar.y;
         acc_im[k][0] = ai.x;
         acc_im[k][1] = ai.y;
+    };
+    pixels(M::kMid, P0, B0);
+#pragma unroll
+    for (int k = 1; k <= M::kMid; ++k) {
+        const float f = static_cast<float>(k);
+        const float2 Ps = __ffma2_rn(splat(f * f), Pb, P0), Bs = __ffma2_rn(splat(f * f), Bb, B0);
+        pixels(M::kMid - k, __ffma2_rn(splat(-f), Pa, Ps), __ffma2_rn(splat(-f), Ba, Bs));
+        if (M::kMid + k < MX) pixels(M::kMid + k, __ffma2_rn(splat(f), Pa, Ps), __ffma2_rn(splat(f), Ba, Bs));
     }
 }
 
 // Store (or add, L.accumulate) a thread's MX x 2 pixels of the tile at
-// (tx0, ty0, slice zz) into the complex64 image: columns lane and lane + 32,
-// so every store of a warp is 32 consecutive pixels.
+// (tx0, ty0, slice zz) into the complex64 image (PixelMap: every store of a
+// warp is 16 consecutive pixels, 128 bytes, of each of two rows).
 template <int MX>
 __device__ __forceinline__ void store_pixels(const BpLaunch &L, int tx0, int ty0, int zz, int warp, int lane,
                                              const float (&re)[MX][2], const float (&im)[MX][2]) {
     float2 *img = static_cast<float2 *>(L.img);
 #pragma unroll
     for (int k = 0; k < MX; ++k) {
-        const int row = tx0 + warp + 8 * k;
+        const int row = tx0 + PixelMap<MX>::row0(warp, lane) + PixelMap<MX>::kStep * k;
         if (row >= L.nx) continue;
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
-            const int col = ty0 + lane + (kTY / 2) * l;
+            const int col = ty0 + PixelMap<MX>::col0(warp, lane) + (kTY / 2) * l;
             if (col >= L.ny) continue;
             const long long o = (static_cast<long long>(zz) * L.nx + row) * L.ny + col;
             float2 v = make_float2(re[k][l], im[k][l]);
@@ -210,9 +215,9 @@ __device__ __forceinline__ void store_pixels(const BpLaunch &L, int tx0, int ty0
     }
 }
 
-// Index of thread (warp, lane)'s pixel pair of row group k in a partial-sum
-// slot of TX x 64 complex64 values (written and read by the same mapping).
-__device__ __forceinline__ int slot_pair(int warp, int lane, int k) { return (warp + 8 * k) * kTY + 2 * lane; }
+// Index of a thread's pixel pair k in a partial-sum slot of TX x 64
+// complex64 values (written and read by the same threads).
+__device__ __forceinline__ int slot_pair(int k) { return k * kThreads + static_cast<int>(threadIdx.x); }
 
 // Unit cursor over one launch (BATCH = false: the kernel parameter's scene)
 // or over the scenes of a batch table, scene-major.
@@ -288,8 +293,17 @@ struct SceneCursor {
 // carries only the batch-wide window size (the largest scene window: the
 // stage buffers' stride) and sk_partial; each scene's image completion time
 // goes to done[scene].
+//
+// Warps 0..7 accumulate; warp 8 produces: per stage it waits until the
+// buffer is empty, puts the stage's records, tables and window copies into
+// it, rewrites the landed windows to intercept form and marks the buffer
+// ready.  As one warp's work the 8 PB row entries of a stage fill the lanes
+// and the PB records, coefficients and copies take one pass (each accumulating
+// warp producing its own pulse slot ran them with 8 of 32 lanes or one), and
+// the accumulating warps carry neither the production's instructions nor its
+// latency.
 template <int MX, int PB, bool CHECKED, int MINB, bool BATCH>
-__global__ void __launch_bounds__(kThreads, MINB)
+__global__ void __launch_bounds__(kFwdThreads, MINB)
     bp_mixed_kernel(const __grid_constant__ BpLaunch L0, const BatchScene *__restrict__ scenes, int nscenes,
                     long long batch_units, unsigned long long *__restrict__ done, int tile_mode) {
     constexpr int TX = 8 * MX;
@@ -297,9 +311,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
     float4 *zero = reinterpret_cast<float4 *>(smem + kHdr - 16);
     PulseGeo *geo = reinterpret_cast<PulseGeo *>(smem + kHdr);
-    float4 *bases = reinterpret_cast<float4 *>(smem + kHdr + 2 * PB * sizeof(PulseGeo));
+    float4 *tabs = reinterpret_cast<float4 *>(smem + kHdr + 2 * PB * sizeof(PulseGeo));
     const uint32_t win_addr = smem_addr(smem + kHdr + 2 * PB * (sizeof(PulseGeo) + kTabEntries * sizeof(float4)));
-    const uint32_t zero_addr = smem_addr(zero);
     const uint32_t buf_bytes = static_cast<uint32_t>(PB) * static_cast<uint32_t>(L0.wsize) * 16u;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -321,52 +334,24 @@ __global__ void __launch_bounds__(kThreads, MINB)
         n = S;
     }
     if (n <= 0) return;
-    const int i0 = warp - TX / 2;
-    const int j0 = lane - kTY / 2;  // column offset of the first pixel (the second is 32 on)
-    const float j0f = static_cast<float>(j0);
 
-    SceneCursor<TX, PB, BATCH> cc, pc;  // consumer at unit i, producer at unit i + 1
-    cc.init(&L0, scenes, nscenes, lo, U);
+    SceneCursor<TX, PB, BATCH> cur;  // this warp's unit
+    cur.init(&L0, scenes, nscenes, lo, U);
     // stage rotation of the tiles this CTA enters at their first stage
     const int rot_later =
-        (!BATCH && kRotate) ? static_cast<int>((cc.g.stages - lo % cc.g.stages) % cc.g.stages) : 0;
-    pc = cc;
+        (!BATCH && kRotate) ? static_cast<int>((cur.g.stages - lo % cur.g.stages) % cur.g.stages) : 0;
 
-    // per-scene constants of the consumer
-    float2 nd2[MX];  // -|d|^2 of the thread's pixel pairs
-    float lam;
-    int wsize;
-    uint32_t pulse_bytes;
-    auto scene_consts = [&]() {
-        const BpLaunch &L = *cc.L;
-        lam = static_cast<float>(L.lambda);
-        wsize = L.wsize;
-        pulse_bytes = static_cast<uint32_t>(wsize) * 16u;
-        const float dxf = static_cast<float>(L.dx), dyf = static_cast<float>(L.dy);
-#pragma unroll
-        for (int k = 0; k < MX; ++k) {
-            const float di = static_cast<float>(i0 + 8 * k) * dxf;
-            const float dj0 = static_cast<float>(j0) * dyf, dj1 = static_cast<float>(j0 + kTY / 2) * dyf;
-            nd2[k] = make_float2(-fmaf(di, di, dj0 * dj0), -fmaf(di, di, dj1 * dj1));
-        }
-    };
-    scene_consts();
-    float acc_re[MX][2], acc_im[MX][2];
-#pragma unroll
-    for (int k = 0; k < MX; ++k)
-#pragma unroll
-        for (int l = 0; l < 2; ++l) acc_re[k][l] = acc_im[k][l] = 0.0f;
-
-    // buffer s: full (windows landed) at bar_base + 8 s, ready at
-    // bar_base + 16 + 8 s, empty at bar_base + 32 + 8 s
+    // buffer s: full (windows landed: PB arrivals and their bytes) at
+    // bar_base + 8 s, ready (intercept form, one arrival) at bar_base + 16 +
+    // 8 s, empty (consumed, one arrival per accumulating warp) at bar_base +
+    // 32 + 8 s
     const uint32_t bar_base = smem_addr(&bars[0]);
     auto ready_bar = [&](int b) { return bar_base + 16u + 8u * b; };
     auto empty_bar = [&](int b) { return bar_base + 32u + 8u * b; };
     if (threadIdx.x == 0) {
-        mbar_init(bar_base, PB);
-        mbar_init(bar_base + 8, PB);
         for (int b = 0; b < 2; ++b) {
-            mbar_init(ready_bar(b), kWarps);
+            mbar_init(bar_base + 8u * b, PB);
+            mbar_init(ready_bar(b), 1);
             mbar_init(empty_bar(b), kWarps);
         }
         *zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -374,178 +359,136 @@ __global__ void __launch_bounds__(kThreads, MINB)
     }
     __syncthreads();
 
-    // records, base tables and windows of the producer cursor's unit into
-    // buffer s
-    // Pre-pass records (single-scene launches: L0.geo_tab; batches: each
-    // scene's L.geo_tab, L0.geo_tab non-null when every scene has them): the
-    // records of the stage after the producer's are copied asynchronously
-    // into the staging ring (two stages of PB records after the stage
-    // buffers' windows) while the current stage accumulates, so their
-    // global-memory latency does not stall the producing warps.
-    const bool pregeo = L0.geo_tab != nullptr;
-    PulseGeo *stg = reinterpret_cast<PulseGeo *>(smem + smem_bytes_of(PB, L0.wsize) - 2 * PB * sizeof(PulseGeo));
-    // stage after the producer cursor's unit (last: the CTA has no more)
-    auto prefetch_next = [&](int slot, bool last) {
-        if (last) return;
-        if constexpr (BATCH) {
-            // the next unit may be the next scene's
-            SceneCursor<TX, PB, BATCH> nx = pc;
-            nx.advance(scenes, nscenes, rot_later);
-            const BpLaunch &L = *nx.L;
+    if (warp == kWarps) {
+        // Pre-pass records (single-scene launches: L0.geo_tab; batches: each
+        // scene's L.geo_tab, L0.geo_tab non-null when every scene has them):
+        // a stage's records, 8 PB words of 16 bytes, are loaded into the
+        // lanes' registers one stage ahead.
+        const bool pregeo = L0.geo_tab != nullptr;
+        constexpr int kPre = (kRecWords * PB + 31) / 32;
+        float4 pre[kPre];
+        auto load_records = [&](const SceneCursor<TX, PB, BATCH> &c) {
+            const BpLaunch &L = *c.L;
             const long long t =
-                ((static_cast<long long>(nx.u.hyp) * L.nz + nx.u.iz) * nx.g.tiles_x + nx.u.tx) * nx.g.tiles_y +
-                nx.u.ty;
-            prefetch_records<PB>(L, static_cast<const PulseGeo *>(L.geo_tab) + t * L.np, nx.stage(),
-                                 stg + slot * PB, warp, lane);
-            return;
+                ((static_cast<long long>(c.u.hyp) * L.nz + c.u.iz) * c.g.tiles_x + c.u.tx) * c.g.tiles_y + c.u.ty;
+            const int p0 = c.stage() * PB;
+            const float4 *src = reinterpret_cast<const float4 *>(static_cast<const PulseGeo *>(L.geo_tab) + t * L.np + p0);
+            const int words = min(PB, L.np - p0) * kRecWords;
+#pragma unroll
+            for (int r = 0; r < kPre; ++r) {
+                const int k = lane + 32 * r;
+                pre[r] = k < words ? src[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        };
+        if (pregeo) load_records(cur);
+        for (int i = 0; i < n; ++i) {
+            const int s = i & 1;
+            const BpLaunch &L = *cur.L;
+            // buffer s last held stage i - 2: every accumulating warp has consumed it
+            if (i >= 2 && !mbar_wait_bounded(empty_bar(s), ((i - 2) >> 1) & 1, L.err)) return;
+            PulseGeo *rec = geo + s * PB;
+            const int p = cur.stage() * PB + lane;  // lane < PB: this lane's pulse
+            if (pregeo) {
+#pragma unroll
+                for (int r = 0; r < kPre; ++r) {
+                    const int k = lane + 32 * r;
+                    if (k < kRecWords * PB) reinterpret_cast<float4 *>(rec)[k] = pre[r];
+                }
+            } else if (lane < PB) {
+                const double cx = L.left + static_cast<double>(cur.u.tx * TX + TX / 2) * L.dx;
+                const double cy = L.bottom + static_cast<double>(cur.u.ty * kTY + kTY / 2) * L.dy;
+                const double cz = L.zlow + static_cast<double>(cur.u.iz) * L.dz;
+                PulseGeo g = {};
+                if (p < L.np) g = make_geo(L, p, static_cast<long long>(cur.u.hyp) * L.np, cx, cy, cz, TX / 2);
+                rec[lane] = g;
+            }
+            __syncwarp();
+            if (lane < PB)
+                issue_window(L, p, lane, rec[lane].flags, rec[lane].wp, rec[lane].ws, win_addr + s * buf_bytes,
+                             bar_base + 8u * s);
+            write_poly_tables<MX, PB>(tabs + s * PB * kTabEntries, rec, lane, L);
+            cur.advance(scenes, nscenes, rot_later);
+            if (pregeo && i + 1 < n) load_records(cur);
+            if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
+            for (int q = 0; q < PB; ++q) {
+                if (!(rec[q].flags & PG_ACTIVE)) continue;
+                rewrite_window<false>(win_addr + s * buf_bytes + static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) * 16u,
+                                      L.W, rec[q].wp, lane, 0.0f);
+            }
+            // the rewrite's generic-proxy stores precede the next bulk copies
+            // (async proxy) into this buffer, which this warp issues
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ready_bar(s));
         }
-        const BpLaunch &L = *pc.L;
-        long long t =
-            ((static_cast<long long>(pc.u.hyp) * L.nz + pc.u.iz) * pc.g.tiles_x + pc.u.tx) * pc.g.tiles_y + pc.u.ty;
-        int st;
-        if (pc.u.b + 1 < pc.g.stages) {
-            st = pc.stage() + 1;
-            if (st == pc.g.stages) st = 0;
-        } else {
-            ++t;  // the next tile, entered at its first stage
-            st = rot_later;
-        }
-        prefetch_records<PB>(L, static_cast<const PulseGeo *>(L.geo_tab) + t * L.np, st, stg + slot * PB, warp, lane);
-    };
-    auto produce = [&](int s, const PulseGeo *staged) {
-        // every lane of the warp enters: the base tables take the whole warp
-        // (the records come from the staging slot, or lane 0 computes them
-        // and shuffles their steps to the warp), lane 0 issues the copy
-        const BpLaunch &L = *pc.L;
-        const double cx = L.left + static_cast<double>(pc.u.tx * TX + TX / 2) * L.dx;
-        const double cy = L.bottom + static_cast<double>(pc.u.ty * kTY + kTY / 2) * L.dy;
-        const double cz = L.zlow + static_cast<double>(pc.u.iz) * L.dz;
-        produce_slots<PB>(L, pc.stage(), geo + s * PB, bases + s * PB * kTabEntries, win_addr + s * buf_bytes,
-                          bar_base + 8 * s, warp, lane, TX / 2, cx, cy, cz,
-                          static_cast<long long>(pc.u.hyp) * L.np, staged);
-    };
-
-    if (pregeo) {
-        // stage 0's records now, stage 1's ahead
-        const BpLaunch &L = *pc.L;
-        const long long t =
-            ((static_cast<long long>(pc.u.hyp) * L.nz + pc.u.iz) * pc.g.tiles_x + pc.u.tx) * pc.g.tiles_y + pc.u.ty;
-        prefetch_records<PB>(L, static_cast<const PulseGeo *>(L.geo_tab) + t * L.np, pc.stage(), stg, warp, lane);
-        produce(0, stg);
-        prefetch_next(1, n < 2);
-    } else {
-        produce(0, nullptr);
-    }
-    const bool ok0 = intercept_slots<PB>(geo, win_addr, bar_base, 0, pc.L->wsize, pc.L->W, warp, lane, pc.L->err);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(ready_bar(0));
-    if (__any_sync(0xffffffffu, !ok0)) {
-        // stage 0's copies never completed (error bit set): leave once the
-        // record prefetches have landed; the other warps leave at their next
-        // wait (every arrival on the incomplete barrier's phase is made)
-        asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
 
-    int last_issued = 0;
+    const uint32_t zero_addr = smem_addr(zero);
+    const int entry = PixelMap<MX>::entry(warp, lane), col = PixelMap<MX>::col0(warp, lane);
+    float acc_re[MX][2], acc_im[MX][2];
+#pragma unroll
+    for (int k = 0; k < MX; ++k)
+#pragma unroll
+        for (int l = 0; l < 2; ++l) acc_re[k][l] = acc_im[k][l] = 0.0f;
     int seg = 0;                 // segments flushed so far
-    int seg_first = cc.u.b;      // first stage of the open segment
+    int seg_first = cur.u.b;     // first stage of the open segment
     for (int i = 0; i < n; ++i) {
         const int s = i & 1;
-        bool ok = true;
-        if (i + 1 < n) {
-            pc.advance(scenes, nscenes, rot_later);
-            // buffer s ^ 1 last held stage i - 1: every warp has consumed it
-            if (i >= 1) ok = mbar_wait_bounded(empty_bar(s ^ 1), ((i - 1) >> 1) & 1, pc.L->err);
-        }
-        if (i + 1 < n && ok) {
-            if (pregeo) {
-                // stage i + 1's records were prefetched into staging slot
-                // (i + 1) & 1; stage i + 2's go to the other one, whose
-                // records this warp read when it produced stage i (a warp
-                // fills and reads only its own pulse slots of the ring)
-                produce(s ^ 1, stg + (s ^ 1) * PB);
-                prefetch_next(s, i + 2 >= n);
-            } else {
-                produce(s ^ 1, nullptr);
-            }
-            last_issued = i + 1;
-        }
-        const BpLaunch &L = *cc.L;
-        const int S = cc.g.stages;
-        const int b = cc.u.b;  // position in the tile's stage order
-        if (ok) ok = mbar_wait_bounded(ready_bar(s), (i >> 1) & 1, L.err);
-        if (ok) {
-            const int nq = min(PB, L.np - cc.stage() * PB);
-            // stage summary: all PB pulses active, none gated or near-field
-            const int my_flags = lane < nq ? geo[s * PB + lane].flags : 0;
-            const int any_f = __reduce_or_sync(0xffffffffu, my_flags);
-            const int all_f = __reduce_and_sync(0xffffffffu, lane < nq ? my_flags : PG_ACTIVE);
-            const uint32_t w0 = win_addr + s * buf_bytes;
-            if (nq == PB && (all_f & PG_ACTIVE) && !(any_f & (PG_GATE | PG_NEAR))) {
-                // the whole stage unrolled (64-row tiles: 1.762 vs 1.771 ms for a
-                // half-stage unroll, no spill either way; 32 rows: 2.250 vs 2.283 ms)
-                constexpr int kUnroll = kFastUnroll > 0 ? kFastUnroll : PB;
-#pragma unroll kUnroll
-                for (int q = 0; q < PB; ++q)
-                    accumulate_pulse<MX, false, false, CHECKED>(geo[s * PB + q], bases + (s * PB + q) * kTabEntries,
-                                                                w0 + q * pulse_bytes, zero_addr, warp, lane, lam, j0f,
-                                                                nd2, acc_re, acc_im, wsize, L.W, L.err);
-            } else {
-                for (int q = 0; q < nq; ++q) {
-                    const PulseGeo &g = geo[s * PB + q];
-                    const float4 *bq = bases + (s * PB + q) * kTabEntries;
-                    const int flags = g.flags;
-                    if (!(flags & PG_ACTIVE)) continue;
-                    const uint32_t w = w0 + q * pulse_bytes;
-                    if (flags & PG_NEAR)
-                        accumulate_pulse<MX, true, true, CHECKED>(g, bq, w, zero_addr, warp, lane, lam, j0f, nd2,
-                                                                  acc_re, acc_im, wsize, L.W, L.err);
-                    else if (flags & PG_GATE)
-                        accumulate_pulse<MX, true, false, CHECKED>(g, bq, w, zero_addr, warp, lane, lam, j0f, nd2,
-                                                                   acc_re, acc_im, wsize, L.W, L.err);
-                    else
-                        accumulate_pulse<MX, false, false, CHECKED>(g, bq, w, zero_addr, warp, lane, lam, j0f, nd2,
-                                                                    acc_re, acc_im, wsize, L.W, L.err);
-                }
+        const BpLaunch &L = *cur.L;
+        const int S = cur.g.stages;
+        const int b = cur.u.b;  // position in the tile's stage order
+        // a wait that runs out (error bit set) ends this warp; the others end at theirs
+        if (!mbar_wait_bounded(ready_bar(s), (i >> 1) & 1, L.err)) return;
+        const int nq = min(PB, L.np - cur.stage() * PB);
+        // stage summary: all PB pulses active, none gated or near-field
+        const int my_flags = lane < nq ? geo[s * PB + lane].flags : 0;
+        const int any_f = __reduce_or_sync(0xffffffffu, my_flags);
+        const int all_f = __reduce_and_sync(0xffffffffu, lane < nq ? my_flags : PG_ACTIVE);
+        const uint32_t w0 = win_addr + s * buf_bytes;
+        const uint32_t pulse_bytes = static_cast<uint32_t>(L.wsize) * 16u;
+        if (nq == PB && (all_f & PG_ACTIVE) && !(any_f & (PG_GATE | PG_NEAR))) {
+            // a loop of one pulse, 230 instructions, stays in the instruction
+            // cache: with the stage's 8 pulses unrolled 1520-1691 us on the
+            // large workload over look directions, as a loop 1511-1649
+#pragma unroll 1
+            for (int q = 0; q < PB; ++q)
+                accumulate_pulse<MX, false, false, CHECKED>(geo[s * PB + q], tabs + (s * PB + q) * kTabEntries,
+                                                            w0 + q * pulse_bytes, zero_addr, entry, col, L, acc_re,
+                                                            acc_im);
+        } else {
+            for (int q = 0; q < nq; ++q) {
+                const PulseGeo &g = geo[s * PB + q];
+                const float4 *tq = tabs + (s * PB + q) * kTabEntries;
+                const int flags = g.flags;
+                if (!(flags & PG_ACTIVE)) continue;
+                const uint32_t w = w0 + q * pulse_bytes;
+                if (flags & PG_NEAR)
+                    accumulate_pulse<MX, true, true, CHECKED>(g, tq, w, zero_addr, entry, col, L, acc_re, acc_im);
+                else if (flags & PG_GATE)
+                    accumulate_pulse<MX, true, false, CHECKED>(g, tq, w, zero_addr, entry, col, L, acc_re, acc_im);
+                else
+                    accumulate_pulse<MX, false, false, CHECKED>(g, tq, w, zero_addr, entry, col, L, acc_re, acc_im);
             }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(s));
-        // the next stage's windows into intercept form, published by the
-        // ready mbarrier
-        if (i + 1 < n && ok) {
-            ok = intercept_slots<PB>(geo + (s ^ 1) * PB, win_addr + (s ^ 1) * buf_bytes, bar_base + 8 * (s ^ 1),
-                                     ((i + 1) >> 1) & 1, pc.L->wsize, pc.L->W, warp, lane, L.err);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(ready_bar(s ^ 1));
-        }
-        // a wait ran out (error bit set): this warp stops, the others at
-        // their next wait for it; its own copies and record prefetches land
-        // before the CTA's shared memory goes away (again bounded)
-        if (__any_sync(0xffffffffu, !ok)) {
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            if (lane == 0 && last_issued > i)
-                mbar_wait_bounded(bar_base + 8 * (last_issued & 1), (last_issued >> 1) & 1, L.err);
-            return;
-        }
         if (i + 1 == n || b == S - 1) {
             // the segment of this tile ends: whole tile -> image, else -> partial slot
             if (seg_first == 0 && b == S - 1) {
-                store_pixels<MX>(L, cc.u.tx * TX, cc.u.ty * kTY, cc.u.hyp * L.nz + cc.u.iz, warp, lane, acc_re,
+                store_pixels<MX>(L, cur.u.tx * TX, cur.u.ty * kTY, cur.u.hyp * L.nz + cur.u.iz, warp, lane, acc_re,
                                  acc_im);
                 // completion time: the latest of the warps' stores
                 if (BATCH && done) {
                     __syncwarp();
-                    if (lane == 0) atomicMax(done + cc.scene, global_timer_ns());
+                    if (lane == 0) atomicMax(done + cur.scene, global_timer_ns());
                 }
             } else {
                 float4 *slot = static_cast<float4 *>(L0.sk_partial) +
                                (2 * static_cast<long long>(blockIdx.x) + (seg > 0 ? 1 : 0)) * (TX * kTY / 2);
 #pragma unroll
                 for (int k = 0; k < MX; ++k)
-                    slot[slot_pair(warp, lane, k) / 2] =
-                        make_float4(acc_re[k][0], acc_im[k][0], acc_re[k][1], acc_im[k][1]);
+                    slot[slot_pair(k)] = make_float4(acc_re[k][0], acc_im[k][0], acc_re[k][1], acc_im[k][1]);
             }
 #pragma unroll
             for (int k = 0; k < MX; ++k)
@@ -554,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
             ++seg;
             seg_first = 0;
         }
-        if (cc.advance(scenes, nscenes, rot_later)) scene_consts();
+        cur.advance(scenes, nscenes, rot_later);
     }
 }
 
@@ -599,7 +542,7 @@ __global__ void __launch_bounds__(kThreads)
         const float4 *slot = part + sk_slot(c, first, units, G) * (TX * kTY / 2);
 #pragma unroll
         for (int k = 0; k < MX; ++k) {
-            const float4 v = slot[slot_pair(warp, lane, k) / 2];
+            const float4 v = slot[slot_pair(k)];
             re[k][0] += v.x;
             im[k][0] += v.y;
             re[k][1] += v.z;
@@ -736,7 +679,7 @@ cudaError_t launch_kernels(const BpLaunch &L0, size_t smem, cudaStream_t s) {
         if (2 * g * TX * kTY * static_cast<long long>(sizeof(float2)) <= L.sk_slot_bytes) G = g;
     }
     if (G > 0x7fffffffLL) return cudaErrorInvalidValue;
-    kern<<<static_cast<unsigned>(G), kThreads, smem, s>>>(L, nullptr, 0, 0, nullptr, 0);
+    kern<<<static_cast<unsigned>(G), kFwdThreads, smem, s>>>(L, nullptr, 0, 0, nullptr, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess || G == tg.tiles) return e;
     bp_sk_fixup_kernel<MX, PB, false>
@@ -761,7 +704,7 @@ int resident_of(K kern, size_t smem) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFwdThreads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -785,12 +728,12 @@ cudaError_t launch_batch_kernels(const BatchScene *scenes, int nscenes, long lon
     if (tiles < 1 || tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
     if (per_tile) {
         // one CTA per tile: no partial sums, scenes finish in order
-        kern<<<static_cast<unsigned>(tiles), kThreads, smem, s>>>(L0, scenes, nscenes, units, done, 1);
+        kern<<<static_cast<unsigned>(tiles), kFwdThreads, smem, s>>>(L0, scenes, nscenes, units, done, 1);
         return cudaGetLastError();
     }
     const long long G = resident < units ? resident : units;
     if (G < 1 || G > 0x7fffffffLL) return cudaErrorInvalidValue;
-    kern<<<static_cast<unsigned>(G), kThreads, smem, s>>>(L0, scenes, nscenes, units, done, 0);
+    kern<<<static_cast<unsigned>(G), kFwdThreads, smem, s>>>(L0, scenes, nscenes, units, done, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     bp_sk_fixup_kernel<MX, PB, true>

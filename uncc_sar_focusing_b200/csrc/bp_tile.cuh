@@ -255,6 +255,120 @@ __device__ __forceinline__ void write_base_table(float4 *tab, int lane, int tx_h
     }
 }
 
+// ---- forward kernel: pixel map and polynomial table -----------------------
+//
+// A thread's pixels: warp w covers rows [2 MX (w >> 1), + 2 MX) and columns
+// 16 (w & 1) + [0, 16) and the same 32 columns on; its lanes are 2 rows x 16
+// columns, each aligned group of 8 lanes a 2 x 4 patch, and a thread steps
+// MX times by two rows.  The 8 lanes of one shared-memory wavefront then look
+// at bins a few entries apart whatever the look direction; as 8 columns of
+// one row they spread over 7 column steps, and where the bin advances about 2
+// entries a column (large workload, look direction along the columns) their
+// 16-byte loads collide two to three ways.
+template <int MX>
+struct PixelMap {
+    static constexpr int kStep = 2;                 // rows between a thread's pixels
+    static constexpr int kMid = MX / 2;             // the row step the polynomials are centred on
+    static constexpr int kGroupRows = kStep * MX;   // rows of a warp
+    // row entry (0..7) of a thread, and the row offset of its middle pixel
+    // from the tile centre
+    static __host__ __device__ constexpr int entry(int warp, int lane) { return (warp >> 1) * 2 + ((lane >> 2) & 1); }
+    static __host__ __device__ constexpr int mid_row(int e) {
+        return (e >> 1) * kGroupRows + (e & 1) + kStep * kMid - 4 * MX;
+    }
+    // first row of the thread within the tile, and its first column (the second is 32 on)
+    static __host__ __device__ constexpr int row0(int warp, int lane) {
+        return (warp >> 1) * kGroupRows + ((lane >> 2) & 1);
+    }
+    static __host__ __device__ constexpr int col0(int warp, int lane) {
+        return (warp & 1) * 16 + ((lane >> 3) << 2) + (lane & 3);
+    }
+};
+
+// Phase and bin of a tile's pixels as polynomials.  With the far-field
+// remainder's phase Q(i, j) = kr g = -kr (t^2 - |d|^2)(h + t hr), a cubic in
+// the pixel's row and column offsets i, j from the tile centre,
+//     Q = i^2 (q20 + i q30) + j i (q11 + i q21) + j^2 (q02 + i q12 + j q03),
+// the phase is 2 pi frac(A + i alpha + j beta) + Q and the window-centred bin
+// B0 - W + i gam + j eta + sigma Q, sigma = lambda / kr.  Around a thread's
+// middle row i = i_c + 2 k both are P0 + k a + k^2 b: the table holds the
+// parts of P0, a, b that depend on i_c only (8 row entries of two float4)
+// and the column phases (32 floats); a thread completes them with its two
+// columns (13 paired operations a pulse), so phase and bin cost 22 paired
+// operations per 16 pixels instead of a full evaluation of t, t^2 - |d|^2 and
+// the remainder for each (64).  The
+// k^3 term of Q (2 k <= 8 rows: 1/64 of the tile's cubic term, < 6e-7 rad at
+// 100 m / 1024 pixels, 8 km) is folded into a by least squares over k.
+//   [2e]     phase, bin, x1 = i (q11 + i q21), x2 = q02 + i q12
+//   [2e + 1] phase step, bin step, step's j term, k^2 phase term
+//   [16..]   2 pi frac(j beta), j = -32..-1
+// and, in the record's first two words (its FP64 steps, no longer needed):
+//   [0]      2 pi frac(32 beta), eta, sigma, q03
+//   [1]      step's j^2 term, k^2 term's j term, lo, hi
+// Near-field pulses keep the linear parts only (their remainder is evaluated
+// per pixel).
+constexpr int kPolyCols = 16, kPolyEntries = kPolyCols + 8;
+constexpr int kRecWords = sizeof(PulseGeo) / sizeof(float4);
+
+// The tables of a stage of PB pulses by one warp, records in rec[0, PB).
+// Lanes q < PB first put the cubic's coefficients of their pulse into words 3
+// and 7 of its record (the forward kernel reads neither), then the 8 PB row
+// entries and the 32 PB column phases are spread over the 32 lanes.
+template <int MX, int PB>
+__device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, int lane, const BpLaunch &L) {
+    using M = PixelMap<MX>;
+    float4 un0 = make_float4(0.f, 0.f, 0.f, 0.f), un1 = un0;
+    if (lane < PB) {
+        float4 *w = reinterpret_cast<float4 *>(rec + lane);
+        const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // a8r, b32r, g8, e32; tx, ty, h, hr; kr, rc, lo, hi
+        const float dx = static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
+        const float m = (rec[lane].flags & PG_NEAR) ? 0.0f : -c2.x;
+        const float n20 = fmaf(c1.x, c1.x, -dx * dx), n11 = 2.0f * c1.x * c1.y, n02 = fmaf(c1.y, c1.y, -dy * dy);
+        const float mh = m * c1.z, mr = m * c1.w;
+        const float q21 = mr * fmaf(c1.x, n11, c1.y * n20), q12 = mr * fmaf(c1.x, n02, c1.y * n11);
+        const float q03 = mr * c1.y * n02, sigma = static_cast<float>(L.lambda) / c2.x;
+        w[7] = make_float4(mh * n20, mh * n11, mh * n02, mr * c1.x * n20);
+        w[3] = make_float4(q21, q12, sigma, 0.0f);
+        un0 = make_float4(c0.y, c0.w * (1.0f / 32.0f), sigma, q03);
+        un1 = make_float4(2.0f * q12, 4.0f * q21, c2.z, c2.w);
+    }
+    __syncwarp();
+    // k^3 ~ kFit k over the thread's rows k = -kMid .. MX - kMid - 1
+    constexpr float kFit = MX == 8 ? 452.0f / 44.0f : (MX == 4 ? 3.0f : (MX == 2 ? 1.0f : 0.0f));
+    for (int t = lane; t < 8 * PB; t += 32) {
+        const int q = t >> 3, e = t & 7;
+        const float4 *w = reinterpret_cast<const float4 *>(rec + q);
+        const double2 d0 = *reinterpret_cast<const double2 *>(w);  // A, alpha
+        const double B0 = rec[q].B0, gam = rec[q].gam;
+        const float4 qa = w[7], qb = w[3];  // q20, q11, q02, q30; q21, q12, sigma
+        const float i = static_cast<float>(M::mid_row(e));
+        const double id = static_cast<double>(i);
+        const double pr = fma(id, d0.y, d0.x), ps = 2.0 * d0.y;
+        const float nl = i * i * fmaf(i, qa.w, qa.x);
+        const float an = fmaf(8.0f * kFit, qa.w, 2.0f * i * fmaf(3.0f * i, qa.w, 2.0f * qa.x));
+        float4 *row = tabs + q * kPolyEntries + 2 * e;
+        row[0] = make_float4(static_cast<float>(kTwoPi * (pr - rint(pr))) + nl,
+                             fmaf(qb.z, nl, static_cast<float>(fma(id, gam, B0 - L.W))), i * fmaf(i, qb.x, qa.y),
+                             fmaf(i, qb.y, qa.z));
+        row[1] = make_float4(static_cast<float>(kTwoPi * (ps - rint(ps))) + an,
+                             fmaf(qb.z, an, static_cast<float>(2.0 * gam)), 2.0f * fmaf(2.0f * i, qb.x, qa.y),
+                             4.0f * fmaf(3.0f * i, qa.w, qa.x));
+    }
+    const double jd = static_cast<double>(lane - kTY / 2);
+#pragma unroll
+    for (int q = 0; q < PB; ++q) {
+        const double pc = jd * rec[q].beta;
+        reinterpret_cast<float *>(tabs + q * kPolyEntries + kPolyCols)[lane] =
+            static_cast<float>(kTwoPi * (pc - rint(pc)));
+    }
+    __syncwarp();
+    if (lane < PB) {
+        float4 *w = reinterpret_cast<float4 *>(rec + lane);
+        w[0] = un0;
+        w[1] = un1;
+    }
+}
+
 // Lane 0: the window copy of pulse p (slot q) into the stage buffer, or a
 // plain arrival when the tile's window misses the pulse's range bins.  The
 // test hook L.drop_pulse expects that pulse's bytes without copying them.
@@ -375,6 +489,28 @@ __device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
 // c_n and Zv = j nu v'_n, so that Z(B) = Zc + B Zv is again one fused
 // multiply-add per component and the pixel loop neither interpolates v nor
 // forms Z.
+template <bool ZFORM>
+__device__ __forceinline__ void rewrite_window(uint32_t w, int W, int wp, int lane, float nu) {
+    uint32_t a = w + static_cast<uint32_t>(W - wp + lane) * 16u;
+    float m = static_cast<float>(lane - wp);
+    auto one = [&](uint32_t at, float mm) {
+        const float4 e = lds128(at);
+        const float cr = fmaf(-mm, e.z, e.x), ci = fmaf(-mm, e.w, e.y);
+        if (ZFORM)
+            sts128(at, fmaf(-nu, ci, e.z), fmaf(nu, cr, e.w), -nu * e.w, nu * e.z);
+        else
+            sts64(at, cr, ci);
+    };
+    int left = 2 * wp + 2 - lane;  // the entries the pulse's tight window copied
+    for (; left > 96; left -= 128, a += 2048u, m += 128.0f) {
+        one(a, m);
+        one(a + 512u, m + 32.0f);
+        one(a + 1024u, m + 64.0f);
+        one(a + 1536u, m + 96.0f);
+    }
+    for (; left > 0; left -= 32, a += 512u, m += 32.0f) one(a, m);
+}
+
 template <int PB, bool ZFORM = false>
 __device__ __forceinline__ bool intercept_slots(const PulseGeo *geo_s, uint32_t win_s, uint32_t bar, uint32_t parity,
                                                 int wsize, int W, int warp, int lane, unsigned *err,
@@ -383,20 +519,8 @@ __device__ __forceinline__ bool intercept_slots(const PulseGeo *geo_s, uint32_t 
     if (!mbar_wait_bounded(bar, parity, err)) return false;
     for (int q = warp; q < PB; q += kWarps) {
         if (!(geo_s[q].flags & PG_ACTIVE)) continue;
-        const uint32_t w = win_s + static_cast<uint32_t>(q) * static_cast<uint32_t>(wsize) * 16u;
-        // the entries the pulse's tight window copied
-        const int wp = geo_s[q].wp;
-        const float nu = ZFORM ? geo_s[q].kr * inv_lam : 0.0f;
-        for (int n = W - wp + lane; n < W + wp + 2; n += 32) {
-            const uint32_t a = w + static_cast<uint32_t>(n) * 16u;
-            const float4 e = lds128(a);
-            const float m = static_cast<float>(n - W);
-            const float cr = fmaf(-m, e.z, e.x), ci = fmaf(-m, e.w, e.y);
-            if (ZFORM)
-                sts128(a, fmaf(-nu, ci, e.z), fmaf(nu, cr, e.w), -nu * e.w, nu * e.z);
-            else
-                sts64(a, cr, ci);
-        }
+        rewrite_window<ZFORM>(win_s + static_cast<uint32_t>(q) * static_cast<uint32_t>(wsize) * 16u, W, geo_s[q].wp,
+                              lane, ZFORM ? geo_s[q].kr * inv_lam : 0.0f);
     }
     // these generic-proxy stores precede the next bulk copy (async proxy) into
     // the same buffer, issued after the CTA barrier
