@@ -66,29 +66,19 @@ __device__ __forceinline__ void produce_slots64(const BpLaunch &L, int b, PulseG
     }
 }
 
-// Store (or add) a thread's MX x 2 pixels of the tile at (tx0, ty0, z-slice iz).
-template <int MX>
-__device__ __forceinline__ void store_pixels64(const BpLaunch &L, int tx0, int ty0, int iz, int warp, int lane,
-                                               const double (&re)[MX][2], const double (&im)[MX][2]) {
+// Store (or add) a thread's pixel (k, l) of the tile at (tx0, ty0, z-slice iz).
+__device__ __forceinline__ void store_pixel64(const BpLaunch &L, int tx0, int ty0, int iz, int warp, int lane, int k,
+                                              int l, double2 v) {
     double2 *img = static_cast<double2 *>(L.img);
-#pragma unroll
-    for (int k = 0; k < MX; ++k) {
-        const int row = tx0 + warp + 8 * k;
-        if (row >= L.nx) continue;
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            const int col = ty0 + 2 * lane + l;
-            if (col >= L.ny) continue;
-            const long long o = (static_cast<long long>(iz) * L.nx + row) * L.ny + col;
-            double2 v = make_double2(re[k][l], im[k][l]);
-            if (L.accumulate) {
-                const double2 old = img[o];
-                v.x += old.x;
-                v.y += old.y;
-            }
-            img[o] = v;
-        }
+    const int row = tx0 + warp + 8 * k, col = ty0 + 2 * lane + l;
+    if (row >= L.nx || col >= L.ny) return;
+    const long long o = (static_cast<long long>(iz) * L.nx + row) * L.ny + col;
+    if (L.accumulate) {
+        const double2 old = img[o];
+        v.x += old.x;
+        v.y += old.y;
     }
+    img[o] = v;
 }
 
 // Tile-local index of pixel (row warp + 8k, column 2 lane + l) in a
@@ -209,7 +199,12 @@ __global__ void __launch_bounds__(kThreads, 1) bp_fp64_kernel(const BpLaunch L) 
         }
         if (i + 1 == n || b == S - 1) {
             if (seg_first == 0 && b == S - 1) {
-                store_pixels64<MX>(L, cc.tx * TX, cc.ty * kTY, cc.iz, warp, lane, acc_re, acc_im);
+#pragma unroll
+                for (int k = 0; k < MX; ++k)
+#pragma unroll
+                    for (int l = 0; l < 2; ++l)
+                        store_pixel64(L, cc.tx * TX, cc.ty * kTY, cc.iz, warp, lane, k, l,
+                                      make_double2(acc_re[k][l], acc_im[k][l]));
             } else {
                 double2 *slot = static_cast<double2 *>(L.sk_partial) +
                                 (2 * static_cast<long long>(blockIdx.x) + (seg > 0 ? 1 : 0)) * (TX * kTY);
@@ -239,27 +234,19 @@ __global__ void __launch_bounds__(kThreads) bp_sk_fixup64_kernel(const BpLaunch 
     const long long c0 = tile::sk_owner(t * tg.stages, tg.units, G);
     const long long c1 = tile::sk_owner(t * tg.stages + tg.stages - 1, tg.units, G);
     if (c0 == c1) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double re[MX][2], im[MX][2];
-#pragma unroll
-    for (int k = 0; k < MX; ++k)
-#pragma unroll
-        for (int l = 0; l < 2; ++l) re[k][l] = im[k][l] = 0.0;
-    const double2 *part = static_cast<const double2 *>(L.sk_partial);
-    for (long long c = c0; c <= c1; ++c) {
-        const double2 *slot = part + tile::sk_slot(c, t * tg.stages, tg.units, G) * (TX * kTY);
-#pragma unroll
-        for (int k = 0; k < MX; ++k)
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                const double2 v = slot[slot_pixel(warp, lane, k, l)];
-                re[k][l] += v.x;
-                im[k][l] += v.y;
-            }
-    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = blockIdx.y;
     int tx0, ty0, iz;
     tile::tile_origin(tg, t, TX, tx0, ty0, iz);
-    store_pixels64<MX>(L, tx0, ty0, iz, warp, lane, re, im);
+    const long long s0 = tile::sk_first_slot(c0, t * tg.stages, tg.units, G);
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const double2 v = tile::sk_sum(static_cast<const double2 *>(L.sk_partial), TX * kTY,
+                                       slot_pixel(warp, lane, k, l), s0, c0, c1, [](double2 &s, const double2 &e) {
+                                           s.x += e.x;
+                                           s.y += e.y;
+                                       });
+        store_pixel64(L, tx0, ty0, iz, warp, lane, k, l, v);
+    }
 }
 
 template <int MX, int PB>
@@ -279,7 +266,7 @@ cudaError_t launch64(const BpLaunch &L, size_t smem, cudaStream_t s) {
     kern<<<static_cast<unsigned>(G), kThreads, smem, s>>>(L);
     e = cudaGetLastError();
     if (e != cudaSuccess || G == tg.tiles) return e;
-    bp_sk_fixup64_kernel<MX><<<static_cast<unsigned>(tg.tiles), kThreads, 0, s>>>(L, G, PB);
+    bp_sk_fixup64_kernel<MX><<<dim3(static_cast<unsigned>(tg.tiles), MX), kThreads, 0, s>>>(L, G, PB);
     return cudaGetLastError();
 }
 

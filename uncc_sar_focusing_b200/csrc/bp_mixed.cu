@@ -188,30 +188,28 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
     }
 }
 
-// Store (or add, L.accumulate) a thread's MX x 2 pixels of the tile at
-// (tx0, ty0, slice zz) into the complex64 image (PixelMap: every store of a
-// warp is 16 consecutive pixels, 128 bytes, of each of two rows).
+// Store (or add, L.accumulate) a thread's pixel pair k of the tile at (tx0,
+// ty0, slice zz) into the complex64 image (PixelMap: every store of a warp is
+// 16 consecutive pixels, 128 bytes, of each of two rows).  v: re, im of the
+// first column, re, im of the second.
 template <int MX>
-__device__ __forceinline__ void store_pixels(const BpLaunch &L, int tx0, int ty0, int zz, int warp, int lane,
-                                             const float (&re)[MX][2], const float (&im)[MX][2]) {
+__device__ __forceinline__ void store_pair(const BpLaunch &L, int tx0, int ty0, int zz, int warp, int lane, int k,
+                                           const float4 &v) {
     float2 *img = static_cast<float2 *>(L.img);
+    const int row = tx0 + PixelMap<MX>::row0(warp, lane) + PixelMap<MX>::kStep * k;
+    if (row >= L.nx) return;
 #pragma unroll
-    for (int k = 0; k < MX; ++k) {
-        const int row = tx0 + PixelMap<MX>::row0(warp, lane) + PixelMap<MX>::kStep * k;
-        if (row >= L.nx) continue;
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            const int col = ty0 + PixelMap<MX>::col0(warp, lane) + (kTY / 2) * l;
-            if (col >= L.ny) continue;
-            const long long o = (static_cast<long long>(zz) * L.nx + row) * L.ny + col;
-            float2 v = make_float2(re[k][l], im[k][l]);
-            if (L.accumulate) {
-                const float2 old = img[o];
-                v.x += old.x;
-                v.y += old.y;
-            }
-            img[o] = v;
+    for (int l = 0; l < 2; ++l) {
+        const int col = ty0 + PixelMap<MX>::col0(warp, lane) + (kTY / 2) * l;
+        if (col >= L.ny) continue;
+        const long long o = (static_cast<long long>(zz) * L.nx + row) * L.ny + col;
+        float2 p = l ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+        if (L.accumulate) {
+            const float2 old = img[o];
+            p.x += old.x;
+            p.y += old.y;
         }
+        img[o] = p;
     }
 }
 
@@ -476,8 +474,10 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
         if (i + 1 == n || b == S - 1) {
             // the segment of this tile ends: whole tile -> image, else -> partial slot
             if (seg_first == 0 && b == S - 1) {
-                store_pixels<MX>(L, cur.u.tx * TX, cur.u.ty * kTY, cur.u.hyp * L.nz + cur.u.iz, warp, lane, acc_re,
-                                 acc_im);
+#pragma unroll
+                for (int k = 0; k < MX; ++k)
+                    store_pair<MX>(L, cur.u.tx * TX, cur.u.ty * kTY, cur.u.hyp * L.nz + cur.u.iz, warp, lane, k,
+                                   make_float4(acc_re[k][0], acc_im[k][0], acc_re[k][1], acc_im[k][1]));
                 // completion time: the latest of the warps' stores
                 if (BATCH && done) {
                     __syncwarp();
@@ -503,8 +503,9 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
 
 // Tiles whose stages were split over several CTAs: add the CTAs' partial
 // sums in CTA order (a fixed order, so results repeat bit for bit) and store
-// the tile.  One CTA per tile of the launch; tiles held whole by one CTA
-// return at once.
+// the tile.  One CTA per (tile of the launch, row step k of its threads), so
+// the few tiles of a small image still fill the SMs; tiles held whole by one
+// CTA return at once.
 template <int MX, int PB, bool BATCH>
 __global__ void __launch_bounds__(kThreads)
     bp_sk_fixup_kernel(const __grid_constant__ BpLaunch L0, const BatchScene *__restrict__ scenes, int nscenes,
@@ -531,27 +532,17 @@ __global__ void __launch_bounds__(kThreads)
     const long long c0 = sk_owner(first, units, G);
     const long long c1 = sk_owner(first + tg.stages - 1, units, G);
     if (c0 == c1) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float re[MX][2], im[MX][2];
-#pragma unroll
-    for (int k = 0; k < MX; ++k)
-#pragma unroll
-        for (int l = 0; l < 2; ++l) re[k][l] = im[k][l] = 0.0f;
-    const float4 *part = static_cast<const float4 *>(L0.sk_partial);
-    for (long long c = c0; c <= c1; ++c) {
-        const float4 *slot = part + sk_slot(c, first, units, G) * (TX * kTY / 2);
-#pragma unroll
-        for (int k = 0; k < MX; ++k) {
-            const float4 v = slot[slot_pair(k)];
-            re[k][0] += v.x;
-            im[k][0] += v.y;
-            re[k][1] += v.z;
-            im[k][1] += v.w;
-        }
-    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = blockIdx.y;
+    const float4 v = sk_sum(static_cast<const float4 *>(L0.sk_partial), TX * kTY / 2, slot_pair(k),
+                            sk_first_slot(c0, first, units, G), c0, c1, [](float4 &s, const float4 &e) {
+                                s.x += e.x;
+                                s.y += e.y;
+                                s.z += e.z;
+                                s.w += e.w;
+                            });
     int tx0, ty0, zz;
     tile_origin(tg, t, TX, tx0, ty0, zz);
-    store_pixels<MX>(L, tx0, ty0, zz, warp, lane, re, im);
+    store_pair<MX>(L, tx0, ty0, zz, warp, lane, k, v);
     if (BATCH && done) {
         __syncthreads();
         if (threadIdx.x == 0) atomicMax(done + scene, global_timer_ns());
@@ -683,7 +674,7 @@ cudaError_t launch_kernels(const BpLaunch &L0, size_t smem, cudaStream_t s) {
     e = cudaGetLastError();
     if (e != cudaSuccess || G == tg.tiles) return e;
     bp_sk_fixup_kernel<MX, PB, false>
-        <<<static_cast<unsigned>(tg.tiles), kThreads, 0, s>>>(L, nullptr, 0, tg.units, G, nullptr);
+        <<<dim3(static_cast<unsigned>(tg.tiles), MX), kThreads, 0, s>>>(L, nullptr, 0, tg.units, G, nullptr);
     return cudaGetLastError();
 }
 
@@ -737,7 +728,7 @@ cudaError_t launch_batch_kernels(const BatchScene *scenes, int nscenes, long lon
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     bp_sk_fixup_kernel<MX, PB, true>
-        <<<static_cast<unsigned>(tiles), kThreads, 0, s>>>(L0, scenes, nscenes, units, G, done);
+        <<<dim3(static_cast<unsigned>(tiles), MX), kThreads, 0, s>>>(L0, scenes, nscenes, units, G, done);
     return cudaGetLastError();
 }
 

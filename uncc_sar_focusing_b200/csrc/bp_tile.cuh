@@ -56,11 +56,32 @@ __device__ __forceinline__ long long sk_owner(long long u, long long units, long
     return c;
 }
 
-// Partial-sum slot of CTA c's segment of the tile whose first unit is
-// `first`: its first segment (the one holding unit lo(c)) uses slot 2c, a
-// later one slot 2c + 1.
-__device__ __forceinline__ long long sk_slot(long long c, long long first, long long units, long long G) {
-    return sk_lo(c, units, G) >= first ? 2 * c : 2 * c + 1;
+// Partial-sum slot of the first CTA c0 = sk_owner(first) of the tile whose
+// first unit is `first`: a CTA's first segment (the one holding unit lo(c))
+// uses slot 2c, a later one slot 2c + 1.  The tile's other CTAs c > c0 start
+// inside it (lo(c) > first), so theirs is slot 2c.
+__device__ __forceinline__ long long sk_first_slot(long long c0, long long first, long long units, long long G) {
+    return sk_lo(c0, units, G) >= first ? 2 * c0 : 2 * c0 + 1;
+}
+
+// Sum of element `at` of a split tile's partial slots (`stride` elements
+// each) in CTA order: slot s0, then those of CTAs c0 + 1 .. c1.  Four loads
+// ahead of their additions: a tile of a small image is spread over 20 or more
+// CTAs, and one load after the other took 34 us for 16 tiles x 18 slots.
+template <typename V, typename ADD>
+__device__ __forceinline__ V sk_sum(const V *part, long long stride, long long at, long long s0, long long c0,
+                                    long long c1, ADD add) {
+    V v = part[s0 * stride + at];
+    long long c = c0 + 1;
+    for (; c + 3 <= c1; c += 4) {
+        V e[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[i] = part[2 * (c + i) * stride + at];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) add(v, e[i]);
+    }
+    for (; c <= c1; ++c) add(v, part[2 * c * stride + at]);
+    return v;
 }
 
 // Pixel origin (row tx0, column ty0) and hypothesis-major slice zz of tile t.
