@@ -28,8 +28,8 @@ void window_for(const sarbp_plan *p, int mx, int *W, int *wsize) {
     tile_window(p->lambda, p->dx, p->dy, mx, W, wsize, &hd);
 }
 
-// Largest stage depth whose shared memory fits 2 CTAs per SM (mixed) or one
-// (FP64); environment SARBP_TILE="mx,pb" overrides (tuning runs).
+// Largest stage depth whose shared memory fits 2 CTAs per SM, else one;
+// environment SARBP_TILE="mx,pb" overrides (tuning runs).
 int choose_tile(sarbp_plan *p) {
     // (mx, pb) candidates, best first; the first pass keeps two CTAs per SM
     // for the mixed kernel, the second accepts one CTA per SM (coarse grids
@@ -47,7 +47,7 @@ int choose_tile(sarbp_plan *p) {
     if (const char *env = std::getenv("SARBP_TILE")) {
         if (std::sscanf(env, "%d,%d", &forced_mx, &forced_pb) != 2) forced_mx = forced_pb = 0;
     }
-    const size_t limits[2] = {fp64 ? 220u * 1024u : 110u * 1024u, 227u * 1024u};
+    const size_t limits[2] = {110u * 1024u, 227u * 1024u};
     for (int pass = -1; pass < 2; ++pass) {
         for (int i = 0; i < ncand; ++i) {
             int mx = cand[i][0], pb = cand[i][1];
@@ -120,7 +120,7 @@ void release(sarbp_plan *p) {
     if (p->fft_ok) cufftDestroy(p->fft);
     cudaFree(p->d_ph);
     cudaFree(p->d_geo);
-    cudaFree(p->d_fft);
+    cudaFree(p->d_fft_base);
     cudaFree(p->d_pairs);
     cudaFree(p->d_fac);
     cudaFree(p->d_img);
@@ -204,7 +204,9 @@ int range_compress_impl(sarbp_plan *p, const void *ph, int np, int memory, cudaS
             : cufftExecC2C(p->fft, static_cast<cufftComplex *>(p->d_fft), static_cast<cufftComplex *>(p->d_fft),
                            CUFFT_INVERSE);
     if (r1 != CUFFT_SUCCESS) return from_cufft(r1);
-    SARBP_TRY_CUDA(launch_rc_pairs(p->precision, p->d_fft, p->d_pairs, p->nfft, np, p->row_stride, p->guard, s));
+    // the FP64 backprojection stages the FFT output itself
+    if (p->precision == SARBP_PRECISION_MIXED)
+        SARBP_TRY_CUDA(launch_rc_pairs(p->d_fft, p->d_pairs, p->nfft, np, p->row_stride, p->guard, s));
     p->np_ready = np;
     if (memory == SARBP_MEMORY_HOST) SARBP_TRY_CUDA(cudaStreamSynchronize(s));
     return SARBP_OK;
@@ -214,9 +216,10 @@ BpLaunch launch_params(const sarbp_plan *p, const double *ax, const double *ay, 
                        const double *f0, int np, void *img, int flags) {
     const sarbp_grid &g = p->desc.grid;
     BpLaunch L{};
-    L.pairs = p->d_pairs;
-    L.row_stride = p->row_stride;
-    L.guard = p->guard;
+    const bool fp64 = p->precision == SARBP_PRECISION_FP64;
+    L.pairs = fp64 ? p->d_fft : p->d_pairs;
+    L.row_stride = fp64 ? p->nfft : p->row_stride;
+    L.guard = fp64 ? 0 : p->guard;
     L.ax = ax;
     L.ay = ay;
     L.az = az;
@@ -705,13 +708,18 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
     p->guard = p->wsize + 2;
     p->row_stride = static_cast<long long>(p->nfft) + 2LL * p->guard;
     const size_t cb = cplx_bytes(p);
-    const size_t entry = p->precision == SARBP_PRECISION_FP64 ? 32 : 16;
+    // mixed: pair rows with guards.  FP64: windows come from the FFT buffer,
+    // rows back to back, where a window past a row's end reads samples of the
+    // neighbouring row that the gate discards; guards at the buffer's ends
+    const bool fp64 = p->precision == SARBP_PRECISION_FP64;
+    const size_t fft_guard = fp64 ? static_cast<size_t>(p->guard) : 0;
     const size_t npix = static_cast<size_t>(g.nx) * g.ny * g.nz;
     const size_t np = static_cast<size_t>(p->np_cap);
+    const size_t pair_bytes = np * static_cast<size_t>(p->row_stride) * 16;
     if ((st = alloc(p, &p->d_ph, np * p->K * 8)) ||
         (st = alloc(p, reinterpret_cast<void **>(&p->d_geo), 5 * np * sizeof(double))) ||
-        (st = alloc(p, &p->d_fft, np * p->nfft * cb)) ||
-        (st = alloc(p, &p->d_pairs, np * static_cast<size_t>(p->row_stride) * entry)) ||
+        (st = alloc(p, &p->d_fft_base, (np * p->nfft + 2 * fft_guard) * cb)) ||
+        (!fp64 && (st = alloc(p, &p->d_pairs, pair_bytes))) ||
         (st = alloc(p, &p->d_fac, static_cast<size_t>(p->K) * cb)) || (st = alloc(p, &p->d_img, npix * cb)) ||
         (st = alloc(p, reinterpret_cast<void **>(&p->d_err), sizeof(unsigned)))) {
         release(p);
@@ -740,8 +748,9 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
                 p->geotab_records = recs;
         }
     }
-    if (cudaMemset(p->d_pairs, 0, np * static_cast<size_t>(p->row_stride) * entry) != cudaSuccess ||
-        cudaMemset(p->d_fft, 0, np * p->nfft * cb) != cudaSuccess ||
+    p->d_fft = static_cast<unsigned char *>(p->d_fft_base) + fft_guard * cb;
+    if ((!fp64 && cudaMemset(p->d_pairs, 0, pair_bytes) != cudaSuccess) ||
+        cudaMemset(p->d_fft_base, 0, (np * p->nfft + 2 * fft_guard) * cb) != cudaSuccess ||
         cudaMemset(p->d_err, 0, sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         release(p);

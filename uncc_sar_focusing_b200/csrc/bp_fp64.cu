@@ -1,12 +1,23 @@
 // bp_fp64.cu -- all-FP64 forward backprojection for sm_100a.
 //
-// Same tiling, shared-memory window staging (cp.async.bulk + mbarrier) and
-// output layout as the mixed kernel in bp_mixed.cu, but every pixel-pulse is
-// computed directly in double: |a_p - x_q| with a double sqrt, the bin
-// index, the linear interpolation of FP64 range profiles and the rotation
-// exp(+j 2 pi k dR) (k = 2 f0 / c, reduced mod one revolution, sincospi),
-// accumulated in double.  It is the accuracy path and the FP64 baseline the
-// mixed kernel is measured against; semantics as bp_mixed.cu.
+// Same tiling, shared-memory window staging (cp.async.bulk + mbarrier), pixel
+// map and output layout as the mixed kernel in bp_mixed.cu, but every
+// pixel-pulse is computed directly in double: |a_p - x_q| with a correctly
+// rounded square root, the bin index, the linear interpolation of FP64 range
+// profiles and the rotation exp(+j 2 pi k dR) (k = 2 f0 / c, reduced mod one
+// revolution), accumulated in double.  It is the accuracy path and the FP64
+// baseline the mixed kernel is measured against; semantics as bp_mixed.cu.
+//
+// What bounds it is the FP64 pipe (64 lanes per SM and cycle): about 40 FP64
+// instructions per pixel-pulse.  The common path has no branch and no library
+// call, so a thread's eight pixels are independent chains the scheduler
+// interleaves, on two CTAs per SM; the square root is a reciprocal-root
+// estimate with one coupled Newton step and a residual correction, the
+// rotation one quadrant reduction and two polynomials; window entries are the
+// range profile's samples themselves (the FFT output), the slope formed per
+// pixel, so no pair rows are written (18-39 us a call) and a window is half
+// the shared memory.  512^2 pixels x 1024 pulses: 2049 us with sqrt(),
+// sincospi() and a gate branch per pixel at one CTA per SM, now NEW us.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -17,11 +28,10 @@ namespace sarbp {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kWarps64 = kThreads / 32;
 constexpr int kTY = 64;
-
-struct __align__(16) PairD {
-    double vr, vi, dr, di;  // rc[b] and rc[b+1] - rc[b]
-};
+// four mbarriers (full, empty; two buffers each), then two zero samples
+constexpr int kHdr64 = 64;
 
 __device__ __forceinline__ PulseGeo64 make_geo64(const BpLaunch &L, int p, double cx, double cy, double cz) {
     PulseGeo64 g;
@@ -32,7 +42,8 @@ __device__ __forceinline__ PulseGeo64 make_geo64(const BpLaunch &L, int p, doubl
     g.r0 = L.r0[p];
     g.k = 2.0 * L.f0[p] / kClight;
     const double vx = g.ax - cx, vy = g.ay - cy, vz = g.az - cz;
-    const double D = sqrt(vx * vx + vy * vy + vz * vz) - g.r0;
+    const double rc = sqrt(vx * vx + vy * vy + vz * vz);
+    const double D = rc - g.r0;
     const double bc = D * L.lambda + L.half_nfft;
     if (!(isfinite(bc) && isfinite(g.k) && fabs(bc) < 1.0e9)) {
         atomicOr(L.err, ERRBIT_NOT_FINITE);
@@ -40,37 +51,118 @@ __device__ __forceinline__ PulseGeo64 make_geo64(const BpLaunch &L, int p, doubl
     }
     g.ws = static_cast<int>(floor(bc)) - L.W;
     if (!(g.ws + L.wsize - 2 <= 0 || g.ws + 1 >= L.nfft - 1)) g.flags = PG_ACTIVE;
+    // the window meets an end of the range bins: test each pixel's bin
+    if (g.ws < 0 || g.ws + L.wsize > L.nfft) g.flags |= PG_GATE;
+    // a pixel may come close to the antenna (or the phase, of a range in the
+    // thousands of kilometres, pass the reduction's range): library functions
+    if (rc <= 0.125 * L.near_hd16 || !(fabs(g.k * D) < 1.0e12)) g.flags |= PG_NEAR;
     return g;
 }
 
-// As produce_slots in bp_mixed.cu: warp w handles pulse slots w, w + 8, ...
-template <int PB>
-__device__ __forceinline__ void produce_slots64(const BpLaunch &L, int b, PulseGeo64 *geo_s, uint32_t win_s,
-                                                uint32_t bar, int warp, int lane, double cx, double cy, double cz) {
-    if (lane != 0) return;
-    for (int q = warp; q < PB; q += kThreads / 32) {
-        const int p = b * PB + q;
-        PulseGeo64 g;
-        g.flags = 0;
-        if (p < L.np) g = make_geo64(L, p, cx, cy, cz);
-        geo_s[q] = g;
-        if (g.flags & PG_ACTIVE) {
-            const uint32_t bytes = static_cast<uint32_t>(L.wsize) * 32u;
-            const PairD *src =
-                static_cast<const PairD *>(L.pairs) + static_cast<long long>(p) * L.row_stride + L.guard + g.ws;
-            mbar_arrive_expect_tx(bar, bytes);
-            bulk_copy_g2s(win_s + static_cast<uint32_t>(q) * bytes, src, bytes, bar);
-        } else {
-            mbar_arrive(bar);
+// Square root of a positive, normal s as sqrt() rounds it: with g ~ sqrt(s)
+// and h ~ 1 / (2 sqrt(s)) from the reciprocal-root estimate (2^-20 or
+// better), r = 1/2 - g h corrects both to 2^-39, and the residual s - g^2,
+// exact by fused multiply-add, corrects g once more (Markstein's scheme).
+__device__ __forceinline__ double sqrt_rn(double s) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    double g = s * y;
+    double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));  // y / 2
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, s), h, g);
+}
+
+// exp(+j 2 pi ph), |ph| < 2^50: ph = n/4 + r exactly, |r| <= 1/8; sin and cos
+// of 2 pi r as polynomials in r^2 (interpolated at the Chebyshev nodes of [0,
+// 1/64] in 60 digits; errors 2e-17 and 5e-17 before rounding), then the
+// quadrant n mod 4 by swap and sign.
+__device__ __forceinline__ void rotation(double ph, double &cs, double &sn) {
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    const double t = fma(ph, 4.0, kMagic);
+    const int q = __double2loint(t);
+    const double r = fma(t - kMagic, -0.25, ph);
+    const double z = r * r;
+    double S = 3.7808689593022957, C = 7.810290968144191;
+    S = fma(S, z, -15.093804209987114);
+    C = fma(C, z, -26.42425703488269);
+    S = fma(S, z, 42.058685020160894);
+    C = fma(C, z, 60.24462008593029);
+    S = fma(S, z, -76.70585970427454);
+    C = fma(C, z, -85.45681709034115);
+    S = fma(S, z, 81.60524927594804);
+    C = fma(C, z, 64.93939402236538);
+    S = fma(S, z, -41.341702240399634);
+    C = fma(C, z, -19.73920880217842);
+    S = r * fma(S, z, 6.283185307179586);
+    C = fma(C, z, 1.0);
+    const bool odd = q & 1;
+    const double c = odd ? S : C, s = odd ? C : S;
+    cs = __hiloint2double(__double2hiint(c) ^ (((q + 1) << 30) & 0x80000000), __double2loint(c));
+    sn = __hiloint2double(__double2hiint(s) ^ ((q << 30) & 0x80000000), __double2loint(s));
+}
+
+__device__ __forceinline__ double2 lds_d2(uint32_t addr) {
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr));
+    return v;
+}
+
+// One pulse into the thread's MX x 2 pixels.  SAFE: pixels gated by the valid
+// range bins, library square root and sine / cosine.
+template <int MX, bool SAFE>
+__device__ __forceinline__ void accumulate_pulse64(const BpLaunch &L, const PulseGeo64 &g, uint32_t w_addr,
+                                                   uint32_t zero_addr, const double (&xs)[MX], const double (&ys)[2],
+                                                   double z, double (&acc_re)[MX][2], double (&acc_im)[MX][2]) {
+    constexpr double kMagic = 6755399441055744.0;
+    const double gax = g.ax, gay = g.ay, gr0 = g.r0, gk = g.k, ez = g.az - z;
+    const uint32_t last = static_cast<uint32_t>(L.wsize - 2);
+    // entry floor(B) - ws: low word of floor(B) + kMagic (its low 32 bits are
+    // the integer itself)
+    const uint32_t base = static_cast<uint32_t>(g.ws);
+#pragma unroll
+    for (int k = 0; k < MX; ++k) {
+        const double ex = gax - xs[k];
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const double ey = gay - ys[l];
+            const double s = ex * ex + ey * ey + ez * ez;
+            const double dR = (SAFE ? sqrt(s) : sqrt_rn(s)) - gr0;
+            const double B = dR * L.lambda + L.half_nfft;
+            const double t = __dadd_rd(B, kMagic);
+            const double a = B - (t - kMagic);
+            const uint32_t idx = static_cast<uint32_t>(__double2loint(t)) - base;
+            uint32_t addr = w_addr + idx * 16u;
+            bool use = true;
+            if (SAFE) use = B > 0.0 && B < static_cast<double>(L.nfft - 1);  // rmin < dR < rmax
+            if (idx > last) {
+                if (use) atomicOr(L.err, ERRBIT_BOUNDS);
+                use = false;
+            }
+            addr = use ? addr : zero_addr;
+            const double2 v = lds_d2(addr), vn = lds_d2(addr + 16u);
+            const double re = fma(SAFE && !use ? 0.0 : a, vn.x - v.x, v.x);
+            const double im = fma(SAFE && !use ? 0.0 : a, vn.y - v.y, v.y);
+            const double ph = gk * dR;
+            double sn, cs;
+            if (SAFE)
+                sincospi(2.0 * (ph - rint(ph)), &sn, &cs);
+            else
+                rotation(ph, cs, sn);
+            acc_re[k][l] = fma(re, cs, fma(-im, sn, acc_re[k][l]));
+            acc_im[k][l] = fma(re, sn, fma(im, cs, acc_im[k][l]));
         }
     }
 }
 
 // Store (or add) a thread's pixel (k, l) of the tile at (tx0, ty0, z-slice iz).
+template <int MX>
 __device__ __forceinline__ void store_pixel64(const BpLaunch &L, int tx0, int ty0, int iz, int warp, int lane, int k,
                                               int l, double2 v) {
+    using M = tile::PixelMap<MX>;
     double2 *img = static_cast<double2 *>(L.img);
-    const int row = tx0 + warp + 8 * k, col = ty0 + 2 * lane + l;
+    const int row = tx0 + M::row0(warp, lane) + M::kStep * k, col = ty0 + M::col0(warp, lane) + (kTY / 2) * l;
     if (row >= L.nx || col >= L.ny) return;
     const long long o = (static_cast<long long>(iz) * L.nx + row) * L.ny + col;
     if (L.accumulate) {
@@ -81,19 +173,26 @@ __device__ __forceinline__ void store_pixel64(const BpLaunch &L, int tx0, int ty
     img[o] = v;
 }
 
-// Tile-local index of pixel (row warp + 8k, column 2 lane + l) in a
-// partial-sum slot of TX x 64 complex128 values.
-__device__ __forceinline__ int slot_pixel(int warp, int lane, int k, int l) { return (warp + 8 * k) * kTY + 2 * lane + l; }
+// Index of a thread's pixel (k, l) in a partial-sum slot of TX x 64
+// complex128 values (written and read by the same threads).
+__device__ __forceinline__ int slot_pixel(int k, int l) {
+    return (2 * k + l) * kThreads + static_cast<int>(threadIdx.x);
+}
 
 // Units of (tile, stage) split over the CTAs as in bp_mixed.cu (tile::sk_lo).
-template <int MX, int PB>
-__global__ void __launch_bounds__(kThreads, 1) bp_fp64_kernel(const BpLaunch L) {
+// Two stage buffers: "full" (PB arrivals and the window bytes) and "empty"
+// (one arrival per warp); warp 0 refills a buffer once every warp has
+// consumed it, its lanes q < PB one pulse each.
+template <int MX, int PB, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) bp_fp64_kernel(const __grid_constant__ BpLaunch L) {
+    using M = tile::PixelMap<MX>;
     constexpr int TX = 8 * MX;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-    PulseGeo64 *geo = reinterpret_cast<PulseGeo64 *>(smem + 32);
-    PairD *win = reinterpret_cast<PairD *>(smem + 32 + 2 * PB * sizeof(PulseGeo64));
-    const int wsize = L.wsize;
+    double2 *zero = reinterpret_cast<double2 *>(smem + 32);
+    PulseGeo64 *geo = reinterpret_cast<PulseGeo64 *>(smem + kHdr64);
+    const uint32_t win_addr = smem_addr(smem + kHdr64 + 2 * PB * sizeof(PulseGeo64));
+    const uint32_t pulse_bytes = static_cast<uint32_t>(L.wsize) * 16u, buf_bytes = PB * pulse_bytes;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const tile::TileGrid tg = tile::tile_grid(L, TX, PB);
@@ -108,111 +207,104 @@ __global__ void __launch_bounds__(kThreads, 1) bp_fp64_kernel(const BpLaunch L) 
     for (int k = 0; k < MX; ++k)
 #pragma unroll
         for (int l = 0; l < 2; ++l) acc_re[k][l] = acc_im[k][l] = 0.0;
-    const double top = static_cast<double>(L.nfft - 1);
 
-    const uint32_t bar_base = smem_addr(&bars[0]);  // buffer s barrier at bar_base + 8*s
+    const uint32_t bar_base = smem_addr(&bars[0]);  // full[s] at bar_base + 8 s, empty[s] at bar_base + 16 + 8 s
+    const uint32_t zero_addr = smem_addr(zero);
     if (threadIdx.x == 0) {
-        mbar_init(bar_base, PB);
-        mbar_init(bar_base + 8, PB);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(bar_base + 8u * s, PB);
+            mbar_init(bar_base + 16u + 8u * s, kWarps64);
+            zero[s] = make_double2(0.0, 0.0);
+        }
         fence_mbar_init();
     }
     __syncthreads();
 
+    // lane q < PB of warp 0: record and window copy of the unit's pulse q into buffer s
     auto produce = [&](const tile::UnitCursor &pc, int s) {
-        if (lane != 0) return;
+        if (lane >= PB) return;
         const double cx = L.left + static_cast<double>(pc.tx * TX + TX / 2) * L.dx;
         const double cy = L.bottom + static_cast<double>(pc.ty * kTY + kTY / 2) * L.dy;
         const double cz = L.zlow + static_cast<double>(pc.iz) * L.dz;
-        produce_slots64<PB>(L, pc.b, geo + s * PB, smem_addr(win + s * PB * wsize), bar_base + 8 * s, warp, lane, cx,
-                            cy, cz);
+        const int p = pc.b * PB + lane;
+        const uint32_t bar = bar_base + 8u * s;
+        PulseGeo64 g;
+        g.flags = 0;
+        if (p < L.np) g = make_geo64(L, p, cx, cy, cz);
+        geo[s * PB + lane] = g;
+        if (g.flags & PG_ACTIVE) {
+            const double2 *src =
+                static_cast<const double2 *>(L.pairs) + static_cast<long long>(p) * L.row_stride + L.guard + g.ws;
+            mbar_arrive_expect_tx(bar, pulse_bytes);
+            bulk_copy_g2s(win_addr + s * buf_bytes + lane * pulse_bytes, src, pulse_bytes, bar);
+        } else {
+            mbar_arrive(bar);
+        }
     };
 
-    tile::UnitCursor cc, pc;  // consumer at unit i, producer at unit i + 1
+    tile::UnitCursor cc, pc;  // consumer at unit i; warp 0's producer at unit i + 1
     cc.init(tg, L, lo);
     pc = cc;
-    produce(pc, 0);
-    __syncthreads();
+    if (warp == 0) produce(pc, 0);
 
-    int last_issued = 0;
     int seg = 0;
     int seg_first = cc.b;
     bool new_tile = true;
     for (int i = 0; i < n; ++i) {
         const int s = i & 1;
-        if (i + 1 < n) {
+        bool ok = true;
+        if (warp == 0 && i + 1 < n) {
             pc.advance(tg, L);
-            produce(pc, s ^ 1);
-            last_issued = i + 1;
+            if (i >= 1) ok = mbar_wait_bounded(bar_base + 16u + 8u * (s ^ 1), ((i - 1) >> 1) & 1, L.err);
+            if (ok) produce(pc, s ^ 1);
+            __syncwarp();
         }
         const int b = cc.b;
         if (new_tile) {
-            const int tx0 = cc.tx * TX, ty0 = cc.ty * kTY;
+            const int tx0 = cc.tx * TX + M::row0(warp, lane), ty0 = cc.ty * kTY + M::col0(warp, lane);
 #pragma unroll
-            for (int k = 0; k < MX; ++k) xs[k] = L.left + static_cast<double>(tx0 + warp + 8 * k) * L.dx;
+            for (int k = 0; k < MX; ++k) xs[k] = L.left + static_cast<double>(tx0 + M::kStep * k) * L.dx;
 #pragma unroll
-            for (int l = 0; l < 2; ++l) ys[l] = L.bottom + static_cast<double>(ty0 + 2 * lane + l) * L.dy;
+            for (int l = 0; l < 2; ++l) ys[l] = L.bottom + static_cast<double>(ty0 + (kTY / 2) * l) * L.dy;
             z = L.zlow + static_cast<double>(cc.iz) * L.dz;
             new_tile = false;
         }
-        const bool ok = mbar_wait_bounded(bar_base + 8 * s, (i >> 1) & 1, L.err);
-        if (ok) {
-            const int nq = min(PB, L.np - b * PB);
-            for (int q = 0; q < nq; ++q) {
-                const PulseGeo64 &g = geo[s * PB + q];
-                if (!(g.flags & PG_ACTIVE)) continue;
-                const PairD *w = win + (s * PB + q) * wsize;
-                const double gax = g.ax, gay = g.ay, gaz = g.az, gr0 = g.r0, gk = g.k;
-                const int gws = g.ws;
-                const double ez = gaz - z;
-#pragma unroll
-                for (int k = 0; k < MX; ++k) {
-                    const double ex = gax - xs[k];
-#pragma unroll
-                    for (int l = 0; l < 2; ++l) {
-                        const double ey = gay - ys[l];
-                        const double dR = sqrt(ex * ex + ey * ey + ez * ez) - gr0;
-                        const double B = dR * L.lambda + L.half_nfft;
-                        if (!(B > 0.0 && B < top)) continue;  // rmin < dR < rmax
-                        const double fl = floor(B);
-                        const int idx = static_cast<int>(fl) - gws;
-                        if (static_cast<unsigned>(idx) > static_cast<unsigned>(wsize - 2)) {
-                            atomicOr(L.err, ERRBIT_BOUNDS);
-                            continue;
-                        }
-                        const double a = B - fl;
-                        const PairD v = w[idx];
-                        const double re = fma(a, v.dr, v.vr);
-                        const double im = fma(a, v.di, v.vi);
-                        const double ph = gk * dR;
-                        double sn, cs;
-                        sincospi(2.0 * (ph - rint(ph)), &sn, &cs);
-                        acc_re[k][l] = fma(re, cs, fma(-im, sn, acc_re[k][l]));
-                        acc_im[k][l] = fma(re, sn, fma(im, cs, acc_im[k][l]));
-                    }
-                }
-            }
-        }
-        if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0 && last_issued > i)
-                mbar_wait_bounded(bar_base + 8 * (last_issued & 1), (last_issued >> 1) & 1, L.err);
+        ok = ok && mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err);
+        if (__any_sync(0xffffffffu, !ok)) {
+            // a wait ran out (error bit set): the other warps end at their own;
+            // warp 0's copies of the next stage land first (again bounded)
+            if (warp == 0 && i + 1 < n) mbar_wait_bounded(bar_base + 8u * (s ^ 1), ((i + 1) >> 1) & 1, L.err);
             return;
         }
+        const int nq = min(PB, L.np - b * PB);
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q) {
+            const PulseGeo64 &g = geo[s * PB + q];
+            const uint32_t w = win_addr + s * buf_bytes + q * pulse_bytes;
+            const int flags = g.flags;
+            if (!(flags & PG_ACTIVE)) continue;
+            if (flags & (PG_GATE | PG_NEAR))
+                accumulate_pulse64<MX, true>(L, g, w, zero_addr, xs, ys, z, acc_re, acc_im);
+            else
+                accumulate_pulse64<MX, false>(L, g, w, zero_addr, xs, ys, z, acc_re, acc_im);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_base + 16u + 8u * s);
         if (i + 1 == n || b == S - 1) {
             if (seg_first == 0 && b == S - 1) {
 #pragma unroll
                 for (int k = 0; k < MX; ++k)
 #pragma unroll
                     for (int l = 0; l < 2; ++l)
-                        store_pixel64(L, cc.tx * TX, cc.ty * kTY, cc.iz, warp, lane, k, l,
-                                      make_double2(acc_re[k][l], acc_im[k][l]));
+                        store_pixel64<MX>(L, cc.tx * TX, cc.ty * kTY, cc.iz, warp, lane, k, l,
+                                          make_double2(acc_re[k][l], acc_im[k][l]));
             } else {
                 double2 *slot = static_cast<double2 *>(L.sk_partial) +
                                 (2 * static_cast<long long>(blockIdx.x) + (seg > 0 ? 1 : 0)) * (TX * kTY);
 #pragma unroll
                 for (int k = 0; k < MX; ++k)
 #pragma unroll
-                    for (int l = 0; l < 2; ++l)
-                        slot[slot_pixel(warp, lane, k, l)] = make_double2(acc_re[k][l], acc_im[k][l]);
+                    for (int l = 0; l < 2; ++l) slot[slot_pixel(k, l)] = make_double2(acc_re[k][l], acc_im[k][l]);
             }
 #pragma unroll
             for (int k = 0; k < MX; ++k)
@@ -227,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_fp64_kernel(const BpLaunch L) 
 }
 
 template <int MX>
-__global__ void __launch_bounds__(kThreads) bp_sk_fixup64_kernel(const BpLaunch L, long long G, int PB) {
+__global__ void __launch_bounds__(kThreads) bp_sk_fixup64_kernel(const __grid_constant__ BpLaunch L, long long G, int PB) {
     constexpr int TX = 8 * MX;
     const tile::TileGrid tg = tile::tile_grid(L, TX, PB);
     const long long t = blockIdx.x;
@@ -240,19 +332,22 @@ __global__ void __launch_bounds__(kThreads) bp_sk_fixup64_kernel(const BpLaunch 
     const long long s0 = tile::sk_first_slot(c0, t * tg.stages, tg.units, G);
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
-        const double2 v = tile::sk_sum(static_cast<const double2 *>(L.sk_partial), TX * kTY,
-                                       slot_pixel(warp, lane, k, l), s0, c0, c1, [](double2 &s, const double2 &e) {
+        const double2 v = tile::sk_sum(static_cast<const double2 *>(L.sk_partial), TX * kTY, slot_pixel(k, l), s0, c0,
+                                       c1, [](double2 &s, const double2 &e) {
                                            s.x += e.x;
                                            s.y += e.y;
                                        });
-        store_pixel64(L, tx0, ty0, iz, warp, lane, k, l, v);
+        store_pixel64<MX>(L, tx0, ty0, iz, warp, lane, k, l, v);
     }
 }
 
-template <int MX, int PB>
-cudaError_t launch64(const BpLaunch &L, size_t smem, cudaStream_t s) {
+// two CTAs per SM (128 registers); one where the windows need its shared memory
+constexpr size_t kTwoCtaSmem = 113u * 1024u;
+
+template <int MX, int PB, int MINB>
+cudaError_t launch64_on(const BpLaunch &L, size_t smem, cudaStream_t s) {
     constexpr int TX = 8 * MX;
-    auto kern = bp_fp64_kernel<MX, PB>;
+    auto kern = bp_fp64_kernel<MX, PB, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     const tile::TileGrid tg = tile::tile_grid(L, TX, PB);
@@ -271,8 +366,13 @@ cudaError_t launch64(const BpLaunch &L, size_t smem, cudaStream_t s) {
 }
 
 template <int MX, int PB>
+cudaError_t launch64(const BpLaunch &L, size_t smem, cudaStream_t s) {
+    return smem > kTwoCtaSmem ? launch64_on<MX, PB, 1>(L, smem, s) : launch64_on<MX, PB, 2>(L, smem, s);
+}
+
+template <int MX, int PB>
 int resident64(size_t smem) {
-    auto kern = bp_fp64_kernel<MX, PB>;
+    auto kern = smem > kTwoCtaSmem ? bp_fp64_kernel<MX, PB, 1> : bp_fp64_kernel<MX, PB, 2>;
     int dev = 0, sms = 0, occ = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -288,8 +388,8 @@ int resident64(size_t smem) {
 }  // namespace
 
 size_t bp_fp64_smem_bytes(const TileConfig &tc, int wsize) {
-    return 32 + 2 * static_cast<size_t>(tc.pb) * sizeof(PulseGeo64) +
-           2 * static_cast<size_t>(tc.pb) * static_cast<size_t>(wsize) * 32;
+    return kHdr64 + 2 * static_cast<size_t>(tc.pb) * sizeof(PulseGeo64) +
+           2 * static_cast<size_t>(tc.pb) * static_cast<size_t>(wsize) * 16;
 }
 
 int bp_fp64_resident(const TileConfig &tc, size_t smem) {

@@ -12,7 +12,7 @@
 //     moved to the input side: ifft(x .* e^{j 2 pi k s/N})[n] = ifft(x)[n + s].
 //     The 1/Nfft scale and the taper ride along, so no normalise or shift pass.
 //  2. cuFFT batched C2C (Z2Z for FP64) inverse, in place.
-//  3. rc_pairs_kernel stores pair entries {rc[b], rc[b+1] - rc[b]} in rows of
+//  3. (mixed precision) rc_pairs_kernel stores pair entries {rc[b], rc[b+1] - rc[b]} in rows of
 //     `row_stride` entries with `guard` zero entries on each side, the layout
 //     the backprojection kernels stage into shared memory.
 #include <cmath>
@@ -43,35 +43,18 @@ __global__ void rc_prep_kernel(const float2 *__restrict__ ph, const C *__restric
     }
 }
 
-struct __align__(16) PairD {
-    double vr, vi, dr, di;
-};
-
 __device__ __forceinline__ void make_pair(const float2 &v, const float2 &vn, float4 *dst) {
     *dst = make_float4(v.x, v.y, vn.x - v.x, vn.y - v.y);
 }
-__device__ __forceinline__ void make_pair(const double2 &v, const double2 &vn, PairD *dst) {
-    PairD e;
-    e.vr = v.x;
-    e.vi = v.y;
-    e.dr = vn.x - v.x;
-    e.di = vn.y - v.y;
-    *dst = e;
-}
 
-template <typename C, typename E>
-__global__ void rc_pairs_kernel(const C *__restrict__ X, E *__restrict__ pairs, int nfft, long long total,
+__global__ void rc_pairs_kernel(const float2 *__restrict__ X, float4 *__restrict__ pairs, int nfft, long long total,
                                 long long row_stride, int guard) {
     const int per = nfft + 1;  // entries b = -1 .. nfft-1 of each row
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         const long long p = i / per;
         const int b = static_cast<int>(i - p * per) - 1;
-        C v, vn;
-        v.x = 0;
-        v.y = 0;
-        vn.x = 0;
-        vn.y = 0;
+        float2 v = make_float2(0.0f, 0.0f), vn = make_float2(0.0f, 0.0f);
         if (b >= 0) v = X[p * nfft + b];
         if (b + 1 < nfft) vn = X[p * nfft + b + 1];
         make_pair(v, vn, pairs + p * row_stride + guard + b);
@@ -371,15 +354,11 @@ cudaError_t launch_rc_prep(int precision, const void *ph, const void *fac, void 
     return cudaGetLastError();
 }
 
-cudaError_t launch_rc_pairs(int precision, const void *fft_buf, void *pairs, int nfft, int np, long long row_stride,
-                            int guard, cudaStream_t s) {
+cudaError_t launch_rc_pairs(const void *fft_buf, void *pairs, int nfft, int np, long long row_stride, int guard,
+                            cudaStream_t s) {
     const long long total = static_cast<long long>(np) * (nfft + 1);
-    if (precision == SARBP_PRECISION_FP64)
-        rc_pairs_kernel<double2, PairD><<<grid_for(total), 256, 0, s>>>(
-            static_cast<const double2 *>(fft_buf), static_cast<PairD *>(pairs), nfft, total, row_stride, guard);
-    else
-        rc_pairs_kernel<float2, float4><<<grid_for(total), 256, 0, s>>>(
-            static_cast<const float2 *>(fft_buf), static_cast<float4 *>(pairs), nfft, total, row_stride, guard);
+    rc_pairs_kernel<<<grid_for(total), 256, 0, s>>>(static_cast<const float2 *>(fft_buf), static_cast<float4 *>(pairs),
+                                                    nfft, total, row_stride, guard);
     return cudaGetLastError();
 }
 

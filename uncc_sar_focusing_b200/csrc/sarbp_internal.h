@@ -12,9 +12,9 @@ namespace sarbp {
 
 // Launch parameters of the forward backprojection kernels.
 struct BpLaunch {
-    const void *pairs;      // float4 (MIXED) / double4 (FP64) pair entries
+    const void *pairs;      // pair entries float4 (MIXED) / range-profile samples double2 (FP64)
     long long row_stride;   // entries per pulse row
-    int guard;              // zero entries before bin 0 of each row
+    int guard;              // zero entries before bin 0 of each row (MIXED)
     const double *ax, *ay, *az, *r0, *f0;
     int np, nfft;
     double lambda;          // nfft / max_wr (bins per metre)
@@ -132,8 +132,8 @@ int bp_fp64_resident(const TileConfig &tc, size_t smem);
 // Range compression kernels (range_compress.cu)
 cudaError_t launch_rc_prep(int precision, const void *ph, const void *fac, void *fft_buf, int K, int nfft, int np,
                            cudaStream_t s);
-cudaError_t launch_rc_pairs(int precision, const void *fft_buf, void *pairs, int nfft, int np, long long row_stride,
-                            int guard, cudaStream_t s);
+cudaError_t launch_rc_pairs(const void *fft_buf, void *pairs, int nfft, int np, long long row_stride, int guard,
+                            cudaStream_t s);
 // Range compression steps 1 and 3 for every scene of a batch in one launch
 // each (blockIdx.y = scene); the FFT in between runs per scene.
 cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStream_t s);
@@ -169,8 +169,9 @@ struct sarbp_plan {
 
     void *d_ph;       // complex64 [np][K] staging for host phase histories
     double *d_geo;    // 5 x np staging for host geometry
-    void *d_fft;      // complex64/128 [np][nfft]
-    void *d_pairs;    // pair entries [np][row_stride]
+    void *d_fft;      // complex64/128 [np][nfft], inside d_fft_base (FP64: guard samples at both ends)
+    void *d_fft_base;
+    void *d_pairs;    // pair entries [np][row_stride] (mixed precision)
     void *d_fac;      // per-sample window * scale * shift twiddle [K]
     void *d_img;      // image staging for host outputs
     unsigned *d_err;  // device error bits
