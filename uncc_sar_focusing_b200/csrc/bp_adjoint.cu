@@ -28,17 +28,26 @@
 //     sum_q s u_q = u (E0 + Et/Rc) - (dx Ei, dy Ej, 0)/Rc
 // with E0 = sum s, Ei = sum s i (Rc/R), Ej = sum s j (Rc/R) and Et = sum s t_eff.
 // In the far field t_eff is linear in (i, j), so a thread accumulates only
-// sum |G| Re(..) per column and sum row * |G| Re(..) over its pixels (two
-// paired FP32 accumulators) and Et follows from Ei and Ej.
+// sum |G| Re(..) per column and row step * |G| Re(..) over its pixels and Et
+// follows from Ei and Ej.
 //
 // Work split: the (tile, pulse-stage) units are divided over the resident
 // CTAs in contiguous ranges (bp_tile.cuh); every unit writes the per-tile
-// partial gradients of its own pulses, so no fix-up pass is needed.  Stages
-// are up to 8 pulses deep (record production and the stage barrier are paid
-// per stage); the warp reduces the 4 sums of each group of up to 4 pulses with
-// one transposed butterfly (each step halves the values a lane holds), the
-// CTA adds its 8 warps, and
-// adjoint_reduce_kernel sums the tiles per pulse in double, in a fixed order.
+// partial gradients of its own pulses, so no fix-up pass is needed.  As in
+// the forward kernel two warps produce the stages; they also add the 8 warps'
+// sums of each consumed stage and write them out.  A warp reduces the 4 sums
+// of a pulse with one transposed butterfly (each step halves the values a
+// lane holds), and adjoint_reduce_kernel sums the tiles per pulse in double,
+// in a fixed order.
+//
+// What bounds it: 21.4 warp instructions per warp-pixel-pulse at 62% of issue
+// slots (20.9 before, where the gathers of the 32 lanes of a row took 9.3
+// shared-memory wavefronts a pixel-pulse instead of 5.8 whenever the look
+// direction lay along the columns).  2048 pulses x 1024^2 pixels, look
+// direction 0 / 45 / 90 degrees from the rows: 2.00 / 2.41 / 2.26 ms before,
+// 2.05 / 2.07 / 2.11 ms now.  The 32 registers of the pixels' |G| and psi
+// leave the 96-register budget of 20 warps short: 3 of the 21.4 instructions
+// are moves that a 142-register build (10 warps, 2.39 ms) does not need.
 #include <algorithm>
 #include <cstdint>
 
@@ -51,54 +60,33 @@ namespace {
 
 using namespace tile;
 
-// Far field: T += |G| s~ per column (x: l = 0, y: l = 1; s~ = Re(Z exp(j
-// theta))) and, after each of the thread's rows k = 0..MX-2, V += T, so that
-// sum_k k |G| s~ = (MX - 1) T - V without per-row weights.
-// Near field: E += (s^, s^ r i, s^ r j, s^ Rc (r - 1)), s^ = |G| s~, r = Rc/R.
+// s^ = |G| s~, s~ = Re(Z exp(j theta)), of the thread's MX x 2 pixels for one
+// pulse.  Far field: S = sum s^ per column (x: l = 0, y: l = 1) and K = sum k
+// s^ over the row steps k - kMid.
+// Near field: E += (s^, s^ r i, s^ r j, s^ Rc (r - 1)), r = Rc/R.
 template <int MX, bool GATE, bool NEAR>
-__device__ __forceinline__ void adjoint_pulse(const PulseGeo &g, const float4 *base, uint32_t w_addr,
-                                              uint32_t zero_addr, int warp, int lane, float lam,
-                                              const float2 (&nd2)[MX], const float2 (&npsi)[MX],
-                                              const float2 (&gm)[MX], float i0f, float j0f, int W,
-                                              float2 &T, float2 &V, float4 &E) {
-    const float4 c0 = *reinterpret_cast<const float4 *>(&g.a8r);  // a8r, b32r, g8, e32
-    const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);   // tx, ty, h, hr
-    const float4 c2 = *reinterpret_cast<const float4 *>(&g.kr);   // kr, rc, lo, hi
-    const float4 rowv = base[warp];
-    const float P00 = rowv.x + reinterpret_cast<const float *>(base + kWarps)[lane];
-    const float B00 = fmaf(j0f, c0.w * (1.0f / 32.0f), rowv.y);
-    const float t00 = fmaf(j0f, c1.y, rowv.z);
-    float2 t2 = make_float2(t00, fmaf(32.0f, c1.y, t00));  // second pixel: 32 columns on
-    float2 Pb = make_float2(P00, P00 + c0.y);
-    float2 Bb = make_float2(B00, B00 + c0.w);
-    const float2 TX8 = splat(8.0f * c1.x), A8 = splat(c0.x), G8 = splat(c0.z);
-    const float2 HR = splat(c1.w), H = splat(c1.z), NKR = splat(-c2.x), NLAM = splat(-lam);
-    const float2 MAGIC = splat(kRoundMagic);
-    // B is the window-centred bin (entry floor(B) + W, intercept form)
-    const uint32_t w_adj = w_addr + (static_cast<uint32_t>(W) - kRoundMagicBits) * 16u;
-#pragma unroll
-    for (int k = 0; k < MX; ++k) {
-        if (k > 0) {
-            t2 = __fadd2_rn(t2, TX8);
-            Pb = __fadd2_rn(Pb, A8);
-            Bb = __fadd2_rn(Bb, G8);
-        }
-        float2 ng;
+__device__ __forceinline__ void adjoint_pulse(const PulseGeo &g, const float4 *tab, uint32_t w_addr,
+                                              uint32_t zero_addr, int entry, int col, const BpLaunch &L,
+                                              const float2 (&npsi)[MX], const float2 (&gm)[MX], float2 &S, float2 &K,
+                                              float4 &E) {
+    using M = PixelMap<MX>;
+    const PixelPoly poly(g, tab, entry, col);
+    // B is the window-centred bin (entry floor(B) + W, Z form)
+    const uint32_t w_adj = w_addr + (static_cast<uint32_t>(L.W) - kRoundMagicBits) * 16u;
+    S = K = make_float2(0.0f, 0.0f);
+    poly.rows<MX>([&](int k, float2 P, float2 B) {
         float2 rr = make_float2(1.0f, 1.0f);  // Rc / R_q (near field only)
+        const float fi = static_cast<float>(M::mid_row(entry) + M::kStep * (k - M::kMid));
         if (NEAR) {
-            const float e0 = -fmaf(t2.x, t2.x, nd2[k].x), e1 = -fmaf(t2.y, t2.y, nd2[k].y);
-            const float s0 = c2.y - t2.x, s1 = c2.y - t2.y;
-            const float g0 = e0 / (s0 + sqrtf(fmaf(s0, s0, e0))), g1 = e1 / (s1 + sqrtf(fmaf(s1, s1, e1)));
-            ng = make_float2(-g0, -g1);
-            rr = make_float2(c2.y / (s0 + g0), c2.y / (s1 + g1));
-        } else {
-            const float2 ne = __ffma2_rn(t2, t2, nd2[k]);
-            ng = __fmul2_rn(ne, __ffma2_rn(t2, HR, H));
+            float2 s;
+            const float2 r = near_remainder(g, L, fi, poly.J, s);
+            P = __ffma2_rn(splat(g.kr), r, P);
+            B = __ffma2_rn(splat(static_cast<float>(L.lambda)), r, B);
+            rr = make_float2(g.rc / (s.x + r.x), g.rc / (s.y + r.y));
         }
         // theta = phi - psi, bin B and its floor split as in the forward kernel
-        const float2 TH = __ffma2_rn(NKR, ng, __fadd2_rn(Pb, npsi[k]));
-        const float2 B = __ffma2_rn(NLAM, ng, Bb);
-        const float2 y = __fadd2_rd(B, MAGIC);
+        const float2 TH = __fadd2_rn(P, npsi[k]);
+        const float2 y = __fadd2_rd(B, splat(kRoundMagic));
         float2 ZR, NZI, CS, SN;  // the pair's Re Z, -Im Z and rotations
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
@@ -107,9 +95,10 @@ __device__ __forceinline__ void adjoint_pulse(const PulseGeo &g, const float4 *b
             const float Bl = l ? B.y : B.x;
             float sn, cs;
             __sincosf(Tl, &sn, &cs);
-            uint32_t addr = __float_as_uint(yl) * 16u + w_adj;
+            uint32_t addr;
+            asm("mad.lo.u32 %0, %1, 16, %2;" : "=r"(addr) : "r"(__float_as_uint(yl)), "r"(w_adj));
             if (GATE) {
-                const bool valid = (Bl > c2.z) && (Bl < c2.w);
+                const bool valid = (Bl > poly.lo) && (Bl < poly.hi);
                 addr = valid ? addr : zero_addr;
             }
             // Z-form entry {Zc, Zv}: Z(B) = v' + j nu v(B) = Zc + B Zv
@@ -132,22 +121,24 @@ __device__ __forceinline__ void adjoint_pulse(const PulseGeo &g, const float4 *b
         const float2 st = __ffma2_rn(ZR, CS, __fmul2_rn(NZI, SN));
         if (NEAR) {
             const float2 sh = __fmul2_rn(gm[k], st);
-            const float ik = i0f + static_cast<float>(8 * k);
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
                 const float s = l ? sh.y : sh.x;
                 const float r = l ? rr.y : rr.x;
                 const float sr = s * r;
                 E.x += s;
-                E.y = fmaf(sr, ik, E.y);
-                E.z = fmaf(sr, j0f + static_cast<float>((kTY / 2) * l), E.z);
-                E.w = fmaf(s, c2.y * (r - 1.0f), E.w);
+                E.y = fmaf(sr, fi, E.y);
+                E.z = fmaf(sr, l ? poly.J.y : poly.J.x, E.z);
+                E.w = fmaf(s, g.rc * (r - 1.0f), E.w);
             }
+        } else if (k != M::kMid) {
+            const float2 sh = __fmul2_rn(gm[k], st);
+            S = __fadd2_rn(S, sh);
+            K = __ffma2_rn(splat(static_cast<float>(k - M::kMid)), sh, K);
         } else {
-            T = __ffma2_rn(gm[k], st, T);
-            if (k < MX - 1) V = __fadd2_rn(V, T);
+            S = __ffma2_rn(gm[k], st, S);
         }
-    }
+    });
 }
 
 // The warp sums of N values (N = 4, 8, 16 or 32) at once: each step swaps
@@ -173,34 +164,29 @@ __device__ __forceinline__ float warp_reduce_scatter(float (&v)[N], int lane) {
     return r;
 }
 
-template <int N>
-struct Log2 {
-    static constexpr int value = N <= 1 ? 0 : 1 + Log2<N / 2>::value;
-};
-template <>
-struct Log2<1> {
-    static constexpr int value = 0;
-};
+// Threads of an adjoint CTA: kThreads accumulating and the producing warps.
+template <int PB>
+constexpr int kAdjThreads = kThreads + 32 * Producers<PB>::kWarps;
+// Shared-memory header: six mbarriers (full, ready, empty; two buffers each)
+// and the zero entry.
+constexpr int kAdjHdr = 64;
 
 template <int MX, int PB>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kAdjThreads<PB>, 2)
     bp_adjoint_kernel(const __grid_constant__ BpLaunch L, const float2 *__restrict__ grad,
                       float4 *__restrict__ partials) {
+    using M = PixelMap<MX>;
     constexpr int TX = 8 * MX;
-    constexpr int RG = PB < 4 ? PB : 4;  // pulses per warp reduction
-    constexpr int NV = 4 * RG;           // its sums: (E0, Ei, Ej, Et) per pulse
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-    float4 *zero = reinterpret_cast<float4 *>(smem + 16);
-    PulseGeo *geo = reinterpret_cast<PulseGeo *>(smem + 32);
-    float4 *bases = reinterpret_cast<float4 *>(smem + 32 + 2 * PB * sizeof(PulseGeo));
-    float *red = reinterpret_cast<float *>(smem + 32 + 2 * PB * (sizeof(PulseGeo) + kBaseEntries * sizeof(float4)));
-    unsigned char *win_ptr = smem + 32 + 2 * PB * (sizeof(PulseGeo) + kBaseEntries * sizeof(float4)) +
-                             2 * kWarps * 4 * PB * sizeof(float);
-    const uint32_t win_addr = smem_addr(win_ptr);
+    float4 *zero = reinterpret_cast<float4 *>(smem + kAdjHdr - 16);
+    PulseGeo *geo = reinterpret_cast<PulseGeo *>(smem + kAdjHdr);
+    float4 *tabs = reinterpret_cast<float4 *>(smem + kAdjHdr + 2 * PB * sizeof(PulseGeo));
+    // the warps' sums of each pulse, [buffer][pulse][sum][warp]
+    float *red = reinterpret_cast<float *>(tabs + 2 * PB * kPolyEntries);
+    const uint32_t win_addr = smem_addr(red + 2 * PB * 4 * kWarps);
     const uint32_t zero_addr = smem_addr(zero);
-    const int wsize = L.wsize;
-    const uint32_t pulse_bytes = static_cast<uint32_t>(wsize) * 16u;
+    const uint32_t pulse_bytes = static_cast<uint32_t>(L.wsize) * 16u;
     const uint32_t buf_bytes = static_cast<uint32_t>(PB) * pulse_bytes;
 
     const TileGrid tg = tile_grid(L, TX, PB);
@@ -210,37 +196,107 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (n <= 0) return;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = warp - TX / 2;
-    const int j0 = lane - kTY / 2;  // columns lane and lane + 32 of the tile
-    const float i0f = static_cast<float>(i0), j0f = static_cast<float>(j0);
-    const float lam = static_cast<float>(L.lambda), inv_lam = static_cast<float>(1.0 / L.lambda);
-    const float dxf = static_cast<float>(L.dx), dyf = static_cast<float>(L.dy);
+    UnitCursor cur;  // this warp's unit
+    cur.init(tg, L, lo);
+    auto tile_of = [&](const UnitCursor &u) {
+        return ((static_cast<long long>(u.hyp) * L.nz + u.iz) * tg.tiles_x + u.tx) * tg.tiles_y + u.ty;
+    };
 
-    float2 nd2[MX];  // -|d|^2 of the thread's pixel pairs
+    // full (windows landed) at bar_base + 8 s, ready (Z form) at + 16 + 8 s,
+    // empty (consumed, sums written) at + 32 + 8 s
+    const uint32_t bar_base = smem_addr(&bars[0]);
+    auto ready_bar = [&](int b) { return bar_base + 16u + 8u * b; };
+    auto empty_bar = [&](int b) { return bar_base + 32u + 8u * b; };
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_base + 8u * b, PB);
+            mbar_init(ready_bar(b), Producers<PB>::kWarps);
+            mbar_init(empty_bar(b), kWarps);
+        }
+        *zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        fence_mbar_init();
+    }
+    __syncthreads();
+
+    if (warp >= kWarps) {
+        // A producing warp (as in bp_mixed.cu) also finishes its pulses of
+        // each consumed stage: lane q adds the 8 warps' sums of pulse q in
+        // warp order and writes the tile's partial gradient, so the
+        // accumulating warps meet at no barrier.
+        constexpr int NQ = Producers<PB>::kPulses;
+        const int q0 = (warp - kWarps) * NQ;  // this warp's pulses of each stage
+        const float lam = static_cast<float>(L.lambda), inv_lam = static_cast<float>(1.0 / L.lambda);
+        const float dx = static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
+        auto finish = [&](int s, const UnitCursor &u) {
+            const int p = u.b * PB + q0 + lane;
+            if (lane < NQ && p < L.np) {
+                const PulseGeo &g = geo[s * PB + q0 + lane];
+                float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (g.flags & PG_ACTIVE) {
+                    const float4 *r = reinterpret_cast<const float4 *>(red + (s * PB + q0 + lane) * 4 * kWarps);
+                    float t[4];
 #pragma unroll
-    for (int k = 0; k < MX; ++k) {
-        const float di = static_cast<float>(i0 + 8 * k) * dxf;
-        const float dj0 = j0f * dyf, dj1 = static_cast<float>(j0 + kTY / 2) * dyf;
-        nd2[k] = make_float2(-fmaf(di, di, dj0 * dj0), -fmaf(di, di, dj1 * dj1));
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 a = r[2 * c], b = r[2 * c + 1];
+                        t[c] = ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+                    }
+                    // sum s u_q = u (E0 + Et/Rc) - (dx Ei, dy Ej, 0)/Rc, times
+                    // lambda; dL/dR0 = -lambda E0
+                    const float Et = (g.flags & PG_NEAR) ? t[3] : fmaf(g.tx, t[1], g.ty * t[2]);
+                    const float c = fmaf(Et, g.rinv, t[0]);
+                    out.x = lam * fmaf(g.ux, c, -dx * t[1] * g.rinv);
+                    out.y = lam * fmaf(g.uy, c, -dy * t[2] * g.rinv);
+                    out.z = lam * g.uz * c;
+                    out.w = -lam * t[0];
+                }
+                partials[tile_of(u) * L.np + p] = out;
+            }
+            __syncwarp();
+        };
+        const bool pregeo = L.geo_tab != nullptr;
+        StageRecords<NQ> pre;
+        if (pregeo) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
+        UnitCursor fin = cur;  // the next stage to finish
+        for (int i = 0; i < n; ++i) {
+            const int s = i & 1;
+            if (i >= 2) {
+                if (!mbar_wait_bounded(empty_bar(s), ((i - 2) >> 1) & 1, L.err)) return;
+                finish(s, fin);
+                fin.advance(tg, L);
+            }
+            PulseGeo *rec = geo + s * PB + q0;
+            const uint32_t win = win_addr + s * buf_bytes + static_cast<uint32_t>(q0) * pulse_bytes;
+            produce_pulses<MX, NQ>(L, cur.b * PB + q0, cur.tx, cur.ty, cur.iz, cur.hyp, pre, pregeo, rec,
+                                   tabs + (s * PB + q0) * kPolyEntries, win, bar_base + 8u * s, lane);
+            cur.advance(tg, L);
+            if (pregeo && i + 1 < n) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
+            if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
+            rewrite_pulses<NQ, true>(L, rec, win, lane, inv_lam);
+            if (lane == 0) mbar_arrive(ready_bar(s));
+        }
+        for (int i = n < 2 ? 0 : n - 2; i < n; ++i) {
+            if (!mbar_wait_bounded(empty_bar(i & 1), (i >> 1) & 1, L.err)) return;
+            finish(i & 1, fin);
+            fin.advance(tg, L);
+        }
+        return;
     }
 
-    UnitCursor cc, pc;  // consumer at unit i, producer at unit i + 1
-    cc.init(tg, L, lo);
-    pc = cc;
-
-    // the consumer tile's upstream gradient as -psi and |G| per pixel pair
+    const int entry = M::entry(warp, lane), col = M::col0(warp, lane);
+    const float i0f = static_cast<float>(M::mid_row(entry)), j0f = static_cast<float>(col - kTY / 2);
+    // the tile's upstream gradient as -psi and |G| per pixel pair
     float2 npsi[MX], gm[MX];
     auto load_tile = [&]() {
-        const int tx0 = cc.tx * TX, ty0 = cc.ty * kTY;
+        const int tx0 = cur.tx * TX + M::row0(warp, lane), ty0 = cur.ty * kTY + col;
 #pragma unroll
         for (int k = 0; k < MX; ++k) {
-            const int row = tx0 + warp + 8 * k;
+            const int row = tx0 + M::kStep * k;
             float ps[2], mg[2];
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
-                const int col = ty0 + lane + (kTY / 2) * l;
-                const float2 q = (row < L.nx && col < L.ny)
-                                     ? grad[(static_cast<long long>(cc.iz) * L.nx + row) * L.ny + col]
+                const int c = ty0 + (kTY / 2) * l;
+                const float2 q = (row < L.nx && c < L.ny)
+                                     ? grad[(static_cast<long long>(cur.iz) * L.nx + row) * L.ny + c]
                                      : make_float2(0.0f, 0.0f);
                 ps[l] = -atan2f(q.y, q.x);
                 mg[l] = sqrtf(fmaf(q.x, q.x, q.y * q.y));
@@ -251,184 +307,50 @@ __global__ void __launch_bounds__(kThreads, 2)
     };
     load_tile();
 
-    const uint32_t bar_base = smem_addr(&bars[0]);  // buffer s barrier at bar_base + 8*s
-    if (threadIdx.x == 0) {
-        mbar_init(bar_base, PB);
-        mbar_init(bar_base + 8, PB);
-        *zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        fence_mbar_init();
-    }
-    __syncthreads();
-
-    // Pre-pass records (BpLaunch::geo_tab, [tile][pulse]): the producing
-    // warps copy them from a staging ring filled a stage ahead, after the
-    // two stage buffers' windows.
-    const bool pregeo = L.geo_tab != nullptr;
-    PulseGeo *stg = reinterpret_cast<PulseGeo *>(win_ptr + 2 * buf_bytes);
-    auto prefetch = [&](const UnitCursor &u, int slot) {
-        const long long t = ((static_cast<long long>(u.hyp) * L.nz + u.iz) * tg.tiles_x + u.tx) * tg.tiles_y + u.ty;
-        prefetch_records<PB>(L, static_cast<const PulseGeo *>(L.geo_tab) + t * L.np, u.b, stg + slot * PB, warp,
-                             lane);
-    };
-    // records, base tables and windows of the producer cursor's unit into
-    // buffer s (every lane of the warp enters produce_slots)
-    auto produce = [&](int s) {
-        const double cx = L.left + static_cast<double>(pc.tx * TX + TX / 2) * L.dx;
-        const double cy = L.bottom + static_cast<double>(pc.ty * kTY + kTY / 2) * L.dy;
-        const double cz = L.zlow + static_cast<double>(pc.iz) * L.dz;
-        produce_slots<PB>(L, pc.b, geo + s * PB, bases + s * PB * kBaseEntries, win_addr + s * buf_bytes,
-                          bar_base + 8 * s, warp, lane, TX / 2, cx, cy, cz, 0, pregeo ? stg + s * PB : nullptr);
-    };
-    if (pregeo) {
-        prefetch(pc, 0);
-        if (n > 1) {
-            UnitCursor nx = pc;
-            nx.advance(tg, L);
-            prefetch(nx, 1);
-        }
-    }
-    produce(0);
-    intercept_slots<PB, true>(geo, win_addr, bar_base, 0, L.wsize, L.W, warp, lane, L.err, inv_lam);
-    __syncthreads();
-
-    int last_issued = 0;
     for (int i = 0; i < n; ++i) {
         const int s = i & 1;
-        if (i + 1 < n) {
-            pc.advance(tg, L);
-            produce(s ^ 1);
-            last_issued = i + 1;
-            // stage i + 2's records into the staging slot stage i's producer
-            // read before the last barrier
-            if (pregeo && i + 2 < n) {
-                UnitCursor nx = pc;
-                nx.advance(tg, L);
-                prefetch(nx, s);
-            }
-        }
-        const int b = cc.b;
-        const bool ok = mbar_wait_bounded(bar_base + 8 * s, (i >> 1) & 1, L.err);
-        const int nq = min(PB, L.np - b * PB);
-        // the record fields the final sum of pulse q = threadIdx.x needs
-        int rflags = 0;
-        float rtx = 0.0f, rty = 0.0f, rux = 0.0f, ruy = 0.0f, ruz = 0.0f, rinv = 0.0f;
-        bool fast = false;
-        if (ok) {
-            const int my_flags = lane < nq ? geo[s * PB + lane].flags : 0;
-            const int any_f = __reduce_or_sync(0xffffffffu, my_flags);
-            const int all_f = __reduce_and_sync(0xffffffffu, lane < nq ? my_flags : PG_ACTIVE);
-            fast = nq == PB && (all_f & PG_ACTIVE) && !(any_f & (PG_GATE | PG_NEAR));
-            if (threadIdx.x < nq) {
-                const PulseGeo &g = geo[s * PB + threadIdx.x];
-                rflags = g.flags;
-                rtx = g.tx;
-                rty = g.ty;
-                rux = g.ux;
-                ruy = g.uy;
-                ruz = g.uz;
-                rinv = g.rinv;
-            }
-        }
-        // pulses in groups of RG: the group's 4 RG sums, then their warp sums
-        // (lane L holds value L >> shift) into this stage's half of red; after
-        // the stage barrier thread q adds the 8 warps for pulse q (the next
-        // stage writes the other half, so one barrier per stage)
-        constexpr int shift = 5 - Log2<NV>::value;
-        float *red_s = red + s * (kWarps * 4 * PB);
+        // a wait that runs out (error bit set) ends this warp; the others end at theirs
+        if (!mbar_wait_bounded(ready_bar(s), (i >> 1) & 1, L.err)) return;
+        const int nq = min(PB, L.np - cur.b * PB);
         const uint32_t w0 = win_addr + s * buf_bytes;
-#pragma unroll
-        for (int gi = 0; gi < PB / RG; ++gi) {
-            float v[NV];
-#pragma unroll
-            for (int c = 0; c < NV; ++c) v[c] = 0.0f;
-            // far field: E0, Ei = i0 E0 + 8 sum k s^, Ej = j0 E0 + 32 sum_(l=1) s^, Et later
-            auto far_sums = [&](int r, float2 T, float2 V) {
-                const float S = T.x + T.y;
-                const float Sk = fmaf(static_cast<float>(MX - 1), S, -(V.x + V.y));
-                v[4 * r + 0] = S;
-                v[4 * r + 1] = fmaf(i0f, S, 8.0f * Sk);
-                v[4 * r + 2] = fmaf(j0f, S, static_cast<float>(kTY / 2) * T.y);
-            };
-            if (fast) {
-#pragma unroll
-                for (int r = 0; r < RG; ++r) {
-                    const int q = gi * RG + r;
-                    float2 T = make_float2(0.0f, 0.0f), V = make_float2(0.0f, 0.0f);
-                    float4 E;
-                    adjoint_pulse<MX, false, false>(geo[s * PB + q], bases + (s * PB + q) * kBaseEntries,
-                                                    w0 + q * pulse_bytes, zero_addr, warp, lane, lam, nd2, npsi, gm,
-                                                    i0f, j0f, L.W, T, V, E);
-                    far_sums(r, T, V);
-                }
-            } else if (ok) {
-#pragma unroll
-                for (int r = 0; r < RG; ++r) {
-                    const int q = gi * RG + r;
-                    const PulseGeo &g = geo[s * PB + q];
-                    if (q >= nq || !(g.flags & PG_ACTIVE)) continue;
-                    const float4 *bq = bases + (s * PB + q) * kBaseEntries;
-                    const uint32_t w = w0 + q * pulse_bytes;
-                    float2 T = make_float2(0.0f, 0.0f), V = make_float2(0.0f, 0.0f);
-                    float4 E = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (g.flags & PG_NEAR) {
-                        adjoint_pulse<MX, true, true>(g, bq, w, zero_addr, warp, lane, lam, nd2, npsi, gm, i0f, j0f,
-                                                      L.W, T, V, E);
-                        v[4 * r + 0] = E.x;
-                        v[4 * r + 1] = E.y;
-                        v[4 * r + 2] = E.z;
-                        v[4 * r + 3] = E.w;
-                    } else {
-                        adjoint_pulse<MX, true, false>(g, bq, w, zero_addr, warp, lane, lam, nd2, npsi, gm, i0f,
-                                                       j0f, L.W, T, V, E);
-                        far_sums(r, T, V);
-                    }
-                }
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q) {
+            const PulseGeo &g = geo[s * PB + q];
+            const float4 *tq = tabs + (s * PB + q) * kPolyEntries;
+            const uint32_t w = w0 + q * pulse_bytes;
+            const int flags = g.flags;
+            if (!(flags & PG_ACTIVE)) continue;
+            float v[4];
+            if (!(flags & PG_NEAR)) {
+                float2 S, K;
+                float4 E;
+                if (flags & PG_GATE)
+                    adjoint_pulse<MX, true, false>(g, tq, w, zero_addr, entry, col, L, npsi, gm, S, K, E);
+                else
+                    adjoint_pulse<MX, false, false>(g, tq, w, zero_addr, entry, col, L, npsi, gm, S, K, E);
+                // E0, Ei = i0 E0 + 2 sum k s^, Ej = j0 E0 + 32 sum_(l=1) s^; Et follows from them
+                v[0] = S.x + S.y;
+                v[1] = fmaf(i0f, v[0], static_cast<float>(M::kStep) * (K.x + K.y));
+                v[2] = fmaf(j0f, v[0], static_cast<float>(kTY / 2) * S.y);
+                v[3] = 0.0f;
+            } else {
+                float2 S, K;
+                float4 E = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                adjoint_pulse<MX, true, true>(g, tq, w, zero_addr, entry, col, L, npsi, gm, S, K, E);
+                v[0] = E.x;
+                v[1] = E.y;
+                v[2] = E.z;
+                v[3] = E.w;
             }
-            const float rs = warp_reduce_scatter<NV>(v, lane);
-            if ((lane & ((1 << shift) - 1)) == 0) red_s[warp * 4 * PB + gi * NV + (lane >> shift)] = rs;
+            // lane 8 c holds the warp's sum c
+            const float rs = warp_reduce_scatter<4>(v, lane);
+            if ((lane & 7) == 0) red[((s * PB + q) * 4 + (lane >> 3)) * kWarps + warp] = rs;
         }
-        // the next stage's windows into intercept form, published by the barrier
-        if (i + 1 < n)
-            intercept_slots<PB, true>(geo + (s ^ 1) * PB, win_addr + (s ^ 1) * buf_bytes, bar_base + 8 * (s ^ 1),
-                                      ((i + 1) >> 1) & 1, wsize, L.W, warp, lane, L.err, inv_lam);
-        if (__syncthreads_or(!ok)) {
-            // let the copies already issued for the other buffer (and the
-            // record prefetches) land before the CTA's shared memory goes
-            // away (again bounded)
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            if (threadIdx.x == 0 && last_issued > i)
-                mbar_wait_bounded(bar_base + 8 * (last_issued & 1), (last_issued >> 1) & 1, L.err);
-            return;
-        }
-        if (threadIdx.x < nq) {
-            const int q = threadIdx.x;
-            float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const float4 x = *reinterpret_cast<const float4 *>(red_s + w * 4 * PB + 4 * q);
-                t.x += x.x;
-                t.y += x.y;
-                t.z += x.z;
-                t.w += x.w;
-            }
-            float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (rflags & PG_ACTIVE) {
-                // sum s u_q = u (E0 + Et/Rc) - (dx Ei, dy Ej, 0)/Rc, times lambda;
-                // dL/dR0 = -lambda E0
-                const float Et = (rflags & PG_NEAR) ? t.w : fmaf(rtx, t.y, rty * t.z);
-                const float c = fmaf(Et, rinv, t.x);
-                out.x = lam * fmaf(rux, c, -dxf * t.y * rinv);
-                out.y = lam * fmaf(ruy, c, -dyf * t.z * rinv);
-                out.z = lam * ruz * c;
-                out.w = -lam * t.x;
-            }
-            const long long tile =
-                ((static_cast<long long>(cc.hyp) * L.nz + cc.iz) * tg.tiles_x + cc.tx) * tg.tiles_y + cc.ty;
-            partials[tile * L.np + b * PB + q] = out;
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty_bar(s));
         if (i + 1 < n) {
-            cc.advance(tg, L);
-            if (cc.b == 0) load_tile();
+            cur.advance(tg, L);
+            if (cur.b == 0) load_tile();
         }
     }
 }
@@ -491,7 +413,7 @@ cudaError_t launch_adj(const BpLaunch &L, const void *grad, void *partials, size
     int dev = 0, sms = 0, occ = 0;
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kAdjThreads<PB>, smem);
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
     const long long units = tile_grid(L, TX, PB).units;
@@ -504,7 +426,7 @@ cudaError_t launch_adj(const BpLaunch &L, const void *grad, void *partials, size
     e = launch_geo_records(La, MX, &pregeo, s);
     if (e != cudaSuccess) return e;
     if (!pregeo) La.geo_tab = nullptr;
-    kern<<<static_cast<unsigned>(ctas), kThreads, smem, s>>>(La, static_cast<const float2 *>(grad),
+    kern<<<static_cast<unsigned>(ctas), kAdjThreads<PB>, smem, s>>>(La, static_cast<const float2 *>(grad),
                                                               static_cast<float4 *>(partials));
     return cudaGetLastError();
 }
@@ -518,8 +440,8 @@ long long bp_tile_count(const BpLaunch &L, const TileConfig &tc) {
 
 size_t bp_adjoint_smem_bytes(const TileConfig &tc, int wsize) {
     const size_t pb = static_cast<size_t>(tc.pb);
-    return 32 + 2 * pb * (sizeof(PulseGeo) + kBaseEntries * sizeof(float4)) + 2 * kWarps * 4 * pb * sizeof(float) +
-           2 * pb * static_cast<size_t>(wsize) * 16 + 2 * pb * sizeof(PulseGeo);
+    return kAdjHdr + 2 * pb * (sizeof(PulseGeo) + kPolyEntries * sizeof(float4)) + 2 * kWarps * 4 * pb * sizeof(float) +
+           2 * pb * static_cast<size_t>(wsize) * 16;
 }
 
 cudaError_t launch_bp_adjoint(const BpLaunch &L, const void *grad, void *partials, const TileConfig &tc, size_t smem,

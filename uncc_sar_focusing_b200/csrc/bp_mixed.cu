@@ -10,13 +10,13 @@
 //     GPU kernel's roundf bracket, cuda_BackProjectionKernels.cuh:68-74).
 //
 // Design (one CTA = one pixel tile of (8*MX) x 64 pixels of one z-slice at a
-// time, 8 accumulating warps of MX x 2 pixels a thread and one producing warp):
+// time, 8 accumulating warps of MX x 2 pixels a thread and two producing warps):
 //  * pulses go through shared memory in stages of PB pulses, two stage
-//    buffers.  For each stage the producing warp writes the FP64 geometry
+//    buffers.  For each stage the producing warps write the FP64 geometry
 //    records (tile-centre range, unit vector, phase and bin steps reduced mod
 //    1), the polynomial tables and one cp.async.bulk copy per pulse of the
-//    window of range bins any pixel of the tile can touch, rewrites the landed
-//    windows to intercept form and marks the buffer ready; the accumulating
+//    window of range bins any pixel of the tile can touch, rewrite the landed
+//    windows to intercept form and mark the buffer ready; the accumulating
 //    warps hand it back through the "empty" mbarrier, so they drift up to a
 //    stage apart and meet nowhere;
 //  * range profiles live in HBM as pair entries {rc[b], rc[b+1]-rc[b]}
@@ -39,7 +39,7 @@
 // 4 of them the 16-byte gather's floor), MUFU 62-65%, 18 warps per SM.  Rows
 // interleaved over the warps, a row of 32 lanes and one evaluation of the
 // range remainder per pixel took 18.0 instructions and 1.70-2.13 ms over the
-// same look directions, this 1.51-1.65 ms.
+// same look directions, this 1.50-1.62 ms.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -64,8 +64,9 @@ constexpr int kTabEntries = kPolyEntries;
 // buffers each) and the zero entry.
 constexpr int kHdr = 64;
 
-// Threads of a forward CTA: kThreads consumers and one producing warp.
-constexpr int kFwdThreads = kThreads + 32;
+// Threads of a forward CTA: kThreads accumulating and the producing warps.
+template <int PB>
+constexpr int kFwdThreads = kThreads + 32 * Producers<PB>::kWarps;
 
 // Dynamic shared memory of the forward kernel: the header and two stage
 // buffers of PB records, tables and windows.
@@ -85,47 +86,23 @@ constexpr bool kRotate = SARBP_STAGE_ROTATION != 0;
 // (32 apart) of a row form a pair whose phase, bin and complex
 // multiply-accumulate run as paired FP32 instructions (__ffma2_rn and
 // friends); the sine/cosine, the shared-memory gather and the interpolation
-// are per pixel.  Phase and bin of row k - kMid are P0 + k a + k^2 b
-// (write_poly_table); rows +-k share P0 + k^2 b.
+// are per pixel.
 template <int MX, bool GATE, bool NEAR, bool CHECKED>
 __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4 *tab, uint32_t w_addr,
                                                  uint32_t zero_addr, int entry, int col, const BpLaunch &L,
                                                  float (&acc_re)[MX][2], float (&acc_im)[MX][2]) {
     using M = PixelMap<MX>;
-    const float4 r0 = tab[2 * entry], r1 = tab[2 * entry + 1];
-    const float4 u0 = reinterpret_cast<const float4 *>(&g)[0], u1 = reinterpret_cast<const float4 *>(&g)[1];
-    const float j0 = static_cast<float>(col - kTY / 2);
-    const float2 J = make_float2(j0, j0 + static_cast<float>(kTY / 2));
-    const float s0 = r0.x + reinterpret_cast<const float *>(tab + kPolyCols)[col];
-    const float2 w = __ffma2_rn(J, __ffma2_rn(J, splat(u0.w), splat(r0.w)), splat(r0.z));
-    const float2 sJ = __fmul2_rn(J, splat(u0.z));
-    const float2 P0 = __ffma2_rn(J, w, make_float2(s0, s0 + u0.x));
-    const float2 B0 = __ffma2_rn(sJ, w, __ffma2_rn(J, splat(u0.y), splat(r0.y)));
-    const float2 v = __ffma2_rn(J, splat(u1.x), splat(r1.z));
-    const float2 Pa = __ffma2_rn(J, v, splat(r1.x)), Ba = __ffma2_rn(sJ, v, splat(r1.y));
-    const float2 Pb = __ffma2_rn(J, splat(u1.y), splat(r1.w)), Bb = __fmul2_rn(Pb, splat(u0.z));
+    const PixelPoly poly(g, tab, entry, col);
     // B is the window-centred bin; shared address of pair entry floor(B) + W:
     // bits(B + 1.5*2^23, rounded down) * 16 + w_adj (mod 2^32)
     const uint32_t w_adj = w_addr + (static_cast<uint32_t>(L.W) - kRoundMagicBits) * 16u;
-    auto pixels = [&](int k, float2 P, float2 B) {
+    poly.rows<MX>([&](int k, float2 P, float2 B) {
         if (NEAR) {
-            // exact remainder of the range, e = |d|^2 - t^2 >= 0
-            const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);  // tx, ty, h, hr
-            const float4 c2 = *reinterpret_cast<const float4 *>(&g.kr);  // kr, rc, lo, hi
-            const float fi = static_cast<float>(M::mid_row(entry) + M::kStep * (k - M::kMid));
-            const float di = fi * static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
-            const float lam = static_cast<float>(L.lambda);
-            float gl[2];
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                const float fj = l ? J.y : J.x, dj = fj * dy;
-                const float t = fmaf(fi, c1.x, fj * c1.y);
-                const float e = -fmaf(t, t, -fmaf(di, di, dj * dj));
-                const float s = c2.y - t;
-                gl[l] = e / (s + sqrtf(fmaf(s, s, e)));
-            }
-            P = make_float2(fmaf(c2.x, gl[0], P.x), fmaf(c2.x, gl[1], P.y));
-            B = make_float2(fmaf(lam, gl[0], B.x), fmaf(lam, gl[1], B.y));
+            float2 s;
+            const float2 r = near_remainder(g, L, static_cast<float>(M::mid_row(entry) + M::kStep * (k - M::kMid)),
+                                            poly.J, s);
+            P = __ffma2_rn(splat(g.kr), r, P);
+            B = __ffma2_rn(splat(static_cast<float>(L.lambda)), r, B);
         }
         const float2 y = __fadd2_rd(B, splat(kRoundMagic));
         float2 RE, IM, CS, SN;  // the pair's interpolated samples and rotations
@@ -140,7 +117,7 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
             uint32_t addr;
             asm("mad.lo.u32 %0, %1, 16, %2;" : "=r"(addr) : "r"(__float_as_uint(yl)), "r"(w_adj));
             if (GATE) {
-                const bool valid = (Bl > u1.z) && (Bl < u1.w);
+                const bool valid = (Bl > poly.lo) && (Bl < poly.hi);
                 addr = valid ? addr : zero_addr;
             }
             if (CHECKED) {
@@ -177,15 +154,7 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
         acc_re[k][1] = ar.y;
         acc_im[k][0] = ai.x;
         acc_im[k][1] = ai.y;
-    };
-    pixels(M::kMid, P0, B0);
-#pragma unroll
-    for (int k = 1; k <= M::kMid; ++k) {
-        const float f = static_cast<float>(k);
-        const float2 Ps = __ffma2_rn(splat(f * f), Pb, P0), Bs = __ffma2_rn(splat(f * f), Bb, B0);
-        pixels(M::kMid - k, __ffma2_rn(splat(-f), Pa, Ps), __ffma2_rn(splat(-f), Ba, Bs));
-        if (M::kMid + k < MX) pixels(M::kMid + k, __ffma2_rn(splat(f), Pa, Ps), __ffma2_rn(splat(f), Ba, Bs));
-    }
+    });
 }
 
 // Store (or add, L.accumulate) a thread's pixel pair k of the tile at (tx0,
@@ -292,16 +261,15 @@ struct SceneCursor {
 // stage buffers' stride) and sk_partial; each scene's image completion time
 // goes to done[scene].
 //
-// Warps 0..7 accumulate; warp 8 produces: per stage it waits until the
-// buffer is empty, puts the stage's records, tables and window copies into
-// it, rewrites the landed windows to intercept form and marks the buffer
-// ready.  As one warp's work the 8 PB row entries of a stage fill the lanes
-// and the PB records, coefficients and copies take one pass (each accumulating
-// warp producing its own pulse slot ran them with 8 of 32 lanes or one), and
-// the accumulating warps carry neither the production's instructions nor its
-// latency.
+// Warps 0..7 accumulate; warps 8 and 9 produce, half of each stage's pulses
+// each (Producers): per stage they wait until the buffer is empty, put its
+// records, tables and window copies into it, rewrite the landed windows to
+// intercept form and mark the buffer ready.  The 32 row entries of 4 pulses
+// fill a warp's lanes (each accumulating warp producing its own pulse slot ran
+// them with 8 of 32 lanes, the records with one), and the accumulating warps
+// carry neither the production's instructions nor its latency.
 template <int MX, int PB, bool CHECKED, int MINB, bool BATCH>
-__global__ void __launch_bounds__(kFwdThreads, MINB)
+__global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
     bp_mixed_kernel(const __grid_constant__ BpLaunch L0, const BatchScene *__restrict__ scenes, int nscenes,
                     long long batch_units, unsigned long long *__restrict__ done, int tile_mode) {
     constexpr int TX = 8 * MX;
@@ -340,7 +308,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
         (!BATCH && kRotate) ? static_cast<int>((cur.g.stages - lo % cur.g.stages) % cur.g.stages) : 0;
 
     // buffer s: full (windows landed: PB arrivals and their bytes) at
-    // bar_base + 8 s, ready (intercept form, one arrival) at bar_base + 16 +
+    // bar_base + 8 s, ready (intercept form, one arrival per producing warp) at bar_base + 16 +
     // 8 s, empty (consumed, one arrival per accumulating warp) at bar_base +
     // 32 + 8 s
     const uint32_t bar_base = smem_addr(&bars[0]);
@@ -349,7 +317,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_base + 8u * b, PB);
-            mbar_init(ready_bar(b), 1);
+            mbar_init(ready_bar(b), Producers<PB>::kWarps);
             mbar_init(empty_bar(b), kWarps);
         }
         *zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -357,66 +325,33 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
     }
     __syncthreads();
 
-    if (warp == kWarps) {
+    if (warp >= kWarps) {
         // Pre-pass records (single-scene launches: L0.geo_tab; batches: each
-        // scene's L.geo_tab, L0.geo_tab non-null when every scene has them):
-        // a stage's records, 8 PB words of 16 bytes, are loaded into the
-        // lanes' registers one stage ahead.
+        // scene's L.geo_tab, L0.geo_tab non-null when every scene has them)
+        // are loaded into the lanes' registers one stage ahead.
+        constexpr int NQ = Producers<PB>::kPulses;
+        const int q0 = (warp - kWarps) * NQ;  // this warp's pulses of each stage
         const bool pregeo = L0.geo_tab != nullptr;
-        constexpr int kPre = (kRecWords * PB + 31) / 32;
-        float4 pre[kPre];
-        auto load_records = [&](const SceneCursor<TX, PB, BATCH> &c) {
-            const BpLaunch &L = *c.L;
-            const long long t =
-                ((static_cast<long long>(c.u.hyp) * L.nz + c.u.iz) * c.g.tiles_x + c.u.tx) * c.g.tiles_y + c.u.ty;
-            const int p0 = c.stage() * PB;
-            const float4 *src = reinterpret_cast<const float4 *>(static_cast<const PulseGeo *>(L.geo_tab) + t * L.np + p0);
-            const int words = min(PB, L.np - p0) * kRecWords;
-#pragma unroll
-            for (int r = 0; r < kPre; ++r) {
-                const int k = lane + 32 * r;
-                pre[r] = k < words ? src[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+        StageRecords<NQ> pre;
+        auto load_records = [&]() {
+            const BpLaunch &L = *cur.L;
+            pre.load(L, ((static_cast<long long>(cur.u.hyp) * L.nz + cur.u.iz) * cur.g.tiles_x + cur.u.tx) * cur.g.tiles_y + cur.u.ty,
+                     cur.stage() * PB + q0, lane);
         };
-        if (pregeo) load_records(cur);
+        if (pregeo) load_records();
         for (int i = 0; i < n; ++i) {
             const int s = i & 1;
             const BpLaunch &L = *cur.L;
             // buffer s last held stage i - 2: every accumulating warp has consumed it
             if (i >= 2 && !mbar_wait_bounded(empty_bar(s), ((i - 2) >> 1) & 1, L.err)) return;
-            PulseGeo *rec = geo + s * PB;
-            const int p = cur.stage() * PB + lane;  // lane < PB: this lane's pulse
-            if (pregeo) {
-#pragma unroll
-                for (int r = 0; r < kPre; ++r) {
-                    const int k = lane + 32 * r;
-                    if (k < kRecWords * PB) reinterpret_cast<float4 *>(rec)[k] = pre[r];
-                }
-            } else if (lane < PB) {
-                const double cx = L.left + static_cast<double>(cur.u.tx * TX + TX / 2) * L.dx;
-                const double cy = L.bottom + static_cast<double>(cur.u.ty * kTY + kTY / 2) * L.dy;
-                const double cz = L.zlow + static_cast<double>(cur.u.iz) * L.dz;
-                PulseGeo g = {};
-                if (p < L.np) g = make_geo(L, p, static_cast<long long>(cur.u.hyp) * L.np, cx, cy, cz, TX / 2);
-                rec[lane] = g;
-            }
-            __syncwarp();
-            if (lane < PB)
-                issue_window(L, p, lane, rec[lane].flags, rec[lane].wp, rec[lane].ws, win_addr + s * buf_bytes,
-                             bar_base + 8u * s);
-            write_poly_tables<MX, PB>(tabs + s * PB * kTabEntries, rec, lane, L);
+            PulseGeo *rec = geo + s * PB + q0;
+            const uint32_t win = win_addr + s * buf_bytes + static_cast<uint32_t>(q0) * static_cast<uint32_t>(L.wsize) * 16u;
+            produce_pulses<MX, NQ>(L, cur.stage() * PB + q0, cur.u.tx, cur.u.ty, cur.u.iz, cur.u.hyp, pre, pregeo, rec,
+                                   tabs + (s * PB + q0) * kTabEntries, win, bar_base + 8u * s, lane);
             cur.advance(scenes, nscenes, rot_later);
-            if (pregeo && i + 1 < n) load_records(cur);
+            if (pregeo && i + 1 < n) load_records();
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            for (int q = 0; q < PB; ++q) {
-                if (!(rec[q].flags & PG_ACTIVE)) continue;
-                rewrite_window<false>(win_addr + s * buf_bytes + static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) * 16u,
-                                      L.W, rec[q].wp, lane, 0.0f);
-            }
-            // the rewrite's generic-proxy stores precede the next bulk copies
-            // (async proxy) into this buffer, which this warp issues
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
+            rewrite_pulses<NQ, false>(L, rec, win, lane);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         return;
@@ -670,7 +605,7 @@ cudaError_t launch_kernels(const BpLaunch &L0, size_t smem, cudaStream_t s) {
         if (2 * g * TX * kTY * static_cast<long long>(sizeof(float2)) <= L.sk_slot_bytes) G = g;
     }
     if (G > 0x7fffffffLL) return cudaErrorInvalidValue;
-    kern<<<static_cast<unsigned>(G), kFwdThreads, smem, s>>>(L, nullptr, 0, 0, nullptr, 0);
+    kern<<<static_cast<unsigned>(G), kFwdThreads<PB>, smem, s>>>(L, nullptr, 0, 0, nullptr, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess || G == tg.tiles) return e;
     bp_sk_fixup_kernel<MX, PB, false>
@@ -688,14 +623,14 @@ cudaError_t launch_mx_pb(const BpLaunch &L, bool checked, size_t smem, cudaStrea
     return one_cta ? launch_kernels<MX, PB, false, 1>(L, smem, s) : launch_kernels<MX, PB, false, kCtasPerSm>(L, smem, s);
 }
 
-template <typename K>
+template <int PB, typename K>
 int resident_of(K kern, size_t smem) {
     int dev = 0, sms = 0, occ = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFwdThreads, smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFwdThreads<PB>, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -705,8 +640,8 @@ int resident_of(K kern, size_t smem) {
 template <int MX, int PB>
 int resident_mx_pb(size_t smem) {
     const bool one_cta = smem > 113u * 1024u;
-    return one_cta ? resident_of(bp_mixed_kernel<MX, PB, false, 1, false>, smem)
-                   : resident_of(bp_mixed_kernel<MX, PB, false, kCtasPerSm, false>, smem);
+    return one_cta ? resident_of<PB>(bp_mixed_kernel<MX, PB, false, 1, false>, smem)
+                   : resident_of<PB>(bp_mixed_kernel<MX, PB, false, kCtasPerSm, false>, smem);
 }
 
 template <int MX, int PB, int MINB>
@@ -719,12 +654,12 @@ cudaError_t launch_batch_kernels(const BatchScene *scenes, int nscenes, long lon
     if (tiles < 1 || tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
     if (per_tile) {
         // one CTA per tile: no partial sums, scenes finish in order
-        kern<<<static_cast<unsigned>(tiles), kFwdThreads, smem, s>>>(L0, scenes, nscenes, units, done, 1);
+        kern<<<static_cast<unsigned>(tiles), kFwdThreads<PB>, smem, s>>>(L0, scenes, nscenes, units, done, 1);
         return cudaGetLastError();
     }
     const long long G = resident < units ? resident : units;
     if (G < 1 || G > 0x7fffffffLL) return cudaErrorInvalidValue;
-    kern<<<static_cast<unsigned>(G), kFwdThreads, smem, s>>>(L0, scenes, nscenes, units, done, 0);
+    kern<<<static_cast<unsigned>(G), kFwdThreads<PB>, smem, s>>>(L0, scenes, nscenes, units, done, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     bp_sk_fixup_kernel<MX, PB, true>
@@ -744,8 +679,8 @@ cudaError_t launch_batch_mx_pb(const BatchScene *scenes, int nscenes, long long 
 
 template <int MX, int PB>
 int batch_resident_mx_pb(size_t smem) {
-    return smem > 113u * 1024u ? resident_of(bp_mixed_kernel<MX, PB, false, 1, true>, smem)
-                               : resident_of(bp_mixed_kernel<MX, PB, false, 2, true>, smem);
+    return smem > 113u * 1024u ? resident_of<PB>(bp_mixed_kernel<MX, PB, false, 1, true>, smem)
+                               : resident_of<PB>(bp_mixed_kernel<MX, PB, false, 2, true>, smem);
 }
 
 }  // namespace

@@ -220,63 +220,7 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     return g;
 }
 
-// Pulse slots of block b handled by this warp (slot q = warp, warp + 8, ...):
-// lane 0 writes the geometry record and either arrives with the window's byte
-// count and issues its bulk copy, or just arrives (inactive / past the end).
-// Per-(tile, pulse) base tables of the mixed kernels (forward and adjoint),
-// kBaseEntries float4 words: row entries 0..7, one per warp, for
-// i0 = warp - TX/2: (2 pi frac(A + i0 alpha), B0 + i0 gam, i0 tx, -kr), then
-// 32 floats, one per lane, for j0 = lane - 32 (a lane's pixels are columns
-// lane and lane + 32 of the tile): the column phase 2 pi frac(j0 beta).  The
-// phase parts are reduced modulo one revolution in FP64; a thread's phase
-// base is row + column, its bin and projection bases row + j0 eta and
-// row + j0 ty, formed in FP32 from the record (eta = e32 / 32 exactly).
-constexpr int kBaseEntries = kWarps + 32 / 4;
-
-// Records (and base tables when base_s != nullptr) and window copies of
-// stage b into one buffer.  Warp w produces slots w, w + 8, ...: lane 0
-// computes the FP64 record (or lanes 0..7 move the prefetched pre-pass
-// record into place), the warp's lanes fill the base tables from it, then
-// lane 0 issues the window's bulk copy (or a plain arrival), whose release
-// on the stage's mbarrier also publishes the record and the tables
-// (__syncwarp orders the other lanes' stores before it).
-// Pre-pass records (BpLaunch::geo_tab) of pulse stage b of the tile whose
-// record row is `rec` into a staging slot of shared memory, asynchronously
-// (cp.async, 16 bytes by each of lanes 0..7 of warp q for slot q): issued a
-// stage ahead of produce_slots, which waits for them.
-template <int PB>
-__device__ __forceinline__ void prefetch_records(const BpLaunch &L, const PulseGeo *rec, int b, PulseGeo *stg,
-                                                 int warp, int lane) {
-    for (int q = warp; q < PB; q += kWarps) {
-        const int p = b * PB + q;
-        if (p < L.np && lane < 8) {
-            const uint32_t dst = smem_addr(reinterpret_cast<const float4 *>(stg + q) + lane);
-            const float4 *src = reinterpret_cast<const float4 *>(rec + p) + lane;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// Base tables of one (tile, pulse) from its record's FP64 steps (every lane
-// of the warp writes its column entry, lanes 0..7 the row entries; the row
-// entries carry -kr in their fourth word, so the forward kernel's
-// consumers read it with the row part).
-__device__ __forceinline__ void write_base_table(float4 *tab, int lane, int tx_half, int W, double A, double alpha,
-                                                 double beta, double B0, double gam, float tx, float kr) {
-    const int j0 = lane - kTY / 2;
-    const double pc = static_cast<double>(j0) * beta;
-    reinterpret_cast<float *>(tab + kWarps)[lane] = static_cast<float>(kTwoPi * (pc - rint(pc)));
-    if (lane < kWarps) {
-        const int i0 = lane - tx_half;
-        const double pr = fma(static_cast<double>(i0), alpha, A);
-        tab[lane] = make_float4(static_cast<float>(kTwoPi * (pr - rint(pr))),
-                                static_cast<float>(fma(static_cast<double>(i0), gam, B0 - W)),
-                                static_cast<float>(i0) * tx, -kr);
-    }
-}
-
-// ---- forward kernel: pixel map and polynomial table -----------------------
+// ---- pixel map and polynomial tables of the mixed kernels ------------------
 //
 // A thread's pixels: warp w covers rows [2 MX (w >> 1), + 2 MX) and columns
 // 16 (w & 1) + [0, 16) and the same 32 columns on; its lanes are 2 rows x 16
@@ -331,15 +275,15 @@ struct PixelMap {
 constexpr int kPolyCols = 16, kPolyEntries = kPolyCols + 8;
 constexpr int kRecWords = sizeof(PulseGeo) / sizeof(float4);
 
-// The tables of a stage of PB pulses by one warp, records in rec[0, PB).
-// Lanes q < PB first put the cubic's coefficients of their pulse into words 3
-// and 7 of its record (the forward kernel reads neither), then the 8 PB row
-// entries and the 32 PB column phases are spread over the 32 lanes.
-template <int MX, int PB>
+// The tables of NQ pulses by one warp, records in rec[0, NQ).  Lanes q < NQ
+// first leave the cubic's coefficients of their pulse where its column phases
+// will be, then the 8 NQ row entries and after them the 32 NQ column phases
+// are spread over the 32 lanes.
+template <int MX, int NQ>
 __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, int lane, const BpLaunch &L) {
     using M = PixelMap<MX>;
     float4 un0 = make_float4(0.f, 0.f, 0.f, 0.f), un1 = un0;
-    if (lane < PB) {
+    if (lane < NQ) {
         float4 *w = reinterpret_cast<float4 *>(rec + lane);
         const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // a8r, b32r, g8, e32; tx, ty, h, hr; kr, rc, lo, hi
         const float dx = static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
@@ -348,26 +292,28 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         const float mh = m * c1.z, mr = m * c1.w;
         const float q21 = mr * fmaf(c1.x, n11, c1.y * n20), q12 = mr * fmaf(c1.x, n02, c1.y * n11);
         const float q03 = mr * c1.y * n02, sigma = static_cast<float>(L.lambda) / c2.x;
-        w[7] = make_float4(mh * n20, mh * n11, mh * n02, mr * c1.x * n20);
-        w[3] = make_float4(q21, q12, sigma, 0.0f);
+        float4 *coef = tabs + lane * kPolyEntries + kPolyCols;
+        coef[0] = make_float4(mh * n20, mh * n11, mh * n02, mr * c1.x * n20);
+        coef[1] = make_float4(q21, q12, sigma, 0.0f);
         un0 = make_float4(c0.y, c0.w * (1.0f / 32.0f), sigma, q03);
         un1 = make_float4(2.0f * q12, 4.0f * q21, c2.z, c2.w);
     }
     __syncwarp();
     // k^3 ~ kFit k over the thread's rows k = -kMid .. MX - kMid - 1
     constexpr float kFit = MX == 8 ? 452.0f / 44.0f : (MX == 4 ? 3.0f : (MX == 2 ? 1.0f : 0.0f));
-    for (int t = lane; t < 8 * PB; t += 32) {
+    for (int t = lane; t < 8 * NQ; t += 32) {
         const int q = t >> 3, e = t & 7;
         const float4 *w = reinterpret_cast<const float4 *>(rec + q);
         const double2 d0 = *reinterpret_cast<const double2 *>(w);  // A, alpha
         const double B0 = rec[q].B0, gam = rec[q].gam;
-        const float4 qa = w[7], qb = w[3];  // q20, q11, q02, q30; q21, q12, sigma
+        float4 *row = tabs + q * kPolyEntries + 2 * e;
+        // q20, q11, q02, q30; q21, q12, sigma
+        const float4 qa = tabs[q * kPolyEntries + kPolyCols], qb = tabs[q * kPolyEntries + kPolyCols + 1];
         const float i = static_cast<float>(M::mid_row(e));
         const double id = static_cast<double>(i);
         const double pr = fma(id, d0.y, d0.x), ps = 2.0 * d0.y;
         const float nl = i * i * fmaf(i, qa.w, qa.x);
         const float an = fmaf(8.0f * kFit, qa.w, 2.0f * i * fmaf(3.0f * i, qa.w, 2.0f * qa.x));
-        float4 *row = tabs + q * kPolyEntries + 2 * e;
         row[0] = make_float4(static_cast<float>(kTwoPi * (pr - rint(pr))) + nl,
                              fmaf(qb.z, nl, static_cast<float>(fma(id, gam, B0 - L.W))), i * fmaf(i, qb.x, qa.y),
                              fmaf(i, qb.y, qa.z));
@@ -375,15 +321,16 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
                              fmaf(qb.z, an, static_cast<float>(2.0 * gam)), 2.0f * fmaf(2.0f * i, qb.x, qa.y),
                              4.0f * fmaf(3.0f * i, qa.w, qa.x));
     }
+    __syncwarp();
     const double jd = static_cast<double>(lane - kTY / 2);
 #pragma unroll
-    for (int q = 0; q < PB; ++q) {
+    for (int q = 0; q < NQ; ++q) {
         const double pc = jd * rec[q].beta;
         reinterpret_cast<float *>(tabs + q * kPolyEntries + kPolyCols)[lane] =
             static_cast<float>(kTwoPi * (pc - rint(pc)));
     }
     __syncwarp();
-    if (lane < PB) {
+    if (lane < NQ) {
         float4 *w = reinterpret_cast<float4 *>(rec + lane);
         w[0] = un0;
         w[1] = un1;
@@ -414,67 +361,64 @@ __device__ __forceinline__ void issue_window(const BpLaunch &L, int p, int q, in
     }
 }
 
-// Records, base tables and window copies of stage b (see below).  stg: the
-// stage's prefetched records (prefetch_records), or nullptr: lane 0 computes
-// them (make_geo).
+// Producing warps of a stage of PB pulses: two, each with half the pulses (one
+// warp alone, 1000 and more instructions a stage, held the accumulating ones
+// up: forward 1583 against 1495 us, adjoint 2175 against 2050 us on 1024^2
+// pixels x 2048 pulses).  With the 8 accumulating warps on two CTAs that is 5
+// warps a scheduler, the most its registers hold at 96 a thread.
 template <int PB>
-__device__ __forceinline__ void produce_slots(const BpLaunch &L, int b, PulseGeo *geo_s, float4 *base_s,
-                                              uint32_t win_s, uint32_t bar, int warp, int lane, int tx_half,
-                                              double cx, double cy, double cz, long long goff = 0,
-                                              const PulseGeo *stg = nullptr) {
-    if (stg) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-        for (int q = warp; q < PB; q += kWarps) {
-            const int p = b * PB + q;
-            const bool valid = p < L.np;
-            // lanes 0..7 move the record's 16-byte words into the stage's
-            // record slot (zeros past the last pulse: flags 0); every lane
-            // reads the steps of the tables itself (broadcast loads)
-            const float4 *rec = reinterpret_cast<const float4 *>(stg + q);
-            if (lane < 8)
-                reinterpret_cast<float4 *>(geo_s + q)[lane] = valid ? rec[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (base_s) {
-                double2 d0 = make_double2(0.0, 0.0), d1 = d0;
-                double gam = 0.0;
-                float tx = 0.0f, kr = 0.0f;
-                if (valid) {
-                    const double2 *rd = reinterpret_cast<const double2 *>(stg + q);
-                    d0 = rd[0];  // A, alpha
-                    d1 = rd[1];  // beta, B0
-                    gam = stg[q].gam;
-                    tx = stg[q].tx;
-                    kr = stg[q].kr;
-                }
-                write_base_table(base_s + q * kBaseEntries, lane, tx_half, L.W, d0.x, d0.y, d1.x, d1.y, gam, tx, kr);
-            }
-            __syncwarp();
-            if (lane == 0 && valid) {
-                const int4 f = *reinterpret_cast<const int4 *>(&stg[q].ws);  // ws, flags, wp, pad
-                issue_window(L, p, q, f.y, f.z, f.x, win_s, bar);
-            } else if (lane == 0) {
-                mbar_arrive(bar);
-            }
+struct Producers {
+    static constexpr int kWarps = PB >= 2 ? 2 : 1;
+    static constexpr int kPulses = PB / kWarps;  // pulses of each
+};
+
+// Pre-pass records (BpLaunch::geo_tab, [tile][pulse]) of pulses p0 .. p0 + NQ - 1
+// of tile t in a producing warp's registers, 8 NQ words of 16 bytes over the
+// lanes; loaded a stage before they are stored.
+template <int NQ>
+struct StageRecords {
+    static constexpr int kPre = (kRecWords * NQ + 31) / 32;
+    float4 w[kPre];
+
+    __device__ __forceinline__ void load(const BpLaunch &L, long long t, int p0, int lane) {
+        const float4 *src = reinterpret_cast<const float4 *>(static_cast<const PulseGeo *>(L.geo_tab) + t * L.np + p0);
+        const int words = min(NQ, L.np - p0) * kRecWords;
+#pragma unroll
+        for (int r = 0; r < kPre; ++r) {
+            const int k = lane + 32 * r;
+            w[r] = k < words ? src[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        return;
     }
-    for (int q = warp; q < PB; q += kWarps) {
-        const int p = b * PB + q;
+    __device__ __forceinline__ void store(PulseGeo *rec, int lane) const {
+#pragma unroll
+        for (int r = 0; r < kPre; ++r) {
+            const int k = lane + 32 * r;
+            if (k < kRecWords * NQ) reinterpret_cast<float4 *>(rec)[k] = w[r];
+        }
+    }
+};
+
+// A producing warp's part of one stage, NQ pulses from p0 of the tile at row
+// tx, column ty (in tiles), slice iz: records (from the pre-pass, or computed
+// by lanes q < NQ), window copies (lane q the one of pulse q) and tables.
+template <int MX, int NQ>
+__device__ __forceinline__ void produce_pulses(const BpLaunch &L, int p0, int tx, int ty, int iz, int hyp,
+                                               const StageRecords<NQ> &pre, bool pregeo, PulseGeo *rec, float4 *tabs,
+                                               uint32_t win, uint32_t bar, int lane) {
+    const int p = p0 + lane;  // lane < NQ: this lane's pulse
+    if (pregeo) {
+        pre.store(rec, lane);
+    } else if (lane < NQ) {
+        const double cx = L.left + static_cast<double>(tx * 8 * MX + 4 * MX) * L.dx;
+        const double cy = L.bottom + static_cast<double>(ty * kTY + kTY / 2) * L.dy;
+        const double cz = L.zlow + static_cast<double>(iz) * L.dz;
         PulseGeo g = {};
-        if (lane == 0 && p < L.np) g = make_geo(L, p, goff, cx, cy, cz, tx_half);
-        if (base_s) {
-            const unsigned full = 0xffffffffu;
-            const double A = __shfl_sync(full, g.A, 0), alpha = __shfl_sync(full, g.alpha, 0);
-            const double beta = __shfl_sync(full, g.beta, 0), B0 = __shfl_sync(full, g.B0, 0);
-            const double gam = __shfl_sync(full, g.gam, 0);
-            const float tx = __shfl_sync(full, g.tx, 0), kr = __shfl_sync(full, g.kr, 0);
-            write_base_table(base_s + q * kBaseEntries, lane, tx_half, L.W, A, alpha, beta, B0, gam, tx, kr);
-            __syncwarp();
-        }
-        if (lane != 0) continue;
-        geo_s[q] = g;
-        issue_window(L, p, q, g.flags, g.wp, g.ws, win_s, bar);
+        if (p < L.np) g = make_geo(L, p, static_cast<long long>(hyp) * L.np, cx, cy, cz, 4 * MX);
+        rec[lane] = g;
     }
+    __syncwarp();
+    if (lane < NQ) issue_window(L, p, lane, rec[lane].flags, rec[lane].wp, rec[lane].ws, win, bar);
+    write_poly_tables<MX, NQ>(tabs, rec, lane, L);
 }
 
 __device__ __forceinline__ float4 lds128(uint32_t addr) {
@@ -495,16 +439,74 @@ __device__ __forceinline__ void sts128(uint32_t addr, float x, float y, float z,
 
 __device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
 
+// Phase and bin polynomials of a thread's pixel pairs for one pulse (columns
+// col and col + 32 of the tile): row step k - kMid takes P0 + k Pa + k^2 Pb
+// and B0 + k Ba + k^2 Bb.
+struct PixelPoly {
+    float2 J, P0, Pa, Pb, B0, Ba, Bb;
+    float lo, hi;  // valid bins
+
+    __device__ __forceinline__ PixelPoly(const PulseGeo &g, const float4 *tab, int entry, int col) {
+        const float4 r0 = tab[2 * entry], r1 = tab[2 * entry + 1];
+        const float4 u0 = reinterpret_cast<const float4 *>(&g)[0], u1 = reinterpret_cast<const float4 *>(&g)[1];
+        const float j0 = static_cast<float>(col - kTY / 2);
+        J = make_float2(j0, j0 + static_cast<float>(kTY / 2));
+        const float s0 = r0.x + reinterpret_cast<const float *>(tab + kPolyCols)[col];
+        const float2 w = __ffma2_rn(J, __ffma2_rn(J, splat(u0.w), splat(r0.w)), splat(r0.z));
+        const float2 sJ = __fmul2_rn(J, splat(u0.z));
+        P0 = __ffma2_rn(J, w, make_float2(s0, s0 + u0.x));
+        B0 = __ffma2_rn(sJ, w, __ffma2_rn(J, splat(u0.y), splat(r0.y)));
+        const float2 v = __ffma2_rn(J, splat(u1.x), splat(r1.z));
+        Pa = __ffma2_rn(J, v, splat(r1.x));
+        Ba = __ffma2_rn(sJ, v, splat(r1.y));
+        Pb = __ffma2_rn(J, splat(u1.y), splat(r1.w));
+        Bb = __fmul2_rn(Pb, splat(u0.z));
+        lo = u1.z;
+        hi = u1.w;
+    }
+
+    // f(k, phase, bin) for the thread's MX pixel pairs, outermost row steps
+    // first, the middle one last; rows +-k share P0 + k^2 Pb.
+    template <int MX, typename F>
+    __device__ __forceinline__ void rows(F f) const {
+        using M = PixelMap<MX>;
+#pragma unroll
+        for (int k = M::kMid; k >= 1; --k) {
+            const float x = static_cast<float>(k);
+            const float2 Ps = __ffma2_rn(splat(x * x), Pb, P0), Bs = __ffma2_rn(splat(x * x), Bb, B0);
+            f(M::kMid - k, __ffma2_rn(splat(-x), Pa, Ps), __ffma2_rn(splat(-x), Ba, Bs));
+            if (M::kMid + k < MX) f(M::kMid + k, __ffma2_rn(splat(x), Pa, Ps), __ffma2_rn(splat(x), Ba, Bs));
+        }
+        f(M::kMid, P0, B0);
+    }
+};
+
+// Near-field pulses: the exact remainder g = e / (s + sqrt(s^2 + e)), s = Rc - t,
+// e = |d|^2 - t^2, of the pixel pair in row offset fi, columns J (and s, for
+// R_q = s + g).
+__device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaunch &L, float fi, float2 J,
+                                                 float2 &s) {
+    const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);  // tx, ty, h, hr
+    const float rc = g.rc, dy = static_cast<float>(L.dy), di = fi * static_cast<float>(L.dx);
+    float gl[2], sl[2];
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const float fj = l ? J.y : J.x, dj = fj * dy;
+        const float t = fmaf(fi, c1.x, fj * c1.y);
+        const float e = -fmaf(t, t, -fmaf(di, di, dj * dj));
+        sl[l] = rc - t;
+        gl[l] = e / (sl[l] + sqrtf(fmaf(sl[l], sl[l], e)));
+    }
+    s = make_float2(sl[0], sl[1]);
+    return make_float2(gl[0], gl[1]);
+}
+
 // Intercept form of the windows: entry n of a pulse's window holds
 // {v_n, v'_n} (v'_n = v_(n+1) - v_n); rewritten in place to
 // {v_n - (n - W) v'_n, v'_n}, a pixel whose window-centred bin is
 // B = bin - ws - W (floor(B) + W = n) interpolates
 //     v(B) = v_n + (B + W - n) v'_n = c_n + B v'_n
-// with one fused multiply-add and no fraction.  Warp `warp` rewrites the
-// slots it produced (q = warp, warp + 8, ...) of one stage buffer once their
-// copies have landed (bounded wait on the buffer's mbarrier; a timeout sets
-// the error bit and leaves the windows as they are).  The barrier that
-// follows publishes them.
+// with one fused multiply-add and no fraction.
 // ZFORM (the adjoint, which needs only Z(B) = v'(B) + j nu v(B), nu = kr /
 // lambda radians per bin): the entry becomes {Zc, Zv} with Zc = v'_n + j nu
 // c_n and Zv = j nu v'_n, so that Z(B) = Zc + B Zv is again one fused
@@ -532,21 +534,19 @@ __device__ __forceinline__ void rewrite_window(uint32_t w, int W, int wp, int la
     for (; left > 0; left -= 32, a += 512u, m += 32.0f) one(a, m);
 }
 
-template <int PB, bool ZFORM = false>
-__device__ __forceinline__ bool intercept_slots(const PulseGeo *geo_s, uint32_t win_s, uint32_t bar, uint32_t parity,
-                                                int wsize, int W, int warp, int lane, unsigned *err,
-                                                float inv_lam = 0.0f) {
-    if (warp >= PB) return true;
-    if (!mbar_wait_bounded(bar, parity, err)) return false;
-    for (int q = warp; q < PB; q += kWarps) {
-        if (!(geo_s[q].flags & PG_ACTIVE)) continue;
-        rewrite_window<ZFORM>(win_s + static_cast<uint32_t>(q) * static_cast<uint32_t>(wsize) * 16u, W, geo_s[q].wp,
-                              lane, ZFORM ? geo_s[q].kr * inv_lam : 0.0f);
+// The windows of NQ pulses, by their producing warp once the copies have landed;
+// the fence orders these generic-proxy stores before the next bulk copies
+// (async proxy) into the buffer, which the same warp issues.
+template <int NQ, bool ZFORM>
+__device__ __forceinline__ void rewrite_pulses(const BpLaunch &L, const PulseGeo *rec, uint32_t win_s, int lane,
+                                              float inv_lam = 0.0f) {
+    for (int q = 0; q < NQ; ++q) {
+        if (!(rec[q].flags & PG_ACTIVE)) continue;
+        rewrite_window<ZFORM>(win_s + static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) * 16u, L.W, rec[q].wp,
+                              lane, ZFORM ? rec[q].kr * inv_lam : 0.0f);
     }
-    // these generic-proxy stores precede the next bulk copy (async proxy) into
-    // the same buffer, issued after the CTA barrier
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    return true;
+    __syncwarp();
 }
 
 }  // namespace tile
