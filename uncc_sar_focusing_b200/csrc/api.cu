@@ -121,7 +121,7 @@ void release(sarbp_plan *p) {
     cudaFree(p->d_ph);
     cudaFree(p->d_geo);
     cudaFree(p->d_fft_base);
-    cudaFree(p->d_pairs);
+    cudaFree(p->d_fft_work);
     cudaFree(p->d_fac);
     cudaFree(p->d_img);
     cudaFree(p->d_err);
@@ -188,8 +188,7 @@ int range_compress_impl(sarbp_plan *p, const void *ph, int np, int memory, cudaS
         src = p->d_ph;
     }
     if (p->d_rctab) {
-        SARBP_TRY_CUDA(launch_rc_fused(src, p->d_fac, p->d_rctab, p->d_pairs, p->K, p->rc_R, np, p->row_stride,
-                                       p->guard, p->rc_grid, s));
+        SARBP_TRY_CUDA(launch_rc_fused(src, p->d_fac, p->d_rctab, p->d_fft, p->K, p->rc_R, np, p->rc_grid, s));
         p->np_ready = np;
         if (memory == SARBP_MEMORY_HOST) SARBP_TRY_CUDA(cudaStreamSynchronize(s));
         return SARBP_OK;
@@ -204,9 +203,6 @@ int range_compress_impl(sarbp_plan *p, const void *ph, int np, int memory, cudaS
             : cufftExecC2C(p->fft, static_cast<cufftComplex *>(p->d_fft), static_cast<cufftComplex *>(p->d_fft),
                            CUFFT_INVERSE);
     if (r1 != CUFFT_SUCCESS) return from_cufft(r1);
-    // the FP64 backprojection stages the FFT output itself
-    if (p->precision == SARBP_PRECISION_MIXED)
-        SARBP_TRY_CUDA(launch_rc_pairs(p->d_fft, p->d_pairs, p->nfft, np, p->row_stride, p->guard, s));
     p->np_ready = np;
     if (memory == SARBP_MEMORY_HOST) SARBP_TRY_CUDA(cudaStreamSynchronize(s));
     return SARBP_OK;
@@ -216,10 +212,7 @@ BpLaunch launch_params(const sarbp_plan *p, const double *ax, const double *ay, 
                        const double *f0, int np, void *img, int flags) {
     const sarbp_grid &g = p->desc.grid;
     BpLaunch L{};
-    const bool fp64 = p->precision == SARBP_PRECISION_FP64;
-    L.pairs = fp64 ? p->d_fft : p->d_pairs;
-    L.row_stride = fp64 ? p->nfft : p->row_stride;
-    L.guard = fp64 ? 0 : p->guard;
+    L.rc = p->d_fft;
     L.ax = ax;
     L.ay = ay;
     L.az = az;
@@ -705,52 +698,21 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
         tile_window(p->lambda, p->dx, p->dy, p->tile.mx, &W, &wsize, &hd);
         near_field_consts(hd, &p->near_hd16, &p->near_coef);
     }
-    p->guard = p->wsize + 2;
-    p->row_stride = static_cast<long long>(p->nfft) + 2LL * p->guard;
     const size_t cb = cplx_bytes(p);
-    // mixed: pair rows with guards.  FP64: windows come from the FFT buffer,
-    // rows back to back, where a window past a row's end reads samples of the
-    // neighbouring row that the gate discards; guards at the buffer's ends
-    const bool fp64 = p->precision == SARBP_PRECISION_FP64;
-    const size_t fft_guard = fp64 ? static_cast<size_t>(p->guard) : 0;
+    const size_t margin = margin_samples(p->wsize);
     const size_t npix = static_cast<size_t>(g.nx) * g.ny * g.nz;
     const size_t np = static_cast<size_t>(p->np_cap);
-    const size_t pair_bytes = np * static_cast<size_t>(p->row_stride) * 16;
+    const size_t rc_bytes = (np * p->nfft + 2 * margin) * cb;
     if ((st = alloc(p, &p->d_ph, np * p->K * 8)) ||
         (st = alloc(p, reinterpret_cast<void **>(&p->d_geo), 5 * np * sizeof(double))) ||
-        (st = alloc(p, &p->d_fft_base, (np * p->nfft + 2 * fft_guard) * cb)) ||
-        (!fp64 && (st = alloc(p, &p->d_pairs, pair_bytes))) ||
+        (st = alloc(p, &p->d_fft_base, rc_bytes)) ||
         (st = alloc(p, &p->d_fac, static_cast<size_t>(p->K) * cb)) || (st = alloc(p, &p->d_img, npix * cb)) ||
         (st = alloc(p, reinterpret_cast<void **>(&p->d_err), sizeof(unsigned)))) {
         release(p);
         return st;
     }
-    // partial-sum slots for launches split over the resident CTAs (two tiles
-    // per CTA); without them every launch runs one CTA per tile
-    p->sk_resident = p->precision == SARBP_PRECISION_FP64 ? bp_fp64_resident(p->tile, p->smem)
-                                                          : bp_mixed_resident(p->tile, p->smem);
-    if (p->sk_resident > 0) {
-        const size_t sk = 2 * static_cast<size_t>(p->sk_resident) * (8 * p->tile.mx) * 64 * cb;
-        if (alloc(p, &p->d_sk, sk) == SARBP_OK) {
-            p->sk_bytes = sk;
-        } else {
-            p->sk_resident = 0;
-        }
-    }
-    // geometry records of a single-image launch from a pre-pass kernel
-    // (environment SARBP_PREGEO=0: computed by the producing lanes instead)
-    if (p->precision == SARBP_PRECISION_MIXED) {
-        const char *env = std::getenv("SARBP_PREGEO");
-        if (!(env && std::strcmp(env, "0") == 0)) {
-            const long long recs = static_cast<long long>((g.ny + 63) / 64) *
-                                   ((g.nx + 8 * p->tile.mx - 1) / (8 * p->tile.mx)) * g.nz * p->np_cap;
-            if (alloc(p, &p->d_geotab, static_cast<size_t>(recs) * sizeof(PulseGeo)) == SARBP_OK)
-                p->geotab_records = recs;
-        }
-    }
-    p->d_fft = static_cast<unsigned char *>(p->d_fft_base) + fft_guard * cb;
-    if ((!fp64 && cudaMemset(p->d_pairs, 0, pair_bytes) != cudaSuccess) ||
-        cudaMemset(p->d_fft_base, 0, (np * p->nfft + 2 * fft_guard) * cb) != cudaSuccess ||
+    p->d_fft = static_cast<unsigned char *>(p->d_fft_base) + margin * cb;
+    if (cudaMemset(p->d_fft_base, 0, rc_bytes) != cudaSuccess ||
         cudaMemset(p->d_err, 0, sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         release(p);
@@ -777,28 +739,66 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
         cudaGetLastError();
         if (want && p->precision == SARBP_PRECISION_MIXED && R >= 1 && rc_fused_shape(K, R, &rc_smem, &tab) &&
             rc_smem <= static_cast<size_t>(dev_smem)) {
-            if (alloc(p, &p->d_rctab, tab.size() * sizeof(float)) == SARBP_OK &&
-                cudaMemcpy(p->d_rctab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess) {
-                p->rc_R = R;
-                // CTAs resident at once: the kernel loops over pulses
-                const int per_sm = rc_smem > 0 ? static_cast<int>((228u * 1024u) / (rc_smem + 1024u)) : 1;
-                p->rc_grid = (sms > 0 ? sms : 148) * (per_sm > 0 ? (per_sm < 4 ? per_sm : 4) : 1);
-            } else {
-                cudaGetLastError();
-                cudaFree(p->d_rctab);
-                p->d_rctab = nullptr;
+            if ((st = alloc(p, &p->d_rctab, tab.size() * sizeof(float))) != SARBP_OK) {
+                release(p);
+                return st;
             }
+            if (cudaMemcpy(p->d_rctab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
+                cudaGetLastError();
+                release(p);
+                return SARBP_ERR_CUDA;
+            }
+            p->rc_R = R;
+            // CTAs resident at once: the kernel loops over pulses
+            const int per_sm = rc_smem > 0 ? static_cast<int>((228u * 1024u) / (rc_smem + 1024u)) : 1;
+            p->rc_grid = (sms > 0 ? sms : 148) * (per_sm > 0 ? (per_sm < 4 ? per_sm : 4) : 1);
         }
     }
-    const cufftResult r = cufftPlan1d(&p->fft, p->nfft, p->precision == SARBP_PRECISION_FP64 ? CUFFT_Z2Z : CUFFT_C2C,
-                                      p->np_cap);
-    if (r != CUFFT_SUCCESS) {
-        release(p);
-        return from_cufft(r);
+    // the other shapes: cuFFT on a work area of the plan's own
+    if (!p->d_rctab) {
+        size_t ws = 0;
+        cufftResult r = cufftCreate(&p->fft);
+        p->fft_ok = r == CUFFT_SUCCESS;
+        if (r == CUFFT_SUCCESS) r = cufftSetAutoAllocation(p->fft, 0);
+        if (r == CUFFT_SUCCESS)
+            r = cufftMakePlan1d(p->fft, p->nfft, p->precision == SARBP_PRECISION_FP64 ? CUFFT_Z2Z : CUFFT_C2C, p->np_cap,
+                                &ws);
+        if (r != CUFFT_SUCCESS) {
+            release(p);
+            return from_cufft(r);
+        }
+        if ((st = alloc(p, &p->d_fft_work, ws > 256 ? ws : 256)) != SARBP_OK) {
+            release(p);
+            return st;
+        }
+        if (cufftSetWorkArea(p->fft, p->d_fft_work) != CUFFT_SUCCESS) {
+            release(p);
+            return SARBP_ERR_CUFFT;
+        }
     }
-    p->fft_ok = true;
-    size_t ws = 0;
-    if (cufftGetSize(p->fft, &ws) == CUFFT_SUCCESS) p->bytes += ws;
+    // partial-sum slots for launches split over the resident CTAs (two tiles
+    // per CTA); without them every launch runs one CTA per tile
+    p->sk_resident = p->precision == SARBP_PRECISION_FP64 ? bp_fp64_resident(p->tile, p->smem)
+                                                          : bp_mixed_resident(p->tile, p->smem);
+    if (p->sk_resident > 0) {
+        const size_t sk = 2 * static_cast<size_t>(p->sk_resident) * (8 * p->tile.mx) * 64 * cb;
+        if (alloc(p, &p->d_sk, sk) == SARBP_OK) {
+            p->sk_bytes = sk;
+        } else {
+            p->sk_resident = 0;
+        }
+    }
+    // geometry records of a single-image launch from a pre-pass kernel
+    // (environment SARBP_PREGEO=0: computed by the producing lanes instead)
+    if (p->precision == SARBP_PRECISION_MIXED) {
+        const char *env = std::getenv("SARBP_PREGEO");
+        if (!(env && std::strcmp(env, "0") == 0)) {
+            const long long recs = static_cast<long long>((g.ny + 63) / 64) *
+                                   ((g.nx + 8 * p->tile.mx - 1) / (8 * p->tile.mx)) * g.nz * p->np_cap;
+            if (alloc(p, &p->d_geotab, static_cast<size_t>(recs) * sizeof(PulseGeo)) == SARBP_OK)
+                p->geotab_records = recs;
+        }
+    }
     *out = p;
     return SARBP_OK;
 }
@@ -883,9 +883,6 @@ int sarbp_get_range_profiles(sarbp_plan *plan, void *out, int memory, void *stre
     SARBP_TRY(drain_pipe(plan));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t bytes = static_cast<size_t>(plan->np_ready) * plan->nfft * cplx_bytes(plan);
-    if (plan->d_rctab)  // fused range compression keeps the profiles only in the pair rows
-        SARBP_TRY_CUDA(launch_pairs_to_rc(plan->d_pairs, plan->d_fft, plan->nfft, plan->np_ready, plan->row_stride,
-                                          plan->guard, s));
     SARBP_TRY_CUDA(cudaMemcpyAsync(out, plan->d_fft, bytes,
                                    memory == SARBP_MEMORY_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
                                    s));

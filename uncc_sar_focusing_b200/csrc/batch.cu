@@ -3,7 +3,7 @@
 // Each scene keeps its own range-compression buffers and cuFFT plan; a
 // device-resident scene table (BatchScene) holds every per-call pointer, so
 // the work of one call -- table upload, batched taper/twiddle/zero-pad, one
-// FFT per scene, batched pair rows, ONE backprojection launch over the
+// FFT per scene, ONE backprojection launch over the
 // (tile, pulse-stage) units of all scenes split evenly over the resident
 // CTAs, the fix-up of split tiles, and the read-back of per-image completion
 // times -- is captured once as a CUDA graph and replayed on later calls with
@@ -29,11 +29,10 @@ struct sarbp_batch {
     int device = 0;
     int n = 0;
     std::vector<sarbp_plan_desc> desc;
-    std::vector<void *> d_pairs, d_fft, d_fac;
+    std::vector<void *> d_rc, d_fac;  // range profiles [np][nfft] with margins at both ends; factor tables
     std::vector<cufftHandle> fft;
     std::vector<char> fft_ok;
-    std::vector<int> guard;
-    std::vector<long long> row_stride;
+    std::vector<size_t> margin;  // readable samples before and after each scene's rows
     std::vector<double> lambda, dx, dy, dz, left, bottom, zlow;
     void *fft_work = nullptr;
     std::vector<void *> rctab;     // per scene: fused range-compression table (null: cuFFT path)
@@ -101,8 +100,7 @@ void release(sarbp_batch *b) {
     drop_graph(b);
     for (int i = 0; i < b->n; ++i) {
         if (i < static_cast<int>(b->fft_ok.size()) && b->fft_ok[i]) cufftDestroy(b->fft[i]);
-        if (i < static_cast<int>(b->d_pairs.size())) cudaFree(b->d_pairs[i]);
-        if (i < static_cast<int>(b->d_fft.size())) cudaFree(b->d_fft[i]);
+        if (i < static_cast<int>(b->d_rc.size())) cudaFree(b->d_rc[i]);
         if (i < static_cast<int>(b->d_fac.size())) cudaFree(b->d_fac[i]);
     }
     cudaFree(b->fft_work);
@@ -131,7 +129,7 @@ bool configure(sarbp_batch *b, const TileConfig &tc) {
         double hd;
         tile_window(b->lambda[i], b->dx[i], b->dy[i], tc.mx, &W[i], &ws[i], &hd);
         near_field_consts(hd, &h16[i], &hc[i]);
-        if (ws[i] + 2 > b->guard[i] || ws[i] > (1 << 16)) return false;
+        if (margin_samples(ws[i]) > b->margin[i] || ws[i] > (1 << 16)) return false;
         wmax = ws[i] > wmax ? ws[i] : wmax;
     }
     const size_t smem = bp_mixed_smem_bytes(tc, wmax);
@@ -221,9 +219,7 @@ int fill_table(sarbp_batch *b, const sarbp_aperture *aps, void *const *images) {
         std::memset(&T, 0, sizeof(T));
         BpLaunch &L = T.L;
         L.drop_pulse = -1;
-        L.pairs = b->d_pairs[i];
-        L.row_stride = b->row_stride[i];
-        L.guard = b->guard[i];
+        L.rc = static_cast<float2 *>(b->d_rc[i]) + b->margin[i];
         L.ax = g.ant_x;
         L.ay = g.ant_y;
         L.az = g.ant_z;
@@ -253,9 +249,7 @@ int fill_table(sarbp_batch *b, const sarbp_aperture *aps, void *const *images) {
         T.fused = b->rctab[i] ? 1 : 0;
         T.ph = a.phase_history;
         T.fac = b->d_fac[i];
-        T.fft = b->d_fft[i];
         T.K = d.num_range_samples;
-        T.row_stride = b->row_stride[i];
         const tile::TileGrid tg = tile::tile_grid(L, 8 * b->tile.mx, b->tile.pb);
         T.unit_begin = units;
         T.tile_begin = tiles;
@@ -310,11 +304,10 @@ int enqueue(sarbp_batch *b, cudaStream_t s) {
         }
         const cufftResult r0 = cufftSetStream(b->fft[i], s);
         if (r0 != CUFFT_SUCCESS) return from_cufft(r0);
-        const cufftResult r1 = cufftExecC2C(b->fft[i], static_cast<cufftComplex *>(b->d_fft[i]),
-                                            static_cast<cufftComplex *>(b->d_fft[i]), CUFFT_INVERSE);
+        cufftComplex *rc = static_cast<cufftComplex *>(b->d_rc[i]) + b->margin[i];
+        const cufftResult r1 = cufftExecC2C(b->fft[i], rc, rc, CUFFT_INVERSE);
         if (r1 != CUFFT_SUCCESS) return from_cufft(r1);
     }
-    SARBP_TRY_CUDA(launch_rc_pairs_batch(b->d_table, n, s));
     SARBP_TRY_CUDA(launch_bp_mixed_batch(b->d_table, n, b->units, b->tiles, b->tile, b->smem, b->resident,
                                          b->d_partial, b->d_times, s, b->max_wsize, per_tile_now(b),
                                          b->records_now ? b->d_geotab : nullptr));
@@ -407,13 +400,11 @@ int sarbp_batch_create(const sarbp_plan_desc *descs, int num_scenes, sarbp_batch
     b->n = num_scenes;
     b->desc.assign(descs, descs + num_scenes);
     const int n = num_scenes;
-    b->d_pairs.assign(n, nullptr);
-    b->d_fft.assign(n, nullptr);
+    b->d_rc.assign(n, nullptr);
     b->d_fac.assign(n, nullptr);
     b->fft.assign(n, 0);
     b->fft_ok.assign(n, 0);
-    b->guard.assign(n, 0);
-    b->row_stride.assign(n, 0);
+    b->margin.assign(n, 0);
     b->np_now.assign(n, 0);
     for (auto *v : {&b->lambda, &b->dx, &b->dy, &b->dz, &b->left, &b->bottom, &b->zlow}) v->assign(n, 0.0);
     b->rctab.assign(n, nullptr);
@@ -436,17 +427,14 @@ int sarbp_batch_create(const sarbp_plan_desc *descs, int num_scenes, sarbp_batch
         axis(d.grid.nx, d.grid.x0, d.grid.wx, &b->left[i], &b->dx[i]);
         axis(d.grid.ny, d.grid.y0, d.grid.wy, &b->bottom[i], &b->dy[i]);
         axis(d.grid.nz, d.grid.z0, d.grid.wz, &b->zlow[i], &b->dz[i]);
-        // rows guarded for the largest tile shape any autotuning may pick
+        // margins for the largest tile shape any autotuning may pick
         int mx_max = 1;
         for (int t = 0; t < bp_batch_tile_count; ++t) mx_max = bp_batch_tiles[t].mx > mx_max ? bp_batch_tiles[t].mx : mx_max;
         int W, ws;
         double hd;
         tile_window(b->lambda[i], b->dx[i], b->dy[i], mx_max, &W, &ws, &hd);
-        b->guard[i] = ws + 2;
-        b->row_stride[i] = static_cast<long long>(d.nfft) + 2LL * b->guard[i];
-        const size_t np = static_cast<size_t>(d.num_pulses);
-        const size_t pair_bytes = np * static_cast<size_t>(b->row_stride[i]) * 16;
-        const size_t fft_bytes = np * d.nfft * sizeof(float2);
+        b->margin[i] = margin_samples(ws);
+        const size_t rc_bytes = (static_cast<size_t>(d.num_pulses) * d.nfft + 2 * b->margin[i]) * sizeof(float2);
         const int R = d.nfft % d.num_range_samples == 0 ? d.nfft / d.num_range_samples : 0;
         size_t rc_smem = 0;
         std::vector<float> tab;
@@ -470,11 +458,10 @@ int sarbp_batch_create(const sarbp_plan_desc *descs, int num_scenes, sarbp_batch
             b->rctab[i] = t;
             b->rc_R[i] = R;
         }
-        if ((st = balloc(b, &b->d_pairs[i], pair_bytes)) || (!fused && (st = balloc(b, &b->d_fft[i], fft_bytes))) ||
+        if ((st = balloc(b, &b->d_rc[i], rc_bytes)) ||
             (st = balloc(b, &b->d_fac[i], static_cast<size_t>(d.num_range_samples) * sizeof(float2))))
             break;
-        if (cudaMemset(b->d_pairs[i], 0, pair_bytes) != cudaSuccess ||
-            (!fused && cudaMemset(b->d_fft[i], 0, fft_bytes) != cudaSuccess)) {
+        if (cudaMemset(b->d_rc[i], 0, rc_bytes) != cudaSuccess) {
             cudaGetLastError();
             st = SARBP_ERR_CUDA;
             break;

@@ -40,14 +40,14 @@
 // lane holds), and adjoint_reduce_kernel sums the tiles per pulse in double,
 // in a fixed order.
 //
-// What bounds it: 21.4 warp instructions per warp-pixel-pulse at 62% of issue
+// What bounds it: 21 warp instructions per warp-pixel-pulse at 62% of issue
 // slots (20.9 before, where the gathers of the 32 lanes of a row took 9.3
 // shared-memory wavefronts a pixel-pulse instead of 5.8 whenever the look
 // direction lay along the columns).  2048 pulses x 1024^2 pixels, look
 // direction 0 / 45 / 90 degrees from the rows: 2.00 / 2.41 / 2.26 ms before,
-// 2.05 / 2.07 / 2.11 ms now.  The 32 registers of the pixels' |G| and psi
-// leave the 96-register budget of 20 warps short: 3 of the 21.4 instructions
-// are moves that a 142-register build (10 warps, 2.39 ms) does not need.
+// 2.00 / 2.02 / 2.07 ms now.  The 32 registers of the pixels' |G| and psi
+// leave the 96-register budget of 20 warps short: 3 of the instructions are
+// moves that a 142-register build (10 warps, 2.39 ms) does not need.
 #include <algorithm>
 #include <cstdint>
 
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
     const int n = static_cast<int>(sk_lo(blockIdx.x + 1, tg.units, G) - lo);
     if (n <= 0) return;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     UnitCursor cur;  // this warp's unit
     cur.init(tg, L, lo);
     auto tile_of = [&](const UnitCursor &u) {
@@ -266,12 +266,13 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
             }
             PulseGeo *rec = geo + s * PB + q0;
             const uint32_t win = win_addr + s * buf_bytes + static_cast<uint32_t>(q0) * pulse_bytes;
-            produce_pulses<MX, NQ>(L, cur.b * PB + q0, cur.tx, cur.ty, cur.iz, cur.hyp, pre, pregeo, rec,
+            const int p0 = cur.b * PB + q0;
+            produce_pulses<MX, NQ>(L, p0, cur.tx, cur.ty, cur.iz, cur.hyp, pre, pregeo, rec,
                                    tabs + (s * PB + q0) * kPolyEntries, win, bar_base + 8u * s, lane);
             cur.advance(tg, L);
             if (pregeo && i + 1 < n) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, true>(L, rec, win, lane, inv_lam);
+            rewrite_pulses<NQ, true>(L, p0, rec, win, lane, inv_lam);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         for (int i = n < 2 ? 0 : n - 2; i < n; ++i) {

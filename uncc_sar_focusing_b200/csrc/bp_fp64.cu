@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_fp64_kernel(const __grid_co
     const uint32_t win_addr = smem_addr(smem + kHdr64 + 2 * PB * sizeof(PulseGeo64));
     const uint32_t pulse_bytes = static_cast<uint32_t>(L.wsize) * 16u, buf_bytes = PB * pulse_bytes;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const tile::TileGrid tg = tile::tile_grid(L, TX, PB);
     const long long G = gridDim.x;
     const long long lo = tile::sk_lo(blockIdx.x, tg.units, G);
@@ -248,8 +248,7 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_fp64_kernel(const __grid_co
         if (p < L.np) g = make_geo64(L, p, cx, cy, cz);
         geo[s * PB + lane] = g;
         if (g.flags & PG_ACTIVE) {
-            const double2 *src =
-                static_cast<const double2 *>(L.pairs) + static_cast<long long>(p) * L.row_stride + L.guard + g.ws;
+            const double2 *src = static_cast<const double2 *>(L.rc) + static_cast<long long>(p) * L.nfft + g.ws;
             mbar_arrive_expect_tx(bar, pulse_bytes);
             bulk_copy_g2s(win_addr + s * buf_bytes + lane * pulse_bytes, src, pulse_bytes, bar);
         } else {

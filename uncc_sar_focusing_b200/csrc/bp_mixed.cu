@@ -19,8 +19,8 @@
 //    windows to intercept form and mark the buffer ready; the accumulating
 //    warps hand it back through the "empty" mbarrier, so they drift up to a
 //    stage apart and meet nowhere;
-//  * range profiles live in HBM as pair entries {rc[b], rc[b+1]-rc[b]}
-//    (float4); intercept form is {rc[b] - (n - W) slope, slope}, so one
+//  * range profiles live in HBM as samples; in shared memory entry n of a
+//    window is {rc[b] - (n - W) slope, slope}, slope = rc[b+1] - rc[b], so one
 //    16-byte load and two FMAs on the window-centred bin interpolate;
 //  * per pixel-pulse all arithmetic is FP32: phase and bin of a thread's
 //    pixels are polynomials in the row step (write_poly_tables), the phase in
@@ -34,12 +34,12 @@
 //    per-(thread, pulse) work is spread over 16 pixels per thread.
 //
 // What bounds it (1024^2 pixels x 2048 pulses, 8 km, look direction along the
-// rows, the columns, ncu): 14.8 warp instructions per warp-pixel-pulse at 58%
-// of issue slots, shared memory's data pipe 80-86% busy (5.1-6.1 wavefronts,
-// 4 of them the 16-byte gather's floor), MUFU 62-65%, 18 warps per SM.  Rows
-// interleaved over the warps, a row of 32 lanes and one evaluation of the
-// range remainder per pixel took 18.0 instructions and 1.70-2.13 ms over the
-// same look directions, this 1.50-1.62 ms.
+// rows / the columns, ncu): 16.0 warp instructions per warp-pixel-pulse at 65%
+// of issue slots, shared memory's data pipe 80-88% busy (5.1-6.1 wavefronts, 4
+// of them the 16-byte gather's floor), MUFU 65%, 20 warps per SM.  With rows
+// interleaved over the warps, a row of 32 lanes and an evaluation of the range
+// remainder per pixel it took 18.0 instructions and 1.70 / 2.29 / 2.13 ms at 0
+// / 45 / 90 degrees, this 1.47 / 1.48 / 1.62 ms.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
     const uint32_t win_addr = smem_addr(smem + kHdr + 2 * PB * (sizeof(PulseGeo) + kTabEntries * sizeof(float4)));
     const uint32_t buf_bytes = static_cast<uint32_t>(PB) * static_cast<uint32_t>(L0.wsize) * 16u;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     // this CTA's units [lo, lo + n) of the launch's (tile, stage) units
     const long long U = BATCH ? batch_units : tile_grid(L0, TX, PB).units;
     const long long G = gridDim.x;
@@ -346,12 +346,13 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
             if (i >= 2 && !mbar_wait_bounded(empty_bar(s), ((i - 2) >> 1) & 1, L.err)) return;
             PulseGeo *rec = geo + s * PB + q0;
             const uint32_t win = win_addr + s * buf_bytes + static_cast<uint32_t>(q0) * static_cast<uint32_t>(L.wsize) * 16u;
-            produce_pulses<MX, NQ>(L, cur.stage() * PB + q0, cur.u.tx, cur.u.ty, cur.u.iz, cur.u.hyp, pre, pregeo, rec,
+            const int p0 = cur.stage() * PB + q0;
+            produce_pulses<MX, NQ>(L, p0, cur.u.tx, cur.u.ty, cur.u.iz, cur.u.hyp, pre, pregeo, rec,
                                    tabs + (s * PB + q0) * kTabEntries, win, bar_base + 8u * s, lane);
             cur.advance(scenes, nscenes, rot_later);
             if (pregeo && i + 1 < n) load_records();
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, false>(L, rec, win, lane);
+            rewrite_pulses<NQ, false>(L, p0, rec, win, lane);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         return;

@@ -343,19 +343,16 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
 __device__ __forceinline__ void issue_window(const BpLaunch &L, int p, int q, int flags, int wp, int ws,
                                              uint32_t win_s, uint32_t bar) {
     if (flags & PG_ACTIVE) {
-        // the pulse's tight window, at its place inside the slot's full one
-        const int off = L.W - wp;
-        const uint32_t bytes = static_cast<uint32_t>(2 * wp + 2) * 16u;
-        if (p == L.drop_pulse) {
-            mbar_arrive_expect_tx(bar, bytes);
-            return;
-        }
-        const float4 *src =
-            static_cast<const float4 *>(L.pairs) + static_cast<long long>(p) * L.row_stride + L.guard + ws + off;
+        // the samples of the pulse's tight window (one more than its 2 wp + 2
+        // entries), from the even sample at or before its first, to where
+        // entry W - wp of the slot will be (rewrite_window)
+        const long long first = static_cast<long long>(p) * L.nfft + ws + (L.W - wp);
+        const int odd = static_cast<int>(first & 1);
+        const uint32_t bytes = static_cast<uint32_t>((2 * wp + 3 + odd + 1) & ~1) * 8u;
         mbar_arrive_expect_tx(bar, bytes);
-        bulk_copy_g2s(win_s + (static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) + static_cast<uint32_t>(off)) *
-                                  16u,
-                      src, bytes, bar);
+        if (p == L.drop_pulse) return;
+        bulk_copy_g2s(win_s + (static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) + static_cast<uint32_t>(L.W - wp)) * 16u,
+                      static_cast<const float2 *>(L.rc) + (first - odd), bytes, bar);
     } else {
         mbar_arrive(bar);
     }
@@ -429,8 +426,10 @@ __device__ __forceinline__ float4 lds128(uint32_t addr) {
     return v;
 }
 
-__device__ __forceinline__ void sts64(uint32_t addr, float x, float y) {
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+__device__ __forceinline__ float2 lds64(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
 }
 
 __device__ __forceinline__ void sts128(uint32_t addr, float x, float y, float z, float w) {
@@ -465,8 +464,9 @@ struct PixelPoly {
         hi = u1.w;
     }
 
-    // f(k, phase, bin) for the thread's MX pixel pairs, outermost row steps
-    // first, the middle one last; rows +-k share P0 + k^2 Pb.
+    // f(k, phase, bin) for the thread's MX pixel pairs, the middle row last
+    // (first: adjoint 2085 instead of 2064 us, forward the same); rows +-k
+    // share P0 + k^2 Pb.
     template <int MX, typename F>
     __device__ __forceinline__ void rows(F f) const {
         using M = PixelMap<MX>;
@@ -501,10 +501,10 @@ __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaun
     return make_float2(gl[0], gl[1]);
 }
 
-// Intercept form of the windows: entry n of a pulse's window holds
-// {v_n, v'_n} (v'_n = v_(n+1) - v_n); rewritten in place to
-// {v_n - (n - W) v'_n, v'_n}, a pixel whose window-centred bin is
-// B = bin - ws - W (floor(B) + W = n) interpolates
+// Intercept form of the windows.  A window arrives as samples v_n; entry n of
+// its slot becomes {v_n - (n - W) v'_n, v'_n}, v'_n = v_(n+1) - v_n, so that a
+// pixel whose window-centred bin is B = bin - ws - W (floor(B) + W = n)
+// interpolates
 //     v(B) = v_n + (B + W - n) v'_n = c_n + B v'_n
 // with one fused multiply-add and no fraction.
 // ZFORM (the adjoint, which needs only Z(B) = v'(B) + j nu v(B), nu = kr /
@@ -512,38 +512,68 @@ __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaun
 // c_n and Zv = j nu v'_n, so that Z(B) = Zc + B Zv is again one fused
 // multiply-add per component and the pixel loop neither interpolates v nor
 // forms Z.
+//
+// In place, from the last entry to the first: the samples (8 bytes) start
+// where the entries (16 bytes) do, so the entries of a group of lanes lie past
+// every sample a lower group still reads; within a group all lanes read before
+// any writes.  Samples instead of pair entries {v_n, v'_n} in HBM halve what
+// range compression writes and the windows copy and need no pass after the
+// FFT (point-target call 106 -> 94 us); the rewrite's second load and
+// difference cost the 1024^2 x 2048 forward kernel 1.9% (1495 -> 1524 us).
+// w: the window's first entry (W - wp); odd: its first sample is the second
+// of those copied (issue_window).
 template <bool ZFORM>
-__device__ __forceinline__ void rewrite_window(uint32_t w, int W, int wp, int lane, float nu) {
-    uint32_t a = w + static_cast<uint32_t>(W - wp + lane) * 16u;
-    float m = static_cast<float>(lane - wp);
-    auto one = [&](uint32_t at, float mm) {
-        const float4 e = lds128(at);
-        const float cr = fmaf(-mm, e.z, e.x), ci = fmaf(-mm, e.w, e.y);
-        if (ZFORM)
-            sts128(at, fmaf(-nu, ci, e.z), fmaf(nu, cr, e.w), -nu * e.w, nu * e.z);
-        else
-            sts64(at, cr, ci);
+__device__ __forceinline__ void rewrite_window(uint32_t w, int wp, uint32_t odd, int lane, float nu) {
+    const int count = 2 * wp + 2;
+    constexpr int kGroup = 4;  // entries of a lane per round
+    int n = (count - 1) / (32 * kGroup) * (32 * kGroup) + lane;  // the lane's first entry of the round
+    uint32_t src = w + (static_cast<uint32_t>(n) + odd) * 8u, dst = w + static_cast<uint32_t>(n) * 16u;
+    float m = static_cast<float>(n - wp);
+    auto round = [&](int entries) {  // entries: those of the lane, at n, n + 32, ...
+        float2 v[kGroup], vn[kGroup];
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i)
+            if (i < entries) {
+                v[i] = lds64(src + 256u * i);
+                vn[i] = lds64(src + 256u * i + 8u);
+            }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i)
+            if (i < entries) {
+                const float2 d = __fadd2_rn(vn[i], make_float2(-v[i].x, -v[i].y));
+                const float2 c = __ffma2_rn(splat(-m - 32.0f * i), d, v[i]);
+                if (ZFORM) {
+                    const float2 z = __fmul2_rn(splat(nu), d);
+                    sts128(dst + 512u * i, fmaf(-nu, c.y, d.x), fmaf(nu, c.x, d.y), -z.y, z.x);
+                } else {
+                    sts128(dst + 512u * i, c.x, c.y, d.x, d.y);
+                }
+            }
+        __syncwarp();
     };
-    int left = 2 * wp + 2 - lane;  // the entries the pulse's tight window copied
-    for (; left > 96; left -= 128, a += 2048u, m += 128.0f) {
-        one(a, m);
-        one(a + 512u, m + 32.0f);
-        one(a + 1024u, m + 64.0f);
-        one(a + 1536u, m + 96.0f);
+    round((count - n + 31) >> 5);
+    for (n -= 32 * kGroup; n >= 0; n -= 32 * kGroup) {
+        src -= 256u * kGroup;
+        dst -= 512u * kGroup;
+        m -= 32.0f * kGroup;
+        round(kGroup);
     }
-    for (; left > 0; left -= 32, a += 512u, m += 32.0f) one(a, m);
 }
 
 // The windows of NQ pulses, by their producing warp once the copies have landed;
 // the fence orders these generic-proxy stores before the next bulk copies
 // (async proxy) into the buffer, which the same warp issues.
 template <int NQ, bool ZFORM>
-__device__ __forceinline__ void rewrite_pulses(const BpLaunch &L, const PulseGeo *rec, uint32_t win_s, int lane,
-                                              float inv_lam = 0.0f) {
+__device__ __forceinline__ void rewrite_pulses(const BpLaunch &L, int p0, const PulseGeo *rec, uint32_t win_s, int lane,
+                                               float inv_lam = 0.0f) {
     for (int q = 0; q < NQ; ++q) {
         if (!(rec[q].flags & PG_ACTIVE)) continue;
-        rewrite_window<ZFORM>(win_s + static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) * 16u, L.W, rec[q].wp,
-                              lane, ZFORM ? rec[q].kr * inv_lam : 0.0f);
+        const int off = L.W - rec[q].wp;
+        const uint32_t odd = (static_cast<uint32_t>(p0 + q) * static_cast<uint32_t>(L.nfft) +
+                              static_cast<uint32_t>(rec[q].ws + off)) & 1u;
+        rewrite_window<ZFORM>(win_s + (static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) + static_cast<uint32_t>(off)) * 16u,
+                              rec[q].wp, odd, lane, ZFORM ? rec[q].kr * inv_lam : 0.0f);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();

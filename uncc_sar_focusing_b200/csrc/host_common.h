@@ -127,6 +127,10 @@ inline void axis(int n, double c, double w, double *lo, double *step) {
     }
 }
 
+// Readable samples the kernels need before and after the range-profile rows
+// for windows of wsize entries (even, so that the rows stay 16-byte aligned).
+inline size_t margin_samples(int wsize) { return static_cast<size_t>(wsize) + 4; }
+
 // Range-bin window of a tile of (8 mx) x 64 pixels with steps dx, dy at
 // lambda bins per metre: W = ceil(lambda * half-diagonal) + 3 bins each side,
 // wsize = 2W + 2 pair entries; hd the half-diagonal in metres.

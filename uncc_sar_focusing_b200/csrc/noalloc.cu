@@ -10,12 +10,12 @@
 // budget does not allow a library to take more behind its back.  For them,
 // sarbp_backproject_noalloc takes range profiles, geometry and the image in
 // memory the caller already owns, and keeps the only scratch it needs -- the
-// pair-entry rows the kernel stages from, plus one error word -- in the
+// rows the kernel stages from, plus one error word -- in the
 // file-scope array below.
 //
 // The array is a fixed 32 MiB per GPU that loads this library, held until the
 // process exits.  Every call shares it and leaves its contents behind, so each
-// call rewrites whole rows (guard bands included) and zeroes the error word
+// call rewrites whole rows (margins included) and zeroes the error word
 // before its kernels run; two calls that overlap on the GPU (different
 // streams, or different host threads on one device) race on it.  The first
 // call on a device looks up the array's device address with
@@ -34,8 +34,8 @@ namespace {
 
 using namespace sarbp;
 
-// 2^21 16-byte entries = 32 MiB.  Entry 0 holds the error word; pair rows
-// start at entry 1 (16-byte aligned, as the bulk copies need).
+// 2^21 16-byte entries = 32 MiB.  Entry 0 holds the error word; the rows start
+// at entry 1 (16-byte aligned, as the bulk copies need).
 constexpr size_t kScratchEntries = size_t(1) << 21;
 constexpr int kMaxDevices = 64;
 
@@ -60,18 +60,14 @@ int scratch_for(int dev, float4 **out) {
     return SARBP_OK;
 }
 
-// Whole pair rows {rc[b], rc[b+1] - rc[b]}, zero outside 0 <= b < nfft
-// (including the guard bands, which a previous call may have filled).
-__global__ void noalloc_pair_rows(const float2 *__restrict__ rc, float4 *__restrict__ rows, int nfft, int guard,
-                                  long long row_stride, long long total) {
+// The caller's rows behind one another with `margin` zeros before and after
+// (a previous call may have filled them): total samples in all.
+__global__ void noalloc_rows(const float2 *__restrict__ rc, float2 *__restrict__ rows, long long margin,
+                             long long samples, long long total) {
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long p = i / row_stride;
-        const int b = static_cast<int>(i - p * row_stride) - guard;
-        float2 v = make_float2(0.0f, 0.0f), vn = make_float2(0.0f, 0.0f);
-        if (b >= 0 && b < nfft) v = rc[p * nfft + b];
-        if (b + 1 >= 0 && b + 1 < nfft) vn = rc[p * nfft + b + 1];
-        rows[i] = make_float4(v.x, v.y, vn.x - v.x, vn.y - v.y);
+        const long long j = i - margin;
+        rows[i] = j >= 0 && j < samples ? rc[j] : make_float2(0.0f, 0.0f);
     }
 }
 
@@ -134,10 +130,13 @@ extern "C" SARBP_API int sarbp_backproject_noalloc(const sarbp_plan_desc *desc, 
         }
     }
     if (!tc.mx) return SARBP_ERR_UNSUPPORTED;
-    const int guard = wsize + 2;
-    const long long row_stride = static_cast<long long>(desc->nfft) + 2LL * guard;
-    const long long total = row_stride * geo->num_pulses;
-    if (total > static_cast<long long>(kScratchEntries) - 1) return SARBP_ERR_UNSUPPORTED;  // beyond 32 MiB
+    // the documented limit (16 bytes per sample of rows with a window's width
+    // each side); the rows themselves take half of it
+    if ((static_cast<long long>(desc->nfft) + 2LL * (wsize + 2)) * geo->num_pulses >
+        static_cast<long long>(kScratchEntries) - 1)
+        return SARBP_ERR_UNSUPPORTED;
+    const long long margin = static_cast<long long>(host::margin_samples(wsize));
+    const long long samples = static_cast<long long>(desc->nfft) * geo->num_pulses, total = samples + 2 * margin;
 
     // desc->device >= 0: run on that device (as sarbp_plan_create does), the
     // caller's current device restored on return; -1: the current device
@@ -165,20 +164,18 @@ extern "C" SARBP_API int sarbp_backproject_noalloc(const sarbp_plan_desc *desc, 
     int st = scratch_for(dev, &scratch);
     if (st != SARBP_OK) return st;
     unsigned *err = reinterpret_cast<unsigned *>(scratch);
-    float4 *rows = scratch + 1;
+    float2 *rows = reinterpret_cast<float2 *>(scratch + 1);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned), s);
     if (e == cudaSuccess) {
         const long long blocks = (total + 255) / 256;
-        noalloc_pair_rows<<<static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(
-            static_cast<const float2 *>(range_profiles), rows, desc->nfft, guard, row_stride, total);
+        noalloc_rows<<<static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(
+            static_cast<const float2 *>(range_profiles), rows, margin, samples, total);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        L.pairs = rows;
-        L.row_stride = row_stride;
-        L.guard = guard;
+        L.rc = rows + margin;
         L.ax = geo->ant_x;
         L.ay = geo->ant_y;
         L.az = geo->ant_z;

@@ -12,9 +12,7 @@
 //     moved to the input side: ifft(x .* e^{j 2 pi k s/N})[n] = ifft(x)[n + s].
 //     The 1/Nfft scale and the taper ride along, so no normalise or shift pass.
 //  2. cuFFT batched C2C (Z2Z for FP64) inverse, in place.
-//  3. (mixed precision) rc_pairs_kernel stores pair entries {rc[b], rc[b+1] - rc[b]} in rows of
-//     `row_stride` entries with `guard` zero entries on each side, the layout
-//     the backprojection kernels stage into shared memory.
+// The backprojection kernels copy their windows straight from these rows.
 #include <cmath>
 #include <vector>
 
@@ -43,31 +41,13 @@ __global__ void rc_prep_kernel(const float2 *__restrict__ ph, const C *__restric
     }
 }
 
-__device__ __forceinline__ void make_pair(const float2 &v, const float2 &vn, float4 *dst) {
-    *dst = make_float4(v.x, v.y, vn.x - v.x, vn.y - v.y);
-}
-
-__global__ void rc_pairs_kernel(const float2 *__restrict__ X, float4 *__restrict__ pairs, int nfft, long long total,
-                                long long row_stride, int guard) {
-    const int per = nfft + 1;  // entries b = -1 .. nfft-1 of each row
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long p = i / per;
-        const int b = static_cast<int>(i - p * per) - 1;
-        float2 v = make_float2(0.0f, 0.0f), vn = make_float2(0.0f, 0.0f);
-        if (b >= 0) v = X[p * nfft + b];
-        if (b + 1 < nfft) vn = X[p * nfft + b + 1];
-        make_pair(v, vn, pairs + p * row_stride + guard + b);
-    }
-}
-
-// Batch forms: scene blockIdx.y of the table, grid-stride over its elements.
+// Batch form: scene blockIdx.y of the table, grid-stride over its elements.
 __global__ void rc_prep_batch_kernel(const BatchScene *__restrict__ scenes) {
     const BatchScene &S = scenes[blockIdx.y];
     if (S.fused) return;  // range-compressed by its own fused launch
     const float2 *__restrict__ ph = static_cast<const float2 *>(S.ph);
     const float2 *__restrict__ fac = static_cast<const float2 *>(S.fac);
-    float2 *__restrict__ out = static_cast<float2 *>(S.fft);
+    float2 *__restrict__ out = static_cast<float2 *>(const_cast<void *>(S.L.rc));
     const int K = S.K, nfft = S.L.nfft;
     const long long total = static_cast<long long>(S.L.np) * nfft;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -85,25 +65,6 @@ __global__ void rc_prep_batch_kernel(const BatchScene *__restrict__ scenes) {
     }
 }
 
-__global__ void rc_pairs_batch_kernel(const BatchScene *__restrict__ scenes) {
-    const BatchScene &S = scenes[blockIdx.y];
-    if (S.fused) return;
-    const float2 *__restrict__ X = static_cast<const float2 *>(S.fft);
-    float4 *__restrict__ pairs = static_cast<float4 *>(const_cast<void *>(S.L.pairs));
-    const int nfft = S.L.nfft, guard = S.L.guard;
-    const int per = nfft + 1;
-    const long long total = static_cast<long long>(S.L.np) * per;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long p = i / per;
-        const int b = static_cast<int>(i - p * per) - 1;
-        float2 v = make_float2(0.0f, 0.0f), vn = make_float2(0.0f, 0.0f);
-        if (b >= 0) v = X[p * nfft + b];
-        if (b + 1 < nfft) vn = X[p * nfft + b + 1];
-        make_pair(v, vn, pairs + p * S.row_stride + guard + b);
-    }
-}
-
 // ---- fused range compression: nfft = R K, K = 32 K2 ------------------------
 //
 // With y[k] = fac[k] ph[k] (taper x 1/N x shift twiddle) and N = R K the
@@ -114,9 +75,8 @@ __global__ void rc_pairs_batch_kernel(const BatchScene *__restrict__ scenes) {
 // m = m2 + K2 m1:  lane k1 transforms its K2 samples in registers (over k2),
 // multiplies by W_K^{k1 m2}, the warp transposes through shared memory, and
 // lane m2 transforms the 32 values over k1 in registers.  The R results are
-// read back interleaved to write the pair entries {rc[b], rc[b+1] - rc[b]},
-// b = -1 .. N-1, straight to HBM: 8 bytes read per input sample, 16 bytes
-// written per pair entry, no FFT buffer.  Twiddles come from one table built
+// read back interleaved to write the profile's samples straight to HBM: 8
+// bytes read per input sample, 8 written per output sample.  Twiddles come from one table built
 // in double on the host and staged into shared memory.
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
@@ -197,20 +157,18 @@ struct RcTable {
     static constexpr int kWn = kTwk + K;           // W_N^i, i < 32 R
     static constexpr int kWnr = kWn + 32 * R;      // W_{N/32}^i, i < N / 32
     static constexpr int kSize = kWnr + NW;
-    // shared row of one sub-transform.  The pair-row writes read element
-    // (r, m) = (b mod R, b / R) for consecutive b: 16 lanes (one 128-byte
-    // wavefront of 8-byte reads) cover R values of r and 16/R of m, first
-    // bank 2 (r kReg + m) mod 32; kReg = 16/R mod 16 makes these 16
-    // distinct even banks for every R (K + 36, right for R = 4, put r and
-    // r + 4 on the same banks for R = 8)
+    // shared row of one sub-transform.  The row writes read element (r, m) =
+    // (b mod R, b / R) for every second b: the 16 lanes of one 128-byte
+    // wavefront of 8-byte reads cover the even (or odd) values of r and 32/R
+    // of m, first bank 2 (r kReg + m) mod 32; kReg = 16/R mod 16 makes these
+    // 16 distinct even banks for R >= 2
     static constexpr int kReg = K + 32 + 16 / R;
     static constexpr size_t kSmem = (static_cast<size_t>(K) + kSize + static_cast<size_t>(R) * kReg) * 8;
 };
 
 template <int K2, int R>
 __device__ __forceinline__ void rc_fused_body(const float2 *__restrict__ ph, const float2 *__restrict__ fac,
-                                              const float2 *__restrict__ tab, float4 *__restrict__ pairs, int np,
-                                              long long row_stride, int guard) {
+                                              const float2 *__restrict__ tab, float2 *__restrict__ rc, int np) {
     using T = RcTable<K2, R>;
     constexpr int K = T::K, N = T::N, REG = T::kReg, LOGR = log2_of<R>();
     extern __shared__ __align__(16) float2 rc_sm[];
@@ -262,13 +220,12 @@ __device__ __forceinline__ void rc_fused_body(const float2 *__restrict__ ph, con
         }
         __syncthreads();
         prefetch(p + gridDim.x);
-        // rc[R m + r] = regions[r][m]
-        float4 *row = pairs + static_cast<long long>(p) * row_stride + guard;
-        for (int b = tid - 1; b < N; b += 32 * R) {
-            float2 u = make_float2(0.0f, 0.0f), un = make_float2(0.0f, 0.0f);
-            if (b >= 0) u = regions[(b & (R - 1)) * REG + (b >> LOGR)];
-            if (b + 1 < N) un = regions[((b + 1) & (R - 1)) * REG + ((b + 1) >> LOGR)];
-            row[b] = make_float4(u.x, u.y, un.x - u.x, un.y - u.y);
+        // rc[R m + r] = regions[r][m], two samples a thread (N is even)
+        float4 *row = reinterpret_cast<float4 *>(rc + static_cast<long long>(p) * N);
+        for (int b = 2 * tid; b < N; b += 64 * R) {
+            const float2 u = regions[(b & (R - 1)) * REG + (b >> LOGR)];
+            const float2 un = regions[((b + 1) & (R - 1)) * REG + ((b + 1) >> LOGR)];
+            row[b >> 1] = make_float4(u.x, u.y, un.x, un.y);
         }
     }
 }
@@ -276,9 +233,9 @@ __device__ __forceinline__ void rc_fused_body(const float2 *__restrict__ ph, con
 template <int K2, int R>
 __global__ void __launch_bounds__(32 * R) rc_fused_kernel(const float2 *__restrict__ ph,
                                                          const float2 *__restrict__ fac,
-                                                         const float2 *__restrict__ tab, float4 *__restrict__ pairs,
-                                                         int np, long long row_stride, int guard) {
-    rc_fused_body<K2, R>(ph, fac, tab, pairs, np, row_stride, guard);
+                                                         const float2 *__restrict__ tab, float2 *__restrict__ rc,
+                                                         int np) {
+    rc_fused_body<K2, R>(ph, fac, tab, rc, np);
 }
 
 // The same for one scene of a batch: every pointer and size from the scene's
@@ -288,7 +245,7 @@ __global__ void __launch_bounds__(32 * R) rc_fused_scene_kernel(const BatchScene
                                                                const float2 *__restrict__ tab) {
     const BatchScene &S = *scene;
     rc_fused_body<K2, R>(static_cast<const float2 *>(S.ph), static_cast<const float2 *>(S.fac), tab,
-                         static_cast<float4 *>(const_cast<void *>(S.L.pairs)), S.L.np, S.row_stride, S.L.guard);
+                         static_cast<float2 *>(const_cast<void *>(S.L.rc)), S.L.np);
 }
 
 template <int K2, int R>
@@ -307,29 +264,16 @@ void fill_rc_table(std::vector<float> &t) {
 }
 
 template <int K2, int R>
-cudaError_t launch_fused(const float2 *ph, const float2 *fac, const float2 *tab, float4 *pairs, int np,
-                         long long row_stride, int guard, int grid, cudaStream_t s) {
+cudaError_t launch_fused(const float2 *ph, const float2 *fac, const float2 *tab, float2 *rc, int np, int grid,
+                         cudaStream_t s) {
     using T = RcTable<K2, R>;
     auto kern = rc_fused_kernel<K2, R>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(T::kSmem));
     if (e != cudaSuccess) return e;
     const int g = np < grid ? np : grid;
-    kern<<<g > 0 ? g : 1, 32 * R, T::kSmem, s>>>(ph, fac, tab, pairs, np, row_stride, guard);
+    kern<<<g > 0 ? g : 1, 32 * R, T::kSmem, s>>>(ph, fac, tab, rc, np);
     return cudaGetLastError();
-}
-
-// Range profiles rc[b] back out of the pair rows (sarbp_get_range_profiles
-// after fused range compression).
-__global__ void pairs_to_rc_kernel(const float4 *__restrict__ pairs, float2 *__restrict__ rc, int nfft,
-                                   long long total, long long row_stride, int guard) {
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long p = i / nfft;
-        const int b = static_cast<int>(i - p * nfft);
-        const float4 e = pairs[p * row_stride + guard + b];
-        rc[i] = make_float2(e.x, e.y);
-    }
 }
 
 int grid_for(long long total) {
@@ -354,23 +298,9 @@ cudaError_t launch_rc_prep(int precision, const void *ph, const void *fac, void 
     return cudaGetLastError();
 }
 
-cudaError_t launch_rc_pairs(const void *fft_buf, void *pairs, int nfft, int np, long long row_stride, int guard,
-                            cudaStream_t s) {
-    const long long total = static_cast<long long>(np) * (nfft + 1);
-    rc_pairs_kernel<<<grid_for(total), 256, 0, s>>>(static_cast<const float2 *>(fft_buf), static_cast<float4 *>(pairs),
-                                                    nfft, total, row_stride, guard);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStream_t s) {
     if (nscenes < 1 || nscenes > 65535) return cudaErrorInvalidValue;
     rc_prep_batch_kernel<<<dim3(128, nscenes), 256, 0, s>>>(scenes);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_rc_pairs_batch(const BatchScene *scenes, int nscenes, cudaStream_t s) {
-    if (nscenes < 1 || nscenes > 65535) return cudaErrorInvalidValue;
-    rc_pairs_batch_kernel<<<dim3(128, nscenes), 256, 0, s>>>(scenes);
     return cudaGetLastError();
 }
 
@@ -390,13 +320,12 @@ bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table) {
     return false;
 }
 
-cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *pairs, int K, int R, int np,
-                            long long row_stride, int guard, int grid, cudaStream_t s) {
+cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
+                            int grid, cudaStream_t s) {
 #define SARBP_RC_CASE(K2_, R_)                                                                                   \
     if (K == 32 * K2_ && R == R_)                                                                                 \
         return launch_fused<K2_, R_>(static_cast<const float2 *>(ph), static_cast<const float2 *>(fac),          \
-                                     static_cast<const float2 *>(table), static_cast<float4 *>(pairs), np,        \
-                                     row_stride, guard, grid, s);
+                                     static_cast<const float2 *>(table), static_cast<float2 *>(rc), np, grid, s);
     SARBP_RC_SHAPES(SARBP_RC_CASE)
 #undef SARBP_RC_CASE
     return cudaErrorInvalidValue;
@@ -417,14 +346,6 @@ cudaError_t launch_rc_fused_scene(const BatchScene *scene, const void *table, in
     SARBP_RC_SHAPES(SARBP_RC_CASE)
 #undef SARBP_RC_CASE
     return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_pairs_to_rc(const void *pairs, void *rc, int nfft, int np, long long row_stride, int guard,
-                               cudaStream_t s) {
-    const long long total = static_cast<long long>(np) * nfft;
-    pairs_to_rc_kernel<<<grid_for(total), 256, 0, s>>>(static_cast<const float4 *>(pairs), static_cast<float2 *>(rc),
-                                                      nfft, total, row_stride, guard);
-    return cudaGetLastError();
 }
 
 }  // namespace sarbp

@@ -12,9 +12,11 @@ namespace sarbp {
 
 // Launch parameters of the forward backprojection kernels.
 struct BpLaunch {
-    const void *pairs;      // pair entries float4 (MIXED) / range-profile samples double2 (FP64)
-    long long row_stride;   // entries per pulse row
-    int guard;              // zero entries before bin 0 of each row (MIXED)
+    // range profiles, complex64 (MIXED) / complex128 (FP64) [np][nfft], 16-byte
+    // aligned, with a window's worth of readable samples before and after: a
+    // window past a row's end reads the neighbouring row's samples (or that
+    // margin), which the gate discards
+    const void *rc;
     const double *ax, *ay, *az, *r0, *f0;
     int np, nfft;
     double lambda;          // nfft / max_wr (bins per metre)
@@ -53,13 +55,11 @@ struct BpLaunch {
 // [unit_begin, unit_begin + its tiles x stages) and tiles
 // [tile_begin, tile_begin + its tiles) of the launch.
 struct BatchScene {
-    BpLaunch L;                 // the scene's backprojection (pairs, geometry, grid, image, window)
+    BpLaunch L;                 // the scene's backprojection (range profiles, geometry, grid, image, window)
     const void *ph;             // complex64 [np][K] phase history (device)
     const void *fac;            // per-sample taper x scale x shift twiddle [K]
-    void *fft;                  // complex64 [np][nfft] FFT buffer
     int K;
-    int fused;                  // 1: range-compressed by its own fused launch (batched taper/pair kernels skip it)
-    long long row_stride;       // pair entries per pulse row
+    int fused;                  // 1: range-compressed by its own fused launch (the batched taper kernel skips it)
     long long unit_begin, tile_begin;
 };
 
@@ -132,26 +132,20 @@ int bp_fp64_resident(const TileConfig &tc, size_t smem);
 // Range compression kernels (range_compress.cu)
 cudaError_t launch_rc_prep(int precision, const void *ph, const void *fac, void *fft_buf, int K, int nfft, int np,
                            cudaStream_t s);
-cudaError_t launch_rc_pairs(const void *fft_buf, void *pairs, int nfft, int np, long long row_stride, int guard,
-                            cudaStream_t s);
-// Range compression steps 1 and 3 for every scene of a batch in one launch
-// each (blockIdx.y = scene); the FFT in between runs per scene.
+// The same for every scene of a batch in one launch (blockIdx.y = scene).
 cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStream_t s);
-// Fused range compression (mixed precision): taper, zero pad, inverse FFT and
-// pair rows in one kernel for nfft = R K with K = 32 K2, K2 in {8, 16, 32},
+// Fused range compression (mixed precision): taper, zero pad and inverse FFT
+// in one kernel for nfft = R K with K = 32 K2, K2 in {8, 16, 32},
 // R in {1, 2, 4, 8, 16}.  rc_fused_shape says whether (K, R) is one of those
 // and fills the twiddle table (interleaved float re, im) and the kernel's
 // shared-memory bytes; grid: CTAs (each loops over pulses).
 bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table);
-cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *pairs, int K, int R, int np,
-                            long long row_stride, int guard, int grid, cudaStream_t s);
-cudaError_t launch_pairs_to_rc(const void *pairs, void *rc, int nfft, int np, long long row_stride, int guard,
-                               cudaStream_t s);
+cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
+                            int grid, cudaStream_t s);
 // Fused range compression of one batch scene, parameters read from its table
 // slot (grid CTAs loop over the scene's pulses).
 cudaError_t launch_rc_fused_scene(const BatchScene *scene, const void *table, int K, int R, int grid,
                                   cudaStream_t s);
-cudaError_t launch_rc_pairs_batch(const BatchScene *scenes, int nscenes, cudaStream_t s);
 
 }  // namespace sarbp
 
@@ -160,8 +154,7 @@ struct sarbp_plan {
     int device;
     int K, np_cap, nfft, precision;
     double lambda;
-    int W, wsize, guard;
-    long long row_stride;
+    int W, wsize;
     sarbp::TileConfig tile;
     size_t smem;
     double near_hd16, near_coef;
@@ -169,9 +162,8 @@ struct sarbp_plan {
 
     void *d_ph;       // complex64 [np][K] staging for host phase histories
     double *d_geo;    // 5 x np staging for host geometry
-    void *d_fft;      // complex64/128 [np][nfft], inside d_fft_base (FP64: guard samples at both ends)
-    void *d_fft_base;
-    void *d_pairs;    // pair entries [np][row_stride] (mixed precision)
+    void *d_fft;      // range profiles complex64/128 [np][nfft] (FFT in place), inside
+    void *d_fft_base; // an allocation with margin_samples of zeros at both ends
     void *d_fac;      // per-sample window * scale * shift twiddle [K]
     void *d_img;      // image staging for host outputs
     unsigned *d_err;  // device error bits
@@ -195,8 +187,9 @@ struct sarbp_plan {
     int sk_resident;  // resident CTAs of the plan's forward kernel
     int drop_pulse = -1;  // test hook: BpLaunch::drop_pulse of the plan's launches
     size_t bytes;     // device bytes held
-    cufftHandle fft;
+    cufftHandle fft;  // shapes without a fused range compression
     bool fft_ok;
+    void *d_fft_work; // its work area
     int np_ready;     // pulses in the current range profiles
     struct sarbp_pipe *pipe;  // pipelined host-buffer focusing (created on first submit)
 };
