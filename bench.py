@@ -828,12 +828,11 @@ def gpu_arm(args):
                     "api": "sarbp_focus_submit/sarbp_focus_wait, pinned host buffers",
                     "synchronous": {"value": world * pp / e2e_sync_s, "ms_per_step": e2e_sync_s * 1e3,
                                     "api": "sarbp_focus, pinned host buffers"}},
-            # per step: range compression (one fused kernel, or taper + pair
-            # rows around cuFFT, whose kernel is the library's and not
-            # counted), the backprojection (+ its fix-up when the tiles are
-            # split over the resident CTAs)
-            "gpu_launches": ((1 if info["fused_range_compression"] else 2) + info["kernels_per_backproject"])
-            * args.steps,
+            # per step: range compression (one fused kernel, or the taper
+            # before cuFFT, whose kernels are the library's and not counted),
+            # the backprojection (+ its fix-up when the tiles are split over
+            # the resident CTAs)
+            "gpu_launches": (1 + info["kernels_per_backproject"]) * args.steps,
             "kernels": {"bp_ms": bp_ms, "range_compress_ms": rc_ms,
                         "adjoint": {"ms": adj_ms, "value": pp / (adj_ms * 1e-3), "unit": UNIT,
                                     "vs_forward_bp_time": adj_ms / bp_ms,

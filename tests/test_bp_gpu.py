@@ -269,3 +269,19 @@ def test_pixel_map_edges(F, monkeypatch, nx, ny, tile):
         got = plan.focus(sc.phase_history, sc.ant_x, sc.ant_y, sc.ant_z, sc.slant_range, sc.start_freq)
     rc = O.range_compress_fp64(sc.phase_history, sc.nfft, O.hamming(sc.num_range_samples))
     assert np.abs(got - O.focus_fp64(sc)).max() < 1e-5 * np.abs(rc).max(axis=1).sum()
+
+
+@pytest.mark.parametrize("K,R,chirp", [(193, 4, 1), (201, 8, 1), (257, 8, 1), (272, 4, 1), (424, 8, 1), (501, 4, 1),
+                                       (509, 8, 1), (424, 5, 0), (192, 8, 0), (500, 8, 0), (521, 4, 0)])
+def test_chirp_range_compression_matches_oracle(F, K, R, chirp):
+    """K <= 512 with a long prime factor, upsampled 4 or 8 times: profiles
+    against the FP64 oracle at the tolerance of the other paths, at both ends
+    of the rule, odd lengths and more pulses than the grid has CTAs."""
+    sc = small_scene(K=K, nfft=R * K, Np=700)
+    sc.window = "none"
+    want = O.range_compress_fp64(sc.phase_history, sc.nfft, None)
+    with F.Plan.for_scene(sc, "mixed") as plan:
+        assert plan.info["chirp_range_compression"] == chirp
+        plan.range_compress(sc.phase_history)
+        got = plan.range_profiles()
+    assert O.rel_l2(got, want) < 2e-6

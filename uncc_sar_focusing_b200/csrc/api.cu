@@ -725,7 +725,7 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
         return st;
     }
     // fused range compression when the shape has a kernel (environment
-    // SARBP_RC=cufft keeps the taper / cuFFT / pair-row path)
+    // SARBP_RC=cufft keeps the taper and cuFFT path)
     {
         const int K = p->K, N = p->nfft;
         const int R = (N % K == 0) ? N / K : 0;
@@ -750,8 +750,8 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
             }
             p->rc_R = R;
             // CTAs resident at once: the kernel loops over pulses
-            const int per_sm = rc_smem > 0 ? static_cast<int>((228u * 1024u) / (rc_smem + 1024u)) : 1;
-            p->rc_grid = (sms > 0 ? sms : 148) * (per_sm > 0 ? (per_sm < 4 ? per_sm : 4) : 1);
+            const int per_sm = rc_fused_resident(K, R);
+            p->rc_grid = (sms > 0 ? sms : 148) * (per_sm > 0 ? per_sm : 1);
         }
     }
     // the other shapes: cuFFT on a work area of the plan's own
@@ -828,7 +828,8 @@ int sarbp_plan_get_info(const sarbp_plan *plan, sarbp_plan_info *info) {
                   g.nz;
     info->smem_bytes = static_cast<long long>(plan->smem);
     info->kernels_per_backproject = (plan->d_sk && plan->sk_resident > 0 && info->tiles % plan->sk_resident != 0) ? 2 : 1;
-    info->fused_range_compression = plan->d_rctab ? 1 : 0;
+    info->fused_range_compression = plan->d_rctab && rc_direct_shape(plan->K) ? 1 : 0;
+    info->chirp_range_compression = plan->d_rctab && !rc_direct_shape(plan->K) ? 1 : 0;
     return SARBP_OK;
 }
 

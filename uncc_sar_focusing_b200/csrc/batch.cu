@@ -295,7 +295,9 @@ int enqueue(sarbp_batch *b, cudaStream_t s) {
     SARBP_TRY_CUDA(cudaGetLastError());
     if (b->records_now)
         SARBP_TRY_CUDA(launch_geo_records_batch(b->d_table, n, b->tile.mx, b->max_records, s));
-    SARBP_TRY_CUDA(launch_rc_prep_batch(b->d_table, n, s));
+    bool any_fft = false;
+    for (int i = 0; i < n; ++i) any_fft = any_fft || !b->rctab[i];
+    if (any_fft) SARBP_TRY_CUDA(launch_rc_prep_batch(b->d_table, n, s));
     for (int i = 0; i < n; ++i) {
         if (b->rctab[i]) {
             SARBP_TRY_CUDA(launch_rc_fused_scene(b->d_table + i, b->rctab[i], b->desc[i].num_range_samples,

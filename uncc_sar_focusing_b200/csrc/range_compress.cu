@@ -14,6 +14,7 @@
 //  2. cuFFT batched C2C (Z2Z for FP64) inverse, in place.
 // The backprojection kernels copy their windows straight from these rows.
 #include <cmath>
+#include <complex>
 #include <vector>
 
 #include "sarbp_internal.h"
@@ -230,22 +231,216 @@ __device__ __forceinline__ void rc_fused_body(const float2 *__restrict__ ph, con
     }
 }
 
+// scene: null, or one scene of a batch whose slot of the device table holds
+// every pointer and size (a captured graph replays with new buffers).
+struct RcArgs {
+    const BatchScene *scene;
+    const float2 *ph, *fac, *tab;
+    float2 *rc;
+    int K, np;
+
+    __device__ __forceinline__ void resolve() {
+        if (!scene) return;
+        ph = static_cast<const float2 *>(scene->ph);
+        fac = static_cast<const float2 *>(scene->fac);
+        rc = static_cast<float2 *>(const_cast<void *>(scene->L.rc));
+        K = scene->K;
+        np = scene->L.np;
+    }
+};
+
 template <int K2, int R>
-__global__ void __launch_bounds__(32 * R) rc_fused_kernel(const float2 *__restrict__ ph,
-                                                         const float2 *__restrict__ fac,
-                                                         const float2 *__restrict__ tab, float2 *__restrict__ rc,
-                                                         int np) {
-    rc_fused_body<K2, R>(ph, fac, tab, rc, np);
+__global__ void __launch_bounds__(32 * R) rc_fused_kernel(RcArgs a) {
+    a.resolve();
+    rc_fused_body<K2, R>(a.ph, a.fac, a.tab, a.rc, a.np);
 }
 
-// The same for one scene of a batch: every pointer and size from the scene's
-// slot of the device table, so a captured graph replays with new buffers.
+// ---- the same for other K <= 512: each sub-transform as a chirp convolution ----
+//
+// The length-K inverse DFT of sub-transform r, with c[k] = W_2K^(k^2) and
+// k m = (k^2 + m^2 - (m - k)^2) / 2 (Bluestein):
+//     rc[R m + r] = c[m] sum_k (y[k] W_N^{k r} c[k]) conj(c[m - k]),
+// a circular convolution of length M = 32 K2 >= 2 K - 1: forward transform,
+// product with the chirp's transform H (1/M included), inverse transform.  One
+// warp per sub-transform; both transforms are the direct kernel's four steps,
+// the first split over k = k1 + 32 k2 (K2 points in the registers of 32 lanes,
+// then 32 points in K2 lanes), the second the other way round, so it starts in
+// the registers where the first ends and two transposes do.  The upper half
+// of the input is zero (the first butterfly of the K2 points is a twiddle) and
+// the upper half of the output is not wanted.
+//
+// K = 424 (8 x 53) and the like went through a zero-padded buffer and cuFFT
+// (radix 53, or its own chirp transform of twice nfft, on data that is 7/8
+// zeros): 512 pulses of 424 samples, 8 times upsampled, 55 us with the pair
+// rows of the time, 40 without, 20 us here; 777 of 501: 96 and 79 to 31 us.
 template <int K2, int R>
-__global__ void __launch_bounds__(32 * R) rc_fused_scene_kernel(const BatchScene *__restrict__ scene,
-                                                               const float2 *__restrict__ tab) {
-    const BatchScene &S = *scene;
-    rc_fused_body<K2, R>(static_cast<const float2 *>(S.ph), static_cast<const float2 *>(S.fac), tab,
-                         static_cast<float2 *>(const_cast<void *>(S.L.rc)), S.L.np);
+struct CztTable {
+    static constexpr int M = 32 * K2, KM = M / 2;
+    static constexpr int kChirp = 0;               // c[k], k < KM
+    static constexpr int kH = KM;                  // H[u], u < M
+    static constexpr int kTwA = kH + M;            // W_M^{k1 m2} at m2 * 32 + k1
+    static constexpr int kTwB = K2 == 32 ? kTwA : kTwA + M;  // W_M^{m2 v1} at v1 * K2 + m2
+    static constexpr int kWn = kTwB + M;           // W_N^i, i < 32 R
+    static constexpr int kWnk = kWn + 32 * R;      // W_N^{32 i}, i < K2 / 2 * R
+    static constexpr int kSize = kWnk + K2 / 2 * R;
+    // row of one sub-transform: K2 x 33 for the transposes, and 16/R mod 16 as RcTable::kReg
+    static constexpr int kReg = (33 * K2 + 15) / 16 * 16 + 16 / R;
+    static constexpr size_t kSmem = (static_cast<size_t>(KM) + kSize + static_cast<size_t>(R) * kReg) * 8;
+};
+
+template <int K2, int R>
+__device__ __forceinline__ void rc_czt_body(const float2 *__restrict__ ph, const float2 *__restrict__ fac,
+                                            const float2 *__restrict__ tab, float2 *__restrict__ rc, int K, int np) {
+    using T = CztTable<K2, R>;
+    constexpr int REG = T::kReg, LOGR = log2_of<R>(), H2 = K2 / 2;
+    extern __shared__ __align__(16) float2 rc_sm[];
+    float2 *y = rc_sm, *tb = y + T::KM, *regions = tb + T::kSize;
+    const int tid = threadIdx.x, r = tid >> 5, lane = tid & 31;
+    for (int i = tid; i < T::kSize; i += 32 * R) tb[i] = tab[i];
+    for (int k = K + tid; k < T::KM; k += 32 * R) y[k] = make_float2(0.0f, 0.0f);
+    const float2 *chirp = tb + T::kChirp;
+    float2 *reg = regions + r * REG;
+    const int N = R * K;
+    // a pulse's input samples, loaded one pulse ahead as in rc_fused_body
+    constexpr int KPT = (T::KM + 32 * R - 1) / (32 * R);
+    float2 pre[KPT];
+    auto prefetch = [&](int q) {
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            const int k = tid + j * 32 * R;
+            pre[j] = (q < np && k < K) ? ph[static_cast<long long>(q) * K + k] : make_float2(0.0f, 0.0f);
+        }
+    };
+    prefetch(blockIdx.x);
+    for (int p = blockIdx.x; p < np; p += gridDim.x) {
+        __syncthreads();  // the previous pulse's reads of the regions are done; the table is staged
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+            const int k = tid + j * 32 * R;
+            if (k < K) y[k] = cmulf(cmulf(pre[j], fac[k]), chirp[k]);
+        }
+        __syncthreads();
+        {
+            // K2 points over k2 in lane k1, the upper half of the input zero
+            const float2 a = tb[T::kWn + lane * r];
+            float2 lo[H2], hi[H2];
+#pragma unroll
+            for (int k2 = 0; k2 < H2; ++k2) {
+                lo[k2] = cmulf(y[lane + 32 * k2], cmulf(a, tb[T::kWnk + k2 * r]));
+                const int e32 = k2 * (32 / K2);
+                hi[k2] = e32 == 0 ? lo[k2]
+                                  : (e32 == 8 ? make_float2(-lo[k2].y, lo[k2].x) : cmulf(lo[k2], w32(e32)));
+            }
+            ifft_dif<H2>(lo);
+            ifft_dif<H2>(hi);
+#pragma unroll
+            for (int m2 = 0; m2 < K2; ++m2) {
+                const int at = bit_reverse<K2>(m2);
+                reg[m2 * 33 + lane] = cmulf(at < H2 ? lo[at < H2 ? at : 0] : hi[at < H2 ? 0 : at - H2],
+                                            tb[T::kTwA + m2 * 32 + lane]);
+            }
+        }
+        __syncwarp();
+        float2 w[32];
+        if (lane < K2) {
+#pragma unroll
+            for (int k1 = 0; k1 < 32; ++k1) w[k1] = reg[lane * 33 + k1];
+        }
+        __syncwarp();
+        if (lane < K2) {
+            ifft_dif<32>(w);
+            // times H, conjugated: the second transform runs in the same direction
+            float2 z[32];
+#pragma unroll
+            for (int m1 = 0; m1 < 32; ++m1) {
+                const float2 x = cmulf(w[bit_reverse<32>(m1)], tb[T::kH + m1 * K2 + lane]);
+                z[m1] = make_float2(x.x, -x.y);
+            }
+            ifft_dif<32>(z);
+#pragma unroll
+            for (int v1 = 0; v1 < 32; ++v1)
+                reg[lane * 33 + v1] = cmulf(z[bit_reverse<32>(v1)], tb[T::kTwB + v1 * K2 + lane]);
+        }
+        __syncwarp();
+        float2 q[K2];
+#pragma unroll
+        for (int m2 = 0; m2 < K2; ++m2) q[m2] = reg[m2 * 33 + lane];
+        __syncwarp();
+        ifft_dif<K2>(q);
+#pragma unroll
+        for (int v2 = 0; v2 < H2; ++v2) {
+            const float2 x = q[bit_reverse<K2>(v2)];
+            reg[lane + 32 * v2] = cmulf(make_float2(x.x, -x.y), chirp[lane + 32 * v2]);
+        }
+        __syncthreads();
+        prefetch(p + gridDim.x);
+        // rc[R m + r] = regions[r][m]
+        if (R > 1) {
+            float4 *row = reinterpret_cast<float4 *>(rc + static_cast<long long>(p) * N);
+            for (int b = 2 * tid; b < N; b += 64 * R) {
+                const float2 u = regions[(b & (R - 1)) * REG + (b >> LOGR)];
+                const float2 un = regions[((b + 1) & (R - 1)) * REG + ((b + 1) >> LOGR)];
+                row[b >> 1] = make_float4(u.x, u.y, un.x, un.y);
+            }
+        } else {
+            for (int b = tid; b < N; b += 32) rc[static_cast<long long>(p) * N + b] = regions[b];
+        }
+    }
+}
+
+// registers for two CTAs of 256 threads per SM
+template <int K2, int R>
+__global__ void __launch_bounds__(32 * R, R <= 8 ? 2 : 1) rc_czt_kernel(RcArgs a) {
+    a.resolve();
+    rc_czt_body<K2, R>(a.ph, a.fac, a.tab, a.rc, a.K, a.np);
+}
+
+// x <- sum_k x[k] exp(+j 2 pi u k / M), M a power of two (double, host)
+void dft_pow2(std::vector<std::complex<double>> &x) {
+    const size_t M = x.size();
+    for (size_t i = 1, j = 0; i < M; ++i) {
+        size_t bit = M >> 1;
+        for (; j & bit; bit >>= 1) j ^= bit;
+        j ^= bit;
+        if (i < j) std::swap(x[i], x[j]);
+    }
+    for (size_t len = 2; len <= M; len <<= 1)
+        for (size_t k = 0; k < len / 2; ++k) {
+            const std::complex<double> w = std::polar(1.0, 2.0 * M_PI * static_cast<double>(k) / static_cast<double>(len));
+            for (size_t i = k; i < M; i += len) {
+                const std::complex<double> a = x[i], b = x[i + len / 2] * w;
+                x[i] = a + b;
+                x[i + len / 2] = a - b;
+            }
+        }
+}
+
+template <int K2, int R>
+void fill_czt_table(int K, std::vector<float> &t) {
+    using T = CztTable<K2, R>;
+    t.assign(2 * static_cast<size_t>(T::kSize), 0.0f);
+    auto put = [&](int at, const std::complex<double> &v) {
+        t[2 * static_cast<size_t>(at)] = static_cast<float>(v.real());
+        t[2 * static_cast<size_t>(at) + 1] = static_cast<float>(v.imag());
+    };
+    auto unit = [](double num, double den) { return std::polar(1.0, 2.0 * M_PI * num / den); };
+    std::vector<std::complex<double>> h(T::M);
+    for (int k = 0; k < K; ++k) {
+        const std::complex<double> c = unit(static_cast<double>((static_cast<long long>(k) * k) % (2 * K)), 2.0 * K);
+        put(T::kChirp + k, c);
+        h[k] = std::conj(c) / static_cast<double>(T::M);
+        if (k > 0) h[T::M - k] = h[k];
+    }
+    dft_pow2(h);
+    for (int u = 0; u < T::M; ++u) put(T::kH + u, h[u]);
+    for (int m2 = 0; m2 < K2; ++m2)
+        for (int k1 = 0; k1 < 32; ++k1) {
+            put(T::kTwA + m2 * 32 + k1, unit(static_cast<double>(k1) * m2, T::M));
+            put(T::kTwB + k1 * K2 + m2, unit(static_cast<double>(k1) * m2, T::M));
+        }
+    const double N = static_cast<double>(R) * K;
+    for (int i = 0; i < 32 * R; ++i) put(T::kWn + i, unit(i, N));
+    for (int i = 0; i < K2 / 2 * R; ++i) put(T::kWnk + i, unit(32.0 * i, N));
 }
 
 template <int K2, int R>
@@ -261,19 +456,6 @@ void fill_rc_table(std::vector<float> &t) {
         for (int k1 = 0; k1 < 32; ++k1) put(T::kTwk + m2 * 32 + k1, static_cast<double>(k1) * m2, T::K);
     for (int i = 0; i < 32 * R; ++i) put(T::kWn + i, i, T::N);
     for (int i = 0; i < T::NW; ++i) put(T::kWnr + i, i, T::NW);
-}
-
-template <int K2, int R>
-cudaError_t launch_fused(const float2 *ph, const float2 *fac, const float2 *tab, float2 *rc, int np, int grid,
-                         cudaStream_t s) {
-    using T = RcTable<K2, R>;
-    auto kern = rc_fused_kernel<K2, R>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(T::kSmem));
-    if (e != cudaSuccess) return e;
-    const int g = np < grid ? np : grid;
-    kern<<<g > 0 ? g : 1, 32 * R, T::kSmem, s>>>(ph, fac, tab, rc, np);
-    return cudaGetLastError();
 }
 
 int grid_for(long long total) {
@@ -304,48 +486,92 @@ cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStre
     return cudaGetLastError();
 }
 
+// (K2, R) of the direct kernels (K = 32 K2) and of the chirp kernels (K <= 16
+// K2, the upsampling factors in use).
 #define SARBP_RC_SHAPES(X) \
     X(8, 1) X(8, 2) X(8, 4) X(8, 8) X(8, 16) X(16, 1) X(16, 2) X(16, 4) X(16, 8) X(16, 16) X(32, 1) X(32, 2) \
         X(32, 4) X(32, 8) X(32, 16)
+#define SARBP_CZT_SHAPES(X) X(32, 4) X(32, 8)
 
-bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table) {
-#define SARBP_RC_CASE(K2_, R_)                                        \
-    if (K == 32 * K2_ && R == R_) {                                   \
-        if (smem) *smem = RcTable<K2_, R_>::kSmem;                    \
-        if (table) fill_rc_table<K2_, R_>(*table);                    \
-        return true;                                                  \
+namespace {
+
+// Calls f(kernel, shared memory, table filler) of shape (K, R); false when
+// there is none.
+template <typename F>
+bool with_rc_shape(int K, int R, F f) {
+#define SARBP_RC_CASE(K2_, R_)                                                             \
+    if (K == 32 * K2_ && R == R_) {                                                        \
+        f(rc_fused_kernel<K2_, R_>, RcTable<K2_, R_>::kSmem,                               \
+          [](int, std::vector<float> &t) { fill_rc_table<K2_, R_>(t); });                  \
+        return true;                                                                       \
     }
     SARBP_RC_SHAPES(SARBP_RC_CASE)
+#undef SARBP_RC_CASE
+    // Chirp kernels where cuFFT has a long prime factor to work through; where
+    // all are small its padded transform is the faster one (2048 pulses, 8
+    // times upsampled, chirp against cuFFT and taper: K = 424 (53) 59 / 133 us,
+    // 509 62 / 176, 201 (67) 46 / 72, but 500 (5) 62 / 42, 247 (19) 47 / 44,
+    // 131 45 / 36).
+    int prime = 1;
+    for (int f = 2, left = K; left > 1; ++f)
+        for (; left % f == 0; left /= f) prime = f;
+    const int k2 = K <= 512 && ((K > 256 && prime >= 17) || (K > 192 && prime >= 53)) ? 32 : 0;
+#define SARBP_RC_CASE(K2_, R_)                                                             \
+    if (k2 == K2_ && R == R_) {                                                            \
+        f(rc_czt_kernel<K2_, R_>, CztTable<K2_, R_>::kSmem,                                \
+          [](int k, std::vector<float> &t) { fill_czt_table<K2_, R_>(k, t); });            \
+        return true;                                                                       \
+    }
+    SARBP_CZT_SHAPES(SARBP_RC_CASE)
 #undef SARBP_RC_CASE
     return false;
 }
 
+cudaError_t launch_rc(const RcArgs &a, int K, int R, int grid, cudaStream_t s) {
+    cudaError_t e = cudaErrorInvalidValue;
+    with_rc_shape(K, R, [&](auto kern, size_t bytes, auto) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+        if (e != cudaSuccess) return;
+        kern<<<grid > 0 ? grid : 1, 32 * R, bytes, s>>>(a);
+        e = cudaGetLastError();
+    });
+    return e;
+}
+
+}  // namespace
+
+bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table) {
+    return with_rc_shape(K, R, [&](auto, size_t bytes, auto fill) {
+        if (smem) *smem = bytes;
+        if (table) fill(K, *table);
+    });
+}
+
+bool rc_direct_shape(int K) { return K == 256 || K == 512 || K == 1024; }
+
+int rc_fused_resident(int K, int R) {
+    int occ = 0;
+    with_rc_shape(K, R, [&](auto kern, size_t bytes, auto) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * R, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            occ = 0;
+        }
+    });
+    return occ;
+}
+
 cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
                             int grid, cudaStream_t s) {
-#define SARBP_RC_CASE(K2_, R_)                                                                                   \
-    if (K == 32 * K2_ && R == R_)                                                                                 \
-        return launch_fused<K2_, R_>(static_cast<const float2 *>(ph), static_cast<const float2 *>(fac),          \
-                                     static_cast<const float2 *>(table), static_cast<float2 *>(rc), np, grid, s);
-    SARBP_RC_SHAPES(SARBP_RC_CASE)
-#undef SARBP_RC_CASE
-    return cudaErrorInvalidValue;
+    const RcArgs a{nullptr, static_cast<const float2 *>(ph), static_cast<const float2 *>(fac),
+                   static_cast<const float2 *>(table), static_cast<float2 *>(rc), K, np};
+    return launch_rc(a, K, R, np < grid ? np : grid, s);
 }
 
 cudaError_t launch_rc_fused_scene(const BatchScene *scene, const void *table, int K, int R, int grid,
                                   cudaStream_t s) {
-#define SARBP_RC_CASE(K2_, R_)                                                                                   \
-    if (K == 32 * K2_ && R == R_) {                                                                               \
-        auto kern = rc_fused_scene_kernel<K2_, R_>;                                                               \
-        const size_t smem = RcTable<K2_, R_>::kSmem;                                                              \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                             static_cast<int>(smem));                                             \
-        if (e != cudaSuccess) return e;                                                                           \
-        kern<<<grid > 0 ? grid : 1, 32 * R_, smem, s>>>(scene, static_cast<const float2 *>(table));               \
-        return cudaGetLastError();                                                                                \
-    }
-    SARBP_RC_SHAPES(SARBP_RC_CASE)
-#undef SARBP_RC_CASE
-    return cudaErrorInvalidValue;
+    return launch_rc(RcArgs{scene, nullptr, nullptr, static_cast<const float2 *>(table), nullptr, 0, 0}, K, R, grid, s);
 }
 
 }  // namespace sarbp
