@@ -66,3 +66,15 @@ def test_matched_filter_and_backprojection_agree(F):
         mf = plan.matched_filter(*args(sc))
         bp = plan.focus(*args(sc))
     assert O.rel_l2(bp * sc.nfft, mf) < 0.03
+
+
+@pytest.mark.parametrize("K,Np,nx,ny", [(2, 2, 1, 1), (127, 9, 11, 13), (128, 65, 16, 8), (129, 130, 40, 33), (300, 7, 90, 101)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-9), ("mixed", 1e-4)])
+def test_matched_filter_block_edges(F, K, Np, nx, ny, precision, tol):
+    """Sample counts around the staged chunk, pulse counts around the warps
+    and CTAs that share them, images that end inside a pixel block."""
+    sc = scene(K=K, Np=Np, nfft=8 * K)
+    sc.grid = S.Grid(nx=nx, ny=ny, wx=0.05 * (nx - 1), wy=0.05 * (ny - 1), x0=0.1, y0=-0.2)
+    with F.Plan.for_scene(sc, precision) as plan:
+        got = plan.matched_filter(*args(sc))
+    assert O.rel_l2(got, O.mf_fp64(sc)) < tol

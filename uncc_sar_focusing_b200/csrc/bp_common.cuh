@@ -103,6 +103,50 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uin
 
 __device__ __forceinline__ double frac_rev(double x) { return x - rint(x); }
 
+// Square root of a positive, normal s as sqrt() rounds it: with g ~ sqrt(s)
+// and h ~ 1 / (2 sqrt(s)) from the reciprocal-root estimate (2^-20 or
+// better), r = 1/2 - g h corrects both to 2^-39, and the residual s - g^2,
+// exact by fused multiply-add, corrects g once more (Markstein's scheme).
+__device__ __forceinline__ double sqrt_rn(double s) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    double g = s * y;
+    double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));  // y / 2
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, s), h, g);
+}
+
+// exp(+j 2 pi ph), |ph| < 2^50: ph = n/4 + r exactly, |r| <= 1/8; sin and cos
+// of 2 pi r as polynomials in r^2 (interpolated at the Chebyshev nodes of [0,
+// 1/64] in 60 digits; errors 2e-17 and 5e-17 before rounding), then the
+// quadrant n mod 4 by swap and sign.
+__device__ __forceinline__ void rotation(double ph, double &cs, double &sn) {
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    const double t = fma(ph, 4.0, kMagic);
+    const int q = __double2loint(t);
+    const double r = fma(t - kMagic, -0.25, ph);
+    const double z = r * r;
+    double S = 3.7808689593022957, C = 7.810290968144191;
+    S = fma(S, z, -15.093804209987114);
+    C = fma(C, z, -26.42425703488269);
+    S = fma(S, z, 42.058685020160894);
+    C = fma(C, z, 60.24462008593029);
+    S = fma(S, z, -76.70585970427454);
+    C = fma(C, z, -85.45681709034115);
+    S = fma(S, z, 81.60524927594804);
+    C = fma(C, z, 64.93939402236538);
+    S = fma(S, z, -41.341702240399634);
+    C = fma(C, z, -19.73920880217842);
+    S = r * fma(S, z, 6.283185307179586);
+    C = fma(C, z, 1.0);
+    const bool odd = q & 1;
+    const double c = odd ? S : C, s = odd ? C : S;
+    cs = __hiloint2double(__double2hiint(c) ^ (((q + 1) << 30) & 0x80000000), __double2loint(c));
+    sn = __hiloint2double(__double2hiint(s) ^ ((q << 30) & 0x80000000), __double2loint(s));
+}
+
 // Flags of a PulseGeo record
 enum : int {
     PG_ACTIVE = 1,  // the tile's window meets the valid range bins
