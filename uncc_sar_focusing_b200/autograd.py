@@ -19,7 +19,7 @@ torch operations.  The reference's own focus metric is a non-differentiable
 """
 from __future__ import annotations
 
-import ctypes
+import contextlib
 
 import torch
 
@@ -30,7 +30,7 @@ from .focusing import Plan
 class _Backproject(torch.autograd.Function):
     @staticmethod
     def forward(ctx, plan: Plan, ant_x, ant_y, ant_z, slant_range, start_freq):
-        img = plan.backproject(ant_x, ant_y, ant_z, slant_range, start_freq, out=plan.new_image(ant_x.device))
+        img = plan.backproject(ant_x, ant_y, ant_z, slant_range, start_freq, out=plan._out_image(ant_x.device))
         ctx.plan = plan
         ctx.save_for_backward(ant_x, ant_y, ant_z, slant_range, start_freq)
         return img
@@ -55,13 +55,12 @@ class _Entropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img):
         x = img.contiguous()
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             work = torch.empty(N.lib().sarbp_image_entropy_work_bytes() // 8, dtype=torch.float64, device=x.device)
             e = torch.empty((), dtype=torch.float32, device=x.device)
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-            N.check(N.lib().sarbp_image_entropy(ctypes.c_void_p(x.data_ptr()), x.numel(),
-                                                ctypes.c_void_p(work.data_ptr()), ctypes.c_void_p(e.data_ptr()),
-                                                ctypes.c_void_p(stream)), "sarbp_image_entropy")
+            N.check(N.lib().sarbp_image_entropy(x.data_ptr(), x.numel(), work.data_ptr(), e.data_ptr(),
+                                                torch.cuda.current_stream(x.device).cuda_stream),
+                    "sarbp_image_entropy")
         ctx.save_for_backward(x, work)
         ctx.shape = img.shape
         return e
@@ -69,15 +68,21 @@ class _Entropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_e):
         x, work = ctx.saved_tensors
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             g = grad_e.detach().to(device=x.device, dtype=torch.float32).contiguous()
             grad = torch.empty_like(x)
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-            N.check(N.lib().sarbp_image_entropy_grad(ctypes.c_void_p(x.data_ptr()), x.numel(),
-                                                     ctypes.c_void_p(work.data_ptr()), ctypes.c_void_p(g.data_ptr()),
-                                                     ctypes.c_void_p(grad.data_ptr()), ctypes.c_void_p(stream)),
+            N.check(N.lib().sarbp_image_entropy_grad(x.data_ptr(), x.numel(), work.data_ptr(), g.data_ptr(),
+                                                     grad.data_ptr(), torch.cuda.current_stream(x.device).cuda_stream),
                     "sarbp_image_entropy_grad")
         return grad.reshape(ctx.shape)
+
+
+def _on(device):
+    """`device` current for a block; nothing to do when it already is."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+_HERE = contextlib.nullcontext()
 
 
 def image_entropy(img: torch.Tensor) -> torch.Tensor:

@@ -38,7 +38,7 @@ struct sarbp_batch {
     std::vector<void *> rctab;     // per scene: fused range-compression table (null: cuFFT path)
     std::vector<int> rc_R;         // per scene: nfft / K of the fused path
     std::vector<void *> rc_tables; // the distinct tables (one per (K, R))
-    int rc_grid = 0;
+    int rc_sms = 0;                // SMs
     // tile shape and the per-scene windows it implies
     TileConfig tile{0, 0};
     size_t smem = 0;
@@ -298,12 +298,22 @@ int enqueue(sarbp_batch *b, cudaStream_t s) {
     bool any_fft = false;
     for (int i = 0; i < n; ++i) any_fft = any_fft || !b->rctab[i];
     if (any_fft) SARBP_TRY_CUDA(launch_rc_prep_batch(b->d_table, n, s));
-    for (int i = 0; i < n; ++i) {
-        if (b->rctab[i]) {
-            SARBP_TRY_CUDA(launch_rc_fused_scene(b->d_table + i, b->rctab[i], b->desc[i].num_range_samples,
-                                                 b->rc_R[i], b->rc_grid, s));
-            continue;
+    // the scenes of each (K, R) together in one launch
+    for (void *tab : b->rc_tables) {
+        std::vector<unsigned short> idx;
+        for (int i = 0; i < n; ++i)
+            if (b->rctab[i] == tab) idx.push_back(static_cast<unsigned short>(i));
+        const int K = b->desc[idx[0]].num_range_samples, R = b->rc_R[idx[0]];
+        const int per_sm = rc_fused_resident(K, R);
+        for (size_t i = 0; i < idx.size(); i += kRcGroup) {
+            const int m = static_cast<int>(idx.size() - i < kRcGroup ? idx.size() - i : kRcGroup);
+            // two waves of the resident CTAs over the group's scenes
+            const int grid = (2 * b->rc_sms * (per_sm > 0 ? per_sm : 1) + m - 1) / m;
+            SARBP_TRY_CUDA(launch_rc_fused_scenes(b->d_table, idx.data() + i, m, tab, K, R, grid, s));
         }
+    }
+    for (int i = 0; i < n; ++i) {
+        if (b->rctab[i]) continue;
         const cufftResult r0 = cufftSetStream(b->fft[i], s);
         if (r0 != CUFFT_SUCCESS) return from_cufft(r0);
         cufftComplex *rc = static_cast<cufftComplex *>(b->d_rc[i]) + b->margin[i];
@@ -421,7 +431,7 @@ int sarbp_batch_create(const sarbp_plan_desc *descs, int num_scenes, sarbp_batch
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
-    b->rc_grid = 2 * (sms > 0 ? sms : 148);
+    b->rc_sms = sms > 0 ? sms : 148;
     std::vector<std::pair<long long, void *>> tab_of;  // key K * 64 + R
     for (int i = 0; i < n && st == SARBP_OK; ++i) {
         const sarbp_plan_desc &d = descs[i];

@@ -231,21 +231,24 @@ __device__ __forceinline__ void rc_fused_body(const float2 *__restrict__ ph, con
     }
 }
 
-// scene: null, or one scene of a batch whose slot of the device table holds
-// every pointer and size (a captured graph replays with new buffers).
+// One aperture, or (scenes non-null) scenes idx[blockIdx.y] of a batch, whose
+// slots of the device table hold every pointer and size (a captured graph
+// replays with new buffers).  blockIdx.x: the aperture's CTAs.
 struct RcArgs {
-    const BatchScene *scene;
+    const BatchScene *scenes;
     const float2 *ph, *fac, *tab;
     float2 *rc;
     int K, np;
+    unsigned short idx[kRcGroup];
 
     __device__ __forceinline__ void resolve() {
-        if (!scene) return;
-        ph = static_cast<const float2 *>(scene->ph);
-        fac = static_cast<const float2 *>(scene->fac);
-        rc = static_cast<float2 *>(const_cast<void *>(scene->L.rc));
-        K = scene->K;
-        np = scene->L.np;
+        if (!scenes) return;
+        const BatchScene &S = scenes[idx[blockIdx.y]];
+        ph = static_cast<const float2 *>(S.ph);
+        fac = static_cast<const float2 *>(S.fac);
+        rc = static_cast<float2 *>(const_cast<void *>(S.L.rc));
+        K = S.K;
+        np = S.L.np;
     }
 };
 
@@ -527,12 +530,12 @@ bool with_rc_shape(int K, int R, F f) {
     return false;
 }
 
-cudaError_t launch_rc(const RcArgs &a, int K, int R, int grid, cudaStream_t s) {
+cudaError_t launch_rc(const RcArgs &a, int K, int R, dim3 grid, cudaStream_t s) {
     cudaError_t e = cudaErrorInvalidValue;
     with_rc_shape(K, R, [&](auto kern, size_t bytes, auto) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
         if (e != cudaSuccess) return;
-        kern<<<grid > 0 ? grid : 1, 32 * R, bytes, s>>>(a);
+        kern<<<grid, 32 * R, bytes, s>>>(a);
         e = cudaGetLastError();
     });
     return e;
@@ -565,13 +568,17 @@ int rc_fused_resident(int K, int R) {
 cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
                             int grid, cudaStream_t s) {
     const RcArgs a{nullptr, static_cast<const float2 *>(ph), static_cast<const float2 *>(fac),
-                   static_cast<const float2 *>(table), static_cast<float2 *>(rc), K, np};
-    return launch_rc(a, K, R, np < grid ? np : grid, s);
+                   static_cast<const float2 *>(table), static_cast<float2 *>(rc), K, np, {}};
+    const int g = np < grid ? np : grid;
+    return launch_rc(a, K, R, dim3(static_cast<unsigned>(g > 0 ? g : 1)), s);
 }
 
-cudaError_t launch_rc_fused_scene(const BatchScene *scene, const void *table, int K, int R, int grid,
-                                  cudaStream_t s) {
-    return launch_rc(RcArgs{scene, nullptr, nullptr, static_cast<const float2 *>(table), nullptr, 0, 0}, K, R, grid, s);
+cudaError_t launch_rc_fused_scenes(const BatchScene *scenes, const unsigned short *idx, int n, const void *table, int K,
+                                   int R, int grid, cudaStream_t s) {
+    if (n < 1 || n > kRcGroup) return cudaErrorInvalidValue;
+    RcArgs a{scenes, nullptr, nullptr, static_cast<const float2 *>(table), nullptr, 0, 0, {}};
+    for (int i = 0; i < n; ++i) a.idx[i] = idx[i];
+    return launch_rc(a, K, R, dim3(static_cast<unsigned>(grid > 0 ? grid : 1), static_cast<unsigned>(n)), s);
 }
 
 }  // namespace sarbp

@@ -145,10 +145,12 @@ bool rc_direct_shape(int K);
 int rc_fused_resident(int K, int R);
 cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
                             int grid, cudaStream_t s);
-// Fused range compression of one batch scene, parameters read from its table
-// slot (grid CTAs loop over the scene's pulses).
-cudaError_t launch_rc_fused_scene(const BatchScene *scene, const void *table, int K, int R, int grid,
-                                  cudaStream_t s);
+// Fused range compression of n <= kRcGroup scenes of one (K, R) of a batch in
+// one launch, parameters read from their table slots: grid CTAs per scene loop
+// over its pulses.
+constexpr int kRcGroup = 64;
+cudaError_t launch_rc_fused_scenes(const BatchScene *scenes, const unsigned short *idx, int n, const void *table, int K,
+                                   int R, int grid, cudaStream_t s);
 
 }  // namespace sarbp
 

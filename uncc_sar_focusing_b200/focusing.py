@@ -10,6 +10,7 @@ happens in libsarbp.so.
 from __future__ import annotations
 
 import ctypes
+import sys
 from typing import Optional
 
 import numpy as np
@@ -21,35 +22,46 @@ _PRECISION = {"mixed": N.PRECISION_MIXED, "fp64": N.PRECISION_FP64}
 _WINDOW = {None: N.WINDOW_NONE, "none": N.WINDOW_NONE, "hamming": N.WINDOW_HAMMING, "taylor": N.WINDOW_TAYLOR}
 
 
+_ITEM = {np.float64: 0, np.complex64: 1, np.complex128: 2}
+
+
+def _torch():
+    """The torch module if the caller's program has loaded it (a tensor can
+    only come from there), else None."""
+    return sys.modules.get("torch")
+
+
 def _is_torch(x) -> bool:
-    return type(x).__module__.startswith("torch")
+    t = _torch()
+    return t is not None and isinstance(x, t.Tensor)
 
 
 def _ptr(x, dtype, count: Optional[int] = None):
     """(pointer, memory kind, keep-alive) of a numpy array or CUDA tensor."""
-    if _is_torch(x):
-        import torch
-
-        want = {np.float64: torch.float64, np.complex64: torch.complex64, np.complex128: torch.complex128}[dtype]
+    t = _torch()
+    if t is not None and isinstance(x, t.Tensor):
+        want = (t.float64, t.complex64, t.complex128)[_ITEM[dtype]]
         if not x.is_cuda:
             raise ValueError("torch tensors passed to the engine must live on a CUDA device")
-        if x.dtype != want or not x.is_contiguous():
+        if x.dtype is not want or not x.is_contiguous():
             raise ValueError(f"expected a contiguous {want} tensor, got {x.dtype}")
         if count is not None and x.numel() < count:
             raise ValueError(f"tensor has {x.numel()} elements, need {count}")
-        return ctypes.c_void_p(x.data_ptr()), N.MEMORY_DEVICE, x
+        return x.data_ptr(), N.MEMORY_DEVICE, x
     a = np.ascontiguousarray(x, dtype=dtype)
     if count is not None and a.size < count:
         raise ValueError(f"array has {a.size} elements, need {count}")
-    return ctypes.c_void_p(a.ctypes.data), N.MEMORY_HOST, a
+    return a.ctypes.data, N.MEMORY_HOST, a
 
 
 def _stream(*arrays):
-    if any(_is_torch(a) for a in arrays):
-        import torch
-
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    return ctypes.c_void_p(0)
+    """Torch's current stream when an array is a CUDA tensor, else the default stream."""
+    t = _torch()
+    if t is not None:
+        for a in arrays:
+            if isinstance(a, t.Tensor):
+                return t.cuda.current_stream().cuda_stream
+    return 0
 
 
 class Plan:
@@ -64,6 +76,7 @@ class Plan:
         self.grid = grid
         self.precision = precision
         self.image_dtype = np.complex128 if precision == "fp64" else np.complex64
+        self._npix = grid.npix
         d = N.PlanDesc()
         d.num_range_samples = self.K
         d.num_pulses = self.np_cap
@@ -126,6 +139,16 @@ class Plan:
         dt = torch.complex128 if self.precision == "fp64" else torch.complex64
         return torch.zeros(self.image_shape(), dtype=dt, device=device)
 
+    def _out_image(self, device=None, lead=()):
+        """Images that a call without accumulation writes every pixel of (no
+        fill): a numpy array, or a tensor on `device`."""
+        shape = (*lead, *self.image_shape())
+        if device is None:
+            return np.empty(shape, dtype=self.image_dtype)
+        import torch
+
+        return torch.empty(shape, dtype=torch.complex128 if self.precision == "fp64" else torch.complex64, device=device)
+
     # -- entry points -------------------------------------------------------
     def set_range_weights(self, weights) -> None:
         """Complex per-sample range weights (a taper, a range reference
@@ -159,18 +182,19 @@ class Plan:
     def _geometry(self, ant_x, ant_y, ant_z, slant_range, start_freq):
         n = int(ant_x.shape[0])
         ptrs = [_ptr(v, np.float64, n) for v in (ant_x, ant_y, ant_z, slant_range, start_freq)]
-        mems = {m for _, m, _ in ptrs}
-        if len(mems) != 1:
+        mem = ptrs[0][1]
+        if any(p[1] != mem for p in ptrs):
             raise ValueError("geometry arrays must all be host arrays or all CUDA tensors")
-        g = N.Geometry(ptrs[0][0], ptrs[1][0], ptrs[2][0], ptrs[3][0], ptrs[4][0], n, mems.pop())
-        return g, [k for _, _, k in ptrs]
+        g = N.Geometry(ptrs[0][0], ptrs[1][0], ptrs[2][0], ptrs[3][0], ptrs[4][0], n, mem)
+        return g, [p[2] for p in ptrs]
 
     def backproject(self, ant_x, ant_y, ant_z, slant_range, start_freq, out=None, accumulate: bool = False,
                     checked: bool = False):
         geo, keep = self._geometry(ant_x, ant_y, ant_z, slant_range, start_freq)
         if out is None:
-            out = self.new_image(None if geo.memory == N.MEMORY_HOST else "cuda")
-        ip, imem, ikeep = _ptr(out, self.image_dtype, int(np.prod(self.image_shape())))
+            dev = None if geo.memory == N.MEMORY_HOST else "cuda"
+            out = self.new_image(dev) if accumulate else self._out_image(dev)
+        ip, imem, ikeep = _ptr(out, self.image_dtype, self._npix)
         flags = (N.ACCUMULATE if accumulate else 0) | (N.CHECKED if checked else 0)
         st = N.lib().sarbp_backproject(self._h, ctypes.byref(geo), ip, imem, flags,
                                        _stream(out, ant_x))
@@ -191,13 +215,14 @@ class Plan:
             raise ValueError("geometry arrays must all be host arrays or all CUDA tensors")
         geo = N.Geometry(ptrs[0][0], ptrs[1][0], ptrs[2][0], ptrs[3][0], ptrs[4][0], n, mems.pop())
         shape = (H,) + tuple(self.image_shape())
-        if out is None:
-            if geo.memory == N.MEMORY_HOST:
-                out = np.zeros(shape, dtype=np.complex64)
-            else:
-                import torch
+        if out is None and not accumulate:
+            out = self._out_image(None if geo.memory == N.MEMORY_HOST else ant_x.device, (H,))
+        elif out is None and geo.memory == N.MEMORY_HOST:
+            out = np.zeros(shape, dtype=np.complex64)
+        elif out is None:
+            import torch
 
-                out = torch.zeros(shape, dtype=torch.complex64, device=ant_x.device)
+            out = torch.zeros(shape, dtype=torch.complex64, device=ant_x.device)
         ip, imem, ikeep = _ptr(out, np.complex64, int(np.prod(shape)))
         st = N.lib().sarbp_backproject_hypotheses(self._h, ctypes.byref(geo), H, ip, imem,
                                                   N.ACCUMULATE if accumulate else 0, _stream(out, ant_x))
@@ -211,18 +236,19 @@ class Plan:
         real loss L whose image gradient is grad_image = dL/dRe + j dL/dIm
         (sarbp_backproject_adjoint, on the plan's current range profiles)."""
         geo, keep = self._geometry(ant_x, ant_y, ant_z, slant_range, start_freq)
-        gp, gmem, gkeep = _ptr(grad_image, np.complex64, int(np.prod(self.image_shape())))
+        gp, gmem, gkeep = _ptr(grad_image, np.complex64, self._npix)
         n = geo.num_pulses
         if gmem == N.MEMORY_DEVICE:
             import torch
 
-            gant = torch.zeros((3, n), dtype=torch.float64, device=grad_image.device)
-            gr0 = torch.zeros(n, dtype=torch.float64, device=grad_image.device)
-            optr = (ctypes.c_void_p(gant.data_ptr()), ctypes.c_void_p(gr0.data_ptr()))
+            make = torch.zeros if accumulate else torch.empty  # else every value is written
+            gant = make((3, n), dtype=torch.float64, device=grad_image.device)
+            gr0 = make(n, dtype=torch.float64, device=grad_image.device)
+            optr = (gant.data_ptr(), gr0.data_ptr())
         else:
             gant = np.zeros((3, n), dtype=np.float64)
             gr0 = np.zeros(n, dtype=np.float64)
-            optr = (ctypes.c_void_p(gant.ctypes.data), ctypes.c_void_p(gr0.ctypes.data))
+            optr = (gant.ctypes.data, gr0.ctypes.data)
         st = N.lib().sarbp_backproject_adjoint(self._h, ctypes.byref(geo), gp, gmem, optr[0], optr[1], gmem,
                                                N.ACCUMULATE if accumulate else 0, _stream(grad_image, ant_x))
         N.check(st, "sarbp_backproject_adjoint")
@@ -235,8 +261,8 @@ class Plan:
         pp, pmem, pkeep = _ptr(phase_history, np.complex64, geo.num_pulses * self.K)
         ap = N.Aperture(pp, pmem, geo)
         if out is None:
-            out = self.new_image(None if pmem == N.MEMORY_HOST and geo.memory == N.MEMORY_HOST else "cuda")
-        ip, imem, ikeep = _ptr(out, self.image_dtype, int(np.prod(self.image_shape())))
+            out = self._out_image(None if pmem == N.MEMORY_HOST and geo.memory == N.MEMORY_HOST else "cuda")
+        ip, imem, ikeep = _ptr(out, self.image_dtype, self._npix)
         st = N.lib().sarbp_focus(self._h, ctypes.byref(ap), ip, imem, _stream(out, phase_history, ant_x))
         N.check(st, "sarbp_focus")
         self.num_pulses_ready = geo.num_pulses
@@ -296,8 +322,8 @@ class Plan:
         pp, pmem, pkeep = _ptr(phase_history, np.complex64, geo.num_pulses * self.K)
         ap = N.Aperture(pp, pmem, geo)
         if out is None:
-            out = self.new_image(None if pmem == N.MEMORY_HOST and geo.memory == N.MEMORY_HOST else "cuda")
-        ip, imem, ikeep = _ptr(out, self.image_dtype, int(np.prod(self.image_shape())))
+            out = self._out_image(None if pmem == N.MEMORY_HOST and geo.memory == N.MEMORY_HOST else "cuda")
+        ip, imem, ikeep = _ptr(out, self.image_dtype, self._npix)
         st = N.lib().sarbp_matched_filter(self._h, ctypes.byref(ap), ip, imem, _stream(out, phase_history, ant_x))
         N.check(st, "sarbp_matched_filter")
         if imem == N.MEMORY_HOST and ikeep is not out:
