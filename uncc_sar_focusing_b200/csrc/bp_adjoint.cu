@@ -45,7 +45,7 @@
 // shared-memory wavefronts a pixel-pulse instead of 5.8 whenever the look
 // direction lay along the columns).  2048 pulses x 1024^2 pixels, look
 // direction 0 / 45 / 90 degrees from the rows: 2.00 / 2.41 / 2.26 ms before,
-// 2.00 / 2.02 / 2.07 ms now.  The 32 registers of the pixels' |G| and psi
+// 1.93 / 1.94 / 1.92 ms now.  The 32 registers of the pixels' |G| and psi
 // leave the 96-register budget of 20 warps short: 3 of the instructions are
 // moves that a 142-register build (10 warps, 2.39 ms) does not need.
 #include <algorithm>
@@ -226,7 +226,6 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
         constexpr int NQ = Producers<PB>::kPulses;
         const int q0 = (warp - kWarps) * NQ;  // this warp's pulses of each stage
         const float lam = static_cast<float>(L.lambda), inv_lam = static_cast<float>(1.0 / L.lambda);
-        const float dx = static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
         auto finish = [&](int s, const UnitCursor &u) {
             const int p = u.b * PB + q0 + lane;
             if (lane < NQ && p < L.np) {
@@ -240,6 +239,10 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
                         const float4 a = r[2 * c], b = r[2 * c + 1];
                         t[c] = ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
                     }
+                    // exchanged tile: the record's x, y and the sums' i, j are
+                    // the image's y, x
+                    const bool ex = g.flags & PG_EXCHANGED;
+                    const float dx = static_cast<float>(ex ? L.dy : L.dx), dy = static_cast<float>(ex ? L.dx : L.dy);
                     // sum s u_q = u (E0 + Et/Rc) - (dx Ei, dy Ej, 0)/Rc, times
                     // lambda; dL/dR0 = -lambda E0
                     const float Et = (g.flags & PG_NEAR) ? t[3] : fmaf(g.tx, t[1], g.ty * t[2]);
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
                     out.y = lam * fmaf(g.uy, c, -dy * t[2] * g.rinv);
                     out.z = lam * g.uz * c;
                     out.w = -lam * t[0];
+                    if (ex) out = make_float4(out.y, out.x, out.z, out.w);
                 }
                 partials[tile_of(u) * L.np + p] = out;
             }
@@ -288,14 +292,15 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
     // the tile's upstream gradient as -psi and |G| per pixel pair
     float2 npsi[MX], gm[MX];
     auto load_tile = [&]() {
-        const int tx0 = cur.tx * TX + M::row0(warp, lane), ty0 = cur.ty * kTY + col;
+        const bool ex = MX == 8 && record_exchanged(L, tile_of(cur));
 #pragma unroll
         for (int k = 0; k < MX; ++k) {
-            const int row = tx0 + M::kStep * k;
+            const int mi = M::row0(warp, lane) + M::kStep * k;
             float ps[2], mg[2];
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
-                const int c = ty0 + (kTY / 2) * l;
+                const int mj = col + (kTY / 2) * l;
+                const int row = cur.tx * TX + (ex ? mj : mi), c = cur.ty * kTY + (ex ? mi : mj);
                 const float2 q = (row < L.nx && c < L.ny)
                                      ? grad[(static_cast<long long>(cur.iz) * L.nx + row) * L.ny + c]
                                      : make_float2(0.0f, 0.0f);

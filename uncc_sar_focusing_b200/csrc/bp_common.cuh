@@ -152,6 +152,7 @@ enum : int {
     PG_ACTIVE = 1,  // the tile's window meets the valid range bins
     PG_GATE = 2,    // some pixels may fall outside (0, nfft-1): test each
     PG_NEAR = 4,    // tile too large for the far-field expansion: exact path
+    PG_EXCHANGED = 8,  // x and y of the record are the image's columns and rows (tile_exchanged)
 };
 
 // Geometry of one pulse relative to one pixel tile (mixed-precision kernel).

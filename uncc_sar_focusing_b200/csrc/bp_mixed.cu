@@ -29,17 +29,18 @@
 //    result bits also form the shared-memory address (near-field pulses add
 //    the exact sqrt form of the remainder per pixel);
 //  * the 8 lanes of a shared-memory wavefront are a 2 x 4 pixel patch
-//    (PixelMap), so their 16-byte gathers rarely collide;
+//    (PixelMap), laid across the look direction (tile_exchanged), so their
+//    16-byte gathers rarely collide;
 //  * MX = 8 (64 x 64-pixel tiles) by default: the per-(tile, pulse) and
 //    per-(thread, pulse) work is spread over 16 pixels per thread.
 //
-// What bounds it (1024^2 pixels x 2048 pulses, 8 km, look direction along the
-// rows / the columns, ncu): 16.0 warp instructions per warp-pixel-pulse at 65%
-// of issue slots, shared memory's data pipe 80-88% busy (5.1-6.1 wavefronts, 4
-// of them the 16-byte gather's floor), MUFU 65%, 20 warps per SM.  With rows
-// interleaved over the warps, a row of 32 lanes and an evaluation of the range
-// remainder per pixel it took 18.0 instructions and 1.70 / 2.29 / 2.13 ms at 0
-// / 45 / 90 degrees, this 1.47 / 1.48 / 1.62 ms.
+// What bounds it (1024^2 pixels x 2048 pulses, 8 km, ncu): 16.0 warp
+// instructions per warp-pixel-pulse at 65% of issue slots, shared memory's data
+// pipe 80% busy (5.1 wavefronts, 4 of them the 16-byte gather's floor), MUFU
+// 65%, 20 warps per SM.  With rows interleaved over the warps, a row of 32
+// lanes and an evaluation of the range remainder per pixel it took 18.0
+// instructions and 1.70 / 2.29 / 2.13 ms at look directions 0 / 45 / 90
+// degrees from the rows, this 1.48 / 1.49 / 1.48 ms.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -159,18 +160,19 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
 
 // Store (or add, L.accumulate) a thread's pixel pair k of the tile at (tx0,
 // ty0, slice zz) into the complex64 image (PixelMap: every store of a warp is
-// 16 consecutive pixels, 128 bytes, of each of two rows).  v: re, im of the
+// 16 consecutive pixels, 128 bytes, of each of two rows; in an exchanged tile
+// 2 pixels of each of 16 rows, once per tile).  v: re, im of the
 // first column, re, im of the second.
 template <int MX>
-__device__ __forceinline__ void store_pair(const BpLaunch &L, int tx0, int ty0, int zz, int warp, int lane, int k,
-                                           const float4 &v) {
+__device__ __forceinline__ void store_pair(const BpLaunch &L, int tx0, int ty0, int zz, bool exchanged, int warp,
+                                           int lane, int k, const float4 &v) {
     float2 *img = static_cast<float2 *>(L.img);
-    const int row = tx0 + PixelMap<MX>::row0(warp, lane) + PixelMap<MX>::kStep * k;
-    if (row >= L.nx) return;
+    const int i = PixelMap<MX>::row0(warp, lane) + PixelMap<MX>::kStep * k;
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
-        const int col = ty0 + PixelMap<MX>::col0(warp, lane) + (kTY / 2) * l;
-        if (col >= L.ny) continue;
+        const int j = PixelMap<MX>::col0(warp, lane) + (kTY / 2) * l;
+        const int row = tx0 + (exchanged ? j : i), col = ty0 + (exchanged ? i : j);
+        if (row >= L.nx || col >= L.ny) continue;
         const long long o = (static_cast<long long>(zz) * L.nx + row) * L.ny + col;
         float2 p = l ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
         if (L.accumulate) {
@@ -405,6 +407,7 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
                     accumulate_pulse<MX, false, false, CHECKED>(g, tq, w, zero_addr, entry, col, L, acc_re, acc_im);
             }
         }
+        const bool exchanged = MX == 8 && (geo[s * PB].flags & PG_EXCHANGED);
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(s));
         if (i + 1 == n || b == S - 1) {
@@ -412,8 +415,8 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
             if (seg_first == 0 && b == S - 1) {
 #pragma unroll
                 for (int k = 0; k < MX; ++k)
-                    store_pair<MX>(L, cur.u.tx * TX, cur.u.ty * kTY, cur.u.hyp * L.nz + cur.u.iz, warp, lane, k,
-                                   make_float4(acc_re[k][0], acc_im[k][0], acc_re[k][1], acc_im[k][1]));
+                    store_pair<MX>(L, cur.u.tx * TX, cur.u.ty * kTY, cur.u.hyp * L.nz + cur.u.iz, exchanged, warp,
+                                   lane, k, make_float4(acc_re[k][0], acc_im[k][0], acc_re[k][1], acc_im[k][1]));
                 // completion time: the latest of the warps' stores
                 if (BATCH && done) {
                     __syncwarp();
@@ -478,7 +481,7 @@ __global__ void __launch_bounds__(kThreads)
                             });
     int tx0, ty0, zz;
     tile_origin(tg, t, TX, tx0, ty0, zz);
-    store_pair<MX>(L, tx0, ty0, zz, warp, lane, k, v);
+    store_pair<MX>(L, tx0, ty0, zz, MX == 8 && record_exchanged(L, t), warp, lane, k, v);
     if (BATCH && done) {
         __syncthreads();
         if (threadIdx.x == 0) atomicMax(done + scene, global_timer_ns());
@@ -511,7 +514,9 @@ __device__ __forceinline__ void geo_records_chunk(const BpLaunch &L, unsigned n,
         const double cx = L.left + static_cast<double>(static_cast<int>(tx) * TX + TX / 2) * L.dx;
         const double cy = L.bottom + static_cast<double>(static_cast<int>(ty) * kTY + kTY / 2) * L.dy;
         const double cz = L.zlow + static_cast<double>(iz) * L.dz;
-        const PulseGeo g = make_geo(L, static_cast<int>(p), static_cast<long long>(hyp) * L.np, cx, cy, cz, TX / 2);
+        const long long goff = static_cast<long long>(hyp) * L.np;
+        const PulseGeo g = make_geo(L, static_cast<int>(p), goff, cx, cy, cz, TX / 2,
+                                    MX == 8 && tile_exchanged(L, goff, cx, cy));
         const float4 *gw = reinterpret_cast<const float4 *>(&g);
 #pragma unroll
         for (int k = 0; k < kWords; ++k) words[k * kStride + threadIdx.x] = gw[k];

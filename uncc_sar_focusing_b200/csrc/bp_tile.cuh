@@ -138,14 +138,17 @@ __device__ __forceinline__ double rsqrt_newton(double s) {
     return y;
 }
 
-// tx_half: half the tile's rows (its columns are 64: 32 each side)
+// tx_half: half the tile's rows (its columns are 64: 32 each side).  exchanged:
+// the record's x (rows of the pixel map) is the image's y and the other way
+// round.
 __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long goff, double cx, double cy,
-                                             double cz, int tx_half) {
+                                             double cz, int tx_half, bool exchanged = false) {
     PulseGeo g;
-    g.flags = 0;
+    g.flags = exchanged ? PG_EXCHANGED : 0;
+    const double dx = exchanged ? L.dy : L.dx, dy = exchanged ? L.dx : L.dy;
     const long long gi = goff + p;  // geometry of hypothesis goff / np
     const double ax = L.ax[gi], ay = L.ay[gi], az = L.az[gi], r0 = L.r0[gi], f0 = L.f0[gi];
-    const double vx = ax - cx, vy = ay - cy, vz = az - cz;
+    const double vx = exchanged ? ay - cy : ax - cx, vy = exchanged ? ax - cx : ay - cy, vz = az - cz;
 #if SARBP_GEO_RSQ
     const double s2 = vx * vx + vy * vy + vz * vz;
     const double inv = rsqrt_newton(s2);
@@ -167,20 +170,20 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
         return g;
     }
     const int ws = static_cast<int>(floor(bc)) - L.W;
-    const double al = frac_rev(-k * ux * L.dx);
-    const double be = frac_rev(-k * uy * L.dy);
+    const double al = frac_rev(-k * ux * dx);
+    const double be = frac_rev(-k * uy * dy);
     g.A = frac_rev(kd);
     g.alpha = al;
     g.beta = be;
     g.B0 = bc - static_cast<double>(ws);
-    g.gam = -L.lambda * ux * L.dx;
-    g.eta = -L.lambda * uy * L.dy;
+    g.gam = -L.lambda * ux * dx;
+    g.eta = -L.lambda * uy * dy;
     g.a8r = static_cast<float>(kTwoPi * frac_rev(8.0 * al));
     g.b32r = static_cast<float>(kTwoPi * frac_rev(32.0 * be));
     g.g8 = static_cast<float>(8.0 * g.gam);
     g.e32 = static_cast<float>(32.0 * g.eta);
-    g.tx = static_cast<float>(ux * L.dx);
-    g.ty = static_cast<float>(uy * L.dy);
+    g.tx = static_cast<float>(ux * dx);
+    g.ty = static_cast<float>(uy * dy);
     g.h = static_cast<float>(0.5 * inv);
     g.hr = static_cast<float>(0.5 * inv * inv);
     g.kr = static_cast<float>(kTwoPi * k);
@@ -194,7 +197,7 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     g.uz = static_cast<float>(vz * inv);
     g.rinv = static_cast<float>(inv);
 
-    int flags = 0;
+    int flags = g.flags;
     if (rc < L.near_hd16 || rc * rc * rc < k * L.near_coef) flags |= PG_NEAR;
     // Tight window: a pixel (i, j) of the tile has bin - bc = i gam + j eta +
     // lambda g with 0 <= g <= hd^2 / (2 (Rc - hd)) (hd the tile
@@ -250,6 +253,28 @@ struct PixelMap {
     }
 };
 
+// 64-row tiles can be taken with rows and columns exchanged (the map's rows run
+// along the image's columns): a wavefront's 4-pixel side then lies along the
+// image's rows.  The pre-pass does it, for all pulses of a tile, where the bins
+// of the tile's first, middle and last pulse advance faster along the columns
+// (|a - c| dx against dy per axis: the ranges are nearly one), so that the short
+// side of the patch is the fast one and its 8 bins stay within 8 entries.
+// 1024^2 x 2048 pulses, look direction along the columns: 1622 -> 1481 us
+// (adjoint 2071 -> 1922), along the rows 1464 -> 1480 (1995 -> 1929).
+__device__ __forceinline__ bool tile_exchanged(const BpLaunch &L, long long goff, double cx, double cy) {
+    const int at[3] = {0, L.np >> 1, L.np - 1};
+    double d = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        d += fabs(L.ay[goff + at[i]] - cy) * L.dy - fabs(L.ax[goff + at[i]] - cx) * L.dx;
+    return d > 0.0;
+}
+
+// Whether tile t of a launch with pre-pass records is exchanged.
+__device__ __forceinline__ bool record_exchanged(const BpLaunch &L, long long t) {
+    return L.geo_tab && (static_cast<const PulseGeo *>(L.geo_tab)[t * L.np].flags & PG_EXCHANGED);
+}
+
 // Phase and bin of a tile's pixels as polynomials.  With the far-field
 // remainder's phase Q(i, j) = kr g = -kr (t^2 - |d|^2)(h + t hr), a cubic in
 // the pixel's row and column offsets i, j from the tile centre,
@@ -286,7 +311,8 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
     if (lane < NQ) {
         float4 *w = reinterpret_cast<float4 *>(rec + lane);
         const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // a8r, b32r, g8, e32; tx, ty, h, hr; kr, rc, lo, hi
-        const float dx = static_cast<float>(L.dx), dy = static_cast<float>(L.dy);
+        const bool ex = rec[lane].flags & PG_EXCHANGED;
+        const float dx = static_cast<float>(ex ? L.dy : L.dx), dy = static_cast<float>(ex ? L.dx : L.dy);
         const float m = (rec[lane].flags & PG_NEAR) ? 0.0f : -c2.x;
         const float n20 = fmaf(c1.x, c1.x, -dx * dx), n11 = 2.0f * c1.x * c1.y, n02 = fmaf(c1.y, c1.y, -dy * dy);
         const float mh = m * c1.z, mr = m * c1.w;
@@ -487,7 +513,8 @@ struct PixelPoly {
 __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaunch &L, float fi, float2 J,
                                                  float2 &s) {
     const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);  // tx, ty, h, hr
-    const float rc = g.rc, dy = static_cast<float>(L.dy), di = fi * static_cast<float>(L.dx);
+    const bool ex = g.flags & PG_EXCHANGED;
+    const float rc = g.rc, dy = static_cast<float>(ex ? L.dx : L.dy), di = fi * static_cast<float>(ex ? L.dy : L.dx);
     float gl[2], sl[2];
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
