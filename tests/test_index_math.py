@@ -332,3 +332,27 @@ def test_polynomials_match_the_exact_range(radius, dx, el, mx):
                 lin = -(tx * row + ty * j)
                 assert np.abs(Q / kr - (exact - lin)).max() * kr < 2e-6
                 assert np.abs(sigma * Q - lam * (exact - lin)).max() < 1e-6
+
+
+# ---- rotation of the all-FP64 kernel (bp_fp64.cu rotation_table) ----
+
+@pytest.mark.parametrize("scale", [1.0, 1.0e3, 1.0e6, 1.0e12])
+def test_rotation_table_matches_sine_and_cosine(scale):
+    """Table entry n mod 512 times two polynomials in r^2, against sine and
+    cosine of the exactly reduced phase in extended precision.  Four roundings
+    of values of at most 1 (entry, polynomial, product, sum): below 5e-16."""
+    rng = np.random.default_rng(5)
+    edges = (np.arange(-600, 600) + 0.5) / 512.0
+    ph = np.concatenate([rng.uniform(-scale, scale, 20000), edges, np.nextafter(edges, 9.0), np.arange(-9, 9) / 4.0])
+    n = np.rint(512.0 * ph)
+    r = ph - n / 512.0
+    z = r * r
+    s = r * ((81.60513954752706 * z - 41.34170224036052) * z + 6.283185307179586)
+    c = (64.93931252474451 * z - 19.739208802169003) * z + 1.0
+    two_pi = 2 * np.longdouble("3.14159265358979323846264338327950288")
+    turn = two_pi * (np.mod(n, 512.0).astype(np.longdouble) / 512)
+    wx, wy = np.cos(turn).astype(np.float64), np.sin(turn).astype(np.float64)
+    exact = two_pi * (ph - np.rint(ph)).astype(np.longdouble)
+    assert np.abs(r).max() <= 1.0 / 1024
+    assert np.abs(wx * c - wy * s - np.cos(exact)).max() < 5e-16
+    assert np.abs(wy * c + wx * s - np.sin(exact)).max() < 5e-16

@@ -8,18 +8,16 @@
 // revolution), accumulated in double.  It is the accuracy path and the FP64
 // baseline the mixed kernel is measured against; semantics as bp_mixed.cu.
 //
-// What bounds it is the FP64 pipe (64 lanes per SM and cycle): about 40 FP64
+// What bounds it is the FP64 pipe (64 lanes per SM and cycle): about 36 FP64
 // instructions per pixel-pulse.  The common path has no branch and no library
 // call, so a thread's eight pixels are independent chains the scheduler
 // interleaves, on two CTAs per SM; the square root is a reciprocal-root
 // estimate with one coupled Newton step and a residual correction, the
-// rotation one quadrant reduction and two polynomials; window entries are the
-// range profile's samples themselves (the FFT output), the slope formed per
-// pixel, so no pair rows are written (18-39 us a call) and a window is half
-// the shared memory.  512^2 pixels x 1024 pulses: 2049 us with sqrt(),
-// sincospi() and a gate branch per pixel at one CTA per SM, now 930 us, 65% of the FP64 pipe; with
-// two issue cycles per FP64 instruction and 27 others the issue slots are 87%
-// taken.
+// rotation an entry of a table of 512 and two short polynomials; window
+// entries are the range profile's samples themselves (the FFT output), the
+// slope formed per pixel, so no pair rows are written (18-39 us a call) and a
+// window is half the shared memory.  512^2 pixels x 1024 pulses: 2049 us with
+// sqrt(), sincospi() and a gate branch per pixel at one CTA per SM, now 825 us.
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -32,8 +30,10 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps64 = kThreads / 32;
 constexpr int kTY = 64;
-// four mbarriers (full, empty; two buffers each), then two zero samples
-constexpr int kHdr64 = 64;
+// four mbarriers (full, empty; two buffers each), two zero samples, and the
+// table exp(+j 2 pi n / 512)
+constexpr int kTurnTable = 512;
+constexpr int kHdr64 = 64 + kTurnTable * 16;
 
 __device__ __forceinline__ PulseGeo64 make_geo64(const BpLaunch &L, int p, double cx, double cy, double cz) {
     PulseGeo64 g;
@@ -67,11 +67,34 @@ __device__ __forceinline__ double2 lds_d2(uint32_t addr) {
     return v;
 }
 
+// exp(+j 2 pi ph), |ph| < 2^42: ph = n/512 + r exactly, |r| <= 1/1024; sin
+// and cos of 2 pi r as polynomials in r^2 (interpolated at the Chebyshev nodes
+// of [0, 1/1024^2] in 60 digits; errors 2e-21 and 1e-17 before rounding), times
+// the table's entry n mod 512.  13 FP64 instructions where quadrants
+// (rotation, bp_common.cuh) take 17 and ten selects; 512^2 pixels x 1024
+// pulses 915 us by quadrants, 853 with 64 entries and polynomials a degree
+// longer (15 instructions), 862 with those 64 once per bank group, 825 with
+// 512: the entries' bank conflicts hide behind the FP64 pipe.
+__device__ __forceinline__ void rotation_table(double ph, uint32_t tab, double &cs, double &sn) {
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    const double t = fma(ph, static_cast<double>(kTurnTable), kMagic);
+    const double2 w = lds_d2(tab + (static_cast<uint32_t>(__double2loint(t)) & (kTurnTable - 1)) * 16u);
+    const double r = fma(t - kMagic, -1.0 / kTurnTable, ph);
+    const double z = r * r;
+    double S = fma(81.60513954752706, z, -41.34170224036052);
+    double C = fma(64.93931252474451, z, -19.739208802169003);
+    S = r * fma(S, z, 6.283185307179586);
+    C = fma(C, z, 1.0);
+    cs = fma(w.x, C, -(w.y * S));
+    sn = fma(w.y, C, w.x * S);
+}
+
 // One pulse into the thread's MX x 2 pixels.  SAFE: pixels gated by the valid
 // range bins, library square root and sine / cosine.
 template <int MX, bool SAFE>
 __device__ __forceinline__ void accumulate_pulse64(const BpLaunch &L, const PulseGeo64 &g, uint32_t w_addr,
-                                                   uint32_t zero_addr, const double (&xs)[MX], const double (&ys)[2],
+                                                   uint32_t zero_addr, uint32_t turn_addr, const double (&xs)[MX],
+                                                   const double (&ys)[2],
                                                    double z, double (&acc_re)[MX][2], double (&acc_im)[MX][2]) {
     constexpr double kMagic = 6755399441055744.0;
     const double gax = g.ax, gay = g.ay, gr0 = g.r0, gk = g.k, ez = g.az - z;
@@ -119,7 +142,7 @@ __device__ __forceinline__ void accumulate_pulse64(const BpLaunch &L, const Puls
             if (SAFE)
                 sincospi(2.0 * (ph - rint(ph)), &sn, &cs);
             else
-                rotation(ph, cs, sn);
+                rotation_table(ph, turn_addr, cs, sn);
             acc_re[k][l] = fma(re, cs, fma(-im, sn, acc_re[k][l]));
             acc_im[k][l] = fma(re, sn, fma(im, cs, acc_im[k][l]));
         }
@@ -180,7 +203,11 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_fp64_kernel(const __grid_co
         for (int l = 0; l < 2; ++l) acc_re[k][l] = acc_im[k][l] = 0.0;
 
     const uint32_t bar_base = smem_addr(&bars[0]);  // full[s] at bar_base + 8 s, empty[s] at bar_base + 16 + 8 s
-    const uint32_t zero_addr = smem_addr(zero);
+    const uint32_t zero_addr = smem_addr(zero), turn_addr = smem_addr(smem + 64);
+    for (int e = threadIdx.x; e < kTurnTable; e += kThreads) {
+        double2 *turn = reinterpret_cast<double2 *>(smem + 64) + e;
+        sincospi(static_cast<double>(e) / (kTurnTable / 2), &turn->y, &turn->x);
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(bar_base + 8u * s, PB);
@@ -254,9 +281,9 @@ __global__ void __launch_bounds__(kThreads, MINB) bp_fp64_kernel(const __grid_co
             const int flags = g.flags;
             if (!(flags & PG_ACTIVE)) continue;
             if (flags & (PG_GATE | PG_NEAR))
-                accumulate_pulse64<MX, true>(L, g, w, zero_addr, xs, ys, z, acc_re, acc_im);
+                accumulate_pulse64<MX, true>(L, g, w, zero_addr, turn_addr, xs, ys, z, acc_re, acc_im);
             else
-                accumulate_pulse64<MX, false>(L, g, w, zero_addr, xs, ys, z, acc_re, acc_im);
+                accumulate_pulse64<MX, false>(L, g, w, zero_addr, turn_addr, xs, ys, z, acc_re, acc_im);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_base + 16u + 8u * s);
