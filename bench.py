@@ -111,7 +111,7 @@ def config_dict(sc, desc: str, world: int) -> dict:
     --config and world size)."""
     return {"workload": desc, "pixels_per_gpu": sc.grid.npix, "pulses": sc.num_pulses,
             "range_samples": sc.num_range_samples, "nfft": sc.nfft, "pixel_pulses_per_step_per_gpu": sc.pixel_pulses,
-            "l2": "inputs larger than L2 (range-profile pair rows of every pulse, 16 B per entry)",
+            "l2": "inputs larger than L2 (range profiles of every pulse, 8 B per sample, and the geometry records)",
             "parallelism": f"{world} image slab(s), one per GPU, no data-path collective"}
 
 
@@ -800,10 +800,9 @@ def gpu_arm(args):
         bp_rate = pp / (bp_ms * 1e-3)
         hbm, hbm_kind = measured_hbm()
         info = plan.info
-        # range compression moves at least the phase history in and the pair
-        # rows the backprojection reads out: 8 B per sample + 16 B per entry
-        # (nfft + 1 entries per pulse)
-        rc_bytes = sc.num_pulses * (sc.num_range_samples * 8 + (sc.nfft + 1) * 16)
+        # range compression moves at least the phase history in and the range
+        # profiles the backprojection reads out: 8 B per sample each
+        rc_bytes = sc.num_pulses * (sc.num_range_samples + sc.nfft) * 8
         mixed_speedup = fp64_ms / bp_ms
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,

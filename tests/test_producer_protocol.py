@@ -1,9 +1,10 @@
-"""The forward kernel's hand-over with one producing warp, replayed on the CPU.
+"""The forward kernel's hand-over with its producing warps, replayed on the CPU.
 
-bp_mixed_kernel (csrc/bp_mixed.cu): per stage i (buffer s = i & 1) the
-producer waits empty[s] for stage i - 2 (from i = 2), writes the records, the
-tables and the copies (PB arrivals on full[s]), waits full[s], rewrites the
-windows and arrives once on ready[s]; each of the 8 accumulating warps waits
+bp_mixed_kernel (csrc/bp_mixed.cu): per stage i (buffer s = i & 1) each
+producer (two, or one for stages of one pulse) waits empty[s] for stage i - 2
+(from i = 2), writes its pulses' records, tables and copies (PB arrivals on
+full[s] between them, one each here), waits full[s], rewrites its windows and
+arrives once on ready[s]; each of the 8 accumulating warps waits
 ready[s], consumes and arrives on empty[s].  Every wait is a parity wait.
 Random interleavings: no deadlock, every wait released by its own stage's
 phase, no buffer refilled while a warp still reads it.
@@ -35,12 +36,12 @@ def consumer(n):
         yield ("arrive", ("empty", s))
 
 
-def replay(n, seed, **kw):
+def replay(n, seed, producers=2, **kw):
     rnd = random.Random(seed)
-    count = {"full": 1, "ready": 1, "empty": WARPS}
+    count = {"full": producers, "ready": producers, "empty": WARPS}
     bars = {(k, b): Barrier(c) for k, c in count.items() for b in range(2)}
     did = {"full": {}, "ready": {}, "empty": {}}
-    progs = [producer(n, **kw)] + [consumer(n) for _ in range(WARPS)]
+    progs = [producer(n, **kw) for _ in range(producers)] + [consumer(n) for _ in range(WARPS)]
     op = [next(p) for p in progs]
     live = set(range(len(progs)))
     while live:
@@ -58,7 +59,7 @@ def replay(n, seed, **kw):
             if what in ("produce", "rewrite") and stage >= 2:
                 assert did["empty"].get(stage - 2, 0) == WARPS
             if what == "consume":
-                assert did["ready"].get(stage, 0) == 1
+                assert did["ready"].get(stage, 0) == producers
             key = {"produce": "full", "rewrite": "ready", "consume": "empty"}[what]
             did[key][stage] = did[key].get(stage, 0) + 1
         try:
@@ -68,10 +69,11 @@ def replay(n, seed, **kw):
     assert all(did["empty"].get(i, 0) == WARPS for i in range(n))
 
 
+@pytest.mark.parametrize("producers", [1, 2])
 @pytest.mark.parametrize("n", [1, 2, 3, 4, 7, 12])
-def test_hand_over(n):
+def test_hand_over(n, producers):
     for seed in range(200):
-        replay(n, seed)
+        replay(n, seed, producers)
 
 
 def test_replay_catches_a_missing_empty_wait():

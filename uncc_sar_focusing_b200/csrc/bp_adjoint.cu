@@ -9,9 +9,9 @@
 //     dL/da_p = sum_q s_pq u_pq (u_pq the unit vector pixel -> antenna),
 //     dL/dR0_p = -sum_q s_pq.
 // v'_p(b) is the slope of the linear interpolation, rc[b+1] - rc[b], which the
-// pair entries already hold.  Nothing per pixel-pulse is stored: the kernel
+// rewritten windows hold.  Nothing per pixel-pulse is stored: the kernel
 // recomputes the geometry of every (tile, pulse) exactly as the forward kernel
-// does (same records, base tables, shared-memory windows and FP32 per-pixel
+// does (same records, polynomial tables, shared-memory windows and FP32 per-pixel
 // arithmetic).
 //
 // Per pixel the kernel holds G_q as |G_q| exp(j psi_q), so that with
@@ -40,8 +40,8 @@
 // lane holds), and adjoint_reduce_kernel sums the tiles per pulse in double,
 // in a fixed order.
 //
-// What bounds it: 21 warp instructions per warp-pixel-pulse at 62% of issue
-// slots (20.9 before, where the gathers of the 32 lanes of a row took 9.3
+// What bounds it: 22 warp instructions per warp-pixel-pulse at 66% of issue
+// slots (20.8 before, where the gathers of the 32 lanes of a row took 9.3
 // shared-memory wavefronts a pixel-pulse instead of 5.8 whenever the look
 // direction lay along the columns).  2048 pulses x 1024^2 pixels, look
 // direction 0 / 45 / 90 degrees from the rows: 2.00 / 2.41 / 2.26 ms before,

@@ -8,16 +8,17 @@
 // revolution), accumulated in double.  It is the accuracy path and the FP64
 // baseline the mixed kernel is measured against; semantics as bp_mixed.cu.
 //
-// What bounds it is the FP64 pipe (64 lanes per SM and cycle): about 36 FP64
-// instructions per pixel-pulse.  The common path has no branch and no library
-// call, so a thread's eight pixels are independent chains the scheduler
-// interleaves, on two CTAs per SM; the square root is a reciprocal-root
-// estimate with one coupled Newton step and a residual correction, the
-// rotation an entry of a table of 512 and two short polynomials; window
-// entries are the range profile's samples themselves (the FFT output), the
-// slope formed per pixel, so no pair rows are written (18-39 us a call) and a
-// window is half the shared memory.  512^2 pixels x 1024 pulses: 2049 us with
-// sqrt(), sincospi() and a gate branch per pixel at one CTA per SM, now 825 us.
+// What bounds it is the FP64 pipe (64 lanes per SM and cycle; 66% busy) at 37
+// FP64 instructions per pixel-pulse, with shared memory's data pipe at 64%.
+// The common path has no branch and no library call, so a thread's eight
+// pixels are independent chains the scheduler interleaves, on two CTAs per SM;
+// the square root is a reciprocal-root estimate with one coupled Newton step
+// and a residual correction, the rotation an entry of a table of 512 and two
+// short polynomials; window entries are the range profile's samples themselves
+// (the FFT output), the slope formed per pixel, so no pair rows are written
+// (18-39 us a call) and a window is half the shared memory.  512^2 pixels x
+// 1024 pulses: 2049 us with sqrt(), sincospi() and a gate branch per pixel at
+// one CTA per SM, now 825 us.
 #include <cstdint>
 
 #include "bp_common.cuh"

@@ -2,7 +2,7 @@
 // forward and adjoint backprojection kernels: tile constants, the FP64
 // geometry record of one pulse relative to one pixel tile, the per-warp
 // producer that writes records and issues the window bulk copies, and the
-// shared-memory load of one pair entry.  See bp_mixed.cu for the design.
+// shared-memory load of one window entry.  See bp_mixed.cu for the design.
 #pragma once
 
 #include <cstdint>

@@ -133,7 +133,7 @@ inline size_t margin_samples(int wsize) { return static_cast<size_t>(wsize) + 4;
 
 // Range-bin window of a tile of (8 mx) x 64 pixels with steps dx, dy at
 // lambda bins per metre: W = ceil(lambda * half-diagonal) + 3 bins each side,
-// wsize = 2W + 2 pair entries; hd the half-diagonal in metres.
+// wsize = 2W + 2 window entries; hd the half-diagonal in metres.
 inline void tile_window(double lambda, double dx, double dy, int mx, int *W, int *wsize, double *hd) {
     const double hx = 0.5 * 8.0 * mx * dx, hy = 0.5 * 64.0 * dy;
     *hd = std::sqrt(hx * hx + hy * hy);
