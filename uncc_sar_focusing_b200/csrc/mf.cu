@@ -14,11 +14,16 @@
 // pixel-pulse.  A warp takes one pulse and 32 P pixels, P = 4 per thread (2 in
 // FP64): each broadcast read of a sample feeds 4 P multiply-adds in P
 // independent chains (one pixel per thread waited out every step of its
-// chain), as paired FP32 instructions from samples stored twice.  The 8 warps
-// of a CTA take different pulses of the same pixels, the CTAs of a cluster
+// chain), as paired FP32 instructions from samples stored twice.  The 16 warps (8
+// in FP64) of a CTA take different pulses of the same pixels, the CTAs of a cluster
 // too, so a small image still fills the SMs; their sums are added in warp and
 // rank order through (distributed) shared memory.  96^2 pixels x 128 pulses x
-// 256 samples: 461 us before, 81 us now, 35 us at the measured FMA rate.
+// 256 samples: 461 us with one pixel a thread, 64 us now, 35 us at the measured FMA rate
+// (256^2 pixels: 387 us, 256 at that rate).  Two CTAs of 16 warps an SM (64
+// registers, 44 bytes spilled outside the sample loop): with 8 warps a CTA and
+// 80 registers the clusters of a small image did not all fit at once, 82 us
+// (256^2: 476).  FP64 keeps 8: 378 us for 128^2 x 256, 443 with 16, and no
+// bound on its registers (it takes 64; 415 us when told to).
 #include <cooperative_groups.h>
 #include <cstdint>
 
@@ -28,13 +33,11 @@
 namespace sarbp {
 namespace {
 
-constexpr int kMfWarps = 8;
-constexpr int kMfThreads = 32 * kMfWarps;
 constexpr int kMfChunk = 128;  // samples a warp stages at a time
 
 // Horner chains of a thread's pixels: FP32 in pairs, FP64 singly.
 struct MfFloat {
-    static constexpr int kPixels = 4;
+    static constexpr int kPixels = 4, kWarps = 16;  // pixels a thread, warps a CTA
     using Sample = float4;  // re, re, im, im
     float2 hr[2], hi[2], zr[2], zi[2];
 
@@ -66,7 +69,7 @@ struct MfFloat {
 };
 
 struct MfDouble {
-    static constexpr int kPixels = 2;
+    static constexpr int kPixels = 2, kWarps = 8;
     using Sample = double2;
     double hr[2], hi[2], zr[2], zi[2];
 
@@ -104,9 +107,8 @@ __device__ __forceinline__ void turn(double ph, double &cs, double &sn) {
 // Pixel block blockIdx.x / (cluster size); the cluster's rank and the warp
 // choose the pulses.  T: float or double.
 template <typename CH, typename T>
-__global__ void __launch_bounds__(kMfThreads) mf_kernel(const float2 *__restrict__ ph, const double *__restrict__ win,
-                                                       MfLaunch M) {
-    constexpr int P = CH::kPixels;
+__device__ __forceinline__ void mf_body(const float2 *__restrict__ ph, const double *__restrict__ win, const MfLaunch &M) {
+    constexpr int P = CH::kPixels, kMfWarps = CH::kWarps;
     namespace cg = cooperative_groups;
     using Sample = typename CH::Sample;
     __shared__ __align__(16) union Smem {
@@ -201,8 +203,18 @@ __global__ void __launch_bounds__(kMfThreads) mf_kernel(const float2 *__restrict
     cluster.sync();  // the other ranks' shared memory stays until it has been read
 }
 
-template <typename CH, typename T>
-cudaError_t launch_mf_on(const float2 *ph, const double *win, const MfLaunch &M, cudaStream_t s) {
+__global__ void __launch_bounds__(32 * MfFloat::kWarps, 2)
+    mf_kernel(const float2 *__restrict__ ph, const double *__restrict__ win, MfLaunch M) {
+    mf_body<MfFloat, float>(ph, win, M);
+}
+
+__global__ void __launch_bounds__(32 * MfDouble::kWarps)
+    mf_kernel64(const float2 *__restrict__ ph, const double *__restrict__ win, MfLaunch M) {
+    mf_body<MfDouble, double>(ph, win, M);
+}
+
+template <typename CH, typename F>
+cudaError_t launch_mf_on(F kern, const float2 *ph, const double *win, const MfLaunch &M, cudaStream_t s) {
     const long long npix = static_cast<long long>(M.nx) * M.ny * M.nz;
     const long long blocks = (npix + 32 * CH::kPixels - 1) / (32 * CH::kPixels);
     int dev = 0, sms = 0;
@@ -211,13 +223,16 @@ cudaError_t launch_mf_on(const float2 *ph, const double *win, const MfLaunch &M,
     if (e != cudaSuccess) return e;
     // CTAs that share the pulses of a pixel block: the number (up to the 8 a
     // portable cluster holds) for which the busiest SM has the fewest pulses,
-    // the larger of equals (96^2 pixels, 128 pulses: 72 blocks leave half the
-    // SMs idle alone; 8 CTAs each give every SM four of two pulses a warp)
+    // but more of them only for a tenth less: large clusters find room on fewer
+    // SMs at a time (mixed, 96^2 pixels x 128 pulses, 72 blocks: 120 / 66 / 91 /
+    // 82 us with 1 / 2 / 4 / 8; 64^2 x 512 455 / 233 / 121 / 118; 256^2 x 128
+    // 437 / 388 / 421 / 470; 160^2 x 100 335 / 265 / 306 / 329).  FP64's CTAs of
+    // 8 warps fit more easily: the most of equals (96^2 x 128: 120 us)
     int ranks = 1;
     long long best = 0;
     for (int r = 1; r <= 8; r *= 2) {
-        const long long cost = ((blocks * r + sms - 1) / sms) * ((M.np + r * kMfWarps - 1) / (r * kMfWarps));
-        if (r == 1 || cost <= best) {
+        const long long cost = ((blocks * r + sms - 1) / sms) * ((M.np + r * CH::kWarps - 1) / (r * CH::kWarps));
+        if (r == 1 || (CH::kWarps == 8 ? cost <= best : 10 * cost < 9 * best)) {
             best = cost;
             ranks = r;
         }
@@ -225,7 +240,7 @@ cudaError_t launch_mf_on(const float2 *ph, const double *win, const MfLaunch &M,
     if (blocks < 1 || blocks * ranks > 0x7fffffffLL) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(blocks * ranks));
-    cfg.blockDim = dim3(kMfThreads);
+    cfg.blockDim = dim3(32 * CH::kWarps);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -233,14 +248,14 @@ cudaError_t launch_mf_on(const float2 *ph, const double *win, const MfLaunch &M,
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, mf_kernel<CH, T>, ph, win, M);
+    return cudaLaunchKernelEx(&cfg, kern, ph, win, M);
 }
 
 }  // namespace
 
 cudaError_t launch_mf(const void *ph, const double *win, const MfLaunch &M, bool fp64, cudaStream_t s) {
     const float2 *x = static_cast<const float2 *>(ph);
-    return fp64 ? launch_mf_on<MfDouble, double>(x, win, M, s) : launch_mf_on<MfFloat, float>(x, win, M, s);
+    return fp64 ? launch_mf_on<MfDouble>(mf_kernel64, x, win, M, s) : launch_mf_on<MfFloat>(mf_kernel, x, win, M, s);
 }
 
 }  // namespace sarbp
