@@ -1,0 +1,104 @@
+"""The mixed kernels' per-(tile, pulse) arithmetic from its own source, on the CPU.
+
+native/tile_probe.cpp builds csrc/bp_tile.cuh for the host: records, polynomial
+tables and every thread's phases and bins of one tile, against the exact range
+in FP64.  A bin becomes a shared-memory address in the kernels, so each must be
+finite and inside the pulse's window whatever the start frequency is.
+"""
+import ctypes
+import math
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+C = 299792458.0
+PG_NEAR = 4
+
+
+@pytest.fixture(scope="module")
+def probe(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("tile_probe") / "libtile_probe.so")
+    subprocess.run(["g++", "-O2", "-std=c++20", "-ffp-contract=off", "-fPIC", "-shared", "-w", "-pthread",
+                    f"-I{CUDA_HOME}/include", "-o", so, os.path.join(HERE, "native", "tile_probe.cpp")], check=True)
+    lib = ctypes.CDLL(so)
+    d, i, p = ctypes.c_double, ctypes.c_int, ctypes.c_void_p
+    lib.tile_probe.argtypes = [p, i, i, d, d, d, d, d, i, d, d, i, i, i, p, p, p]
+    return lib.tile_probe
+
+
+def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392, lam=32.1, el=30.0, look=(0.0, 30.0, 88.0, 200.0)):
+    """The tile's phases, bins and pulse words, with their exact values:
+    phase modulo one turn, window-centred bin (float64)."""
+    az = np.radians(np.asarray(look))
+    n = len(az)
+    x = radius * math.cos(math.radians(el)) * np.cos(az)
+    y = radius * math.cos(math.radians(el)) * np.sin(az)
+    z = np.full(n, radius * math.sin(math.radians(el)))
+    r0 = np.sqrt(x * x + y * y + z * z)
+    f = np.broadcast_to(np.asarray(f0, dtype=np.float64), (n,))
+    geo = np.ascontiguousarray(np.stack([x, y, z, r0, f]))
+    dx, dy = spacing, 1.1 * spacing
+    left, bottom = 0.3, -0.7
+    hd = math.hypot(4 * mx * dx, 32 * dy)
+    W = int(math.ceil(lam * hd)) + 3
+    P = np.full((n, 8 * mx, 64), np.nan, dtype=np.float32)
+    B = P.copy()
+    words = np.zeros((n, 3), dtype=np.int32)
+    err = probe(geo.ctypes.data, n, nfft, lam, dx, dy, left, bottom, W, 16.0 * hd, 0.625 * hd ** 4 / 1e-7, mx,
+                int(exchanged), int(split), P.ctypes.data, B.ctypes.data, words.ctypes.data)
+    assert err == 0
+    if exchanged:  # the map's rows run along the image's columns
+        P, B = P.transpose(0, 2, 1), B.transpose(0, 2, 1)
+    px = left + dx * np.arange(8 * mx)[None, :, None]
+    py = bottom + dy * np.arange(64)[None, None, :]
+    R = np.sqrt((x[:, None, None] - px) ** 2 + (y[:, None, None] - py) ** 2 + z[:, None, None] ** 2)
+    dR = R - r0[:, None, None]
+    rev = 2.0 * f[:, None, None] / C * dR
+    bin_ = lam * dR + 0.5 * nfft - words[:, 1, None, None] - W
+    rc = np.sqrt((x - left - 4 * mx * dx) ** 2 + (y - bottom - 32 * dy) ** 2 + z * z)
+    far = (0.625 * hd ** 4 / rc ** 3)[:, None, None]  # metres the expansion may be off
+    return dict(P=P, B=B, words=words, rev=rev, bin=bin_, far=far, kr=4.0 * math.pi * f[:, None, None] / C, lam=lam, W=W)
+
+
+def check(t):
+    assert np.isfinite(t["P"]).all() and np.isfinite(t["B"]).all()
+    wp = t["words"][:, 2, None, None]
+    fl = np.floor(t["B"])
+    assert (fl >= -wp).all() and (fl <= wp).all(), "a bin outside its pulse's window"
+    far = np.where(t["words"][:, 0, None, None] & PG_NEAR, 0.0, t["far"])
+    # bins: four roundings at the window's half-width; phases: five at the
+    # largest phase and 1e-6 rad for the cubic term's fit; and the expansion
+    tol_bin = 4.0 * 2.0 ** -24 * t["W"] + t["lam"] * far
+    tol_phase = 5.0 * 2.0 ** -24 * np.abs(t["P"]).max() + 1e-6 + np.abs(t["kr"]) * far
+    assert (np.abs(t["B"] - t["bin"]) <= tol_bin).all(), np.abs(t["B"] - t["bin"]).max()
+    turn = t["P"].astype(np.float64) / (2.0 * math.pi) - t["rev"]
+    off = 2.0 * math.pi * np.abs(turn - np.rint(turn))
+    assert (off <= tol_phase).all(), off.max()
+
+
+@pytest.mark.parametrize("mx,exchanged", [(1, False), (2, False), (4, False), (8, False), (8, True)])
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("radius,spacing", [(8e3, 0.1), (10e3, 0.08), (60.0, 0.1), (3e3, 0.4)])
+def test_phases_and_bins(probe, mx, exchanged, split, radius, spacing):
+    check(tile(probe, 9.28e9, radius, spacing, mx, exchanged, split))
+
+
+@pytest.mark.parametrize("radius,spacing", [(8e3, 0.1), (60.0, 0.1)])
+@pytest.mark.parametrize("f0", [0.0, 1e-30, -1e-30, 1e-9, 25.0, -3.0e8, -9.28e9, [9.28e9, 0.0, -3.0e8, 0.0]])
+def test_any_start_frequency(probe, f0, radius, spacing):
+    """Baseband data and blanked pulses: the bin does not depend on the start
+    frequency, the phase is zero at zero."""
+    for mx, split in ((2, False), (8, False), (8, True)):
+        t = tile(probe, f0, radius, spacing, mx, split=split)
+        check(t)
+        assert (t["P"][np.broadcast_to(t["kr"] == 0.0, t["P"].shape)] == 0.0).all()
+
+
+@pytest.mark.parametrize("lam", [1e-30, 1e-14, 1e-6])
+def test_wide_swaths(probe, lam):
+    """Range bins of kilometres and more: the phase does not depend on them."""
+    check(tile(probe, 9.28e9, 8e3, 0.1, 8, lam=lam))

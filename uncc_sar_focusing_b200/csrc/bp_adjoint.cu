@@ -70,7 +70,7 @@ __device__ __forceinline__ void adjoint_pulse(const PulseGeo &g, const float4 *t
                                               const float2 (&npsi)[MX], const float2 (&gm)[MX], float2 &S, float2 &K,
                                               float4 &E) {
     using M = PixelMap<MX>;
-    const PixelPoly poly(g, tab, entry, col);
+    const PixelPoly<true> poly(g, tab, entry, col);
     // B is the window-centred bin (entry floor(B) + W, Z form)
     const uint32_t w_adj = w_addr + (static_cast<uint32_t>(L.W) - kRoundMagicBits) * 16u;
     S = K = make_float2(0.0f, 0.0f);

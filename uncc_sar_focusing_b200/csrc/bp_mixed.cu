@@ -93,7 +93,7 @@ __device__ __forceinline__ void accumulate_pulse(const PulseGeo &g, const float4
                                                  uint32_t zero_addr, int entry, int col, const BpLaunch &L,
                                                  float (&acc_re)[MX][2], float (&acc_im)[MX][2]) {
     using M = PixelMap<MX>;
-    const PixelPoly poly(g, tab, entry, col);
+    const PixelPoly<false> poly(g, tab, entry, col);
     // B is the window-centred bin; shared address of entry floor(B) + W:
     // bits(B + 1.5*2^23, rounded down) * 16 + w_adj (mod 2^32)
     const uint32_t w_adj = w_addr + (static_cast<uint32_t>(L.W) - kRoundMagicBits) * 16u;

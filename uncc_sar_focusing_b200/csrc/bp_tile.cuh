@@ -198,7 +198,10 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     g.rinv = static_cast<float>(inv);
 
     int flags = g.flags;
-    if (rc < L.near_hd16 || rc * rc * rc < k * L.near_coef) flags |= PG_NEAR;
+    // (bins of less than 1e-12 or more than 1e12 to the metre would leave the
+    // polynomials' FP32 range; the exact path does without their ratio)
+    if (rc < L.near_hd16 || rc * rc * rc < k * L.near_coef || !(L.lambda > 1.0e-12 && L.lambda < 1.0e12))
+        flags |= PG_NEAR;
     // Tight window: a pixel (i, j) of the tile has bin - bc = i gam + j eta +
     // lambda g with 0 <= g <= hd^2 / (2 (Rc - hd)) (hd the tile
     // half-diagonal), |i| <= tx_half, |j| <= 32, so its floor(bin) and
@@ -276,24 +279,25 @@ __device__ __forceinline__ bool record_exchanged(const BpLaunch &L, long long t)
 }
 
 // Phase and bin of a tile's pixels as polynomials.  With the far-field
-// remainder's phase Q(i, j) = kr g = -kr (t^2 - |d|^2)(h + t hr), a cubic in
-// the pixel's row and column offsets i, j from the tile centre,
+// remainder in bins Q(i, j) = lambda g = -lambda (t^2 - |d|^2)(h + t hr), a cubic
+// in the pixel's row and column offsets i, j from the tile centre,
 //     Q = i^2 (q20 + i q30) + j i (q11 + i q21) + j^2 (q02 + i q12 + j q03),
-// the phase is 2 pi frac(A + i alpha + j beta) + Q and the window-centred bin
-// B0 - W + i gam + j eta + sigma Q, sigma = lambda / kr.  Around a thread's
-// middle row i = i_c + 2 k both are P0 + k a + k^2 b: the table holds the
-// parts of P0, a, b that depend on i_c only (8 row entries of two float4)
-// and the column phases (32 floats); a thread completes them with its two
-// columns (13 paired operations a pulse), so phase and bin cost 22 paired
-// operations per 16 pixels instead of a full evaluation of t, t^2 - |d|^2 and
-// the remainder for each (64).  The
-// k^3 term of Q (2 k <= 8 rows: 1/64 of the tile's cubic term, < 6e-7 rad at
+// the window-centred bin is B0 - W + i gam + j eta + Q and the phase
+// 2 pi frac(A + i alpha + j beta) + tau Q, tau = kr / lambda.  (Not the phase
+// and its lambda / kr: kr is zero at baseband, and a bin becomes an address.)
+// Around a thread's middle row i = i_c + 2 k both are P0 + k a + k^2 b: the
+// table holds the parts of P0, a, b that depend on i_c only (8 row entries of
+// two float4) and the column phases (32 floats); a thread completes them with
+// its two columns (13 paired operations a pulse), so phase and bin cost 22
+// paired operations per 16 pixels instead of a full evaluation of t, t^2 -
+// |d|^2 and the remainder for each (64).  The
+// k^3 term of tau Q (2 k <= 8 rows: 1/64 of the tile's cubic term, < 6e-7 rad at
 // 100 m / 1024 pixels, 8 km) is folded into a by least squares over k.
 //   [2e]     phase, bin, x1 = i (q11 + i q21), x2 = q02 + i q12
-//   [2e + 1] phase step, bin step, step's j term, k^2 phase term
+//   [2e + 1] phase step, bin step, step's j term, k^2 term
 //   [16..]   2 pi frac(j beta), j = -32..-1
 // and, in the record's first two words (its FP64 steps, no longer needed):
-//   [0]      2 pi frac(32 beta), eta, sigma, q03
+//   [0]      2 pi frac(32 beta), eta, tau, q03
 //   [1]      step's j^2 term, k^2 term's j term, lo, hi
 // Near-field pulses keep the linear parts only (their remainder is evaluated
 // per pixel).
@@ -313,15 +317,16 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // a8r, b32r, g8, e32; tx, ty, h, hr; kr, rc, lo, hi
         const bool ex = rec[lane].flags & PG_EXCHANGED;
         const float dx = static_cast<float>(ex ? L.dy : L.dx), dy = static_cast<float>(ex ? L.dx : L.dy);
-        const float m = (rec[lane].flags & PG_NEAR) ? 0.0f : -c2.x;
+        const bool near = rec[lane].flags & PG_NEAR;
+        const float lam = static_cast<float>(L.lambda);
         const float n20 = fmaf(c1.x, c1.x, -dx * dx), n11 = 2.0f * c1.x * c1.y, n02 = fmaf(c1.y, c1.y, -dy * dy);
-        const float mh = m * c1.z, mr = m * c1.w;
+        const float mh = near ? 0.0f : -lam * c1.z, mr = near ? 0.0f : -lam * c1.w;
         const float q21 = mr * fmaf(c1.x, n11, c1.y * n20), q12 = mr * fmaf(c1.x, n02, c1.y * n11);
-        const float q03 = mr * c1.y * n02, sigma = static_cast<float>(L.lambda) / c2.x;
+        const float q03 = mr * c1.y * n02, tau = near ? 0.0f : c2.x / lam;
         float4 *coef = tabs + lane * kPolyEntries + kPolyCols;
         coef[0] = make_float4(mh * n20, mh * n11, mh * n02, mr * c1.x * n20);
-        coef[1] = make_float4(q21, q12, sigma, 0.0f);
-        un0 = make_float4(c0.y, c0.w * (1.0f / 32.0f), sigma, q03);
+        coef[1] = make_float4(q21, q12, tau, 0.0f);
+        un0 = make_float4(c0.y, c0.w * (1.0f / 32.0f), tau, q03);
         un1 = make_float4(2.0f * q12, 4.0f * q21, c2.z, c2.w);
     }
     __syncwarp();
@@ -333,18 +338,18 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         const double2 d0 = *reinterpret_cast<const double2 *>(w);  // A, alpha
         const double B0 = rec[q].B0, gam = rec[q].gam;
         float4 *row = tabs + q * kPolyEntries + 2 * e;
-        // q20, q11, q02, q30; q21, q12, sigma
+        // q20, q11, q02, q30; q21, q12, tau
         const float4 qa = tabs[q * kPolyEntries + kPolyCols], qb = tabs[q * kPolyEntries + kPolyCols + 1];
         const float i = static_cast<float>(M::mid_row(e));
         const double id = static_cast<double>(i);
         const double pr = fma(id, d0.y, d0.x), ps = 2.0 * d0.y;
         const float nl = i * i * fmaf(i, qa.w, qa.x);
         const float an = fmaf(8.0f * kFit, qa.w, 2.0f * i * fmaf(3.0f * i, qa.w, 2.0f * qa.x));
-        row[0] = make_float4(static_cast<float>(kTwoPi * (pr - rint(pr))) + nl,
-                             fmaf(qb.z, nl, static_cast<float>(fma(id, gam, B0 - L.W))), i * fmaf(i, qb.x, qa.y),
+        row[0] = make_float4(fmaf(qb.z, nl, static_cast<float>(kTwoPi * (pr - rint(pr)))),
+                             static_cast<float>(fma(id, gam, B0 - L.W)) + nl, i * fmaf(i, qb.x, qa.y),
                              fmaf(i, qb.y, qa.z));
-        row[1] = make_float4(static_cast<float>(kTwoPi * (ps - rint(ps))) + an,
-                             fmaf(qb.z, an, static_cast<float>(2.0 * gam)), 2.0f * fmaf(2.0f * i, qb.x, qa.y),
+        row[1] = make_float4(fmaf(qb.z, an, static_cast<float>(kTwoPi * (ps - rint(ps)))),
+                             static_cast<float>(2.0 * gam) + an, 2.0f * fmaf(2.0f * i, qb.x, qa.y),
                              4.0f * fmaf(3.0f * i, qa.w, qa.x));
     }
     __syncwarp();
@@ -466,7 +471,10 @@ __device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
 
 // Phase and bin polynomials of a thread's pixel pairs for one pulse (columns
 // col and col + 32 of the tile): row step k - kMid takes P0 + k Pa + k^2 Pb
-// and B0 + k Ba + k^2 Bb.
+// and B0 + k Ba + k^2 Bb.  SPLIT: Pb beside Bb instead of from it, for the
+// adjoint, whose registers it suits (1950 against 1964 us on 1024^2 pixels x
+// 2048 pulses; forward 1508 against 1484).
+template <bool SPLIT>
 struct PixelPoly {
     float2 J, P0, Pa, Pb, B0, Ba, Bb;
     float lo, hi;  // valid bins
@@ -478,14 +486,14 @@ struct PixelPoly {
         J = make_float2(j0, j0 + static_cast<float>(kTY / 2));
         const float s0 = r0.x + reinterpret_cast<const float *>(tab + kPolyCols)[col];
         const float2 w = __ffma2_rn(J, __ffma2_rn(J, splat(u0.w), splat(r0.w)), splat(r0.z));
-        const float2 sJ = __fmul2_rn(J, splat(u0.z));
-        P0 = __ffma2_rn(J, w, make_float2(s0, s0 + u0.x));
-        B0 = __ffma2_rn(sJ, w, __ffma2_rn(J, splat(u0.y), splat(r0.y)));
+        const float2 tJ = __fmul2_rn(J, splat(u0.z));
+        P0 = __ffma2_rn(tJ, w, make_float2(s0, s0 + u0.x));
+        B0 = __ffma2_rn(J, w, __ffma2_rn(J, splat(u0.y), splat(r0.y)));
         const float2 v = __ffma2_rn(J, splat(u1.x), splat(r1.z));
-        Pa = __ffma2_rn(J, v, splat(r1.x));
-        Ba = __ffma2_rn(sJ, v, splat(r1.y));
-        Pb = __ffma2_rn(J, splat(u1.y), splat(r1.w));
-        Bb = __fmul2_rn(Pb, splat(u0.z));
+        Pa = __ffma2_rn(tJ, v, splat(r1.x));
+        Ba = __ffma2_rn(J, v, splat(r1.y));
+        Bb = __ffma2_rn(J, splat(u1.y), splat(r1.w));
+        Pb = SPLIT ? __ffma2_rn(tJ, splat(u1.y), splat(r1.w * u0.z)) : __fmul2_rn(Bb, splat(u0.z));
         lo = u1.z;
         hi = u1.w;
     }
