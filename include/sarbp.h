@@ -169,7 +169,7 @@ typedef struct sarbp_plan_info {
                                     precision, nfft = R K, K in {256, 512, 1024}, R in
                                     {1, 2, 4, 8, 16}); 0: see chirp_range_compression */
     int chirp_range_compression; /* 1: one kernel does them by a chirp convolution (mixed
-                                    precision, K <= 512 with a long prime factor, R in
+                                    precision, K <= 512 with long prime factors, R in
                                     {4, 8}); 0 with
                                     fused_range_compression 0: taper kernel and cuFFT */
     int reserved[3];

@@ -760,7 +760,7 @@ int sarbp_plan_create(const sarbp_plan_desc *desc, sarbp_plan **out) {
         cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaGetLastError();
-        if (want && p->precision == SARBP_PRECISION_MIXED && R >= 1 && rc_fused_shape(K, R, &rc_smem, &tab) &&
+        if (want && p->precision == SARBP_PRECISION_MIXED && R >= 1 && rc_fused_shape(K, R, p->np_cap, &rc_smem, &tab) &&
             rc_smem <= static_cast<size_t>(dev_smem)) {
             if ((st = alloc(p, &p->d_rctab, tab.size() * sizeof(float))) != SARBP_OK) {
                 release(p);

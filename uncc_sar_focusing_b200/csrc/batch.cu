@@ -450,7 +450,8 @@ int sarbp_batch_create(const sarbp_plan_desc *descs, int num_scenes, sarbp_batch
         const int R = d.nfft % d.num_range_samples == 0 ? d.nfft / d.num_range_samples : 0;
         size_t rc_smem = 0;
         std::vector<float> tab;
-        const bool fused = want_fused && R >= 1 && rc_fused_shape(d.num_range_samples, R, &rc_smem, &tab) &&
+        const bool fused = want_fused && R >= 1 &&
+                           rc_fused_shape(d.num_range_samples, R, d.num_pulses, &rc_smem, &tab) &&
                            rc_smem <= static_cast<size_t>(dev_smem);
         if (fused) {
             const long long key = static_cast<long long>(d.num_range_samples) * 64 + R;

@@ -529,7 +529,30 @@ cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStre
         X(32, 4) X(32, 8) X(32, 16)
 #define SARBP_CZT_SHAPES(X) X(32, 4) X(32, 8)
 
+bool rc_direct_shape(int K) { return K == 256 || K == 512 || K == 1024; }
+
 namespace {
+
+// Whether `pulses` pulses of K samples take the chirp kernel: where cuFFT has
+// long prime factors to work through.  The chirp kernel's time hardly depends
+// on K, cuFFT's on the factors (2048 pulses, 4 / 8 times upsampled, chirp 42 /
+// 63 us; taper and cuFFT: K = 424 (53) 71 / 144, 244 (61) 47 / 79, 301 (43) 56 /
+// 73, 319 (11 29) 55 / 61, 377 (13 29) 48 / 75; but 285 (19) 21 / 35, 276 (23)
+// 21 / 31, 372 (31) 28 / 58, 260 (13) 24 / 32).  With a
+// factor of 17 to 31 alone the smaller K go either way, by the number of
+// pulses: K = 304, 8 times, 350 pulses 20 against 17 us, 1024 39 / 27; from 385
+// on cuFFT's 8 times upsampled transforms fall behind (399 63 / 71, 460 65 /
+// 73, 483 66 / 83).
+bool chirp_pays(int K, int pulses) {
+    if (K <= 192 || K > 512) return false;
+    int prime = 1, sum = 0;  // the longest factor; the sum of those from 11 on
+    for (int f = 2, left = K; left > 1; ++f) {
+        if (left % f == 0 && f >= 11) sum += f;
+        for (; left % f == 0; left /= f) prime = f;
+    }
+    if (prime >= 53) return true;
+    return K > 256 && (sum >= 37 || (prime >= 17 && (K >= 385 || pulses <= 768)));
+}
 
 // Calls f(kernel, shared memory, table filler) of shape (K, R); false when
 // there is none.
@@ -543,17 +566,8 @@ bool with_rc_shape(int K, int R, F f) {
     }
     SARBP_RC_SHAPES(SARBP_RC_CASE)
 #undef SARBP_RC_CASE
-    // Chirp kernels where cuFFT has a long prime factor to work through; where
-    // all are small its padded transform is the faster one (2048 pulses, 8
-    // times upsampled, chirp against cuFFT and taper: K = 424 (53) 59 / 133 us,
-    // 509 62 / 176, 201 (67) 46 / 72, but 500 (5) 62 / 42, 247 (19) 47 / 44,
-    // 131 45 / 36).
-    int prime = 1;
-    for (int f = 2, left = K; left > 1; ++f)
-        for (; left % f == 0; left /= f) prime = f;
-    const int k2 = K <= 512 && ((K > 256 && prime >= 17) || (K > 192 && prime >= 53)) ? 32 : 0;
 #define SARBP_RC_CASE(K2_, R_)                                                             \
-    if (k2 == K2_ && R == R_) {                                                            \
+    if (K <= 16 * K2_ && !rc_direct_shape(K) && R == R_) {                                 \
         f(rc_czt_kernel<K2_, R_>, CztTable<K2_, R_>::kSmem,                                \
           [](int k, std::vector<float> &t) { fill_czt_table<K2_, R_>(k, t); });            \
         return true;                                                                       \
@@ -576,14 +590,13 @@ cudaError_t launch_rc(const RcArgs &a, int K, int R, dim3 grid, cudaStream_t s) 
 
 }  // namespace
 
-bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table) {
+bool rc_fused_shape(int K, int R, int pulses, size_t *smem, std::vector<float> *table) {
+    if (!rc_direct_shape(K) && !chirp_pays(K, pulses)) return false;
     return with_rc_shape(K, R, [&](auto, size_t bytes, auto fill) {
         if (smem) *smem = bytes;
         if (table) fill(K, *table);
     });
 }
-
-bool rc_direct_shape(int K) { return K == 256 || K == 512 || K == 1024; }
 
 int rc_fused_resident(int K, int R) {
     int occ = 0;

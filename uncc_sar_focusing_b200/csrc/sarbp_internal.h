@@ -136,11 +136,12 @@ cudaError_t launch_rc_prep(int precision, const void *ph, const void *fac, void 
 cudaError_t launch_rc_prep_batch(const BatchScene *scenes, int nscenes, cudaStream_t s);
 // Fused range compression (mixed precision): taper, zero pad and inverse FFT
 // in one kernel for nfft = R K: K in {256, 512, 1024} and R in {1, 2, 4, 8, 16}
-// (rc_direct_shape), or another K <= 512 with a long prime factor and R in {4,
-// 8} (chirp convolution).  rc_fused_shape says whether (K, R) is one of those and fills the twiddle table (interleaved float
-// re, im) and the kernel's shared-memory bytes; rc_fused_resident: its CTAs
-// resident per SM; grid: CTAs (each loops over pulses).
-bool rc_fused_shape(int K, int R, size_t *smem, std::vector<float> *table);
+// (rc_direct_shape), or another K <= 512 with long prime factors and R in {4,
+// 8} (chirp convolution).  rc_fused_shape says whether `pulses` pulses of (K, R)
+// take one of those and fills the twiddle table (interleaved float re, im) and
+// the kernel's shared-memory bytes; rc_fused_resident: its CTAs resident per
+// SM; grid: CTAs (each loops over pulses).
+bool rc_fused_shape(int K, int R, int pulses, size_t *smem, std::vector<float> *table);
 bool rc_direct_shape(int K);
 int rc_fused_resident(int K, int R);
 cudaError_t launch_rc_fused(const void *ph, const void *fac, const void *table, void *rc, int K, int R, int np,
