@@ -26,8 +26,15 @@ static inline float2 __ffma2_rn(float2 a, float2 b, float2 c) {
 }
 static inline float2 __fmul2_rn(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 static inline float2 __fadd2_rn(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-// the device's estimate, good to 2^-22; a value off by as much stands in for it
-static inline float rsqrtf(float x) { return static_cast<float>(1.0 / std::sqrt(static_cast<double>(x))) * (1.0f + 0x1p-22f); }
+// the device's estimates: values off by 2^-22, up or down, stand in for them
+static inline float off(double v) {
+    static thread_local unsigned n = 0;
+    return static_cast<float>(v * (1.0 + (++n & 1 ? 0x1p-22 : -0x1p-22)));
+}
+static inline float rsqrtf(float x) { return off(1.0 / std::sqrt(static_cast<double>(x))); }
+#define SARBP_HOST_ESTIMATES
+static inline float sqrt_estimate(float x) { return off(std::sqrt(static_cast<double>(x))); }
+static inline float rcp_estimate(float x) { return off(1.0 / static_cast<double>(x)); }
 static inline int __shfl_sync(unsigned, int v, int) { return v; }
 static inline unsigned atomicOr(unsigned *p, unsigned v) {
     const unsigned o = *p;

@@ -87,6 +87,23 @@ def test_phases_and_bins(probe, mx, exchanged, split, radius, spacing):
     check(tile(probe, 9.28e9, radius, spacing, mx, exchanged, split))
 
 
+@pytest.mark.parametrize("radius,spacing,el,mx", [(8e3, 0.3, 45.0, 8), (8e3, 2.0, 30.0, 4), (300.0, 0.2, 20.0, 8),
+                                                  (30.0, 0.1, 40.0, 8), (9.0, 0.1, 60.0, 8), (5.0, 0.1, 88.0, 1)])
+def test_near_field_remainder(probe, radius, spacing, el, mx):
+    """The exact path from a tile's far side to an antenna above it: bins as
+    elsewhere; phases at the roundings of the remainder, six at its largest
+    value (offset, its square, the difference, root, step and product) beside
+    those of the linear part."""
+    t = tile(probe, 9.28e9, radius, spacing, mx, el=el)
+    assert (t["words"][:, 0] & PG_NEAR).all()
+    assert np.isfinite(t["P"]).all() and np.isfinite(t["B"]).all()
+    tol_bin = 4.0 * 2.0 ** -24 * t["W"]
+    assert (np.abs(t["B"] - t["bin"]) <= tol_bin).all(), np.abs(t["B"] - t["bin"]).max()
+    turn = t["P"].astype(np.float64) / (2.0 * math.pi) - t["rev"]
+    off = 2.0 * math.pi * np.abs(turn - np.rint(turn))
+    assert (off <= 2.0 ** -24 * (5.0 * 40.0 + 6.0 * np.abs(t["P"]).max())).all(), off.max()
+
+
 @pytest.mark.parametrize("radius,spacing", [(8e3, 0.1), (60.0, 0.1)])
 @pytest.mark.parametrize("f0", [0.0, 1e-30, -1e-30, 1e-9, 25.0, -3.0e8, -9.28e9, [9.28e9, 0.0, -3.0e8, 0.0]])
 def test_any_start_frequency(probe, f0, radius, spacing):

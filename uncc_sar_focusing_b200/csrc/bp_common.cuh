@@ -103,6 +103,22 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uin
 
 __device__ __forceinline__ double frac_rev(double x) { return x - rint(x); }
 
+// The hardware's estimates of sqrt(x) and 1/x, one instruction each (relative
+// error about 2^-23; 0, infinities and NaN as the exact functions).  A host
+// build of the kernels' arithmetic brings its own.
+#ifndef SARBP_HOST_ESTIMATES
+__device__ __forceinline__ float sqrt_estimate(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_estimate(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+#endif
+
 // Square root of a positive, normal s as sqrt() rounds it: with g ~ sqrt(s)
 // and h ~ 1 / (2 sqrt(s)) from the reciprocal-root estimate (2^-20 or
 // better), r = 1/2 - g h corrects both to 2^-39, and the residual s - g^2,
