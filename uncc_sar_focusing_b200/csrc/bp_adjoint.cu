@@ -171,8 +171,8 @@ constexpr int kAdjThreads = kThreads + 32 * Producers<PB>::kWarps;
 // and the zero entry.
 constexpr int kAdjHdr = 64;
 
-template <int MX, int PB>
-__global__ void __launch_bounds__(kAdjThreads<PB>, 2)
+template <int MX, int PB, int MINB>
+__global__ void __launch_bounds__(kAdjThreads<PB>, MINB)
     bp_adjoint_kernel(const __grid_constant__ BpLaunch L, const float2 *__restrict__ grad,
                       float4 *__restrict__ partials) {
     using M = PixelMap<MX>;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, 2)
             cur.advance(tg, L);
             if (pregeo && i + 1 < n) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, true>(L, p0, rec, win, lane, inv_lam);
+            rewrite_pulses<NQ, true, PB == 1 && MINB == 1 ? 8 : 4>(L, p0, rec, win, lane, inv_lam);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         for (int i = n < 2 ? 0 : n - 2; i < n; ++i) {
@@ -412,7 +412,12 @@ __global__ void __launch_bounds__(32 * kRedWarps)
 template <int MX, int PB>
 cudaError_t launch_adj(const BpLaunch &L, const void *grad, void *partials, size_t smem, cudaStream_t s) {
     constexpr int TX = 8 * MX;
-    auto kern = bp_adjoint_kernel<MX, PB>;
+    // two CTAs per SM (96 registers) unless a stage of one pulse needs more
+    // shared memory than two get
+    auto kern = bp_adjoint_kernel<MX, PB, 2>;
+    if constexpr (PB == 1) {
+        if (smem > 113u * 1024u) kern = bp_adjoint_kernel<MX, PB, 1>;
+    }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     // one CTA per resident slot, each taking a contiguous range of units

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
             cur.advance(scenes, nscenes, rot_later);
             if (pregeo && i + 1 < n) load_records();
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, false>(L, p0, rec, win, lane);
+            rewrite_pulses<NQ, false, PB == 1 ? 8 : 4>(L, p0, rec, win, lane);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         return;

@@ -564,11 +564,15 @@ __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaun
 // FFT (point-target call 106 -> 94 us); the rewrite's second load and
 // difference cost the 1024^2 x 2048 forward kernel 1.9% (1495 -> 1524 us).
 // w: the window's first entry (W - wp); odd: its first sample is the second
-// of those copied (issue_window).
-template <bool ZFORM>
+// of those copied (issue_window).  kGroup: entries of a lane per round.  A
+// stage of one pulse has its one window of 2500 entries and more rewritten by
+// one warp, which the others wait for: there 8 where the registers allow (128
+// 8-row tiles x 256 pulses, 4978 entries: forward 878 -> 738 us, 789 when range
+// profiles were stored as entries; with 96 registers and 2660 entries 208 ->
+// 202, but the adjoint 269 -> 294).
+template <bool ZFORM, int kGroup>
 __device__ __forceinline__ void rewrite_window(uint32_t w, int wp, uint32_t odd, int lane, float nu) {
     const int count = 2 * wp + 2;
-    constexpr int kGroup = 4;  // entries of a lane per round
     int n = (count - 1) / (32 * kGroup) * (32 * kGroup) + lane;  // the lane's first entry of the round
     uint32_t src = w + (static_cast<uint32_t>(n) + odd) * 8u, dst = w + static_cast<uint32_t>(n) * 16u;
     float m = static_cast<float>(n - wp);
@@ -607,7 +611,7 @@ __device__ __forceinline__ void rewrite_window(uint32_t w, int wp, uint32_t odd,
 // The windows of NQ pulses, by their producing warp once the copies have landed;
 // the fence orders these generic-proxy stores before the next bulk copies
 // (async proxy) into the buffer, which the same warp issues.
-template <int NQ, bool ZFORM>
+template <int NQ, bool ZFORM, int GROUP>
 __device__ __forceinline__ void rewrite_pulses(const BpLaunch &L, int p0, const PulseGeo *rec, uint32_t win_s, int lane,
                                                float inv_lam = 0.0f) {
     for (int q = 0; q < NQ; ++q) {
@@ -615,7 +619,7 @@ __device__ __forceinline__ void rewrite_pulses(const BpLaunch &L, int p0, const 
         const int off = L.W - rec[q].wp;
         const uint32_t odd = (static_cast<uint32_t>(p0 + q) * static_cast<uint32_t>(L.nfft) +
                               static_cast<uint32_t>(rec[q].ws + off)) & 1u;
-        rewrite_window<ZFORM>(win_s + (static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) + static_cast<uint32_t>(off)) * 16u,
+        rewrite_window<ZFORM, GROUP>(win_s + (static_cast<uint32_t>(q) * static_cast<uint32_t>(L.wsize) + static_cast<uint32_t>(off)) * 16u,
                               rec[q].wp, odd, lane, ZFORM ? rec[q].kr * inv_lam : 0.0f);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
