@@ -23,7 +23,8 @@
 // registers, 44 bytes spilled outside the sample loop): with 8 warps a CTA and
 // 80 registers the clusters of a small image did not all fit at once, 82 us
 // (256^2: 476).  FP64 keeps 8: 378 us for 128^2 x 256, 443 with 16, and no
-// bound on its registers (it takes 64; 415 us when told to).
+// bound on its registers (it takes 64; 415 us when told to).  Few pulses take
+// CTAs of fewer warps (launch_mf_on).
 #include <cooperative_groups.h>
 #include <cstdint>
 
@@ -105,10 +106,10 @@ __device__ __forceinline__ void turn(double ph, double &cs, double &sn) {
 }
 
 // Pixel block blockIdx.x / (cluster size); the cluster's rank and the warp
-// choose the pulses.  T: float or double.
-template <typename CH, typename T>
+// choose the pulses.  T: float or double; kMfWarps: warps of the CTA.
+template <typename CH, typename T, int kMfWarps>
 __device__ __forceinline__ void mf_body(const float2 *__restrict__ ph, const double *__restrict__ win, const MfLaunch &M) {
-    constexpr int P = CH::kPixels, kMfWarps = CH::kWarps;
+    constexpr int P = CH::kPixels;
     namespace cg = cooperative_groups;
     using Sample = typename CH::Sample;
     __shared__ __align__(16) union Smem {
@@ -187,34 +188,60 @@ __device__ __forceinline__ void mf_body(const float2 *__restrict__ ph, const dou
         sm.sum[warp][j][1][lane] = im[j];
     }
     __syncthreads();
-    const int j = warp >> 1, c = warp & 1;  // this thread's pixel and component of the CTA's sum
-    T t = 0;
-    if (j < P) {
+    // component i & 1 of pixel i >> 1 of the CTA's sum: warp i mod kMfWarps
+#pragma unroll
+    for (int i = warp; i < 2 * P; i += kMfWarps) {
+        const int j = i >> 1, c = i & 1;
+        T t = 0;
         for (int w = 0; w < kMfWarps; ++w) t += sm.sum[w][j][c][lane];
-        __syncwarp();
-        sm.sum[0][j][c][lane] = t;  // read by this warp only before now
+        sm.sum[0][j][c][lane] = t;  // read by this thread only before now
     }
-    cluster.sync();
-    if (rank == 0 && j < P) {
-        for (int r = 1; r < ranks; ++r) t += *cluster.map_shared_rank(&sm.sum[0][j][c][lane], r);
-        const long long q = q0 + 32 * j;
-        if (q < npix) static_cast<T *>(M.img)[2 * q + c] = t;
+    if (ranks > 1) cluster.sync();
+    if (rank == 0) {
+#pragma unroll
+        for (int i = warp; i < 2 * P; i += kMfWarps) {
+            const int j = i >> 1, c = i & 1;
+            T t = sm.sum[0][j][c][lane];
+            for (int r = 1; r < ranks; ++r) t += *cluster.map_shared_rank(&sm.sum[0][j][c][lane], r);
+            const long long q = q0 + 32 * j;
+            if (q < npix) static_cast<T *>(M.img)[2 * q + c] = t;
+        }
     }
-    cluster.sync();  // the other ranks' shared memory stays until it has been read
+    if (ranks > 1) cluster.sync();  // the other ranks' shared memory stays until it has been read
 }
 
-__global__ void __launch_bounds__(32 * MfFloat::kWarps, 2)
+// W warps a CTA: CH::kWarps, 4 or 1.  The small CTAs take 128 registers: one
+// pulse x 256 samples on 16^2 pixels 8.7 us, with 64 (44 bytes spilled, the
+// sample loads not ahead) 12.2; 512^2 pixels x 12 pulses 61 against 57.
+template <int W>
+__global__ void __launch_bounds__(32 * W, W == MfFloat::kWarps ? 2 : MfFloat::kWarps / W)
     mf_kernel(const float2 *__restrict__ ph, const double *__restrict__ win, MfLaunch M) {
-    mf_body<MfFloat, float>(ph, win, M);
+    mf_body<MfFloat, float, W>(ph, win, M);
 }
 
-__global__ void __launch_bounds__(32 * MfDouble::kWarps)
+template <int W>
+__global__ void __launch_bounds__(32 * W)
     mf_kernel64(const float2 *__restrict__ ph, const double *__restrict__ win, MfLaunch M) {
-    mf_body<MfDouble, double>(ph, win, M);
+    mf_body<MfDouble, double, W>(ph, win, M);
+}
+
+// Warps of a CTA for np pulses.  All CTAs there are running at once: the fewest
+// rounds of pulses.  More than fit: fewer slots (rounds x warps) by a fifth,
+// since a warp without a pulse holds its place until the others are done (512^2
+// pixels x 64 samples: one pulse 49 us on CTAs of 16 warps, 9 on CTAs of one; 3
+// pulses 50 / 20; 12 73, 61 on CTAs of 4; 30 140, 165 on CTAs of one; FP64 12
+// pulses 123 on 8, 85 on 4).
+int mf_warps(int full, int np, long long blocks, int sms) {
+    if (np >= 2 * full) return full;
+    if (blocks < 2LL * sms) return np == 1 ? 1 : (np <= 4 ? 4 : full);
+    int best = full;
+    for (const int w : {4, 1})
+        if (5 * ((np + w - 1) / w * w) < 4 * ((np + best - 1) / best * best)) best = w;
+    return best;
 }
 
 template <typename CH, typename F>
-cudaError_t launch_mf_on(F kern, const float2 *ph, const double *win, const MfLaunch &M, cudaStream_t s) {
+cudaError_t launch_mf_on(F full, F four, F one, const float2 *ph, const double *win, const MfLaunch &M, cudaStream_t s) {
     const long long npix = static_cast<long long>(M.nx) * M.ny * M.nz;
     const long long blocks = (npix + 32 * CH::kPixels - 1) / (32 * CH::kPixels);
     int dev = 0, sms = 0;
@@ -237,25 +264,28 @@ cudaError_t launch_mf_on(F kern, const float2 *ph, const double *win, const MfLa
             ranks = r;
         }
     }
+    const int warps = mf_warps(CH::kWarps, M.np, blocks, sms);
+    if (warps < CH::kWarps) ranks = 1;
     if (blocks < 1 || blocks * ranks > 0x7fffffffLL) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(blocks * ranks));
-    cfg.blockDim = dim3(32 * CH::kWarps);
+    cfg.blockDim = dim3(32 * warps);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = static_cast<unsigned>(ranks);
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, ph, win, M);
+    cfg.numAttrs = ranks > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, warps == CH::kWarps ? full : (warps == 4 ? four : one), ph, win, M);
 }
 
 }  // namespace
 
 cudaError_t launch_mf(const void *ph, const double *win, const MfLaunch &M, bool fp64, cudaStream_t s) {
     const float2 *x = static_cast<const float2 *>(ph);
-    return fp64 ? launch_mf_on<MfDouble>(mf_kernel64, x, win, M, s) : launch_mf_on<MfFloat>(mf_kernel, x, win, M, s);
+    return fp64 ? launch_mf_on<MfDouble>(mf_kernel64<MfDouble::kWarps>, mf_kernel64<4>, mf_kernel64<1>, x, win, M, s)
+                : launch_mf_on<MfFloat>(mf_kernel<MfFloat::kWarps>, mf_kernel<4>, mf_kernel<1>, x, win, M, s);
 }
 
 }  // namespace sarbp
