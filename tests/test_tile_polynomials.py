@@ -30,9 +30,11 @@ def probe(tmp_path_factory):
     return lib.tile_probe
 
 
-def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392, lam=32.1, el=30.0, look=(0.0, 30.0, 88.0, 200.0)):
+def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392, lam=32.1, el=30.0,
+         look=(0.0, 30.0, 88.0, 200.0), near=1.0):
     """The tile's phases, bins and pulse words, with their exact values:
-    phase modulo one turn, window-centred bin (float64)."""
+    phase modulo one turn, window-centred bin (float64).  near: a factor on the
+    far-field test's constant."""
     az = np.radians(np.asarray(look))
     n = len(az)
     x = radius * math.cos(math.radians(el)) * np.cos(az)
@@ -48,7 +50,7 @@ def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392
     P = np.full((n, 8 * mx, 64), np.nan, dtype=np.float32)
     B = P.copy()
     words = np.zeros((n, 3), dtype=np.int32)
-    err = probe(geo.ctypes.data, n, nfft, lam, dx, dy, left, bottom, W, 16.0 * hd, 0.625 * hd ** 4 / 1e-7, mx,
+    err = probe(geo.ctypes.data, n, nfft, lam, dx, dy, left, bottom, W, 16.0 * hd, near * 0.625 * hd ** 4 / 1e-7, mx,
                 int(exchanged), int(split), P.ctypes.data, B.ctypes.data, words.ctypes.data)
     assert err == 0
     if exchanged:  # the map's rows run along the image's columns
@@ -61,7 +63,8 @@ def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392
     bin_ = lam * dR + 0.5 * nfft - words[:, 1, None, None] - W
     rc = np.sqrt((x - left - 4 * mx * dx) ** 2 + (y - bottom - 32 * dy) ** 2 + z * z)
     far = (0.625 * hd ** 4 / rc ** 3)[:, None, None]  # metres the expansion may be off
-    return dict(P=P, B=B, words=words, rev=rev, bin=bin_, far=far, kr=4.0 * math.pi * f[:, None, None] / C, lam=lam, W=W)
+    v = np.stack([x - left - 4 * mx * dx, y - bottom - 32 * dy, z], 1)
+    return dict(rc=rc, r0=r0, v=v, P=P, B=B, words=words, rev=rev, bin=bin_, far=far, kr=4.0 * math.pi * f[:, None, None] / C, lam=lam, W=W)
 
 
 def check(t):
@@ -119,3 +122,28 @@ def test_any_start_frequency(probe, f0, radius, spacing):
 def test_wide_swaths(probe, lam):
     """Range bins of kilometres and more: the phase does not depend on them."""
     check(tile(probe, 9.28e9, 8e3, 0.1, 8, lam=lam))
+
+
+@pytest.mark.parametrize("mx,bound", [(8, 10.5), (4, 0.9), (2, 0.0)])
+def test_cubic_term_of_the_row_steps(probe, mx, bound):
+    """The k^3 term over a thread's rows k = -mx/2 .. mx/2 - 1 is carried by the
+    lower terms: what is left of k^3 is `bound` at most, and the phase is off
+    by 8 q30 kr / lambda times that.  At 20 half-diagonals (with the far-field
+    test turned down to 16) it stands far above the roundings, against the
+    expansion itself in FP64."""
+    spacing, f0, lam = 0.1, 9.28e9, 32.1
+    hd = math.hypot(4 * mx * spacing, 32 * 1.1 * spacing)
+    radius, el = 20.0 * hd, math.degrees(math.acos(math.sqrt(1.0 / 3.0)))  # the largest cubic term along the rows
+    t = tile(probe, f0, radius, spacing, mx, el=el, lam=lam, look=(-20.0, 0.0, 15.0, 170.0), near=0.0)
+    assert not (t["words"][:, 0] & PG_NEAR).any()
+    i = (np.arange(8 * mx) - 4 * mx)[None, :, None] * spacing
+    j = (np.arange(64) - 32)[None, None, :] * 1.1 * spacing
+    v, rc = t["v"], t["rc"][:, None, None]
+    along = (v[:, 0, None, None] * i + v[:, 1, None, None] * j) / rc
+    e = i * i + j * j - along * along
+    rev = 2.0 * f0 / C * (rc - t["r0"][:, None, None] - along + e * (0.5 / rc + along * 0.5 / rc ** 2))
+    turn = t["P"].astype(np.float64) / (2.0 * math.pi) - rev
+    off = 2.0 * math.pi * np.abs(turn - np.rint(turn))
+    u = np.abs(v[:, 0]) / t["rc"]
+    q30 = (2.0 * math.pi * f0 / C / t["rc"] ** 2 * u * (1.0 - u * u)).max() * spacing ** 3
+    assert off.max() <= 8.0 * bound * q30 + 5.0 * 2.0 ** -24 * np.abs(t["P"]).max(), (off.max(), 8.0 * bound * q30)

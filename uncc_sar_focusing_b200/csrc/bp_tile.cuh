@@ -291,8 +291,10 @@ __device__ __forceinline__ bool record_exchanged(const BpLaunch &L, long long t)
 // its two columns (13 paired operations a pulse), so phase and bin cost 22
 // paired operations per 16 pixels instead of a full evaluation of t, t^2 -
 // |d|^2 and the remainder for each (64).  The
-// k^3 term of tau Q (2 k <= 8 rows: 1/64 of the tile's cubic term, < 6e-7 rad at
-// 100 m / 1024 pixels, 8 km) is folded into a by least squares over k.
+// k^3 term of tau Q is carried by the lower ones (least squares): at most 10.5 of
+// its 64 at the outer row is left, 2e-7 rad at 0.12 m and 8 km, 3e-7 at 0.5 m and
+// 50 km, 6e-7 at 3.9 m and 800 km, the coarsest tiles of 64 rows that are far
+// field there.
 //   [2e]     phase, bin, x1 = i (q11 + i q21), x2 = q02 + i q12
 //   [2e + 1] phase step, bin step, step's j term, k^2 term
 //   [16..]   2 pi frac(j beta), j = -32..-1
@@ -330,8 +332,10 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         un1 = make_float4(2.0f * q12, 4.0f * q21, c2.z, c2.w);
     }
     __syncwarp();
-    // k^3 ~ kFit k over the thread's rows k = -kMid .. MX - kMid - 1
-    constexpr float kFit = MX == 8 ? 452.0f / 44.0f : (MX == 4 ? 3.0f : (MX == 2 ? 1.0f : 0.0f));
+    // over the thread's rows, m = k + 1/2 = -(MX - 1)/2 .. (MX - 1)/2, m^3 ~ beta
+    // m by least squares; so k^3 ~ kC0 + kC1 k - 3/2 k^2
+    constexpr float kBeta = MX == 8 ? 9.25f : (MX == 4 ? 2.05f : 0.25f);
+    constexpr float kC0 = 0.5f * kBeta - 0.125f, kC1 = kBeta - 0.75f;
     for (int t = lane; t < 8 * NQ; t += 32) {
         const int q = t >> 3, e = t & 7;
         const float4 *w = reinterpret_cast<const float4 *>(rec + q);
@@ -343,14 +347,14 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         const float i = static_cast<float>(M::mid_row(e));
         const double id = static_cast<double>(i);
         const double pr = fma(id, d0.y, d0.x), ps = 2.0 * d0.y;
-        const float nl = i * i * fmaf(i, qa.w, qa.x);
-        const float an = fmaf(8.0f * kFit, qa.w, 2.0f * i * fmaf(3.0f * i, qa.w, 2.0f * qa.x));
+        const float nl = fmaf(8.0f * kC0, qa.w, i * i * fmaf(i, qa.w, qa.x));
+        const float an = fmaf(8.0f * kC1, qa.w, 2.0f * i * fmaf(3.0f * i, qa.w, 2.0f * qa.x));
         row[0] = make_float4(fmaf(qb.z, nl, static_cast<float>(kTwoPi * (pr - rint(pr)))),
                              static_cast<float>(fma(id, gam, B0 - L.W)) + nl, i * fmaf(i, qb.x, qa.y),
                              fmaf(i, qb.y, qa.z));
         row[1] = make_float4(fmaf(qb.z, an, static_cast<float>(kTwoPi * (ps - rint(ps)))),
                              static_cast<float>(2.0 * gam) + an, 2.0f * fmaf(2.0f * i, qb.x, qa.y),
-                             4.0f * fmaf(3.0f * i, qa.w, qa.x));
+                             4.0f * fmaf(3.0f * (i - 1.0f), qa.w, qa.x));
     }
     __syncwarp();
     const double jd = static_cast<double>(lane - kTY / 2);
