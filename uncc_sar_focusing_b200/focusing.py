@@ -25,22 +25,18 @@ _WINDOW = {None: N.WINDOW_NONE, "none": N.WINDOW_NONE, "hamming": N.WINDOW_HAMMI
 _ITEM = {np.float64: 0, np.complex64: 1, np.complex128: 2}
 
 
-def _torch():
-    """The torch module if the caller's program has loaded it (a tensor can
-    only come from there), else None."""
-    return sys.modules.get("torch")
-
-
 def _is_torch(x) -> bool:
-    t = _torch()
-    return t is not None and isinstance(x, t.Tensor)
+    """By the type's own module, without the torch module, which another thread
+    may be half way through importing while there are only arrays here."""
+    m = type(x).__module__
+    return m == "torch" or m.startswith("torch")
 
 
 def _ptr(x, dtype, count: Optional[int] = None):
     """(pointer, memory kind, keep-alive) of a numpy array or CUDA tensor."""
-    t = _torch()
-    if t is not None and isinstance(x, t.Tensor):
-        want = (t.float64, t.complex64, t.complex128)[_ITEM[dtype]]
+    if _is_torch(x):
+        torch = sys.modules["torch"]
+        want = (torch.float64, torch.complex64, torch.complex128)[_ITEM[dtype]]
         if not x.is_cuda:
             raise ValueError("torch tensors passed to the engine must live on a CUDA device")
         if x.dtype is not want or not x.is_contiguous():
@@ -56,11 +52,10 @@ def _ptr(x, dtype, count: Optional[int] = None):
 
 def _stream(*arrays):
     """Torch's current stream when an array is a CUDA tensor, else the default stream."""
-    t = _torch()
-    if t is not None:
-        for a in arrays:
-            if isinstance(a, t.Tensor):
-                return t.cuda.current_stream().cuda_stream
+    for a in arrays:
+        if _is_torch(a):
+            torch = sys.modules["torch"]
+            return torch.cuda.current_stream().cuda_stream
     return 0
 
 
