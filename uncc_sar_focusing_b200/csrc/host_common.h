@@ -133,11 +133,14 @@ inline size_t margin_samples(int wsize) { return static_cast<size_t>(wsize) + 4;
 
 // Range-bin window of a tile of (8 mx) x 64 pixels with steps dx, dy at
 // lambda bins per metre: W = ceil(lambda * half-diagonal) + 3 bins each side,
-// wsize = 2W + 2 window entries; hd the half-diagonal in metres.
+// wsize = 2W + 2 window entries; hd the half-diagonal in metres.  Any window
+// past the 65536 entries that callers refuse gets the same W (a bin scale of
+// 2^31 bins and more to the half-diagonal would wrap around).
 inline void tile_window(double lambda, double dx, double dy, int mx, int *W, int *wsize, double *hd) {
     const double hx = 0.5 * 8.0 * mx * dx, hy = 0.5 * 64.0 * dy;
     *hd = std::sqrt(hx * hx + hy * hy);
-    *W = static_cast<int>(std::ceil(lambda * *hd)) + 3;
+    const double w = std::ceil(lambda * *hd) + 3.0;
+    *W = w < 65536.0 ? static_cast<int>(w) : 65536;
     *wsize = 2 * (*W) + 2;
 }
 

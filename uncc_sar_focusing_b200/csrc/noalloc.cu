@@ -117,14 +117,15 @@ extern "C" SARBP_API int sarbp_backproject_noalloc(const sarbp_plan_desc *desc, 
     for (int pass = 0; pass < 2 && !tc.mx; ++pass) {
         const size_t limit = pass == 0 ? 110u * 1024u : 227u * 1024u;
         for (const auto &c : cand) {
-            const double hx = 0.5 * 8.0 * c[0] * dx, hy = 0.5 * 64.0 * dy;
-            const int w = static_cast<int>(std::ceil(lambda * std::sqrt(hx * hx + hy * hy))) + 3;
+            int w, ws;
+            double hd;
+            host::tile_window(lambda, dx, dy, c[0], &w, &ws, &hd);
             const TileConfig t{c[0], c[1]};
-            const size_t sm = bp_mixed_smem_bytes(t, 2 * w + 2);
-            if (2 * w + 2 > (1 << 16) || sm > limit) continue;
+            const size_t sm = bp_mixed_smem_bytes(t, ws);
+            if (ws > (1 << 16) || sm > limit) continue;
             tc = t;
             W = w;
-            wsize = 2 * w + 2;
+            wsize = ws;
             smem = sm;
             break;
         }
