@@ -35,6 +35,18 @@ static inline float rsqrtf(float x) { return off(1.0 / std::sqrt(static_cast<dou
 #define SARBP_HOST_ESTIMATES
 static inline float sqrt_estimate(float x) { return off(std::sqrt(static_cast<double>(x))); }
 static inline float rcp_estimate(float x) { return off(1.0 / static_cast<double>(x)); }
+// off by up to 2^-20, the low word zero
+static inline double rsqrt_estimate(double x) {
+    static thread_local uint64_t n = 1;
+    n = n * 6364136223846793005ull + 1442695040888963407ull;
+    const double e = (static_cast<double>(n >> 11) * 0x1p-53 * 2.0 - 1.0) * (0x1p-20 - 0x1p-21);
+    double y = 1.0 / std::sqrt(x) * (1.0 + e);
+    uint64_t b;
+    std::memcpy(&b, &y, 8);
+    b &= ~0xffffffffull;
+    std::memcpy(&y, &b, 8);
+    return y;
+}
 static inline int __shfl_sync(unsigned, int v, int) { return v; }
 static inline unsigned atomicOr(unsigned *p, unsigned v) {
     const unsigned o = *p;
@@ -155,4 +167,12 @@ extern "C" int tile_probe(const double *geo, int np, int nfft, double lambda, do
         default: (split ? run<1, true> : run<1, false>)(L, exchanged != 0, phase, bin, words); break;
     }
     return static_cast<int>(err);
+}
+
+extern "C" void sqrt_probe(const double *x, double *out, int n) {
+    for (int i = 0; i < n; ++i) out[i] = sqrt_rn(x[i]);
+}
+
+extern "C" void rotation_probe(const double *x, double *cs, double *sn, int n) {
+    for (int i = 0; i < n; ++i) rotation(x[i], cs[i], sn[i]);
 }

@@ -3,6 +3,7 @@
 #define SARBP_HOST_ESTIMATES
 static inline float sqrt_estimate(float x) { return x; }
 static inline float rcp_estimate(float x) { return x; }
+static inline double rsqrt_estimate(double x) { return x; }
 static inline int __shfl_sync(unsigned, int v, int) { return v; }
 static inline unsigned atomicOr(unsigned *p, unsigned v) { return *p |= v; }
 static inline size_t __cvta_generic_to_shared(const void *p) { return reinterpret_cast<size_t>(p); }

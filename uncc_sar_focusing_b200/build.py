@@ -90,7 +90,7 @@ def build_lib(force: bool = False, jobs: int = 8) -> str:
 
 def build_probes(force: bool = False) -> str:
     src = os.path.join(CSRC, "probes.cu")
-    if force or _newer(PROBE_LIB, [src, __file__]):
+    if force or _newer(PROBE_LIB, [src, os.path.join(CSRC, "bp_common.cuh"), __file__]):
         _run([NVCC] + CUFLAGS + ["-shared", "-o", PROBE_LIB, src, "-cudart", "static"])
     return PROBE_LIB
 

@@ -103,9 +103,10 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uin
 
 __device__ __forceinline__ double frac_rev(double x) { return x - rint(x); }
 
-// The hardware's estimates of sqrt(x) and 1/x, one instruction each (relative
-// error about 2^-23; 0, infinities and NaN as the exact functions).  A host
-// build of the kernels' arithmetic brings its own.
+// The hardware's estimates of sqrt(x), 1/x (relative error about 2^-23; 0,
+// infinities and NaN as the exact functions) and, in double, 1/sqrt(x) (2^-20 or
+// better), one instruction each.  A host build of the kernels' arithmetic brings
+// its own.
 #ifndef SARBP_HOST_ESTIMATES
 __device__ __forceinline__ float sqrt_estimate(float x) {
     float y;
@@ -117,15 +118,21 @@ __device__ __forceinline__ float rcp_estimate(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ double rsqrt_estimate(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
 #endif
 
-// Square root of a positive, normal s as sqrt() rounds it: with g ~ sqrt(s)
-// and h ~ 1 / (2 sqrt(s)) from the reciprocal-root estimate (2^-20 or
-// better), r = 1/2 - g h corrects both to 2^-39, and the residual s - g^2,
-// exact by fused multiply-add, corrects g once more (Markstein's scheme).
+// Square root of a positive, normal s, rounded as sqrt() rounds it but for
+// about one argument in 2^25, where it is the neighbour: with g ~ sqrt(s) and h
+// ~ 1 / (2 sqrt(s)) from the reciprocal-root estimate (2^-20 or better), r = 1/2
+// - g h corrects both to 2^-39, and the residual s - g^2 by fused multiply-add
+// corrects g once more, to 2^-78 before the last rounding (Markstein's scheme,
+// whose proof wants a better estimate).
 __device__ __forceinline__ double sqrt_rn(double s) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    const double y = rsqrt_estimate(s);
     double g = s * y;
     double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));  // y / 2
     const double r = fma(-g, h, 0.5);
@@ -134,7 +141,7 @@ __device__ __forceinline__ double sqrt_rn(double s) {
     return fma(fma(-g, g, s), h, g);
 }
 
-// exp(+j 2 pi ph), |ph| < 2^50: ph = n/4 + r exactly, |r| <= 1/8; sin and cos
+// exp(+j 2 pi ph), |ph| <= 2^49: ph = n/4 + r exactly, |r| <= 1/8; sin and cos
 // of 2 pi r as polynomials in r^2 (interpolated at the Chebyshev nodes of [0,
 // 1/64] in 60 digits; errors 2e-17 and 5e-17 before rounding), then the
 // quadrant n mod 4 by swap and sign.

@@ -2,8 +2,8 @@
 //
 // Same tiling, shared-memory window staging (cp.async.bulk + mbarrier), pixel
 // map and output layout as the mixed kernel in bp_mixed.cu, but every
-// pixel-pulse is computed directly in double: |a_p - x_q| with a correctly
-// rounded square root, the bin index, the linear interpolation of FP64 range
+// pixel-pulse is computed directly in double: |a_p - x_q| with a square root
+// rounded as sqrt() rounds it (sqrt_rn), the bin index, the linear interpolation of FP64 range
 // profiles and the rotation exp(+j 2 pi k dR) (k = 2 f0 / c, reduced mod one
 // revolution), accumulated in double.  It is the accuracy path and the FP64
 // baseline the mixed kernel is measured against; semantics as bp_mixed.cu.

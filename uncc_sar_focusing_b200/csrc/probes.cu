@@ -6,7 +6,10 @@
 // independent chains per thread; sarbp_probe times it with CUDA events and
 // returns the operation rate, so the bench divides by peaks measured on the
 // same GPU in the same run.  Built into libsarbp_probes.so, used by bench.py.
+// sarbp_probe_math evaluates the kernels' own square root and rotation for tests.
 #include <cuda_runtime.h>
+
+#include "bp_common.cuh"
 
 namespace {
 
@@ -82,9 +85,29 @@ __global__ void probe_lds128(float *out, int iters) {
     if (s == 123.456f) out[0] = s;
 }
 
+__global__ void probe_math(int which, const double *x, double *a, double *b, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (which == 0) {
+            a[i] = sarbp::sqrt_rn(x[i]);
+            b[i] = sqrt(x[i]);
+        } else {
+            sarbp::rotation(x[i], a[i], b[i]);
+        }
+    }
+}
+
 }  // namespace
 
 extern "C" {
+
+// n values in device memory.  which 0: a = sqrt_rn(x), b = sqrt(x); 1: a, b =
+// cosine and sine of 2 pi x by rotation().  Returns 0 or a CUDA error code.
+__attribute__((visibility("default"))) int sarbp_probe_math(int which, const double *x, double *a, double *b, int n) {
+    if (which < 0 || which > 1 || !x || !a || !b || n < 1) return -1;
+    probe_math<<<148 * 8, 256>>>(which, x, a, b, n);
+    const cudaError_t e = cudaGetLastError();
+    return static_cast<int>(e == cudaSuccess ? cudaDeviceSynchronize() : e);
+}
 
 // which: 0 FP32 FMA, 1 FP64 FMA, 2 __sincosf, 3 LDS.128.
 // Returns 0 and *ops_per_s (FMA, sincos or 16-byte loads per second) and
