@@ -193,7 +193,8 @@ struct __align__(16) PulseGeo {
     double A, alpha;   // frac(k (Rc - R0)); frac(-k ux dx): revolutions per x step
     double beta, B0;   // frac(-k uy dy); tile-centre bin relative to the window start
     double gam, eta;   // -lambda ux dx, -lambda uy dy: bins per x / y step
-    float a8r, b32r, g8, e32;  // 2 pi frac(8 alpha), 2 pi frac(32 beta) (rad); 8 gam, 32 eta (bins)
+    float b32r, e32;         // 2 pi frac(32 beta) (rad), 32 eta (bins)
+    float pad2, pad3;
     float tx, ty, h, hr;     // ux dx, uy dy (m); 1/(2 Rc), 1/(2 Rc^2)
     float kr, rc, lo, hi;    // 2 pi k (rad/m); Rc; valid iff lo < B_rel < hi
     int ws;                  // start bin of the tile's full window (W bins each side; may be negative)

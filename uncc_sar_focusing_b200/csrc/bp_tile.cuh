@@ -178,9 +178,7 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     g.B0 = bc - static_cast<double>(ws);
     g.gam = -L.lambda * ux * dx;
     g.eta = -L.lambda * uy * dy;
-    g.a8r = static_cast<float>(kTwoPi * frac_rev(8.0 * al));
     g.b32r = static_cast<float>(kTwoPi * frac_rev(32.0 * be));
-    g.g8 = static_cast<float>(8.0 * g.gam);
     g.e32 = static_cast<float>(32.0 * g.eta);
     g.tx = static_cast<float>(ux * dx);
     g.ty = static_cast<float>(uy * dy);
@@ -316,7 +314,7 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
     float4 un0 = make_float4(0.f, 0.f, 0.f, 0.f), un1 = un0;
     if (lane < NQ) {
         float4 *w = reinterpret_cast<float4 *>(rec + lane);
-        const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // a8r, b32r, g8, e32; tx, ty, h, hr; kr, rc, lo, hi
+        const float4 c0 = w[3], c1 = w[4], c2 = w[5];  // b32r, e32; tx, ty, h, hr; kr, rc, lo, hi
         const bool ex = rec[lane].flags & PG_EXCHANGED;
         const float dx = static_cast<float>(ex ? L.dy : L.dx), dy = static_cast<float>(ex ? L.dx : L.dy);
         const bool near = rec[lane].flags & PG_NEAR;
@@ -328,7 +326,7 @@ __device__ __forceinline__ void write_poly_tables(float4 *tabs, PulseGeo *rec, i
         float4 *coef = tabs + lane * kPolyEntries + kPolyCols;
         coef[0] = make_float4(mh * n20, mh * n11, mh * n02, mr * c1.x * n20);
         coef[1] = make_float4(q21, q12, tau, 0.0f);
-        un0 = make_float4(c0.y, c0.w * (1.0f / 32.0f), tau, q03);
+        un0 = make_float4(c0.x, c0.y * (1.0f / 32.0f), tau, q03);
         un1 = make_float4(2.0f * q12, 4.0f * q21, c2.z, c2.w);
     }
     __syncwarp();

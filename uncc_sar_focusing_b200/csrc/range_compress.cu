@@ -304,12 +304,12 @@ __global__ void __launch_bounds__(32 * R) rc_fused_kernel(const __grid_constant_
 // rows of the time, 40 without, 20 us here; 777 of 501: 96 and 79 to 31 us.
 template <int K2, int R>
 struct CztTable {
+    static_assert(K2 == 32 && (R == 4 || R == 8), "the chirp kernel's shapes");
     static constexpr int M = 32 * K2, KM = M / 2;
     static constexpr int kChirp = 0;               // c[k], k < KM
     static constexpr int kH = KM;                  // H[u], u < M
-    static constexpr int kTwA = kH + M;            // W_M^{k1 m2} at m2 * 32 + k1
-    static constexpr int kTwB = K2 == 32 ? kTwA : kTwA + M;  // W_M^{m2 v1} at v1 * K2 + m2
-    static constexpr int kWn = kTwB + M;           // W_N^i, i < 32 R
+    static constexpr int kTw = kH + M;             // W_M^{k1 m2} at m2 * 32 + k1
+    static constexpr int kWn = kTw + M;            // W_N^i, i < 32 R
     static constexpr int kWnk = kWn + 32 * R;      // W_N^{32 i}, i < K2 / 2 * R
     static constexpr int kSize = kWnk + K2 / 2 * R;
     // row of one sub-transform: K2 x 33 for the transposes, and 16/R mod 16 as RcTable::kReg
@@ -373,17 +373,15 @@ __device__ __forceinline__ void rc_czt_body(const float2 *__restrict__ ph, const
             for (int m2 = 0; m2 < K2; ++m2) {
                 const int at = bit_reverse<K2>(m2);
                 reg[m2 * 33 + lane] = cmulf(at < H2 ? lo[at < H2 ? at : 0] : hi[at < H2 ? 0 : at - H2],
-                                            tb[T::kTwA + m2 * 32 + lane]);
+                                            tb[T::kTw + m2 * 32 + lane]);
             }
         }
         __syncwarp();
-        float2 w[32];
-        if (lane < K2) {
+        {
+            float2 w[32];
 #pragma unroll
             for (int k1 = 0; k1 < 32; ++k1) w[k1] = reg[lane * 33 + k1];
-        }
-        __syncwarp();
-        if (lane < K2) {
+            __syncwarp();
             ifft_dif<32>(w);
             // times H, conjugated: the second transform runs in the same direction
             float2 z[32];
@@ -395,7 +393,7 @@ __device__ __forceinline__ void rc_czt_body(const float2 *__restrict__ ph, const
             ifft_dif<32>(z);
 #pragma unroll
             for (int v1 = 0; v1 < 32; ++v1)
-                reg[lane * 33 + v1] = cmulf(z[bit_reverse<32>(v1)], tb[T::kTwB + v1 * K2 + lane]);
+                reg[lane * 33 + v1] = cmulf(z[bit_reverse<32>(v1)], tb[T::kTw + v1 * 32 + lane]);
         }
         __syncwarp();
         float2 q[K2];
@@ -411,22 +409,18 @@ __device__ __forceinline__ void rc_czt_body(const float2 *__restrict__ ph, const
         __syncthreads();
         prefetch(p + gridDim.x);
         // rc[R m + r] = regions[r][m]
-        if (R > 1) {
-            float4 *row = reinterpret_cast<float4 *>(rc + static_cast<long long>(p) * N);
-            for (int b = 2 * tid; b < N; b += 64 * R) {
-                const float2 u = regions[(b & (R - 1)) * REG + (b >> LOGR)];
-                const float2 un = regions[((b + 1) & (R - 1)) * REG + ((b + 1) >> LOGR)];
-                row[b >> 1] = make_float4(u.x, u.y, un.x, un.y);
-            }
-        } else {
-            for (int b = tid; b < N; b += 32) rc[static_cast<long long>(p) * N + b] = regions[b];
+        float4 *row = reinterpret_cast<float4 *>(rc + static_cast<long long>(p) * N);
+        for (int b = 2 * tid; b < N; b += 64 * R) {
+            const float2 u = regions[(b & (R - 1)) * REG + (b >> LOGR)];
+            const float2 un = regions[((b + 1) & (R - 1)) * REG + ((b + 1) >> LOGR)];
+            row[b >> 1] = make_float4(u.x, u.y, un.x, un.y);
         }
     }
 }
 
 // registers for two CTAs of 256 threads per SM
 template <int K2, int R>
-__global__ void __launch_bounds__(32 * R, R <= 8 ? 2 : 1) rc_czt_kernel(const __grid_constant__ RcArgs a) {
+__global__ void __launch_bounds__(32 * R, 2) rc_czt_kernel(const __grid_constant__ RcArgs a) {
     const RcJob j(a);
     rc_czt_body<K2, R>(j.ph, j.fac, a.tab, j.rc, j.K, j.np);
 }
@@ -470,10 +464,8 @@ void fill_czt_table(int K, std::vector<float> &t) {
     dft_pow2(h);
     for (int u = 0; u < T::M; ++u) put(T::kH + u, h[u]);
     for (int m2 = 0; m2 < K2; ++m2)
-        for (int k1 = 0; k1 < 32; ++k1) {
-            put(T::kTwA + m2 * 32 + k1, unit(static_cast<double>(k1) * m2, T::M));
-            put(T::kTwB + k1 * K2 + m2, unit(static_cast<double>(k1) * m2, T::M));
-        }
+        for (int k1 = 0; k1 < 32; ++k1)
+            put(T::kTw + m2 * 32 + k1, unit(static_cast<double>(k1) * m2, T::M));
     const double N = static_cast<double>(R) * K;
     for (int i = 0; i < 32 * R; ++i) put(T::kWn + i, unit(i, N));
     for (int i = 0; i < K2 / 2 * R; ++i) put(T::kWnk + i, unit(32.0 * i, N));
