@@ -568,10 +568,10 @@ __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaun
 // w: the window's first entry (W - wp); odd: its first sample is the second
 // of those copied (issue_window).  kGroup: entries of a lane per round.  A
 // stage of one pulse has its one window of 2500 entries and more rewritten by
-// one warp, which the others wait for: there 8 where the registers allow (128
-// 8-row tiles x 256 pulses, 4978 entries: forward 878 -> 738 us, 789 when range
-// profiles were stored as entries; with 96 registers and 2660 entries 208 ->
-// 202, but the adjoint 269 -> 294).
+// one warp, which the others wait for: there 8 (128 8-row tiles x 256 pulses,
+// 4978 entries: forward 823 -> 692 us, 787 when range profiles were stored as
+// entries; adjoint 1066 -> 879), 6 for the adjoint on 96 registers (2660
+// entries: 3 267, 4 282, 6 255, 8 278 us).
 template <bool ZFORM, int kGroup>
 __device__ __forceinline__ void rewrite_window(uint32_t w, int wp, uint32_t odd, int lane, float nu) {
     const int count = 2 * wp + 2;
