@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, MINB)
             cur.advance(tg, L);
             if (pregeo && i + 1 < n) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, true, PB > 1 ? 4 : (MINB == 1 ? 8 : 6)>(L, p0, rec, win, lane, inv_lam);
+            rewrite_pulses<NQ, true, (PB > 1 ? 4 : (MINB == 1 ? 8 : 6))>(L, p0, rec, win, lane, inv_lam);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         for (int i = n < 2 ? 0 : n - 2; i < n; ++i) {
