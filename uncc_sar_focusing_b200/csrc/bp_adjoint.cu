@@ -164,6 +164,10 @@ __device__ __forceinline__ float warp_reduce_scatter(float (&v)[N], int lane) {
     return r;
 }
 
+// Entries of a lane per round of the window rewrite (tile::rewrite_window).
+template <int PB, int MINB>
+constexpr int kAdjRewriteGroup = PB >= 4 ? 2 : (PB == 2 ? 4 : (MINB == 1 ? 8 : 6));
+
 // Threads of an adjoint CTA: kThreads accumulating and the producing warps.
 template <int PB>
 constexpr int kAdjThreads = kThreads + 32 * Producers<PB>::kWarps;
@@ -276,7 +280,7 @@ __global__ void __launch_bounds__(kAdjThreads<PB>, MINB)
             cur.advance(tg, L);
             if (pregeo && i + 1 < n) pre.load(L, tile_of(cur), cur.b * PB + q0, lane);
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, true, (PB > 1 ? 4 : (MINB == 1 ? 8 : 6))>(L, p0, rec, win, lane, inv_lam);
+            rewrite_pulses<NQ, true, kAdjRewriteGroup<PB, MINB>>(L, p0, rec, win, lane, inv_lam);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         for (int i = n < 2 ? 0 : n - 2; i < n; ++i) {

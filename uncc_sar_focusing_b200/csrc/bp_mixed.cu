@@ -61,6 +61,10 @@ constexpr int kCtasPerSm = SARBP_CTAS_PER_SM;
 
 constexpr int kTabEntries = kPolyEntries;
 
+// Entries of a lane per round of the window rewrite (tile::rewrite_window).
+template <int PB>
+constexpr int kRewriteGroup = PB == 1 ? 8 : (PB == 4 ? 2 : 4);
+
 // Header of the shared memory: six mbarriers (full, ready and empty, two
 // buffers each) and the zero entry.
 constexpr int kHdr = 64;
@@ -354,7 +358,7 @@ __global__ void __launch_bounds__(kFwdThreads<PB>, MINB)
             cur.advance(scenes, nscenes, rot_later);
             if (pregeo && i + 1 < n) load_records();
             if (!mbar_wait_bounded(bar_base + 8u * s, (i >> 1) & 1, L.err)) return;
-            rewrite_pulses<NQ, false, PB == 1 ? 8 : 4>(L, p0, rec, win, lane);
+            rewrite_pulses<NQ, false, kRewriteGroup<PB>>(L, p0, rec, win, lane);
             if (lane == 0) mbar_arrive(ready_bar(s));
         }
         return;

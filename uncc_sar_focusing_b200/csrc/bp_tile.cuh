@@ -566,12 +566,13 @@ __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaun
 // FFT (point-target call 106 -> 94 us); the rewrite's second load and
 // difference cost the 1024^2 x 2048 forward kernel 1.9% (1495 -> 1524 us).
 // w: the window's first entry (W - wp); odd: its first sample is the second
-// of those copied (issue_window).  kGroup: entries of a lane per round.  A
-// stage of one pulse has its one window of 2500 entries and more rewritten by
-// one warp, which the others wait for: there 8 (128 8-row tiles x 256 pulses,
-// 4978 entries: forward 823 -> 692 us, 787 when range profiles were stored as
-// entries; adjoint 1066 -> 879), 6 for the adjoint on 96 registers (2660
-// entries: 3 267, 4 282, 6 255, 8 278 us).
+// of those copied (issue_window).  kGroup: entries of a lane per round, more for
+// wide windows, where the accumulating warps wait for this, fewer where the
+// registers it takes cost them spills.  Forward, stages of 8 pulses (1024^2 x
+// 2048): 2 1485, 3 1497, 4 1462 us; 4 pulses (windows of 474): 2 145, 4 149; 2
+// (1278): 2 165, 4 151; 1 (4978): 4 823, 8 692.  Adjoint, 8: 2 1930, 4 1943; 2:
+// 2 193, 4 189; 1, two CTAs an SM (2660): 3 267, 4 282, 6 255, 8 278; one CTA
+// (4978): 4 1066, 8 879.
 template <bool ZFORM, int kGroup>
 __device__ __forceinline__ void rewrite_window(uint32_t w, int wp, uint32_t odd, int lane, float nu) {
     const int count = 2 * wp + 2;
