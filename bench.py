@@ -829,9 +829,9 @@ def gpu_arm(args):
                                     "api": "sarbp_focus, pinned host buffers"}},
             # per step: range compression (one fused kernel, or the taper
             # before cuFFT, whose kernels are the library's and not counted),
-            # the backprojection (+ its fix-up when the tiles are split over
-            # the resident CTAs)
-            "gpu_launches": (1 + info["kernels_per_backproject"]) * args.steps,
+            # the geometry records' pre-pass, the backprojection (+ its
+            # fix-up when the tiles are split over the resident CTAs)
+            "gpu_launches": (1 + info["geometry_record_kernels"] + info["kernels_per_backproject"]) * args.steps,
             "kernels": {"bp_ms": bp_ms, "range_compress_ms": rc_ms,
                         "adjoint": {"ms": adj_ms, "value": pp / (adj_ms * 1e-3), "unit": UNIT,
                                     "vs_forward_bp_time": adj_ms / bp_ms,

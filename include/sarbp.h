@@ -156,7 +156,9 @@ SARBP_API int sarbp_plan_workspace_bytes(const sarbp_plan *plan, size_t *bytes);
  * per CTA, resident_ctas CTAs resident at once on the device, tiles per
  * image, and kernels_per_backproject (2 when a launch's (tile, stage) units
  * are split over the resident CTAs and a fix-up kernel adds the split tiles,
- * else 1).  No counterpart in the reference. */
+ * else 1), and geometry_record_kernels (1 when a pre-pass kernel writes the
+ * geometry records of every (tile, pulse) before them, else 0: FP64 plans, or
+ * no room for the records).  No counterpart in the reference. */
 typedef struct sarbp_plan_info {
     int tile_mx;
     int stage_pulses;
@@ -172,7 +174,8 @@ typedef struct sarbp_plan_info {
                                     precision, K <= 512 with long prime factors, R in
                                     {4, 8}); 0 with
                                     fused_range_compression 0: taper kernel and cuFFT */
-    int reserved[3];
+    int geometry_record_kernels;
+    int reserved[2];
 } sarbp_plan_info;
 SARBP_API int sarbp_plan_get_info(const sarbp_plan *plan, sarbp_plan_info *info);
 

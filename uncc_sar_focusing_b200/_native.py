@@ -64,7 +64,8 @@ class PlanInfo(ctypes.Structure):
     _fields_ = [("tile_mx", ctypes.c_int), ("stage_pulses", ctypes.c_int), ("window_bins", ctypes.c_int),
                 ("resident_ctas", ctypes.c_int), ("tiles", ctypes.c_longlong), ("smem_bytes", ctypes.c_longlong),
                 ("kernels_per_backproject", ctypes.c_int), ("fused_range_compression", ctypes.c_int),
-                ("chirp_range_compression", ctypes.c_int), ("reserved", ctypes.c_int * 3)]
+                ("chirp_range_compression", ctypes.c_int), ("geometry_record_kernels", ctypes.c_int),
+                ("reserved", ctypes.c_int * 2)]
 
 
 class BatchInfo(ctypes.Structure):

@@ -853,6 +853,7 @@ int sarbp_plan_get_info(const sarbp_plan *plan, sarbp_plan_info *info) {
     info->kernels_per_backproject = (plan->d_sk && plan->sk_resident > 0 && info->tiles % plan->sk_resident != 0) ? 2 : 1;
     info->fused_range_compression = plan->d_rctab && rc_direct_shape(plan->K) ? 1 : 0;
     info->chirp_range_compression = plan->d_rctab && !rc_direct_shape(plan->K) ? 1 : 0;
+    info->geometry_record_kernels = plan->d_geotab ? 1 : 0;
     return SARBP_OK;
 }
 
