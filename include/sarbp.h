@@ -258,8 +258,9 @@ SARBP_API int sarbp_focus_submit(sarbp_plan *plan, const sarbp_aperture *apertur
 SARBP_API int sarbp_focus_wait(sarbp_plan *plan, unsigned long long ticket);
 
 /* Batches of independent scenes of uneven sizes (different K, pulse counts,
- * nfft, grids) focused together: one range-compression launch pair for all
- * scenes (plus one FFT per scene) and ONE backprojection launch whose
+ * nfft, grids) focused together: one range-compression launch for the scenes
+ * of each fused shape (up to 64 of them; one taper launch and one FFT per scene
+ * for the others) and ONE backprojection launch whose
  * (tile, pulse-stage) units of all scenes are split evenly over the resident
  * CTAs, captured once as a CUDA graph and replayed per call.  The reference
  * focuses one aperture per call (cuda_sar_focusing.hpp:526-723).

@@ -40,13 +40,13 @@
 // lane holds), and adjoint_reduce_kernel sums the tiles per pulse in double,
 // in a fixed order.
 //
-// What bounds it: 22 warp instructions per warp-pixel-pulse at 66% of issue
+// What bounds it: 21.7 warp instructions per warp-pixel-pulse at 65% of issue
 // slots (20.8 before, where the gathers of the 32 lanes of a row took 9.3
 // shared-memory wavefronts a pixel-pulse instead of 5.8 whenever the look
 // direction lay along the columns).  2048 pulses x 1024^2 pixels, look
 // direction 0 / 45 / 90 degrees from the rows: 2.00 / 2.41 / 2.26 ms before,
-// 1.93 / 1.94 / 1.92 ms now.  The 32 registers of the pixels' |G| and psi
-// leave the 96-register budget of 20 warps short: 3 of the instructions are
+// 1.93 / 1.95 / 1.93 ms now.  The 32 registers of the pixels' |G| and psi
+// leave the 96-register budget of 20 warps short: some 3 of the instructions are
 // moves that a 142-register build (10 warps, 2.39 ms) does not need.
 #include <algorithm>
 #include <cstdint>

@@ -92,8 +92,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 
 // Plain (non-multicast) bulk copy global -> this CTA's shared memory,
 // completing transaction bytes on `bar`.  dst, src and bytes are multiples
-// of 16 (the callers copy whole 16- or 32-byte entries from 256-byte aligned
-// allocations).
+// of 16 (FP64 windows are 16-byte samples; mixed ones 8-byte samples, an even
+// number from an even one on, of rows that start on 16 bytes).
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),

@@ -34,13 +34,15 @@
 //  * MX = 8 (64 x 64-pixel tiles) by default: the per-(tile, pulse) and
 //    per-(thread, pulse) work is spread over 16 pixels per thread.
 //
-// What bounds it (1024^2 pixels x 2048 pulses, 8 km, ncu): 16.0 warp
+// What bounds it (1024^2 pixels x 2048 pulses, 8 km, ncu): 16.1 warp
 // instructions per warp-pixel-pulse at 65% of issue slots, shared memory's data
-// pipe 80% busy (5.1 wavefronts, 4 of them the 16-byte gather's floor), MUFU
-// 65%, 20 warps per SM.  With rows interleaved over the warps, a row of 32
+// pipe 83% busy (5.2 wavefronts, 4 of them the 16-byte gather's floor), MUFU
+// 66%, 20 warps per SM.  With rows interleaved over the warps, a row of 32
 // lanes and an evaluation of the range remainder per pixel it took 18.0
 // instructions and 1.70 / 2.29 / 2.13 ms at look directions 0 / 45 / 90
-// degrees from the rows, this 1.48 / 1.49 / 1.48 ms.
+// degrees from the rows, this 1.46 / 1.48 / 1.46 ms.  The 96 registers of 20
+// warps are short: 24 bytes a thread are spilled and 44 loaded back (batches,
+// whose accumulating warps carry the scene cursor too, 132 / 160).
 #include <cstdint>
 
 #include "bp_common.cuh"
@@ -625,7 +627,7 @@ cudaError_t launch_kernels(const BpLaunch &L0, size_t smem, cudaStream_t s) {
 
 template <int MX, int PB>
 cudaError_t launch_mx_pb(const BpLaunch &L, bool checked, size_t smem, cudaStream_t s) {
-    // two CTAs per SM (128 registers) by default; one CTA per SM (up to 255
+    // two CTAs per SM (96 registers) by default; one CTA per SM (up to 200
     // registers) when the stage needs more shared memory than two CTAs get
     const bool one_cta = smem > 113u * 1024u;
     if (checked)

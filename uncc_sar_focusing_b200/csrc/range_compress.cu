@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(32 * R) rc_fused_kernel(const __grid_constant_
 // K = 424 (8 x 53) and the like went through a zero-padded buffer and cuFFT
 // (radix 53, or its own chirp transform of twice nfft, on data that is 7/8
 // zeros): 512 pulses of 424 samples, 8 times upsampled, 55 us with the pair
-// rows of the time, 40 without, 20 us here; 777 of 501: 96 and 79 to 31 us.
+// rows of the time, 50 without, 23 us here; 777 of 501: 96 and 79 to 31 us.
 template <int K2, int R>
 struct CztTable {
     static_assert(K2 == 32 && (R == 4 || R == 8), "the chirp kernel's shapes");
