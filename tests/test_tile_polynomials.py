@@ -147,3 +147,18 @@ def test_cubic_term_of_the_row_steps(probe, mx, bound):
     u = np.abs(v[:, 0]) / t["rc"]
     q30 = (2.0 * math.pi * f0 / C / t["rc"] ** 2 * u * (1.0 - u * u)).max() * spacing ** 3
     assert off.max() <= 8.0 * bound * q30 + 5.0 * 2.0 ** -24 * np.abs(t["P"]).max(), (off.max(), 8.0 * bound * q30)
+
+
+@pytest.mark.parametrize("f0", [0.0, 25.0, -1.0e6, -9.28e9])
+@pytest.mark.parametrize("radius,spacing,lam,mx", [(4e3, 3.0, 2.0, 8), (2.5e3, 1.5, 6.0, 8), (900.0, 0.6, 20.0, 4)])
+def test_far_field_test_of_any_start_frequency(probe, f0, radius, spacing, lam, mx):
+    """Coarse tiles at 17 and more half-diagonals: with a start frequency of
+    zero or below it the expansion is taken only where it leaves bins within
+    1e-4 and phases within 1e-7 turns, as it is above."""
+    t = tile(probe, f0, radius, spacing, mx, lam=lam)
+    tol_bin = 4.0 * 2.0 ** -24 * t["W"] + 1e-4
+    assert (np.abs(t["B"] - t["bin"]) <= tol_bin).all(), np.abs(t["B"] - t["bin"]).max()
+    turn = t["P"].astype(np.float64) / (2.0 * math.pi) - t["rev"]
+    off = 2.0 * math.pi * np.abs(turn - np.rint(turn))
+    tol = 2.0 ** -24 * (5.0 * 40.0 + 6.0 * np.abs(t["P"]).max()) + 2.0 * math.pi * 1e-7 + 1e-6
+    assert (off <= tol).all(), off.max()

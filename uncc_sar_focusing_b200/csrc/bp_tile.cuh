@@ -196,9 +196,12 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     g.rinv = static_cast<float>(inv);
 
     int flags = g.flags;
-    // (bins of less than 1e-12 or more than 1e12 to the metre would leave the
-    // polynomials' FP32 range; the exact path does without their ratio)
-    if (rc < L.near_hd16 || rc * rc * rc < k * L.near_coef || !(L.lambda > 1.0e-12 && L.lambda < 1.0e12))
+    // near field: the expansion would be off by 1e-7 turns, or (start frequencies
+    // next to zero) 1e-4 bins.  (Bins of less than 1e-12 or more than 1e12 to the
+    // metre would leave the polynomials' FP32 range; the exact path does without
+    // their ratio.)
+    const double reach = fmax(fabs(k), 1.0e-3 * L.lambda);
+    if (rc < L.near_hd16 || rc * rc * rc < reach * L.near_coef || !(L.lambda > 1.0e-12 && L.lambda < 1.0e12))
         flags |= PG_NEAR;
     // Tight window: a pixel (i, j) of the tile has bin - bc = i gam + j eta +
     // lambda g with 0 <= g <= hd^2 / (2 (Rc - hd)) (hd the tile
