@@ -146,8 +146,8 @@ inline void tile_window(double lambda, double dx, double dy, int mx, int *W, int
 
 // Far-field test constants of the mixed kernel for a tile half-diagonal hd:
 // the remainder after the e (h + t hr) expansion is <= 0.625 hd^4 / Rc^3
-// metres; a pulse whose k times that exceeds 1e-7 revolutions takes the
-// exact path.
+// metres; a pulse for which that is more than 1e-7 revolutions (or 1e-4 bins)
+// takes the exact path.
 inline void near_field_consts(double hd, double *near_hd16, double *near_coef) {
     *near_hd16 = 16.0 * hd;
     *near_coef = 0.625 * hd * hd * hd * hd / 1.0e-7;
