@@ -31,7 +31,7 @@ def probe(tmp_path_factory):
 
 
 def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392, lam=32.1, el=30.0,
-         look=(0.0, 30.0, 88.0, 200.0), near=1.0):
+         look=(0.0, 30.0, 88.0, 200.0), near=1.0, origin=(0.3, -0.7)):
     """The tile's phases, bins and pulse words, with their exact values:
     phase modulo one turn, window-centred bin (float64).  near: a factor on the
     far-field test's constant."""
@@ -44,7 +44,7 @@ def tile(probe, f0, radius, spacing, mx, exchanged=False, split=False, nfft=3392
     f = np.broadcast_to(np.asarray(f0, dtype=np.float64), (n,))
     geo = np.ascontiguousarray(np.stack([x, y, z, r0, f]))
     dx, dy = spacing, 1.1 * spacing
-    left, bottom = 0.3, -0.7
+    left, bottom = origin
     hd = math.hypot(4 * mx * dx, 32 * dy)
     W = int(math.ceil(lam * hd)) + 3
     P = np.full((n, 8 * mx, 64), np.nan, dtype=np.float32)
@@ -162,3 +162,12 @@ def test_far_field_test_of_any_start_frequency(probe, f0, radius, spacing, lam, 
     off = 2.0 * math.pi * np.abs(turn - np.rint(turn))
     tol = 2.0 ** -24 * (5.0 * 40.0 + 6.0 * np.abs(t["P"]).max()) + 2.0 * math.pi * 1e-7 + 1e-6
     assert (off <= tol).all(), off.max()
+
+
+@pytest.mark.parametrize("radius", [1e-21, 1e-19, 1e-12, 1e-3])
+def test_one_pixel_next_to_the_antenna(probe, radius):
+    """A grid of one pixel has a tile of no extent: no range is near field by
+    its diagonal, and 1 / Rc^2 leaves FP32 at 1e-19 m.  (Below 1e-22 m the record
+    itself is refused as not finite.)"""
+    t = tile(probe, 9.28e9, radius, 0.0, 1, origin=(0.0, 0.0))
+    assert np.isfinite(t["P"]).all() and (np.abs(t["B"] - t["bin"]) <= 1e-4).all()

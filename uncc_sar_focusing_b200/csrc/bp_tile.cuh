@@ -198,10 +198,10 @@ __device__ __forceinline__ PulseGeo make_geo(const BpLaunch &L, int p, long long
     int flags = g.flags;
     // near field: the expansion would be off by 1e-7 turns, or (start frequencies
     // next to zero) 1e-4 bins.  (Bins of less than 1e-12 or more than 1e12 to the
-    // metre would leave the polynomials' FP32 range; the exact path does without
-    // their ratio.)
+    // metre, and 1 / Rc^2 next to the one pixel of a grid without extent, would
+    // leave the polynomials' FP32 range; the exact path does without.)
     const double reach = fmax(fabs(k), 1.0e-3 * L.lambda);
-    if (rc < L.near_hd16 || rc * rc * rc < reach * L.near_coef || !(L.lambda > 1.0e-12 && L.lambda < 1.0e12))
+    if (rc < fmax(L.near_hd16, 1.0e-9) || rc * rc * rc < reach * L.near_coef || !(L.lambda > 1.0e-12 && L.lambda < 1.0e12))
         flags |= PG_NEAR;
     // Tight window: a pixel (i, j) of the tile has bin - bc = i gam + j eta +
     // lambda g with 0 <= g <= hd^2 / (2 (Rc - hd)) (hd the tile
