@@ -528,7 +528,7 @@ struct PixelPoly {
 // with 1 / (2 s + 2 g0) ~ r (1 - g0 r), leaves its own rounding: no further off
 // than sqrtf() and a division, whose special cases end the block in which the
 // pixels' chains are interleaved.  512^2 pixels x 1024 pulses at 0.15 m, 8 km:
-// forward 674 -> 441 us, adjoint 921 -> 739.
+// forward 674 -> 449 us, adjoint 921 -> 740.
 __device__ __forceinline__ float2 near_remainder(const PulseGeo &g, const BpLaunch &L, float fi, float2 J,
                                                  float2 &s) {
     const float4 c1 = *reinterpret_cast<const float4 *>(&g.tx);  // tx, ty, h, hr
